@@ -1,4 +1,6 @@
-// irc_exact.cu -- EXACT-mode site kNN and the kNN-list delta.
+// irc_exact.cu -- EXACT-mode site kNN and the kNN-list delta.  (Plans large
+// enough are served by the proven search of irc_cert.cu; the kernel here then
+// finishes the tiles it leaves open.)
 //
 // EXACT kNN: the true k nearest candidates (squared distance > 0, the irc2
 // GPU convention) under the reference FP32 arithmetic, ordered by the key
@@ -21,6 +23,7 @@
 #include <cstdio>
 #include <mutex>
 
+#include "irc_cert.cuh"
 #include "irc_common.cuh"
 #include "irc_plan.cuh"
 #include "irc_scan.cuh"
@@ -120,7 +123,7 @@ __device__ __forceinline__ void warp_sort_keys(unsigned long long *keys, int lan
 __global__ void __launch_bounds__(kThreads)
 k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
                  float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
-                 float *__restrict__ d2Knn, int *__restrict__ ovf_count, int *__restrict__ ovf_list)
+                 float *__restrict__ d2Knn, int *__restrict__ ovf_count, int *__restrict__ ovf_list, irc::TileQueue tq)
 {
     __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
     __shared__ float sTau[kQB];
@@ -128,87 +131,90 @@ k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
     extern __shared__ __align__(16) unsigned char dyn[];
     unsigned long long *sList = reinterpret_cast<unsigned long long *>(dyn);   // [kQB][kCap]
     float *sMin = reinterpret_cast<float *>(sList + kQB * kCap);              // [kQB][kThreads]
-    int chunk, qs, n;
-    irc::tile_lookup<kQB>(p, blockIdx.x, chunk, qs, n);
-    const int r0 = __ldg(p.roff + chunk), r1 = __ldg(p.roff + chunk + 1);
-    irc::stage_queries<kQB>(F, nC, qs, n, sA);
-    if (threadIdx.x < kQB) sCnt[threadIdx.x] = 0;
-    __syncthreads();
-    const int t = threadIdx.x;
-    // pass 1: stripe minima
-    float mn[kQB];
+    for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
+        int chunk, qs, n;
+        irc::tile_lookup<kQB>(p, tq.tile(w), chunk, qs, n);
+        const int r0 = __ldg(p.roff + chunk), r1 = __ldg(p.roff + chunk + 1);
+        irc::stage_queries<kQB>(F, nC, qs, n, sA);
+        if (threadIdx.x < kQB) sCnt[threadIdx.x] = 0;
+        __syncthreads();
+        const int t = threadIdx.x;
+        // pass 1: stripe minima
+        float mn[kQB];
 #pragma unroll
-    for (int q = 0; q < kQB; ++q) mn[q] = __int_as_float(0x7f800000);
-    walk_stripe(p, r0, r1, t, [&](int iB) {
-        float acc[kQB];
-        dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
+        for (int q = 0; q < kQB; ++q) mn[q] = __int_as_float(0x7f800000);
+        walk_stripe(p, r0, r1, t, [&](int iB) {
+            float acc[kQB];
+            dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
 #pragma unroll
-        for (int q = 0; q < kQB; ++q)
-            if (acc[q] > 0.0f && acc[q] < mn[q]) mn[q] = acc[q];
-    });
+            for (int q = 0; q < kQB; ++q)
+                if (acc[q] > 0.0f && acc[q] < mn[q]) mn[q] = acc[q];
+        });
 #pragma unroll
-    for (int q = 0; q < kQB; ++q) sMin[q * kThreads + t] = mn[q];
-    __syncthreads();
-    // tau = k-th smallest stripe minimum (by value); +inf if fewer than k finite
-    const int lane = t & 31, warp = t >> 5, nw = kThreads / 32;
-    for (int q = warp; q < kQB; q += nw) {
-        float *m = sMin + q * kThreads;
-        float kth = __int_as_float(0x7f800000);
-        for (int k = 0; k < knn; ++k) {
-            unsigned long long best = ~0ull;
-            for (int s = lane; s < kThreads; s += 32) {
-                const unsigned long long key = dkey(m[s], s);
-                best = key < best ? key : best;
+        for (int q = 0; q < kQB; ++q) sMin[q * kThreads + t] = mn[q];
+        __syncthreads();
+        // tau = k-th smallest stripe minimum (by value); +inf if fewer than k finite
+        const int lane = t & 31, warp = t >> 5, nw = kThreads / 32;
+        for (int q = warp; q < kQB; q += nw) {
+            float *m = sMin + q * kThreads;
+            float kth = __int_as_float(0x7f800000);
+            for (int k = 0; k < knn; ++k) {
+                unsigned long long best = ~0ull;
+                for (int s = lane; s < kThreads; s += 32) {
+                    const unsigned long long key = dkey(m[s], s);
+                    best = key < best ? key : best;
+                }
+                best = irc::warp_min_u64(best);
+                const int s = (int)(best & 0xffffffffu);
+                kth = __uint_as_float((unsigned)(best >> 32));
+                __syncwarp();
+                if (lane == 0) m[s] = __int_as_float(0x7fffffff);      // NaN bits: sorts last
+                __syncwarp();
+                if (!(kth < __int_as_float(0x7f800000))) break;
             }
-            best = irc::warp_min_u64(best);
-            const int s = (int)(best & 0xffffffffu);
-            kth = __uint_as_float((unsigned)(best >> 32));
+            if (lane == 0) sTau[q] = kth;
+        }
+        __syncthreads();
+        // pass 2: collect d2 <= tau
+        walk_stripe(p, r0, r1, t, [&](int iB) {
+            float acc[kQB];
+            dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
+#pragma unroll
+            for (int q = 0; q < kQB; ++q)
+                if (acc[q] > 0.0f && acc[q] <= sTau[q]) {
+                    const int slot = atomicAdd(&sCnt[q], 1);
+                    if (slot < kCap) sList[q * kCap + slot] = dkey(acc[q], iB);
+                }
+        });
+        __syncthreads();
+        for (int q = warp; q < n; q += nw) {
+            const int cnt = sCnt[q];
+            const size_t o = (size_t)(qs + q - p.q_base);
+            if (cnt > kCap) {                          // overflow: finished by the fallback kernel
+                if (lane == 0) { int i = atomicAdd(ovf_count, 1); ovf_list[i] = qs + q; }
+                continue;
+            }
+            unsigned long long *L = sList + q * kCap;
+            for (int i = cnt + lane; i < kCap; i += 32) L[i] = ~0ull;
             __syncwarp();
-            if (lane == 0) m[s] = __int_as_float(0x7fffffff);      // NaN bits: sorts last
+            warp_sort_keys(L, lane);
             __syncwarp();
-            if (!(kth < __int_as_float(0x7f800000))) break;
-        }
-        if (lane == 0) sTau[q] = kth;
-    }
-    __syncthreads();
-    // pass 2: collect d2 <= tau
-    walk_stripe(p, r0, r1, t, [&](int iB) {
-        float acc[kQB];
-        dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
-#pragma unroll
-        for (int q = 0; q < kQB; ++q)
-            if (acc[q] > 0.0f && acc[q] <= sTau[q]) {
-                const int slot = atomicAdd(&sCnt[q], 1);
-                if (slot < kCap) sList[q * kCap + slot] = dkey(acc[q], iB);
+            for (int k = lane; k < knn; k += 32) {
+                const unsigned long long key = L[k];
+                const bool ok = k < cnt;
+                const float d2 = ok ? __uint_as_float((unsigned)(key >> 32)) : kInfSentinel;
+                const int idx = ok ? (int)(key & 0xffffffffu) : qs + q;
+                miKnn[(size_t)k + (size_t)knn * o] = idx + 1;
+                if (d2Knn) d2Knn[(size_t)k + (size_t)knn * o] = d2;
+                if (k == knn - 1) {
+                    const float v = irc::ref_sqrt_abs(d2);
+                    vrKnn[o] = v;
+                    if (rho) rho[o] = __fdiv_rn(1.0f, v);
+                }
             }
-    });
-    __syncthreads();
-    for (int q = warp; q < n; q += nw) {
-        const int cnt = sCnt[q];
-        const size_t o = (size_t)(qs + q - p.q_base);
-        if (cnt > kCap) {                          // overflow: finished by the fallback kernel
-            if (lane == 0) { int i = atomicAdd(ovf_count, 1); ovf_list[i] = qs + q; }
-            continue;
+            __syncwarp();
         }
-        unsigned long long *L = sList + q * kCap;
-        for (int i = cnt + lane; i < kCap; i += 32) L[i] = ~0ull;
-        __syncwarp();
-        warp_sort_keys(L, lane);
-        __syncwarp();
-        for (int k = lane; k < knn; k += 32) {
-            const unsigned long long key = L[k];
-            const bool ok = k < cnt;
-            const float d2 = ok ? __uint_as_float((unsigned)(key >> 32)) : kInfSentinel;
-            const int idx = ok ? (int)(key & 0xffffffffu) : qs + q;
-            miKnn[(size_t)k + (size_t)knn * o] = idx + 1;
-            if (d2Knn) d2Knn[(size_t)k + (size_t)knn * o] = d2;
-            if (k == knn - 1) {
-                const float v = irc::ref_sqrt_abs(d2);
-                vrKnn[o] = v;
-                if (rho) rho[o] = __fdiv_rn(1.0f, v);
-            }
-        }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -340,6 +346,20 @@ k_delta_compact(irc::PlanDev p, const int *__restrict__ fb_flag, int *__restrict
     }
 }
 
+// The reference's tie rule of the delta search (REF): the smallest
+// sqrt(d2), then the lowest bin, then inside the bin the smallest d2 and the
+// first row.  One 64-bit key orders them: sqrt bits (31, positive) | bin (10)
+// | d2 among the at most 5 FP32 values that share a square root (3: its offset
+// from the rounded square) | step inside the bin (20; row = run start + bin /
+// runs + step * stride).
+__device__ __forceinline__ unsigned long long ref_key(float d2, int bin, int step)
+{
+    const float v = irc::ref_sqrt_abs(d2);
+    const unsigned dd = __float_as_uint(d2) - __float_as_uint(__fmul_rn(v, v)) + 4u;
+    return ((unsigned long long)__float_as_uint(v) << 33) | ((unsigned long long)bin << 23) |
+           ((unsigned long long)(dd & 7u) << 20) | (unsigned)step;
+}
+
 // Drift-window fallback for the queued queries, one unit per (16-query tile
 // of a chunk, part of its candidate window; long windows have up to kParts
 // parts of at least kMinPart candidates): a unit loads every candidate of its
@@ -351,10 +371,11 @@ k_delta_compact(irc::PlanDev p, const int *__restrict__ fb_flag, int *__restrict
 // (a probe holds ~1,000 fallback tiles per site, too few to fill 152 SMs
 // when each scans a whole ~30K-candidate window).
 
+template <bool REF>
 __global__ void __launch_bounds__(kThreads)
 k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restrict__ R, int nC,
               const uint8_t *__restrict__ row_dims, const int *__restrict__ n_items, const int2 *__restrict__ items,
-              const int *__restrict__ fb_list, unsigned long long *__restrict__ keys)
+              const int *__restrict__ fb_list, unsigned long long *__restrict__ keys, int nT)
 {
     __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
     __shared__ float sRA[kQB];
@@ -367,7 +388,10 @@ k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restri
         const int chunk = item.x & 0x0fffffff, part = item.x >> 28, first = item.y >> 5, n = item.y & 31;
         const int ntot = __ldg(p.ncand + chunk);
         const int np = min(kParts, max(1, ntot / kMinPart));
-        const int r0 = __ldg(p.roff + chunk), r1 = __ldg(p.roff + chunk + 1);
+        // REF: the runs as the reference passes them (its bins depend on them)
+        const int32_t *prs = REF ? p.rsr : p.rs, *prn = REF ? p.rnr : p.rn;
+        const int r0 = __ldg((REF ? p.roffr : p.roff) + chunk), r1 = __ldg((REF ? p.roffr : p.roff) + chunk + 1);
+        const int nBB = r1 - r0, nT0 = REF ? nT / nBB : 1;
         const int seg = __ldg(p.q0 + chunk) - p.q_base;
         // features that can be non-zero for this chunk's queries and candidates
         // (their site's width, irc_plan_set_site_dims): the rest add exactly 0
@@ -386,10 +410,13 @@ k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restri
         unsigned long long best[kQB];
 #pragma unroll
         for (int q = 0; q < kQB; ++q) best[q] = ~0ull;
+        float thr[kQB];                                      // REF: distances above it cannot be the minimum
+#pragma unroll
+        for (int q = 0; q < kQB; ++q) thr[q] = kInfSentinel;
         const int per = (ntot + np - 1) / np, lo = part * per, hi = min(ntot, lo + per);
         int pos = 0;                                         // position of run r's first candidate
         for (int r = r0; r < r1 && pos < hi; ++r) {
-            const int rs = __ldg(p.rs + r), rn = __ldg(p.rn + r);
+            const int rs = __ldg(prs + r), rn = __ldg(prn + r);
             const int a = max(lo - pos, 0), b = min(hi - pos, rn);
             for (int i = a + (int)threadIdx.x; i < b; i += kThreads) {
                 const int iB = rs + i;
@@ -404,8 +431,16 @@ k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restri
 #pragma unroll
                 for (int q = 0; q < kQB; ++q)
                     if (((live >> q) & 1u) && acc[q] > 0.0f && acc[q] < kInfSentinel) {
-                        const unsigned long long key = dkey(acc[q], iB);
-                        best[q] = key < best[q] ? key : best[q];
+                        if (REF) {
+                            if (acc[q] <= thr[q]) {
+                                const unsigned long long key = ref_key(acc[q], (i % nT0) * nBB + (r - r0), i / nT0);
+                                best[q] = key < best[q] ? key : best[q];
+                                thr[q] = fminf(thr[q], acc[q] * (1.0f + 0x1p-20f));   // every d2 sharing its root
+                            }
+                        } else {
+                            const unsigned long long key = dkey(acc[q], iB);
+                            best[q] = key < best[q] ? key : best[q];
+                        }
                     }
             }
             pos += rn;
@@ -427,10 +462,11 @@ k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restri
 
 // delta and nneigh of the queued queries from their keys (no candidate:
 // sqrt(SINGLE_INF) .* rho and the query itself, as search_delta_drift_).
+template <bool REF>
 __global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, const int *__restrict__ n_items,
                                const int2 *__restrict__ items, const int *__restrict__ fb_list,
                                const unsigned long long *__restrict__ keys, float *__restrict__ delta,
-                               int *__restrict__ nneigh)
+                               int *__restrict__ nneigh, int nT)
 {
     const int total = *n_items * kQB;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -442,6 +478,18 @@ __global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, cons
         const size_t o = (size_t)(qq - p.q_base);
         const unsigned long long b = keys[o];
         const bool ok = b != ~0ull;
+        if (REF) {
+            int row = qq;
+            if (ok) {
+                const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
+                const int bin = (int)(b >> 23) & 1023;
+                row = __ldg(p.rsr + r0 + bin % nBB) + bin / nBB + (int)(b & 0xfffffu) * (nT / nBB);
+            }
+            const float v = ok ? __uint_as_float((unsigned)(b >> 33)) : irc::ref_sqrt_abs(kInfSentinel);
+            delta[o] = __fmul_rn(v, __ldg(R + qq));
+            nneigh[o] = row + 1;
+            continue;
+        }
         const float d2 = ok ? __uint_as_float((unsigned)(b >> 32)) : kInfSentinel;
         delta[o] = __fmul_rn(irc::ref_sqrt_abs(d2), __ldg(R + qq));
         nneigh[o] = (ok ? (int)(b & 0xffffffffu) : qq) + 1;
@@ -459,6 +507,25 @@ static int irc_plan_scratch(irc_plan *pl, int **counters, int **list_a, int **li
     return IRC_OK;
 }
 
+// The EXACT kernel over the tiles of tq (all of the plan's by default) and its
+// overflow queue (*cnt, zeroed; up to n_out entries).
+int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
+                    float *d2Knn, const irc::TileQueue &tq, int *cnt, int *ovf_list, cudaStream_t s)
+{
+    const size_t smem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
+    cudaError_t e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): smem attribute");
+    const int tiles = pl->ntiles[irc::tile_slot(kQB)];
+    const int grid = tq.list && tiles > kQueueBlocks ? kQueueBlocks : tiles;
+    k_site_knn_exact<<<grid, kThreads, smem, s>>>(pl->dev, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, ovf_list, tq);
+    IRC_CHECK_LAUNCH("irc_site_knn(EXACT)");
+    // the overflow list is usually empty; size the grid for the worst case
+    k_exact_overflow<<<kQueueBlocks, 256, 0, s>>>(
+        pl->dev, F, nC, knn, cnt, ovf_list, vrKnn, rho, miKnn, d2Knn);
+    IRC_CHECK_LAUNCH("irc_site_knn(EXACT) overflow");
+    return IRC_OK;
+}
+
 int irc_site_knn_exact(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho,
                        int32_t *miKnn, float *d2Knn, cudaStream_t s)
 {
@@ -468,17 +535,7 @@ int irc_site_knn_exact(irc_plan *pl, const float *F, int nC, int knn, float *vrK
     if (rc != IRC_OK) return rc;
     cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * sizeof(int), s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): memset");
-    const size_t smem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
-    e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): smem attribute");
-    const int tiles = pl->ntiles[irc::tile_slot(kQB)];
-    k_site_knn_exact<<<tiles, kThreads, smem, s>>>(pl->dev, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, la);
-    IRC_CHECK_LAUNCH("irc_site_knn(EXACT)");
-    // the overflow list is usually empty; size the grid for the worst case
-    k_exact_overflow<<<kQueueBlocks, 256, 0, s>>>(
-        pl->dev, F, nC, knn, cnt, la, vrKnn, rho, miKnn, d2Knn);
-    IRC_CHECK_LAUNCH("irc_site_knn(EXACT) overflow");
-    return IRC_OK;
+    return irc_exact_tiles(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, irc::TileQueue{}, cnt, la, s);
 }
 
 int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, int knn,
@@ -488,21 +545,33 @@ int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, in
     int *cnt, *la, *lb;
     int rc = irc_plan_scratch(pl, &cnt, &la, &lb);
     if (rc != IRC_OK) return rc;
-    // flags in list a, compacted queries in list b, (chunk, tile) items after them
-    int *n_items = cnt + irc::kScratchItems;
-    int2 *items = reinterpret_cast<int2 *>(lb + pl->dev.n_out);
-    unsigned long long *keys = reinterpret_cast<unsigned long long *>(
-        lb + pl->dev.n_out + 16 * ((size_t)pl->dev.n_out / 16 + pl->dev.nChunks + 1));
-    cudaError_t e = cudaMemsetAsync(n_items, 0, sizeof(int), s);
-    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: memset");
+    // flags in list a, compacted queries in list b, (chunk, tile) items and keys after them
+    irc_delta_scratch sc;
+    sc.n_items = cnt + irc::kScratchItems;
     const int n = pl->dev.n_out;
+    sc.flags = la;
+    sc.list = lb;
+    sc.items = reinterpret_cast<int2 *>(lb + n);      // (8-byte aligned: the two lists hold 2 n words)
+    sc.keys = reinterpret_cast<unsigned long long *>(sc.items + delta_items(n, pl->dev.nChunks));
     k_delta_list<<<(n + 255) / 256, 256, 0, s>>>(pl->dev, R, knn, miKnn, d2Knn, delta, nneigh, la);
     IRC_CHECK_LAUNCH("irc_site_delta list");
-    k_delta_compact<<<pl->dev.nChunks, kThreads, 0, s>>>(pl->dev, la, lb, n_items, items, keys);
+    return irc_delta_window(pl, F, nC, R, 0, sc, delta, nneigh, s);
+}
+
+// The drift-window search of the flagged queries: ties by (d2, row), or by the
+// reference's rule over nT bins (nT > 0).
+int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int nT, const irc_delta_scratch &sc,
+                     float *delta, int32_t *nneigh, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(sc.n_items, 0, sizeof(int), s);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: memset");
+    k_delta_compact<<<pl->dev.nChunks, kThreads, 0, s>>>(pl->dev, sc.flags, sc.list, sc.n_items, sc.items, sc.keys);
     IRC_CHECK_LAUNCH("irc_site_delta compact");
-    k_delta_tiles<<<kQueueBlocks, kThreads, 0, s>>>(pl->dev, F, R, nC, pl->row_dims, n_items, items, lb, keys);
+    auto tiles = nT > 0 ? k_delta_tiles<true> : k_delta_tiles<false>;
+    auto finish = nT > 0 ? k_delta_finish<true> : k_delta_finish<false>;
+    tiles<<<kQueueBlocks, kThreads, 0, s>>>(pl->dev, F, R, nC, pl->row_dims, sc.n_items, sc.items, sc.list, sc.keys, nT);
     IRC_CHECK_LAUNCH("irc_site_delta tiles");
-    k_delta_finish<<<kQueueBlocks, kThreads, 0, s>>>(pl->dev, R, n_items, items, lb, keys, delta, nneigh);
+    finish<<<kQueueBlocks, kThreads, 0, s>>>(pl->dev, R, sc.n_items, sc.items, sc.list, sc.keys, delta, nneigh, nT);
     IRC_CHECK_LAUNCH("irc_site_delta finish");
     return IRC_OK;
 }
@@ -660,7 +729,7 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn_exact_noalloc: smem attribute");
     int32_t *cnt = base, *queue = base + irc::kScratchLists;
-    k_site_knn_exact<<<(unsigned)tiles, kThreads, smem, s>>>(p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue);
+    k_site_knn_exact<<<(unsigned)tiles, kThreads, smem, s>>>(p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, irc::TileQueue{});
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc");
     k_exact_overflow<<<kQueueBlocks, 256, 0, s>>>(p, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc overflow");

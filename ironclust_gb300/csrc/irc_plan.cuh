@@ -50,6 +50,16 @@ struct PlanDev {
     int nChunks, q_base, n_out, nF, nRuns;
 };
 
+// The 16-query tiles a plain-form kernel works on: every tile of the plan, one
+// per block (list null), or the tiles a proven search left open (irc_cert.cu):
+// list[0 .. *count), or all ntiles of them when *all is set.
+struct TileQueue {
+    const int *list, *count, *all;
+    int ntiles;
+    __device__ __forceinline__ int size() const { return !list ? (int)gridDim.x : *all ? ntiles : *count; }
+    __device__ __forceinline__ int tile(int w) const { return !list || *all ? w : list[w]; }
+};
+
 // Map a flat tile id to (chunk, first query, query count) for tile size QB.
 template <int QB>
 __device__ __forceinline__ void tile_lookup(const PlanDev &p, int tile, int &chunk, int &qs, int &n)
@@ -81,13 +91,15 @@ struct irc_plan {
     void *tc_items_buf;                    // items of irc_plan_tc_layout, when called
     void *tc_buf;                          // tensor-core operand rows (2 x nF x tc_row_bytes) and the
                                            // padded FP32 rows of the re-rank, allocated lazily
-    size_t tc_row_bytes;
     size_t tc_bytes;                       // allocated size of tc_buf
     int tc_external;                       // tc_buf belongs to the caller (irc_plan_set_tc_buffer)
     int n_row_iv;                          // rows of F the plan reads: n_row_iv intervals
     int row_iv[2 * 8];                     // [lo, hi) pairs, ascending (at most 8; else one hull)
     int ntiles[irc::kNumTileSizes];        // host copy of tile counts
     int max_nq;                            // largest query chunk
+    int max_rn;                            // longest candidate run
+    int runs_ascend;                       // every chunk's runs ascend without overlap (a row is in at most one)
+    int uses_pool;                         // the plan took working memory from the library's pool (irc_cert.cu)
     long long pairs;                       // (query, candidate) pairs of the plan
     int device;
     // host copies (for the per-chunk drop-in emulation and validation)

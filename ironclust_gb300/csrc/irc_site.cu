@@ -8,12 +8,14 @@
 // the chunk into shared memory, and performs the MATLAB sort/min on the
 // device with warp arg-min reductions over (value, bin) keys -- the stable
 // ascending order of MATLAB's sort.  Results equal the reference kernels +
-// MATLAB post-processing bit for bit.
+// MATLAB post-processing bit for bit.  (Plans large enough are served by the
+// proven search of irc_cert.cu; the kernels here take the rest.)
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
 
+#include "irc_cert.cuh"
 #include "irc_common.cuh"
 #include "irc_plan.cuh"
 #include "irc_scan.cuh"
@@ -28,59 +30,62 @@ constexpr int kDeltaQB = 16;   // queries per CTA, delta kernel
 // kNN (search_min_drift + sort): bin table sV/sI [QB][nT] in dynamic smem.
 __global__ void __launch_bounds__(kThreads)
 k_site_knn_ref(irc::PlanDev p, const float *__restrict__ F, int nC, int nT, int knn,
-               float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn)
+               float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn, irc::TileQueue tq)
 {
     constexpr int QB = kKnnQB;
     __shared__ __align__(16) float sA[IRC_NC_MAX * QB];
     extern __shared__ __align__(16) unsigned char dyn[];
     float *sV = reinterpret_cast<float *>(dyn);            // [QB][nT]  sqrt(|bin min|)
     int *sI = reinterpret_cast<int *>(sV + QB * nT);       // [QB][nT]  1-based index
-    int chunk, qs, n;
-    irc::tile_lookup<QB>(p, blockIdx.x, chunk, qs, n);
-    const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
-    irc::stage_queries<QB>(F, nC, qs, n, sA);
-    __syncthreads();
-    const int nT0 = nT / nBB;
-    for (int t = threadIdx.x; t < nT; t += blockDim.x) {
-        const int b = t % nBB;
-        const int ib0 = __ldg(p.rsr + r0 + b), nb0 = __ldg(p.rnr + r0 + b);
-        float mn[QB];
-        int mi[QB];
+    for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
+        int chunk, qs, n;
+        irc::tile_lookup<QB>(p, tq.tile(w), chunk, qs, n);
+        const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
+        irc::stage_queries<QB>(F, nC, qs, n, sA);
+        __syncthreads();
+        const int nT0 = nT / nBB;
+        for (int t = threadIdx.x; t < nT; t += blockDim.x) {
+            const int b = t % nBB;
+            const int ib0 = __ldg(p.rsr + r0 + b), nb0 = __ldg(p.rnr + r0 + b);
+            float mn[QB];
+            int mi[QB];
 #pragma unroll
-        for (int q = 0; q < QB; ++q) { mn[q] = IRC_SINGLE_INF_F; mi[q] = qs + min(q, n - 1); }
-        irc::scan_bin<QB, false>(F, nullptr, nC, ib0 + t / nBB, ib0 + nb0, nT0, sA, nullptr, mn, mi);
+            for (int q = 0; q < QB; ++q) { mn[q] = IRC_SINGLE_INF_F; mi[q] = qs + min(q, n - 1); }
+            irc::scan_bin<QB, false>(F, nullptr, nC, ib0 + t / nBB, ib0 + nb0, nT0, sA, nullptr, mn, mi);
 #pragma unroll
-        for (int q = 0; q < QB; ++q) { sV[q * nT + t] = irc::ref_sqrt_abs(mn[q]); sI[q * nT + t] = mi[q] + 1; }
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const float kTaken = -1.0f;
-    for (int q = warp; q < n; q += nw) {
-        float *v = sV + q * nT;
-        const int *ix = sI + q * nT;
-        const size_t o = (size_t)(qs + q - p.q_base);
-        float last = 0.0f;
-        for (int k = 0; k < knn; ++k) {
-            unsigned long long best = ~0ull;
-            for (int t = lane; t < nT; t += 32) {
-                const float x = v[t];
-                const unsigned long long key = (x == kTaken) ? ~0ull : irc::sort_key(x, t);
-                best = key < best ? key : best;
+            for (int q = 0; q < QB; ++q) { sV[q * nT + t] = irc::ref_sqrt_abs(mn[q]); sI[q * nT + t] = mi[q] + 1; }
+        }
+        __syncthreads();
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        const float kTaken = -1.0f;
+        for (int q = warp; q < n; q += nw) {
+            float *v = sV + q * nT;
+            const int *ix = sI + q * nT;
+            const size_t o = (size_t)(qs + q - p.q_base);
+            float last = 0.0f;
+            for (int k = 0; k < knn; ++k) {
+                unsigned long long best = ~0ull;
+                for (int t = lane; t < nT; t += 32) {
+                    const float x = v[t];
+                    const unsigned long long key = (x == kTaken) ? ~0ull : irc::sort_key(x, t);
+                    best = key < best ? key : best;
+                }
+                best = irc::warp_min_u64(best);
+                const int t = (int)(best & 0xffffffffu);
+                last = v[t];
+                __syncwarp();
+                if (lane == 0) {
+                    miKnn[(size_t)k + (size_t)knn * o] = ix[t];
+                    v[t] = kTaken;
+                }
+                __syncwarp();
             }
-            best = irc::warp_min_u64(best);
-            const int t = (int)(best & 0xffffffffu);
-            last = v[t];
-            __syncwarp();
             if (lane == 0) {
-                miKnn[(size_t)k + (size_t)knn * o] = ix[t];
-                v[t] = kTaken;
+                vrKnn[o] = last;
+                if (rho) rho[o] = __fdiv_rn(1.0f, last);
             }
-            __syncwarp();
         }
-        if (lane == 0) {
-            vrKnn[o] = last;
-            if (rho) rho[o] = __fdiv_rn(1.0f, last);
-        }
+        __syncthreads();
     }
 }
 
@@ -247,37 +252,26 @@ void merge_runs(const int32_t *roff, const int32_t *rs, const int32_t *rn, int n
 
 }  // namespace
 
-// Tensor-core operand rows (two [nF x row_bytes] matrices) followed by the
-// re-rank's FP32 rows padded to 16-byte multiples ([nF x fp_row_bytes]) and
-// extra_bytes of working space (256-byte aligned);
-// allocated on the first tensor-core call of a plan, grown when a call
-// needs more, kept until irc_plan_destroy.
-int irc_plan_tc_buffers(irc_plan *pl, void **fq, void **fc, void **fp, void **extra, size_t row_bytes,
-                        size_t fp_row_bytes, size_t extra_bytes)
+// The plan's tensor-core working memory, `need` bytes: the caller's buffer
+// (irc_plan_set_tc_buffer), or one allocated on the first tensor-core call of
+// the plan, grown when a call needs more, kept until irc_plan_destroy.
+int irc_plan_tc_buffer(irc_plan *pl, size_t need, void **buf)
 {
-    const size_t one = (size_t)pl->dev.nF * row_bytes;
-    const size_t fpb = ((size_t)pl->dev.nF * fp_row_bytes + 255) & ~(size_t)255;
-    const size_t need = 2 * one + fpb + extra_bytes;
     if (pl->tc_external) {
         if (pl->tc_bytes < need) {
             irc_host::set_error("irc_site_knn: the shared operand buffer holds %zu bytes, %zu needed",
                                 pl->tc_bytes, need);
             return IRC_E_INVAL;
         }
-        pl->tc_row_bytes = row_bytes;
-    } else if (!pl->tc_buf || pl->tc_bytes < need || pl->tc_row_bytes != row_bytes) {
+    } else if (!pl->tc_buf || pl->tc_bytes < need) {
         if (pl->tc_buf) cudaFree(pl->tc_buf);
         pl->tc_buf = nullptr;
         pl->tc_bytes = 0;
         cudaError_t e = cudaMalloc(&pl->tc_buf, need);
         if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: operand buffers");
-        pl->tc_row_bytes = row_bytes;
         pl->tc_bytes = need;
     }
-    *fq = pl->tc_buf;
-    *fc = (char *)pl->tc_buf + one;
-    *fp = (char *)pl->tc_buf + 2 * one;
-    *extra = (char *)pl->tc_buf + 2 * one + fpb;
+    *buf = pl->tc_buf;
     return IRC_OK;
 }
 
@@ -341,6 +335,19 @@ int irc_exact_chunk_fill(float *D, int32_t *I, const float *F, const int32_t *IB
     cudaStreamSynchronize(s);                    // the plan's image is released with the call
     irc_plan_destroy(pl);
     return rc;
+}
+
+// search_min_drift + sort over the tiles of tq (all of the plan's by default).
+int irc_ref_tiles(irc_plan *pl, const float *F, int nC, int knn, int nThreads, float *vrKnn, float *rho,
+                  int32_t *miKnn, const irc::TileQueue &tq, cudaStream_t s)
+{
+    const size_t smem = (size_t)kKnnQB * nThreads * 8;
+    cudaError_t e = cudaFuncSetAttribute(k_site_knn_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: smem attribute");
+    const int tiles = tiles_for(pl, kKnnQB), grid = tq.list ? std::min(tiles, 152) : tiles;
+    k_site_knn_ref<<<grid, kThreads, smem, s>>>(pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
+    IRC_CHECK_LAUNCH("irc_site_knn(REF)");
+    return IRC_OK;
 }
 
 // Exact / tensor-core site kernels (irc_exact.cu, irc_tc.cu).
@@ -471,8 +478,8 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     // counters, two query lists, the delta fallback's (tile, part) units (up to 8 parts per
     // 16-query tile) and its per-query 64-bit best keys (8-byte aligned: every term before
     // them is even)
-    const size_t scratch_ints = irc::kScratchLists + 2 * (size_t)n_out +
-                                16 * ((size_t)n_out / 16 + nChunks + 1) + 2 * (size_t)n_out;
+    const size_t scratch_ints = irc::kScratchLists + 2 * (size_t)n_out + 2 * delta_items(n_out, nChunks) +
+                                2 * (size_t)n_out;
     cudaError_t e = cudaMalloc(&pl->dmem, (img.size() + scratch_ints) * sizeof(int32_t));
     if (e != cudaSuccess) {
         free(pl->h_q0); free(pl->h_nq); free(pl->h_roff); free(pl->h_rs); free(pl->h_rn); free(pl);
@@ -509,6 +516,12 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     pl->max_nq = max_nq;
     pl->pairs = pairs;
     row_intervals(q0, nq, rs, rn, nChunks, nRuns, pl);
+    pl->runs_ascend = 1;
+    for (int i = 0; i < nChunks; ++i)
+        for (int r = roff[i]; r < roff[i + 1]; ++r) {
+            pl->max_rn = std::max(pl->max_rn, rn[r]);
+            if (r > roff[i] && rs[r] < rs[r - 1] + rn[r - 1]) pl->runs_ascend = 0;
+        }
     *out = pl;
     return IRC_OK;
 }
@@ -517,6 +530,7 @@ int irc_plan_destroy(irc_plan *pl)
 {
     if (!pl) return IRC_OK;
     cudaError_t e = cudaFree(pl->dmem);
+    irc_cert_release(pl);
     if (pl->tc_buf && !pl->tc_external) cudaFree(pl->tc_buf);
     if (pl->tc_items_buf) cudaFree(pl->tc_items_buf);
     if (pl->row_dims) cudaFree(pl->row_dims);
@@ -528,9 +542,7 @@ int irc_plan_destroy(irc_plan *pl)
 size_t irc_plan_tc_bytes(const irc_plan *pl, int nC)
 {
     if (!pl || nC < 1) return 0;
-    const size_t one = (size_t)pl->dev.nF * 128;
-    const size_t fpb = ((size_t)pl->dev.nF * (size_t)irc_tc::fp_row4(nC) * 16 + 255) & ~(size_t)255;
-    return 2 * one + fpb + (size_t)256 * 64 * 4 + 256 + irc_tc::list_area_bytes(pl->dev.n_out);
+    return irc_tc::ops_bytes(pl, nC, irc_tc::Fmt::bf16) + irc_tc::list_area_bytes(pl->dev.n_out);
 }
 
 int irc_plan_set_tc_buffer(irc_plan *pl, void *buf, size_t bytes)
@@ -542,7 +554,6 @@ int irc_plan_set_tc_buffer(irc_plan *pl, void *buf, size_t bytes)
     if (pl->tc_buf && !pl->tc_external) cudaFree(pl->tc_buf);
     pl->tc_buf = buf;
     pl->tc_bytes = bytes;
-    pl->tc_row_bytes = 0;
     pl->tc_external = 1;
     return IRC_OK;
 }
@@ -665,14 +676,15 @@ int irc_site_knn(irc_plan *pl, const float *F, int nC, int knn, int nThreads, in
                 irc_host::set_error("irc_site_knn: chunk %d has more runs than bins", i);
                 return IRC_E_INVAL;
             }
-        const size_t smem = (size_t)kKnnQB * nThreads * 8;
-        cudaError_t e = cudaFuncSetAttribute(k_site_knn_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: smem attribute");
-        k_site_knn_ref<<<tiles_for(pl, kKnnQB), kThreads, smem, s>>>(pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn);
-        IRC_CHECK_LAUNCH("irc_site_knn(REF)");
-        return IRC_OK;
+        const int rc = irc_cert_site_knn(pl, F, nC, knn, nThreads, mode, vrKnn, rho, miKnn, nullptr, s);
+        if (rc != IRC_CERT_PASS) return rc;
+        return irc_ref_tiles(pl, F, nC, knn, nThreads, vrKnn, rho, miKnn, irc::TileQueue{}, s);
     }
-    if (mode == IRC_MODE_EXACT) return irc_site_knn_exact(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, s);
+    if (mode == IRC_MODE_EXACT) {
+        const int rc = irc_cert_site_knn(pl, F, nC, knn, 0, mode, vrKnn, rho, miKnn, d2Knn, s);
+        if (rc != IRC_CERT_PASS) return rc;
+        return irc_site_knn_exact(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, s);
+    }
     if (mode == IRC_MODE_BF16 || mode == IRC_MODE_FP8)
         return irc_site_knn_tc(pl, F, nC, knn, mode, vrKnn, rho, miKnn, d2Knn, s);
     irc_host::set_error("irc_site_knn: unknown mode %d", mode);
@@ -694,6 +706,8 @@ int irc_site_delta(irc_plan *pl, const float *F, int nC, const float *R, int nTh
                 irc_host::set_error("irc_site_delta: chunk %d has more runs than bins", i);
                 return IRC_E_INVAL;
             }
+        const int rc = irc_cert_site_delta_ref(pl, F, nC, R, nThreads, delta, nneigh, s);
+        if (rc != IRC_CERT_PASS) return rc;
         k_site_delta_ref<<<tiles_for(pl, kDeltaQB), kThreads, 0, s>>>(pl->dev, F, R, nC, nThreads, delta, nneigh);
         IRC_CHECK_LAUNCH("irc_site_delta(REF)");
         return IRC_OK;

@@ -53,6 +53,7 @@
 // tensor pipe.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <mutex>
 #include <type_traits>
@@ -60,6 +61,7 @@
 
 #include "irc_common.cuh"
 #include "irc_plan.cuh"
+#include "irc_rerank.cuh"
 #include "irc_sm100.cuh"
 #include "irc_tc.cuh"
 
@@ -70,7 +72,12 @@ __constant__ uint32_t c_wait_polls = 1u << 22;
 namespace {
 
 using irc_tc::BM;
+using irc_tc::Fmt;
 using irc_tc::KP;
+using irc_rr::emit;
+using irc_rr::QROW4;
+using irc_rr::TAU_LOW_BIT;
+using irc_rr::WARP_KEYS;
 constexpr int PARTS = 4;                          // epilogue warps per TMEM lane quarter
 constexpr int PART = 32;                          // columns of a 128-tile per epilogue warp (one minimum each)
 constexpr int BROW = 128 + 1;                     // minima row of a query (f32, 4 parts x 32) in the threshold step
@@ -82,9 +89,6 @@ constexpr uint32_t TMEM_COLS = 512;               // all TMEM columns (one CTA p
 constexpr int LISTCAP = 192;                      // candidate-list capacity per query (the four warps' hits pooled)
 constexpr int LROW = LISTCAP + 1;                 // list row (u32), padded
 constexpr size_t LIST_BYTES = (size_t)LROW * BM * 4;
-constexpr int WARP_KEYS = 64;                     // sorted re-rank keys kept per epilogue warp
-constexpr int QROW4 = 16;                         // float4 of a staged query row (nC <= 64)
-constexpr int TAU_LOW_BIT = 12;                   // threshold search stops at this bit (2^-11 relative)
 // The threshold is the tau_rank-th smallest per-column minimum: tau_rank
 // distinct candidates lie at or below it, a margin over knn (<= 32) for the
 // rounding of the filter.  A list it cut must hold at least knn +
@@ -97,10 +101,11 @@ constexpr int TAU_LOW_BIT = 12;                   // threshold search stops at t
 // BF16 distance error, ~2^-8 |a| / d relative, crossed the gap between the
 // 30th and 40th neighbour), rank 44 did not.  FP8 (3 mantissa bits) keeps
 // rank 64.
-__host__ __device__ constexpr int tau_rank(bool fp8) { return fp8 ? 64 : 48; }
-__host__ __device__ constexpr int crowd_margin(bool fp8) { return fp8 ? 16 : 8; }
-static_assert(tau_rank(false) >= irc_tc::KNN_MAX + crowd_margin(false), "rank covers knn plus the margin");
-static_assert(tau_rank(true) >= irc_tc::KNN_MAX + crowd_margin(true), "rank covers knn plus the margin");
+// F16 takes BF16's rank: its callers prove each query's list complete.
+__host__ __device__ constexpr int tau_rank(Fmt f) { return f == Fmt::fp8 ? 64 : 48; }
+__host__ __device__ constexpr int crowd_margin(Fmt f) { return f == Fmt::fp8 ? 16 : 8; }
+static_assert(tau_rank(Fmt::bf16) >= irc_tc::KNN_MAX + crowd_margin(Fmt::bf16), "rank covers knn plus the margin");
+static_assert(tau_rank(Fmt::fp8) >= irc_tc::KNN_MAX + crowd_margin(Fmt::fp8), "rank covers knn plus the margin");
 static_assert((size_t)BROW * BM * 4 <= LIST_BYTES, "minima rows alias the list area");
 static_assert(LISTCAP <= irc_tc::LIST_MAX, "the re-rank takes every list the filter hands over");
 
@@ -146,42 +151,6 @@ __device__ __forceinline__ bool pipe_wait(uint64_t *bar, uint32_t parity, volati
     return sm100::mbar_wait(bar, parity, abort_flag, lim, lim < 64u ? lim : 0u);
 }
 
-// Ascending bitonic sort of 32*PER keys held PER per lane (element e = lane*PER + i).
-template <class T, int PER>
-__device__ __forceinline__ void warp_bitonic(T (&v)[PER], int lane)
-{
-    constexpr int N = 32 * PER;
-#pragma unroll
-    for (int size = 2; size <= N; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= PER) {
-                const int ls = stride / PER;
-#pragma unroll
-                for (int i = 0; i < PER; ++i) {
-                    const int e = lane * PER + i;
-                    const T o = __shfl_xor_sync(0xffffffffu, v[i], ls);
-                    const bool up = (e & size) == 0, lower = (e & stride) == 0;
-                    v[i] = (lower == up) ? (o < v[i] ? o : v[i]) : (o > v[i] ? o : v[i]);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < PER; ++i) {
-                    const int j = i ^ stride;
-                    if (j > i) {
-                        const int e = lane * PER + i;
-                        const bool up = (e & size) == 0;
-                        const T a = v[i], b = v[j];
-                        const bool sw = up ? (a > b) : (a < b);
-                        v[i] = sw ? b : a;
-                        v[j] = sw ? a : b;
-                    }
-                }
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ double dist2_f64(const float *__restrict__ b, const float *__restrict__ a, int nd)
 {
     double acc = 0.0;
@@ -190,31 +159,6 @@ __device__ __forceinline__ double dist2_f64(const float *__restrict__ b, const f
         acc = __dadd_rn(acc, __dmul_rn(d, d));
     }
     return acc;
-}
-
-__device__ __forceinline__ void emit(int e, unsigned long long key, int q, int knn, size_t o, int *miKnn,
-                                     float *d2Knn, float *vrKnn, float *rho)
-{
-    const bool have = key != ~0ull;
-    const float d2 = have ? __uint_as_float((unsigned)(key >> 32)) : IRC_SINGLE_INF_F;
-    const int idx = have ? (int)(key & 0xffffffffu) : q;
-    // streaming stores: the outputs are not read again by this kernel and
-    // should not push the gathered feature rows out of L2
-    __stcs(miKnn + (size_t)e + (size_t)knn * o, idx + 1);
-    if (d2Knn) __stcs(d2Knn + (size_t)e + (size_t)knn * o, d2);
-    if (e == knn - 1) {
-        const float vk = irc::ref_sqrt_abs(d2);
-        __stcs(vrKnn + o, vk);
-        if (rho) __stcs(rho + o, __fdiv_rn(1.0f, vk));
-    }
-}
-
-// 256-bit read-only load of 8 floats (32-byte aligned).
-__device__ __forceinline__ void ld_nc_v8(const float *p, float (&v)[8])
-{
-    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                 : "l"(p));
 }
 
 // Exact re-rank of the cL candidates listed for query q (list[0 .. cL)),
@@ -231,47 +175,8 @@ __device__ __forceinline__ void rerank(const uint32_t *__restrict__ list, int cL
                                        float *vrKnn, float *rho, int *scratch)
 {
     const float *a = F + (size_t)q * nC;
-    // the query row, staged once per warp (broadcast reads below)
-    if (lane < Dp4) qs[lane] = __ldg(Fp + (size_t)q * Dp4 + lane);
-    // exact FP32 distances with the reference arithmetic (d = b - a, fused
-    // accumulate in feature order)
-    const int nbatch = (cL + 31) / 32;                // <= PER (checked by the caller)
     unsigned long long kv[PER];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) kv[i] = ~0ull;
-    __syncwarp();
-#pragma unroll
-    for (int bi = 0; bi < PER; ++bi) {
-        if (bi >= nbatch) break;
-        const int e = bi * 32 + lane;
-        if (e < cL) {
-            const int idx = (int)__ldg(list + e);
-            // whole 32-byte sectors: rows are padded to a multiple of 8 floats
-            const float *bs = reinterpret_cast<const float *>(Fp + (size_t)idx * Dp4);
-            float acc = 0.0f;
-            const int full = nd >> 3, tail = nd & 7;   // whole groups of 8 features, then the rest
-#pragma unroll 2
-            for (int c8 = 0; c8 < full; ++c8) {
-                float bv[8];
-                ld_nc_v8(bs + 8 * c8, bv);
-                const float4 a0 = qs[2 * c8], a1 = qs[2 * c8 + 1];
-                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-                for (int u = 0; u < 8; ++u) acc = irc::dterm(acc, bv[u], av[u]);
-            }
-            if (tail) {
-                float bv[8];
-                ld_nc_v8(bs + 8 * full, bv);
-                const float4 a0 = qs[2 * full], a1 = qs[2 * full + 1];
-                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (u < tail) acc = irc::dterm(acc, bv[u], av[u]);
-            }
-            if (acc > 0.0f && acc < IRC_SINGLE_INF_F)
-                kv[bi] = ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned)idx;
-        }
-    }
+    irc_rr::list_keys<PER>(list, cL, Fp, Dp4, q, qs, nd, lane, kv);
     // A list cut by tau that holds fewer than knn + margin positive distances
     // (exact copies of the query, at distance 0 and excluded like the
     // reference's d > 0 test, crowded the threshold) may miss nearer
@@ -288,76 +193,11 @@ __device__ __forceinline__ void rerank(const uint32_t *__restrict__ list, int cL
             return;
         }
     }
-    // ws[0 .. WARP_KEYS) <- the smallest keys, ascending, selection first:
-    // a bitwise search (stopped at TAU_LOW_BIT,
-    // rounded up) bounds the k-th distance from above, and the keys at or
-    // below that bound plus 2^-16 relative -- the band below lies inside it
-    // -- are compacted into ws and sorted alone, one per lane when at most 32
-    // pass (the usual case: about knn of them), else two per lane.  They are
-    // the first positions of the full sort, so the result is the same; if
-    // more than WARP_KEYS pass, the full sort runs.
-    bool sorted = false;
-    if (PER >= 2) {
-        // the bits above the highest one in which the keys' distances differ
-        // are common to all of them, hence the answer's: start below them
-        unsigned lo = 0xffffffffu, hi = 0u;
-#pragma unroll
-        for (int i = 0; i < PER; ++i)
-            if (kv[i] != ~0ull) {
-                lo = min(lo, (unsigned)(kv[i] >> 32));
-                hi = max(hi, (unsigned)(kv[i] >> 32));
-            }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        unsigned ans = 0;
-        int top = 30;
-        if (lo <= hi) {                           // some key: distances are below 2^31 as bit patterns
-            const unsigned x = lo ^ hi;
-            top = x ? 31 - __clz(x) : TAU_LOW_BIT;
-            ans = top < 31 ? lo & ~((2u << top) - 1u) : 0u;
-            top = min(top, 30);
-        }
-#pragma unroll 1
-        for (int b = top; b >= TAU_LOW_BIT; --b) {
-            const unsigned t = ans | (1u << b);
-            unsigned c = 0;
-#pragma unroll
-            for (int i = 0; i < PER; ++i) c += (unsigned)((unsigned)(kv[i] >> 32) < t);
-            if (__reduce_add_sync(0xffffffffu, c) < (unsigned)knn) ans = t;
-        }
-        const unsigned ub = ans | ((1u << TAU_LOW_BIT) - 1u);
-        const unsigned tb = ub >= 0x7f800000u ? 0x7f800000u
-                                              : __float_as_uint(__uint_as_float(ub) * (1.0f + 0x1p-16f));
-        int n = 0;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const bool pr = (unsigned)(kv[i] >> 32) <= tb;          // never an empty slot (~0)
-            const unsigned bal = __ballot_sync(0xffffffffu, pr);
-            const int pos = n + __popc(bal & ((1u << lane) - 1u));
-            if (pr && pos < WARP_KEYS) ws[pos] = kv[i];
-            n += __popc(bal);
-        }
-        __syncwarp();
-        if (n <= 32) {                            // the common case: ~knn keys, one per lane
-            unsigned long long v1[1] = {lane < n ? ws[lane] : ~0ull};
-            __syncwarp();
-            warp_bitonic<unsigned long long, 1>(v1, lane);
-            ws[lane] = v1[0];
-            ws[32 + lane] = ~0ull;
-            sorted = true;
-        } else if (n <= WARP_KEYS) {
-            unsigned long long v2[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) v2[i] = lane * 2 + i < n ? ws[lane * 2 + i] : ~0ull;
-            __syncwarp();
-            warp_bitonic<unsigned long long, 2>(v2, lane);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) ws[lane * 2 + i] = v2[i];
-            sorted = true;
-        }
-    }
-    if (!sorted) {
-        warp_bitonic<unsigned long long, PER>(kv, lane);
+    // ws[0 .. WARP_KEYS) <- the smallest keys, ascending; if more than
+    // WARP_KEYS pass the selection's bound, the full sort runs
+    unsigned tb;
+    if (irc_rr::select_keys<PER>(kv, knn, ws, lane, tb) > WARP_KEYS) {
+        irc_rr::warp_bitonic<unsigned long long, PER>(kv, lane);
 #pragma unroll
         for (int i = 0; i < PER; ++i)
             if (lane * PER + i < WARP_KEYS) ws[lane * PER + i] = kv[i];
@@ -523,26 +363,36 @@ __device__ __forceinline__ void mark2x32_signs(uint32_t ta, int la, uint32_t tb,
 }
 
 // The pass-2 threshold of query row `row` into the query tile in shared
-// memory: -tau' split exactly into three BF16 terms at K positions tau_k ..
+// memory: -tau' split into three BF16 (exactly) or F16 terms (to 2^-25
+// absolute) at K positions tau_k ..
 // tau_k + 2, against 1, 1, 1 in every candidate row, so the pass-2
-// accumulators are d2 - tau'.  tau' = tau (1 + 2^-10), capped at 1e30: the
+// accumulators are d2 - tau'.  tau' = tau (1 + 2^-10), capped at 1e30 (F16:
+// 60000, above every distance its scaled operands can form): the
 // small margin keeps every candidate at or below tau negative whatever the
 // rounding of the extra terms.  The tile is 128-byte swizzled: the 16-byte
 // piece c of row r sits at piece c ^ (r % 8).
+template <Fmt FMT>
 __device__ __forceinline__ void put_tau(uint8_t *sA, int row, int tau_k, float tau)
 {
-    const float x = -fminf(tau * (1.0f + 0x1p-10f), 1e30f);
-    const __nv_bfloat16 h = __float2bfloat16_rn(x);
-    const float r1 = x - __bfloat162float(h);
-    const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-    const __nv_bfloat16 l = __float2bfloat16_rn(r1 - __bfloat162float(m));
-    const __nv_bfloat16 v[3] = {h, m, l};
+    const float x = -fminf(tau * (1.0f + 0x1p-10f), FMT == Fmt::f16 ? 60000.0f : 1e30f);
+    uint16_t v[3];
+    float rem = x;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        if (FMT == Fmt::f16) {
+            const __half h = __float2half_rn(rem);
+            rem -= __half2float(h);
+            v[t] = __half_as_ushort(h);
+        } else {
+            const __nv_bfloat16 h = __float2bfloat16_rn(rem);
+            rem -= __bfloat162float(h);
+            v[t] = __bfloat16_as_ushort(h);
+        }
+    }
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
         const int k = tau_k + t;
-        __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(sA + (size_t)row * 128 +
-                                                               (((k >> 3) ^ (row & 7)) << 4) + (k & 7) * 2);
-        *dst = v[t];
+        *reinterpret_cast<uint16_t *>(sA + (size_t)row * 128 + (((k >> 3) ^ (row & 7)) << 4) + (k & 7) * 2) = v[t];
     }
 }
 
@@ -585,7 +435,7 @@ __device__ __forceinline__ bool slot_barrier_and(int slot, int nthreads, bool v)
 // sends the query to the exact fallback instead.
 __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::TcItem &it, int s, int quarter, int part,
                                          int qrow, int nq_s, const uint32_t *lists, const int *sCnt,
-                                         const irc_tc::ListOut &lo, int *scratch, int lane)
+                                         const float *sTau, const irc_tc::ListOut &lo, int *scratch, int lane)
 {
     constexpr int RL = 32 / PARTS;
     int cL = -1;                                  // -1: no query in this lane, -2: to the fallback
@@ -607,9 +457,13 @@ __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::Tc
     const bool fits = (unsigned long long)base + total <= (unsigned long long)lo.cap;
     if (lane < RL && cL != -1) {
         const int q = it.qs[s] + qrow + part * RL + lane;
+        if (lo.cert)                              // the list's bound and its chunk, for the proof of completeness
+            lo.cert[q - p.q_base] = make_int2(__float_as_int(sTau[quarter * 32 + part * RL + lane]), it.chunk[s]);
         if (cL == -2 || !fits) {
-            const int k = atomicAdd(scratch + 0, 1);
-            scratch[irc::kScratchLists + k] = q;
+            if (!lo.cert) {                       // (with the record above, its tile is searched again)
+                const int k = atomicAdd(scratch + 0, 1);
+                scratch[irc::kScratchLists + k] = q;
+            }
         } else {
             // bit 30: the list holds every candidate of the chunk (nothing was cut by tau)
             const int complete = cL == __ldg(p.ncand + it.chunk[s]) ? (1 << 30) : 0;
@@ -653,7 +507,7 @@ struct Shared {
 // synchronise only among themselves (named barrier 1 + slot).  Unit g of a
 // slot (counted over all its items, both passes) goes to accumulator
 // s * BPS + g % BPS, whose barriers are in phase g / BPS.
-template <int BN, int NS, bool TAU>
+template <int BN, int NS, Fmt FMT, bool TAU>
 __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::TcItem *__restrict__ items, int rank,
                                          uint32_t tmem, int tau_k, const Shared &sh, const irc_tc::ListOut &lo,
                                          int *scratch, int warp, int lane)
@@ -787,7 +641,7 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             // the thresholds into the item's query tile; visible to the tensor
             // core (async proxy) before the MMA thread, released by tau_ready,
             // issues the slot's pass-2 MMAs (one phase per item with units)
-            put_tau(sh.sA + (size_t)r * A_BYTES, row, tau_k, tau);
+            put_tau<FMT>(sh.sA + (size_t)r * A_BYTES, row, tau_k, tau);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) sm100::mbar_arrive(&sh.tau_ready[s]);
@@ -816,7 +670,7 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             if (lane == 0) sm100::mbar_arrive(&sh.acc_empty[b]);
         }
         slot_barrier(s, slot_threads);
-        if (__all_sync(0xffffffffu, ok)) hand_off(p, it, s, quarter, part, qrow, nq_s, sh.lists, sh.sCnt, lo, scratch, lane);
+        if (__all_sync(0xffffffffu, ok)) hand_off(p, it, s, quarter, part, qrow, nq_s, sh.lists, sh.sCnt, sh.sTau, lo, scratch, lane);
         g0 += 2u * (unsigned)U;
         // every warp of the slot is done with this item's lists before the
         // next item's minima overwrite them; after a timed-out wait all stop
@@ -905,15 +759,15 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
 // wrote the thresholds into the query tile (tau_ready[s], one phase per item
 // in which the slot has units).  After an item's last MMA a commit frees its
 // query tile.
-template <int BN, int NS, bool FP8, bool TAU>
+template <int BN, int NS, Fmt FMT, bool TAU>
 __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcItem *__restrict__ items, int nk,
                                       uint32_t tmem, const Shared &sh)
 {
     using T = Tile<BN>;
     constexpr int BPS = T::NBUF / NS;
-    // bf16 x bf16 (kind::f16, K = 16) or e4m3 x e4m3 (kind::f8f6f4, K = 32) -> f32;
-    // either way one MMA consumes 32 bytes of every 128-byte operand row
-    constexpr uint32_t idesc = FP8 ? sm100::idesc_make(BM, BN, 0, 0) : sm100::idesc_make(BM, BN, 1, 1);
+    // bf16 x bf16 or f16 x f16 (kind::f16, K = 16) or e4m3 x e4m3 (kind::f8f6f4, K = 32)
+    // -> f32; either way one MMA consumes 32 bytes of every 128-byte operand row
+    constexpr uint32_t idesc = FMT == Fmt::bf16 ? sm100::idesc_make(BM, BN, 1, 1) : sm100::idesc_make(BM, BN, 0, 0);
     unsigned g0[NS], taus[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) g0[s] = taus[s] = 0;
@@ -952,7 +806,7 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
                         for (int kk = 0; kk < KP / 16; ++kk)
                             if (kk >= nk)
                                 break;                    // the rest of every operand row is zero
-                            else if (FP8)
+                            else if (FMT == Fmt::fp8)
                                 sm100::mma_f8(tmem + b * BN, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk > 0 ? 1u : 0u);
                             else
                                 sm100::mma_f16(tmem + b * BN, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk > 0 ? 1u : 0u);
@@ -983,7 +837,7 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
 // is empty.  TAU: pass 2 reads the signs of d2 - tau (the thresholds written
 // into the query tile at K position tau_k), else it compares d2 with tau in
 // the epilogue.
-template <bool FP8, int BN, bool TAU, int NS>
+template <Fmt FMT, int BN, bool TAU, int NS>
 __global__ void __launch_bounds__(THREADS, 1)
 k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmC, irc::PlanDev p,
          const irc_tc::TcItem *__restrict__ items, int n_items, unsigned *queue, int nk, int tau_k, irc_tc::ListOut lo,
@@ -1042,10 +896,10 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
         if (lane == 0) produce<BN, NS>(tmQ, tmC, p, items, n_items, queue, sh);
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) issue<BN, NS, FP8, TAU>(p, items, nk, tmem, sh);
+        if (lane == 0) issue<BN, NS, FMT, TAU>(p, items, nk, tmem, sh);
         __syncwarp();
     } else {
-        epilogue<BN, NS, TAU>(p, items, tau_rank(FP8), tmem, tau_k, sh, lo, scratch, warp, lane);
+        epilogue<BN, NS, FMT, TAU>(p, items, tau_rank(FMT), tmem, tau_k, sh, lo, scratch, warp, lane);
     }
     sm100::tc_fence_before();
     __syncthreads();
@@ -1111,12 +965,12 @@ static cudaEvent_t *profile_slot()
     return &g_prof_ev[3 * g_prof_used++];
 }
 
-template <bool FP8, int BN, bool TAU, int NS>
+template <Fmt FMT, int BN, bool TAU, int NS>
 static int launch_filter(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, const irc_tc::TcItem *items,
-                         int n_items, unsigned *queue, int nk, int tau_k, const ListOut &lo, cudaStream_t s)
+                         int n_items, unsigned *queue, int nk, int tau_k, const ListOut &lo, int *scratch, cudaStream_t s)
 {
     if (n_items <= 0) return IRC_OK;
-    auto kern = k_knn_tc<FP8, BN, TAU, NS>;
+    auto kern = k_knn_tc<FMT, BN, TAU, NS>;
     const int smem = (int)Tile<BN>::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int sms = 0;
@@ -1125,28 +979,27 @@ static int launch_filter(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan 
     // persistent: one CTA per SM (shared memory and TMEM allow one), each
     // taking items from the queue until it is empty
     const int grid = n_items < sms ? n_items : sms;
-    kern<<<grid, THREADS, smem, s>>>(mq, mc, pl->dev, items, n_items, queue, nk, tau_k, lo, pl->scratch);
+    kern<<<grid, THREADS, smem, s>>>(mq, mc, pl->dev, items, n_items, queue, nk, tau_k, lo, scratch);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core)");
     return IRC_OK;
 }
 
-int launch_knn_tc(bool fp8, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, const float *F,
-                  const float4 *Fp, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn, float *d2Knn,
-                  const ListOut &lo, cudaStream_t s)
+// The filter of every packing class of the plan on stream s.
+int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, int nC, const ListOut &lo,
+                   int *scratch, cudaStream_t s)
 {
     const int n_out = pl->dev.n_out;
     cudaError_t e = cudaMemsetAsync(lo.qinfo, 0xff, (size_t)n_out * sizeof(int2), s);   // (-1, -1): no list
     if (e == cudaSuccess) e = cudaMemsetAsync(lo.count, 0, 4 * sizeof(unsigned), s);     // count, queue heads
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): memset");
-    // BF16: the pass-2 thresholds go into K positions nC + 6 .. nC + 8 of the
-    // query rows when they fit (else, and for FP8, pass 2 compares in the
+    // BF16, F16: the pass-2 thresholds go into K positions nC + 6 .. nC + 8 of
+    // the query rows when they fit (else, and for FP8, pass 2 compares in the
     // epilogue).  MMAs per unit: only the 32-byte K slices that hold data
-    // (nC features, 6 BF16 / 12 FP8 norm entries, the threshold terms).
+    // (nC features, 6 BF16 / F16 or 12 FP8 norm entries, the threshold terms).
+    const bool fp8 = fmt == Fmt::fp8;
     const int tau_k = (!fp8 && nC + 9 <= KP) ? nC + 6 : -1;
     const int used = fp8 ? nC + 12 : 2 * (nC + (tau_k >= 0 ? 9 : 6));
     const int nk = (used + 31) / 32;
-    cudaEvent_t *ev = profile_slot();
-    if (ev) cudaEventRecord(ev[0], s);
     // one persistent launch per packing class: one-slot and two-slot items on
     // 256-candidate units (or 128, irc_plan_tc_units), then four-slot items
     // on 128.  The threshold goes into the MMA only on 256-wide units; the
@@ -1157,34 +1010,40 @@ int launch_knn_tc(bool fp8, const CUtensorMap &mq, const CUtensorMap &mc, irc_pl
     const int n1 = pl->n_tc_one, n2 = pl->n_tc_wide - pl->n_tc_one, n4 = pl->n_tc_items - pl->n_tc_wide;
     const irc_tc::TcItem *it1 = pl->tc_items, *it2 = it1 + n1, *it4 = it2 + n2;
     const bool narrow = pl->tc_wide_bn == 128;
+    auto run = [&](auto fmt_c, auto tau_c) {
+        constexpr Fmt F = decltype(fmt_c)::value;
+        constexpr bool T = decltype(tau_c)::value;
+        int r = narrow ? launch_filter<F, 128, false, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, scratch, s)
+                       : launch_filter<F, 256, T, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, scratch, s);
+        if (r != IRC_OK) return r;
+        r = narrow ? launch_filter<F, 128, false, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, scratch, s)
+                   : launch_filter<F, 256, T, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, scratch, s);
+        if (r != IRC_OK) return r;
+        return launch_filter<F, 128, false, 4>(mq, mc, pl, it4, n4, lo.count + 3, nk, tau_k, lo, scratch, s);
+    };
     using yes = std::true_type;
     using no = std::false_type;
-    auto run = [&](auto tau_c) {
-        constexpr bool T = decltype(tau_c)::value;
-        int r;
-        if (narrow)
-            r = fp8 ? launch_filter<true, 128, false, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, s)
-                    : launch_filter<false, 128, false, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, s);
-        else
-            r = fp8 ? launch_filter<true, 256, false, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, s)
-                    : launch_filter<false, 256, T, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, s);
-        if (r != IRC_OK) return r;
-        if (narrow)
-            r = fp8 ? launch_filter<true, 128, false, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, s)
-                    : launch_filter<false, 128, false, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, s);
-        else
-            r = fp8 ? launch_filter<true, 256, false, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, s)
-                    : launch_filter<false, 256, T, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, s);
-        if (r != IRC_OK) return r;
-        return fp8 ? launch_filter<true, 128, false, 4>(mq, mc, pl, it4, n4, lo.count + 3, nk, tau_k, lo, s)
-                   : launch_filter<false, 128, false, 4>(mq, mc, pl, it4, n4, lo.count + 3, nk, tau_k, lo, s);
-    };
-    const int rc = tau_k >= 0 ? run(yes{}) : run(no{});
+    if (fp8) return run(std::integral_constant<Fmt, Fmt::fp8>{}, no{});
+    if (fmt == Fmt::f16)
+        return tau_k >= 0 ? run(std::integral_constant<Fmt, Fmt::f16>{}, yes{})
+                          : run(std::integral_constant<Fmt, Fmt::f16>{}, no{});
+    return tau_k >= 0 ? run(std::integral_constant<Fmt, Fmt::bf16>{}, yes{})
+                      : run(std::integral_constant<Fmt, Fmt::bf16>{}, no{});
+}
+
+int launch_knn_tc(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, const float *F,
+                  const float4 *Fp, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn, float *d2Knn,
+                  const ListOut &lo, cudaStream_t s)
+{
+    const int n_out = pl->dev.n_out;
+    cudaEvent_t *ev = profile_slot();
+    if (ev) cudaEventRecord(ev[0], s);
+    const int rc = launch_filters(fmt, mq, mc, pl, nC, lo, pl->scratch, s);
     if (rc != IRC_OK) return rc;
     if (ev) cudaEventRecord(ev[1], s);
     k_rerank<<<(n_out + RR_WARPS - 1) / RR_WARPS, 32 * RR_WARPS, 0, s>>>(
         lo.qinfo, lo.lists, n_out, pl->dev.q_base, F, Fp, nC, pl->row_dims, knn, vrKnn, rho, miKnn, d2Knn,
-        crowd_margin(fp8), pl->scratch);
+        crowd_margin(fmt), pl->scratch);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core) re-rank");
     if (ev) cudaEventRecord(ev[2], s);
     return IRC_OK;

@@ -13,6 +13,12 @@ constexpr int LIST_MAX = 256;    // longest candidate list re-ranked (else: the 
 constexpr int LIST_AVG = 128;    // list area per plan: LIST_AVG entries per query
 using TcItem = irc::TcItem;
 
+// Operand formats of the filter (128-byte rows in all of them).  f16: the
+// BF16 row layout in half precision, the features scaled by a power of two to
+// at most 8 in magnitude; 8 times BF16's resolution at the same MMA cost, so
+// that a query's candidate list can be proven complete (irc_cert.cu).
+enum class Fmt : int { bf16 = 0, fp8 = 1, f16 = 2 };
+
 // The re-rank's FP32 copy of a feature row, zero-padded to a multiple of 8
 // floats (32 bytes) so that it is read with whole-sector 256-bit loads:
 // width in float4.
@@ -26,6 +32,7 @@ struct ListOut {
     uint32_t *lists;
     unsigned *count;             // count[0]: list entries used; count[1..3]: work-queue heads of the
     unsigned cap;                // filter's one-, two- and four-slot launches
+    int2 *cert;                  // per query (threshold bits, chunk), or null when nobody asks
 };
 
 // Entries of the list area of a plan with n_out queries (offsets are int32).
@@ -51,14 +58,33 @@ inline ListOut list_area(void *base, long long n_out)
     lo.count = (unsigned *)b;
     lo.lists = (uint32_t *)(b + 256);
     lo.cap = (unsigned)list_cap(n_out);
+    lo.cert = nullptr;
     return lo;
 }
 
 // The filter (one persistent launch per packing class: items of one or two
 // slots on 256-candidate units, four-slot items on 128-candidate units; mc is
 // the candidate-row map with 128-row boxes) and the re-rank, on stream s.
-int launch_knn_tc(bool fp8, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, const float *F,
+int launch_knn_tc(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, const float *F,
                   const float4 *Fp, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn, float *d2Knn,
                   const ListOut &lo, cudaStream_t s);
+
+// The filter alone; scratch: the counter words of its overflow queue and error
+// word (irc_plan.cuh), the queue after them (unused when lo.cert is set).
+int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, int nC, const ListOut &lo,
+                   int *scratch, cudaStream_t s);
+
+// Operand rows of the plan's rows of F and the tensor maps over them
+// (irc_tc_host.cu); buf: ops_bytes(...) of device memory.
+struct Operands {
+    CUtensorMap mq, mc;
+    const float4 *fp;            // padded FP32 rows of the re-rank
+    const float *ref;            // the centre, [nC]
+    const float *scale;          // f16: the power of two the features were scaled by
+    const float *qnorm;          // f16: upper bound of every query's scaled norm, [n_out]
+};
+size_t ops_bytes(const irc_plan *pl, int nC, Fmt fmt);
+int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, Operands *out,
+                  cudaStream_t s);
 
 }  // namespace irc_tc

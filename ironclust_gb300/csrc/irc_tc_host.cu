@@ -21,6 +21,8 @@
 
 namespace {
 
+using irc_tc::Fmt;
+
 // F (f32 [nF x nC]) -> query / candidate BF16 rows of 64.
 // Centring of the tensor-core operands.  Distances do not change when every
 // feature vector is shifted by the same reference point, but the rounding
@@ -32,6 +34,9 @@ namespace {
 // features.
 constexpr int kMeanBlocks = 256;
 
+// FINITE: values that are not finite are left out of the sums (f16 operands:
+// one such spike must not spoil the centre and with it every proof).
+template <bool FINITE>
 __global__ void k_colsum_part(const float *__restrict__ F, int nC, int stride, int nS, float *__restrict__ part)
 {
     __shared__ float red[4][64];
@@ -40,7 +45,10 @@ __global__ void k_colsum_part(const float *__restrict__ F, int nC, int stride, i
     const int k0 = blockIdx.x * per, k1 = min(nS, k0 + per);
     float acc = 0.0f;
     if (c < nC)
-        for (int k = k0 + lane_r; k < k1; k += 4) acc += __ldg(F + (size_t)k * stride * nC + c);
+        for (int k = k0 + lane_r; k < k1; k += 4) {
+            const float v = __ldg(F + (size_t)k * stride * nC + c);
+            if (!FINITE || isfinite(v)) acc += v;
+        }
     red[lane_r][c] = acc;
     __syncthreads();
     if (threadIdx.x < 64)
@@ -54,6 +62,37 @@ __global__ void k_colsum_final(const float *__restrict__ part, int nb, int nC, i
     double acc = 0.0;
     for (int b = 0; b < nb; ++b) acc += (double)part[(size_t)b * 64 + c];
     ref[c] = nS > 0 ? (float)(acc / (double)nS) : 0.0f;
+}
+
+// The power of two that brings every finite |F - ref| to at most 8, from the
+// finite |F| maximum and the largest |ref| (their sum bounds the differences;
+// what the bound loses, a factor of two at most, only costs half-precision
+// subnormals).  0 when features reach 2^62, whose squared distances leave
+// FP32's range: nothing is proven with it.
+__global__ void k_scale(const unsigned *__restrict__ amax, const float *__restrict__ ref, int nC,
+                        float *__restrict__ scale)
+{
+    float m = 0.0f;
+    for (int c = threadIdx.x; c < nC; c += 32) m = fmaxf(m, fabsf(ref[c]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) {
+        const float b = __uint_as_float(*amax) + m;
+        *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
+    }
+}
+
+// |F| maximum over the finite values (bits of a non-negative float, so
+// integer max == float max).
+__global__ void k_absmax_finite(const float *__restrict__ F, size_t n, unsigned *__restrict__ out)
+{
+    unsigned m = 0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const unsigned b = __float_as_uint(fabsf(__ldg(F + i)));
+        if (b < 0x7f800000u) m = max(m, b);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
 // |F| maximum (bits of a non-negative float, so integer max == float max).
@@ -105,11 +144,27 @@ size_t prep_smem(int nC)
     return (size_t)kPrepWarps * (2 * 32 * 128 + 32 * (size_t)(nC | 1) * 4) + 64 * 4;
 }
 
-template <bool FP8>
+// The 16-bit operand value of x: its bits, and the value they stand for.
+template <Fmt FMT>
+__device__ __forceinline__ unsigned short op16(float x)
+{
+    return FMT == Fmt::f16 ? __half_as_ushort(__float2half_rn(x)) : __bfloat16_as_ushort(__float2bfloat16_rn(x));
+}
+
+template <Fmt FMT>
+__device__ __forceinline__ float val16(unsigned short v)
+{
+    return FMT == Fmt::f16 ? __half2float(__ushort_as_half(v)) : __bfloat162float(__ushort_as_bfloat16(v));
+}
+
+// qnorm (f16): an upper bound of every query's scaled norm |s (a - ref)|: the
+// rounded row's norm, plus the rounding (2^-11 relative, 2^-25 absolute per
+// feature), with room.
+template <Fmt FMT>
 __global__ void __launch_bounds__(32 * kPrepWarps)
 k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restrict__ ref,
        const unsigned *__restrict__ amax, uint4 *__restrict__ Fq, uint4 *__restrict__ Fc, float *__restrict__ Fp,
-       int Dp4, int q_lo, int q_hi)
+       int Dp4, int q_lo, int q_hi, const float *__restrict__ scale, float *__restrict__ qnorm)
 {
     extern __shared__ __align__(16) unsigned char prep_sm[];
     const int nCs = nC | 1;
@@ -139,28 +194,28 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
         const float *a = w + lane * nCs;
         uint4 *oq = sq + lane * 8, *oc = sc + lane * 8;
         const int sw = lane & 7;
-        if (!FP8) {
+        if (FMT != Fmt::fp8) {
+            const float s16 = FMT == Fmt::f16 ? *scale : 1.0f;         // a power of two: exact
             float na = 0.0f;
             for (int k = 0; k < nC; ++k) {
-                const float f = __bfloat162float(__float2bfloat16_rn(a[k] - sref[k]));
+                const float f = val16<FMT>(op16<FMT>((a[k] - sref[k]) * s16));
                 na = __fmaf_rn(f, f, na);
             }
-            const __nv_bfloat16 h = __float2bfloat16_rn(na);
-            const float rem1 = na - __bfloat162float(h);
-            const __nv_bfloat16 m = __float2bfloat16_rn(rem1);
-            const __nv_bfloat16 l = __float2bfloat16_rn(rem1 - __bfloat162float(m));
-            const __nv_bfloat16 one = __float2bfloat16_rn(1.0f), zero = __float2bfloat16_rn(0.0f);
+            const unsigned short h = op16<FMT>(na);
+            const float rem1 = na - val16<FMT>(h);
+            const unsigned short m = op16<FMT>(rem1);
+            const unsigned short l = op16<FMT>(rem1 - val16<FMT>(m));
+            const unsigned short one = op16<FMT>(1.0f), zero = 0;
 #pragma unroll 1
             for (int j = 0; j < irc_tc::KP / 8; ++j) {
-                __align__(16) __nv_bfloat16 wq[8], wc[8];
+                __align__(16) unsigned short wq[8], wc[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const int k = j * 8 + e;
-                    __nv_bfloat16 vq = zero, vc = zero;
+                    unsigned short vq = zero, vc = zero;
                     if (k < nC) {
-                        const __nv_bfloat16 bf = __float2bfloat16_rn(a[k] - sref[k]);
-                        vc = bf;
-                        vq = __float2bfloat16_rn(-2.0f * __bfloat162float(bf));
+                        vc = op16<FMT>((a[k] - sref[k]) * s16);
+                        vq = op16<FMT>(-2.0f * val16<FMT>(vc));
                     } else if (k < nC + 3) {
                         vq = (k == nC) ? h : (k == nC + 1) ? m : l;
                         vc = one;
@@ -176,6 +231,9 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
                 oq[j ^ sw] = *reinterpret_cast<uint4 *>(wq);
                 oc[j ^ sw] = *reinterpret_cast<uint4 *>(wc);
             }
+            const long long row = r0 + lane;
+            if (FMT == Fmt::f16 && row >= q_lo && row < q_hi)
+                qnorm[row - q_lo] = __fsqrt_ru(na) * (1.0f + 0x1p-9f) + 1e-6f;
         } else {
             const float am = __uint_as_float(*amax);
             const float scl = am > 0.0f ? 32.0f / am : 1.0f;
@@ -247,10 +305,11 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-// Tensor map over [rows x 128 bytes] operand rows (64 BF16 or 128 e4m3 values),
+// Tensor map over [rows x 128 bytes] operand rows (64 BF16 or F16, or 128 e4m3 values),
 // box_rows-row boxes, 128-byte swizzle.
-int make_map(CUtensorMap *m, void *base, int rows, int box_rows, bool fp8)
+int make_map(CUtensorMap *m, void *base, int rows, int box_rows, Fmt fmt)
 {
+    const bool fp8 = fmt == Fmt::fp8;
     EncodeTiledFn enc = encode_fn();
     if (!enc) { irc_host::set_error("cuTensorMapEncodeTiled unavailable"); return IRC_E_CUDA; }
     const int inner = fp8 ? 128 : irc_tc::KP;
@@ -258,8 +317,9 @@ int make_map(CUtensorMap *m, void *base, int rows, int box_rows, bool fp8)
     cuuint64_t strides[1] = {(cuuint64_t)128};
     cuuint32_t box[2] = {(cuuint32_t)inner, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(m, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims,
-                     strides, box, estr,
+    CUresult r = enc(m, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                            : fmt == Fmt::f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                     2, base, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { irc_host::set_error("cuTensorMapEncodeTiled failed (%d)", (int)r); return IRC_E_CUDA; }
@@ -268,67 +328,103 @@ int make_map(CUtensorMap *m, void *base, int rows, int box_rows, bool fp8)
 
 }  // namespace
 
-// Plan-owned tensor-core operand buffers (irc_site.cu) and the exact
+// The plan's tensor-core working memory (irc_site.cu) and the exact
 // fallback for queries whose candidate list overflowed (irc_exact.cu).
-int irc_plan_tc_buffers(irc_plan *pl, void **fq, void **fc, void **fp, void **extra, size_t row_bytes,
-                        size_t fp_row_bytes, size_t extra_bytes);
+int irc_plan_tc_buffer(irc_plan *pl, size_t need, void **buf);
 int irc_exact_overflow_drain(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho,
                              int32_t *miKnn, float *d2Knn, cudaStream_t s);
 
-int irc_site_knn_tc(irc_plan *pl, const float *F, int nC, int knn, int mode, float *vrKnn, float *rho,
-                    int32_t *miKnn, float *d2Knn, cudaStream_t s)
+namespace irc_tc {
+
+constexpr size_t kPartBytes = sizeof(float) * kMeanBlocks * 64;
+
+static size_t fp_bytes(const irc_plan *pl, int nC)
 {
-    const bool fp8 = mode == IRC_MODE_FP8;
-    if (nC + (fp8 ? 2 * kFp8Pieces : 6) > (fp8 ? 128 : irc_tc::KP)) {
-        irc_host::set_error("irc_site_knn(tensor core): nC=%d too large", nC);
-        return IRC_E_NC;
-    }
-    if (knn > irc_tc::KNN_MAX) { irc_host::set_error("irc_site_knn(BF16): knn %d > %d", knn, irc_tc::KNN_MAX); return IRC_E_INVAL; }
-    const int nF = pl->dev.nF;
-    void *fq, *fc, *fp, *ex;
-    const int Dp4 = irc_tc::fp_row4(nC);                               // padded FP32 row, float4
-    const size_t part_bytes = sizeof(float) * kMeanBlocks * 64;
-    int rc = irc_plan_tc_buffers(pl, &fq, &fc, &fp, &ex, irc_tc::KP * 2, (size_t)Dp4 * 16,
-                                 part_bytes + 256 + irc_tc::list_area_bytes(pl->dev.n_out));
-    float *part = (float *)ex;
-    float *ref = (float *)((char *)ex + part_bytes);
-    const irc_tc::ListOut lo = irc_tc::list_area((char *)ex + part_bytes + 256, pl->dev.n_out);
-    if (rc != IRC_OK) return rc;
-    cudaError_t e = cudaMemsetAsync(pl->scratch, 0, sizeof(int), s);       // overflow-queue count
-    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(BF16): memset");
+    return ((size_t)pl->dev.nF * (size_t)fp_row4(nC) * 16 + 255) & ~(size_t)255;
+}
+
+// query rows | candidate rows | padded FP32 rows | column sums | centre (256
+// bytes) | f16: scale (256 bytes), query norms
+size_t ops_bytes(const irc_plan *pl, int nC, Fmt fmt)
+{
+    const size_t q = fmt == Fmt::f16 ? 256 + (((size_t)pl->dev.n_out * 4 + 255) & ~(size_t)255) : 0;
+    return 2 * (size_t)pl->dev.nF * 128 + fp_bytes(pl, nC) + kPartBytes + 256 + q;
+}
+
+int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, Operands *out,
+                  cudaStream_t s)
+{
+    const bool fp8 = fmt == Fmt::fp8, f16 = fmt == Fmt::f16;
+    const int nF = pl->dev.nF, Dp4 = fp_row4(nC);
+    const size_t one = (size_t)nF * 128;
+    char *b = (char *)buf;
+    void *fq = b, *fc = b + one, *fp = b + 2 * one;
+    float *part = (float *)(b + 2 * one + fp_bytes(pl, nC));
+    float *ref = (float *)((char *)part + kPartBytes);
+    float *scale = ref + 64, *qnorm = ref + 128;
     const int nQ = pl->dev.n_out;                                     // the query rows q_base ..
     const int stride = nQ > 65536 ? (nQ + 65535) / 65536 : 1;
     const int nS = (nQ + stride - 1) / stride;                        // sampled: q_base + k * stride
-    k_colsum_part<<<kMeanBlocks, 256, 0, s>>>(F + (size_t)pl->dev.q_base * nC, nC, stride, nS, part);
+    (f16 ? k_colsum_part<true> : k_colsum_part<false>)<<<kMeanBlocks, 256, 0, s>>>(F + (size_t)pl->dev.q_base * nC, nC,
+                                                                                   stride, nS, part);
     k_colsum_final<<<1, 64, 0, s>>>(part, kMeanBlocks, nC, nS, ref);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core) centre");
     // operand rows for the rows the plan reads (its row intervals)
-    unsigned *amax = reinterpret_cast<unsigned *>(pl->scratch + 1);       // free word of the plan scratch
-    if (fp8) {
-        e = cudaMemsetAsync(amax, 0, sizeof(unsigned), s);
-        if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(FP8): memset");
+    if (fp8 || f16) {
+        cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned), s);
+        if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): memset");
         for (int v = 0; v < pl->n_row_iv; ++v) {
             const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
-            k_absmax<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
+            if (fp8) k_absmax<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
+            else k_absmax_finite<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, amax);
         }
-        IRC_CHECK_LAUNCH("irc_site_knn(FP8) absmax");
+        if (f16) k_scale<<<1, 32, 0, s>>>(amax, ref, nC, scale);
+        IRC_CHECK_LAUNCH("irc_site_knn(tensor core) absmax");
     }
     const size_t psm = prep_smem(nC);
-    auto prep = fp8 ? k_prep<true> : k_prep<false>;
-    e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
+    auto prep = fp8 ? k_prep<Fmt::fp8> : f16 ? k_prep<Fmt::f16> : k_prep<Fmt::bf16>;
+    cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): prep smem attribute");
     for (int v = 0; v < pl->n_row_iv; ++v) {
         const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
         const int rows_per_block = 32 * kPrepWarps;
         prep<<<(n + rows_per_block - 1) / rows_per_block, 32 * kPrepWarps, psm, s>>>(
             F, lo, n, nC, ref, amax, (uint4 *)fq, (uint4 *)fc, (float *)fp, Dp4, pl->dev.q_base,
-            pl->dev.q_base + pl->dev.n_out);
+            pl->dev.q_base + pl->dev.n_out, scale, qnorm);
     }
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core) prep");
-    CUtensorMap mq, mc;
-    if ((rc = make_map(&mq, fq, nF, 32, fp8)) != IRC_OK) return rc;       // 32 query rows per lane quarter
-    if ((rc = make_map(&mc, fc, nF, 128, fp8)) != IRC_OK) return rc;     // 128-row candidate tiles
-    rc = irc_tc::launch_knn_tc(fp8, mq, mc, pl, F, (const float4 *)fp, nC, knn, vrKnn, rho, miKnn, d2Knn, lo, s);
+    int rc = make_map(&out->mq, fq, nF, 32, fmt);                     // 32 query rows per lane quarter
+    if (rc == IRC_OK) rc = make_map(&out->mc, fc, nF, 128, fmt);      // 128-row candidate tiles
+    out->fp = (const float4 *)fp;
+    out->ref = ref;
+    out->scale = scale;
+    out->qnorm = qnorm;
+    return rc;
+}
+
+}  // namespace irc_tc
+
+int irc_site_knn_tc(irc_plan *pl, const float *F, int nC, int knn, int mode, float *vrKnn, float *rho,
+                    int32_t *miKnn, float *d2Knn, cudaStream_t s)
+{
+    const bool fp8 = mode == IRC_MODE_FP8;
+    const Fmt fmt = fp8 ? Fmt::fp8 : Fmt::bf16;
+    if (nC + (fp8 ? 2 * kFp8Pieces : 6) > (fp8 ? 128 : irc_tc::KP)) {
+        irc_host::set_error("irc_site_knn(tensor core): nC=%d too large", nC);
+        return IRC_E_NC;
+    }
+    if (knn > irc_tc::KNN_MAX) { irc_host::set_error("irc_site_knn(BF16): knn %d > %d", knn, irc_tc::KNN_MAX); return IRC_E_INVAL; }
+    void *buf;
+    const size_t ops = irc_tc::ops_bytes(pl, nC, fmt);
+    int rc = irc_plan_tc_buffer(pl, ops + irc_tc::list_area_bytes(pl->dev.n_out), &buf);
+    if (rc != IRC_OK) return rc;
+    const irc_tc::ListOut lo = irc_tc::list_area((char *)buf + ops, pl->dev.n_out);
+    cudaError_t e = cudaMemsetAsync(pl->scratch, 0, sizeof(int), s);       // overflow-queue count
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(BF16): memset");
+    irc_tc::Operands op;
+    unsigned *amax = reinterpret_cast<unsigned *>(pl->scratch + 1);       // free word of the plan scratch
+    if ((rc = irc_tc::make_operands(fmt, pl, F, nC, buf, amax, &op, s)) != IRC_OK) return rc;
+    rc = irc_tc::launch_knn_tc(fmt, op.mq, op.mc, pl, F, op.fp, nC, knn, vrKnn, rho, miKnn, d2Knn, lo, s);
     if (rc != IRC_OK) return rc;
     return irc_exact_overflow_drain(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, s);
 }
