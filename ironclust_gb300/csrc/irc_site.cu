@@ -445,6 +445,7 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
                 tiles.push_back(ms[r] + t);
                 tiles.push_back(std::min(128, mn[r] - t));
             }
+        pl->tc_max_tiles = std::max(pl->tc_max_tiles, (int)(tiles.size() / 2) - img.back());
         if ((tiles.size() / 2) & 1) { tiles.push_back(0); tiles.push_back(0); }
     }
     img.push_back((int32_t)(tiles.size() / 2));

@@ -187,6 +187,17 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[16], uint32_t (&b)[16
                  : "memory");
 }
 
+// The same for one 16-register load.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]),
+                   "+r"(a[15])
+                 :
+                 : "memory");
+}
+
 // min(a, b, c) in one instruction (three-input min.f32, sm_100 family); NaN
 // operands are ignored as by fminf.
 __device__ __forceinline__ float fmin3(float a, float b, float c)

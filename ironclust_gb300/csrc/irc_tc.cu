@@ -25,10 +25,12 @@
 // N = 256 as at 128, so this halves it per pair -- unless the plan asks for
 // 128-wide units (irc_plan_tc_units), and four-slot items 128-wide units
 // (four accumulators, one per slot).  Warp roles: warp 0 claims items and
-// issues TMA loads (a 3- or 4-stage ring, four 32-row query boxes per item),
-// warp 1 owns TMEM and issues tcgen05.mma from one thread, warps 2-17 are the
-// epilogue: four per TMEM lane quarter, warp w of a quarter reading columns
-// 32w .. 32w + 31 of every 128-tile.  Each slot's units are streamed twice:
+// issues TMA loads (a ring of 4 wide or 6 narrow stages, four 32-row query
+// boxes per item), warps 1 and 18 issue tcgen05.mma from one thread each, unit
+// by unit in turn (warp 1 also owns TMEM), warps 2-17 are the epilogue: four
+// per TMEM lane quarter, warp w of a quarter reading columns 32w .. 32w + 31
+// of every 128-tile.  A warp releases an accumulator as soon as its values are
+// in registers.  Each slot's units are streamed twice:
 //   pass 1  every thread folds its columns into 32 per-column minima (the two
 //           tiles of a wide unit with one three-input min); per query, the
 //           r-th smallest of the 128 minima (r = 48 for BF16, 64 for FP8; a
@@ -45,7 +47,11 @@
 //           d2 - tau and a hit is a sign bit (one funnel shift per pair);
 //           elsewhere every pair is compared with tau in the epilogue.
 // The minima partition is the same at both widths, so results never depend
-// on the width or the work layout.  Every listed candidate is then re-ranked
+// on the width or the work layout.  Measured on 400,000 spikes, D = 33 (1.2e10
+// pairs, one launch): 3.65 ms with one MMA issuer, three stages and late
+// releases, 3.10 ms as above; without any epilogue work the pipeline takes
+// 1.81, and folding, marking and appending add 0.35, 0.48 and 0.46.
+// Every listed candidate is then re-ranked
 // with the reference FP32 arithmetic (exact), zero distances dropped, sorted
 // by (distance, index) with a warp bitonic network; candidates within 16 ulps
 // of the k-th distance are re-ordered by their FP64 distance.  The kernel is
@@ -82,13 +88,13 @@ constexpr int PARTS = 4;                          // epilogue warps per TMEM lan
 constexpr int PART = 32;                          // columns of a 128-tile per epilogue warp (one minimum each)
 constexpr int BROW = 128 + 1;                     // minima row of a query (f32, 4 parts x 32) in the threshold step
 constexpr int EPI_WARPS = 4 * PARTS;
-constexpr int THREADS = 32 * (2 + EPI_WARPS);
+constexpr int MMA_WARPS = 2;                      // MMA issuers: warp 1 and the last warp, alternate units
+constexpr int THREADS = 32 * (1 + MMA_WARPS + EPI_WARPS);
 constexpr uint32_t A_BYTES = BM * KP * 2;         // the query tile: 128 rows x 128 bytes
 constexpr uint32_t HALF_BYTES = 128 * KP * 2;     // one 128-candidate tile
 constexpr uint32_t TMEM_COLS = 512;               // all TMEM columns (one CTA per SM)
 constexpr int LISTCAP = 192;                      // candidate-list capacity per query (the four warps' hits pooled)
-constexpr int LROW = LISTCAP + 1;                 // list row (u32), padded
-constexpr size_t LIST_BYTES = (size_t)LROW * BM * 4;
+constexpr int MAX_SHORT_TILES = 512;              // tiles per chunk that a 16-bit list entry can name
 // The threshold is the tau_rank-th smallest per-column minimum: tau_rank
 // distinct candidates lie at or below it, a margin over knn (<= 32) for the
 // rounding of the filter.  A list it cut must hold at least knn +
@@ -106,23 +112,37 @@ __host__ __device__ constexpr int tau_rank(Fmt f) { return f == Fmt::fp8 ? 64 : 
 __host__ __device__ constexpr int crowd_margin(Fmt f) { return f == Fmt::fp8 ? 16 : 8; }
 static_assert(tau_rank(Fmt::bf16) >= irc_tc::KNN_MAX + crowd_margin(Fmt::bf16), "rank covers knn plus the margin");
 static_assert(tau_rank(Fmt::fp8) >= irc_tc::KNN_MAX + crowd_margin(Fmt::fp8), "rank covers knn plus the margin");
-static_assert((size_t)BROW * BM * 4 <= LIST_BYTES, "minima rows alias the list area");
 static_assert(LISTCAP <= irc_tc::LIST_MAX, "the re-rank takes every list the filter hands over");
 
 // Shapes of the filter for a unit width BN (MMA N): 256 for items of one or
 // two slots (two 256-column accumulators; the MMA issue cost per instruction
 // is the same at N = 256 as at 128, so the wider unit halves it per pair), 128
 // for four-slot items (one accumulator per slot).
-template <int BN>
+// A list entry is 16 bits -- place of the tile in the chunk's list (9 bits) and
+// column (7) -- unless a chunk has more tiles than that (BIG: 32 bits, the
+// candidate's row); the half-size lists make room for a fourth stage of a wide
+// unit.  Stages matter because a load takes ~900 cycles from issue to arrival,
+// and freeing a stage, waking the producer and issuing its loads ~700 more:
+// three 32 KB stages held the pipeline at ~1,200 cycles a unit.
+template <int BN, bool BIG>
 struct Tile {
     static_assert(BN == 128 || BN == 256, "unit width");
     static constexpr int NBUF = TMEM_COLS / BN;   // accumulator buffers, split among the slots
-    static constexpr int STAGES = BN == 256 ? 3 : 4;
+    static constexpr int STAGES = BN == 256 ? (BIG ? 3 : 4) : (BIG ? 4 : 6);
     static constexpr uint32_t STAGE_BYTES = BN * KP * 2;
+    using Entry = typename std::conditional<BIG, uint32_t, uint16_t>::type;
+    static constexpr int LROW = LISTCAP + 4 / (int)sizeof(Entry);     // entries of a list row, an odd number of words
+    // list rows of a lane quarter; its minima rows (threshold step) share the space
+    static constexpr size_t MIN_BYTES = (size_t)BROW * 32 * 4, ROWS_BYTES = (size_t)LROW * 32 * sizeof(Entry);
+    static constexpr size_t QUARTER_BYTES = ROWS_BYTES > MIN_BYTES ? ROWS_BYTES : MIN_BYTES;
     // two query tiles (the next item's loads while this one's MMAs run)
     static constexpr size_t SMEM_BYTES = 1024 /*align slack*/ + 2 * A_BYTES + (size_t)STAGE_BYTES * STAGES +
-                                         LIST_BYTES + BM * 4 /*tau*/ + BM * 4 /*counts*/ + 256 /*barriers*/;
+                                         4 * QUARTER_BYTES + BM * 4 /*tau*/ + BM * 4 /*counts*/ + 384 /*barriers*/;
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+    static __device__ __forceinline__ const Entry *row(const unsigned char *lists, int quarter, int l)
+    {
+        return reinterpret_cast<const Entry *>(lists + quarter * QUARTER_BYTES) + l * LROW;
+    }
 };
 
 // Work units of a slot per pass over its chunk's sequence of 128-candidate
@@ -139,16 +159,37 @@ __device__ __forceinline__ int units_per_pass(int nts)
     return BN == 256 ? (nts + 1) >> 1 : nts;
 }
 
+// The MMA issuer of unit k (both passes counted) of slot s: alternate units of
+// a one-slot item, whose accumulators alternate too, alternate slots else.  A
+// slot's unit count over both passes is even, so an accumulator stays with
+// its issuer from item to item.
+template <int NS>
+__device__ __forceinline__ int issuer_of(int k, int s)
+{
+    static_assert(MMA_WARPS == 2, "two issuers");
+    return (NS == 1 ? k : s) & 1;
+}
+
 // A wait of the filter's pipeline (see sm100::mbar_wait), bounded by the
-// poll limit set with irc_set_wait_limit.  It starts with try_wait (no
-// non-blocking probes): a probing warp would take issue slots from the
-// epilogue warps sharing its scheduler.  A limit below 64 polls makes every
-// poll a non-blocking test instead, so such a limit gives up at the first
-// phase that is not already complete (how the tests force the timeout path).
+// poll limit set with irc_set_wait_limit.  One non-blocking test first: the
+// producer's and the MMA threads' waits mostly find their phase complete, and
+// a bare test costs a fraction of the bounded loop (147 cycles for a complete
+// phase).  The loop then starts with try_wait (no more probes): a probing warp
+// would take issue slots from the epilogue warps sharing its scheduler.  A
+// limit below 64 polls makes every poll a non-blocking test, so such a limit
+// gives up at the first phase that is not already complete (how the tests
+// force the timeout path).
 __device__ __forceinline__ bool pipe_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
 {
+    if (sm100::mbar_test_wait(bar, parity)) return true;
     const uint32_t lim = c_wait_polls;
     return sm100::mbar_wait(bar, parity, abort_flag, lim, lim < 64u ? lim : 0u);
+}
+
+// The same by a whole warp: one answer for all lanes.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
+{
+    return __all_sync(0xffffffffu, pipe_wait(bar, parity, abort_flag));
 }
 
 __device__ __forceinline__ double dist2_f64(const float *__restrict__ b, const float *__restrict__ a, int nd)
@@ -257,14 +298,24 @@ __device__ __forceinline__ int chunk_tiles(const irc::PlanDev &p, int chunk)
     return n;
 }
 
+// The accumulator goes back to the MMA issuer as soon as this warp's values
+// are in registers: the rest of the unit's work then overlaps the next MMAs.
+__device__ __forceinline__ void release_acc(uint64_t *empty, int lane)
+{
+    sm100::tc_fence_before();
+    __syncwarp();
+    if (lane == 0) sm100::mbar_arrive(empty);
+}
+
 // Pass 1 of one warp and 128-tile (BN = 128): fold its 32 columns (taddr:
 // the first) into the per-column minima; lim = valid columns of the 32.
-__device__ __forceinline__ void fold32(uint32_t taddr, int lim, float (&bm)[PART])
+__device__ __forceinline__ void fold32(uint32_t taddr, int lim, uint64_t *empty, int lane, float (&bm)[PART])
 {
     uint32_t x[16], y[16];
     sm100::tmem_ld16_nowait(taddr, x);
     sm100::tmem_ld16_nowait(taddr + 16, y);
     sm100::tmem_wait_ld(x, y);
+    release_acc(empty, lane);
     if (lim >= 32) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -283,7 +334,8 @@ __device__ __forceinline__ void fold32(uint32_t taddr, int lim, float (&bm)[PART
 // Pass 1 of one warp and 256-wide unit: its 32 columns of both 128-tiles
 // (ta, tb: the first column of each; la, lb: valid columns) folded into the
 // same minima with three-input mins.
-__device__ __forceinline__ void fold2x32(uint32_t ta, int la, uint32_t tb, int lb, float (&bm)[PART])
+__device__ __forceinline__ void fold2x32(uint32_t ta, int la, uint32_t tb, int lb, uint64_t *empty, int lane,
+                                         float (&bm)[PART])
 {
     const float inf = __int_as_float(0x7f800000);
 #pragma unroll
@@ -292,6 +344,7 @@ __device__ __forceinline__ void fold2x32(uint32_t ta, int la, uint32_t tb, int l
         sm100::tmem_ld16_nowait(ta + 16 * r, x);
         sm100::tmem_ld16_nowait(tb + 16 * r, y);
         sm100::tmem_wait_ld(x, y);
+        if (r == 1) release_acc(empty, lane);
         if (la >= 32 && lb >= 32) {
 #pragma unroll
             for (int i = 0; i < 16; ++i)
@@ -312,12 +365,8 @@ __device__ __forceinline__ unsigned lim_mask(int lim)
 
 // Pass 2 of one warp and 128-tile: the mask of its 32 columns at or below
 // tau, limited to the lim valid columns.
-__device__ __forceinline__ unsigned mark32(uint32_t taddr, int lim, float tau)
+__device__ __forceinline__ unsigned mark_regs(const uint32_t (&x)[16], const uint32_t (&y)[16], int lim, float tau)
 {
-    uint32_t x[16], y[16];
-    sm100::tmem_ld16_nowait(taddr, x);
-    sm100::tmem_ld16_nowait(taddr + 16, y);
-    sm100::tmem_wait_ld(x, y);
     // four independent partial masks: short dependency chains
     unsigned a0 = 0u, a1 = 0u, a2 = 0u, a3 = 0u;
 #pragma unroll
@@ -331,7 +380,8 @@ __device__ __forceinline__ unsigned mark32(uint32_t taddr, int lim, float tau)
 }
 
 // Bit c of the result = sign bit of v[c], one funnel shift per value in two
-// independent chains.
+// independent chains.  (Half of the values through the carry of an add, on the
+// other pipe, measured 1.6 times the rate alone and 1% slower here.)
 __device__ __forceinline__ unsigned signs16(const uint32_t (&v)[16])
 {
     unsigned c0 = 0u, c1 = 0u;                    // values 0-7, 8-15
@@ -343,23 +393,30 @@ __device__ __forceinline__ unsigned signs16(const uint32_t (&v)[16])
     return c0 | (c1 << 8);
 }
 
-// Pass 2 with the threshold folded into the MMA (accumulators d2 - tau) of
-// one warp and 256-wide unit: the masks of its 32 columns of each tile with a
-// negative accumulator, limited to the valid columns.
-__device__ __forceinline__ void mark2x32_signs(uint32_t ta, int la, uint32_t tb, int lb, unsigned &ma, unsigned &mb)
+// Pass 2 of one warp and unit: the masks of its 32 columns of each tile (the
+// second of a 256-wide unit) that are hits, limited to the valid columns.
+// Every value is loaded before the accumulator is released; SIGNS: the
+// threshold is folded into the MMA (accumulators d2 - tau), a hit is a sign bit.
+template <int BN, bool SIGNS>
+__device__ __forceinline__ void mark(uint32_t ta, int la, uint32_t tb, int lb, float tau, uint64_t *empty, int lane,
+                                     unsigned &ma, unsigned &mb)
 {
-    unsigned a[2], b[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {                 // columns 16r .. 16r + 15 of both tiles
-        uint32_t x[16], y[16];
-        sm100::tmem_ld16_nowait(ta + 16 * r, x);
-        sm100::tmem_ld16_nowait(tb + 16 * r, y);
-        sm100::tmem_wait_ld(x, y);
-        a[r] = signs16(x);
-        b[r] = signs16(y);
+    uint32_t x[2][16], y[2][16];                  // columns 16r .. 16r + 15 of the two tiles
+    sm100::tmem_ld16_nowait(ta, x[0]);
+    sm100::tmem_ld16_nowait(ta + 16, x[1]);
+    if constexpr (BN == 256) {
+        sm100::tmem_ld16_nowait(tb, y[0]);
+        sm100::tmem_ld16_nowait(tb + 16, y[1]);
     }
-    ma = (a[0] | (a[1] << 16)) & lim_mask(la);
-    mb = (b[0] | (b[1] << 16)) & lim_mask(lb);
+    sm100::tmem_wait_ld(x[0], x[1]);
+    if constexpr (BN == 256) sm100::tmem_wait_ld(y[0], y[1]);
+    release_acc(empty, lane);
+    if constexpr (SIGNS) ma = (signs16(x[0]) | (signs16(x[1]) << 16)) & lim_mask(la);
+    else ma = mark_regs(x[0], x[1], la, tau);
+    if constexpr (BN == 256) {
+        if constexpr (SIGNS) mb = (signs16(y[0]) | (signs16(y[1]) << 16)) & lim_mask(lb);
+        else mb = mark_regs(y[0], y[1], lb, tau);
+    }
 }
 
 // The pass-2 threshold of query row `row` into the query tile in shared
@@ -396,18 +453,24 @@ __device__ __forceinline__ void put_tau(uint8_t *sA, int row, int tau_k, float t
     }
 }
 
-// Append the hits of a 32-column mask (columns c0 + bit) to the query's
-// pooled list (its four epilogue warps share it): one shared-memory atomic
-// reserves the room; entries past LISTCAP are dropped, and a count past it
-// sends the query to the exact fallback.
-__device__ __forceinline__ void append_hits(uint32_t *lrow, int *cnt, unsigned m, uint32_t c0)
+// Append the hits of a unit's two 32-column masks (entries ca + bit, cb + bit)
+// to the query's pooled list (its four epilogue warps share it): one
+// shared-memory atomic reserves the room; entries past LISTCAP are dropped,
+// and a count past it sends the query to the exact fallback.  (A share per
+// warp with the count in a register measured the same.)
+template <class E>
+__device__ __forceinline__ void append_hits(E *lrow, int *cnt, unsigned ma, uint32_t ca, unsigned mb, uint32_t cb)
 {
-    int e = atomicAdd(cnt, __popc(m));
-    while (m) {
-        const int jj = __ffs(m) - 1;
-        m &= m - 1u;
-        if (e < LISTCAP) lrow[e] = c0 + (uint32_t)jj;
+    if (!(ma | mb)) return;
+    int e = atomicAdd(cnt, __popc(ma) + __popc(mb));
+#pragma unroll 1
+    while (ma | mb) {
+        const bool first = ma != 0u;
+        const unsigned m = first ? ma : mb;
+        if (e < LISTCAP) lrow[e] = (E)((first ? ca : cb) + (uint32_t)(__ffs(m) - 1));
         ++e;
+        if (first) ma &= ma - 1u;
+        else mb &= mb - 1u;
     }
 }
 
@@ -433,8 +496,9 @@ __device__ __forceinline__ bool slot_barrier_and(int slot, int nthreads, bool v)
 // its quarter's queries (query L in lane L) into one bump allocation and
 // records (offset, length) per query; a list past LISTCAP or a full list area
 // sends the query to the exact fallback instead.
+template <class T>
 __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::TcItem &it, int s, int quarter, int part,
-                                         int qrow, int nq_s, const uint32_t *lists, const int *sCnt,
+                                         int qrow, int nq_s, const int2 *__restrict__ tl, const unsigned char *lists, const int *sCnt,
                                          const float *sTau, const irc_tc::ListOut &lo, int *scratch, int lane)
 {
     constexpr int RL = 32 / PARTS;
@@ -476,8 +540,11 @@ __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::Tc
         const int n = __shfl_sync(0xffffffffu, cL, L);
         const unsigned off = base + __shfl_sync(0xffffffffu, incl - len, L);
         if (n <= 0) continue;                     // warp-uniform
-        const uint32_t *lr = lists + (size_t)(quarter * 32 + part * RL + L) * LROW;
-        for (int e = lane; e < n; e += 32) lo.lists[off + e] = lr[e];
+        const typename T::Entry *lr = T::row(lists, quarter, part * RL + L);
+        for (int e = lane; e < n; e += 32) {
+            const uint32_t v = lr[e];
+            lo.lists[off + e] = sizeof(typename T::Entry) == 4 ? v : (uint32_t)__ldg(tl + (v >> 7)).x + (v & 127u);
+        }
     }
 }
 
@@ -487,15 +554,15 @@ __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::Tc
 struct Shared {
     uint8_t *sA;                                  // two query tiles, A_BYTES each
     uint8_t *sB;                                  // candidate stages
-    uint32_t *lists;                              // [BM][LROW]
+    unsigned char *lists;                         // list rows, QUARTER_BYTES a lane quarter
     float *sTau;                                  // [BM]
     int *sCnt;                                    // [BM] list counts
-    uint64_t *full, *empty;                       // [STAGES] candidate stages loaded / consumed
+    uint64_t *full, *empty;                       // [MMA_WARPS][STAGES] a unit loaded (per issuer), [STAGES] stage consumed
     uint64_t *a_full, *a_empty;                   // [2] query tile loaded / its item's MMAs done
     uint64_t *acc_full, *acc_empty;               // [NBUF] accumulator written / read
     uint64_t *tau_ready;                          // [4] a slot's thresholds are in its query tile
     uint64_t *item_full, *item_empty;             // [2] item index published / read by every consumer
-    uint64_t *mma_done;
+    uint64_t *mma_done;                           // [MMA_WARPS]
     int *item_idx;                                // [2]
     uint32_t *tmem_slot;
     volatile int *abort_flag;
@@ -507,12 +574,12 @@ struct Shared {
 // synchronise only among themselves (named barrier 1 + slot).  Unit g of a
 // slot (counted over all its items, both passes) goes to accumulator
 // s * BPS + g % BPS, whose barriers are in phase g / BPS.
-template <int BN, int NS, Fmt FMT, bool TAU>
+template <int BN, int NS, Fmt FMT, bool TAU, bool BIG>
 __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::TcItem *__restrict__ items, int rank,
                                          uint32_t tmem, int tau_k, const Shared &sh, const irc_tc::ListOut &lo,
                                          int *scratch, int warp, int lane)
 {
-    using T = Tile<BN>;
+    using T = Tile<BN, BIG>;
     constexpr int QPS = 4 / NS;                   // lane quarters per slot
     constexpr int BPS = T::NBUF / NS;             // accumulator buffers per slot
     const int ew = warp - 2;                      // 0..15
@@ -524,8 +591,8 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
     const int row = quarter * 32 + lane;
     const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + part * PART;
     // the minima rows of a quarter alias that quarter's own list rows
-    float *qarea = reinterpret_cast<float *>(sh.lists + (size_t)quarter * 32 * LROW);
-    uint32_t *lrow = sh.lists + (size_t)row * LROW;
+    float *qarea = reinterpret_cast<float *>(sh.lists + quarter * T::QUARTER_BYTES);
+    typename T::Entry *lrow = const_cast<typename T::Entry *>(T::row(sh.lists, quarter, lane));
     unsigned g0 = 0;                              // this slot's units of the earlier items
     for (int seq = 0;; ++seq) {
         const int r = seq & 1;
@@ -578,17 +645,14 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             const int b = s * BPS + (int)(g % BPS);
             if (!(ok = pipe_wait(&sh.acc_full[b], (g / BPS) & 1, sh.abort_flag))) break;
             sm100::tc_fence_after();
-            if (active) {
-                if constexpr (BN == 256) {
-                    // either tile may be the short one (the first when it ends a run)
-                    if (na > 0 || nb > 0) fold2x32(tbase + b * BN, na, tbase + b * BN + 128, nb, bm);
-                } else {
-                    if (na > 0) fold32(tbase + b * BN, na, bm);
-                }
+            uint64_t *empty = &sh.acc_empty[b];
+            // (either tile may be the short one: the first when it ends a run)
+            if (active && (na > 0 || nb > 0)) {
+                if constexpr (BN == 256) fold2x32(tbase + b * BN, na, tbase + b * BN + 128, nb, empty, lane, bm);
+                else fold32(tbase + b * BN, na, empty, lane, bm);
+            } else {
+                release_acc(empty, lane);
             }
-            sm100::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) sm100::mbar_arrive(&sh.acc_empty[b]);
         }
         // threshold: rank-th smallest of the 128 column minima of every query
         {
@@ -616,8 +680,23 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
                 ans[L] = 0u;
             }
             const int lowb = nts <= 16 ? TAU_LOW_BIT + 4 : TAU_LOW_BIT;   // uniform over the slot
+            // bits above the highest one in which any two minima of the warp's
+            // rows differ are common to every answer: start below them
+            unsigned lo_v = 0xffffffffu, hi_v = 0u;
+#pragma unroll
+            for (int L = 0; L < RL; ++L)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    lo_v = min(lo_v, v4[L][u]);
+                    hi_v = max(hi_v, v4[L][u]);
+                }
+            lo_v = __reduce_min_sync(0xffffffffu, lo_v);
+            hi_v = __reduce_max_sync(0xffffffffu, hi_v);
+            const int top = min(30, 31 - __clz((lo_v ^ hi_v) | 1u));
+#pragma unroll
+            for (int L = 0; L < RL; ++L) ans[L] = lo_v & ~((2u << top) - 1u);
 #pragma unroll 1
-            for (int b = 30; b >= lowb; --b) {
+            for (int b = top; b >= lowb; --b) {
 #pragma unroll
                 for (int L = 0; L < RL; ++L) {
                     const unsigned t = ans[L] | (1u << b);
@@ -654,23 +733,20 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             const int b = s * BPS + (int)(g % BPS);
             if (!(ok = pipe_wait(&sh.acc_full[b], (g / BPS) & 1, sh.abort_flag))) break;
             sm100::tc_fence_after();
+            uint64_t *empty = &sh.acc_empty[b];
             if (active && (na > 0 || nb > 0)) {
                 unsigned ma = 0u, mb = 0u;
-                if constexpr (BN == 256 && TAU) {
-                    mark2x32_signs(tbase + b * BN, na, tbase + b * BN + 128, nb, ma, mb);
-                } else {
-                    if (na > 0) ma = mark32(tbase + b * BN, na, tau);
-                    if (BN == 256 && nb > 0) mb = mark32(tbase + b * BN + 128, nb, tau);
-                }
-                if (ma) append_hits(lrow, sh.sCnt + row, ma, (uint32_t)(ra + part * PART));
-                if (mb) append_hits(lrow, sh.sCnt + row, mb, (uint32_t)(rb + part * PART));
+                mark<BN, BN == 256 && TAU>(tbase + b * BN, na, tbase + b * BN + 128, nb, tau, empty, lane, ma, mb);
+                // entries: rows, or (place of the tile in the list, column)
+                const uint32_t ea = BIG ? (uint32_t)ra : (uint32_t)((k - U) * (BN / 128)) << 7;
+                const uint32_t eb = BIG ? (uint32_t)rb : ea + 128u;
+                append_hits(lrow, sh.sCnt + row, ma, ea + part * PART, mb, eb + part * PART);
+            } else {
+                release_acc(empty, lane);
             }
-            sm100::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) sm100::mbar_arrive(&sh.acc_empty[b]);
         }
         slot_barrier(s, slot_threads);
-        if (__all_sync(0xffffffffu, ok)) hand_off(p, it, s, quarter, part, qrow, nq_s, sh.lists, sh.sCnt, sh.sTau, lo, scratch, lane);
+        if (__all_sync(0xffffffffu, ok)) hand_off<T>(p, it, s, quarter, part, qrow, nq_s, tl, sh.lists, sh.sCnt, sh.sTau, lo, scratch, lane);
         g0 += 2u * (unsigned)U;
         // every warp of the slot is done with this item's lists before the
         // next item's minima overwrite them; after a timed-out wait all stop
@@ -678,49 +754,63 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
     }
 }
 
-// TMA producer (one thread): claims items from the launch's work queue and
+// TMA producer (one warp): claims items from the launch's work queue and
 // publishes their indices (a two-entry ring), loads each item's four 32-row
 // query boxes into the free query tile, then the slots' units round-robin,
 // each slot's sequence twice (both passes).  A unit's 128-candidate tiles land
-// in consecutive 128-row halves of its stage.  Stage and tile counters run on
+// in consecutive 128-row halves of its stage, lane h loading half h from its
+// tile's first row, which it fetched a unit ahead (the table lookup is off the
+// path between a free stage and its loads).  Stage and tile counters run on
 // across items, so the ring never drains between them.
-template <int BN, int NS>
+template <int BN, int NS, bool BIG>
 __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMap &tmC, const irc::PlanDev &p,
                                         const irc_tc::TcItem *__restrict__ items, int n_items, unsigned *queue,
-                                        const Shared &sh)
+                                        const Shared &sh, int lane)
 {
-    using T = Tile<BN>;
+    using T = Tile<BN, BIG>;
     constexpr int QPS = 4 / NS;
-    sm100::prefetch_tmap(&tmQ);
-    sm100::prefetch_tmap(&tmC);
-    int i = 0, n_a = 0;                           // candidate stages and query tiles loaded
+    constexpr int NH = BN / 128;                  // 128-tiles of a unit
+    if (lane == 0) {
+        sm100::prefetch_tmap(&tmQ);
+        sm100::prefetch_tmap(&tmC);
+    }
+    int n_a = 0, n_w[MMA_WARPS] = {};             // query tiles loaded, units loaded for each issuer
+    int st = 0;                                   // stage of the next unit
+    uint32_t ph = 1;                              // parity of the stage's last release
     bool ok = true;
     for (int seq = 0; ok; ++seq) {
         const int r = seq & 1;
-        const unsigned claim = atomicAdd(queue, 1u);
+        unsigned claim = 0;
+        if (lane == 0) claim = atomicAdd(queue, 1u);
+        claim = __shfl_sync(0xffffffffu, claim, 0);
         const int idx = claim < (unsigned)n_items ? (int)claim : -1;
-        if (!(ok = pipe_wait(&sh.item_empty[r], ((seq >> 1) & 1) ^ 1, sh.abort_flag))) break;
-        sh.item_idx[r] = idx;
-        sm100::mbar_arrive(&sh.item_full[r]);     // release: the index is visible to the waiters
+        if (!(ok = warp_wait(&sh.item_empty[r], ((seq >> 1) & 1) ^ 1, sh.abort_flag))) break;
+        if (lane == 0) {
+            sh.item_idx[r] = idx;
+            sm100::mbar_arrive(&sh.item_full[r]); // release: the index is visible to the waiters
+        }
         if (idx < 0) break;
         const irc_tc::TcItem it = items[idx];
         const int2 *tl[NS];
-        int U[NS], nt[NS];
+        int U[NS], nt[NS], row[NS];               // row: this lane's tile of the slot's next unit
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             nt[s] = chunk_tiles(p, it.chunk[s]);
             U[s] = units_per_pass<BN>(nt[s]);
             tl[s] = nt[s] ? p.tc_tiles + __ldg(p.tc_toff + it.chunk[s]) : p.tc_tiles;
+            row[s] = lane < NH && lane < nt[s] ? __ldg(tl[s] + lane).x : 0;
         }
         // the query tile of item seq - 2 is free once that item's MMAs are done
-        if (!(ok = pipe_wait(&sh.a_empty[r], ((seq >> 1) & 1) ^ 1, sh.abort_flag))) break;
+        if (!(ok = warp_wait(&sh.a_empty[r], ((seq >> 1) & 1) ^ 1, sh.abort_flag))) break;
         uint8_t *sA = sh.sA + (size_t)r * A_BYTES;
-        sm100::mbar_arrive_expect_tx(&sh.a_full[r], A_BYTES);
+        if (lane == 0) sm100::mbar_arrive_expect_tx(&sh.a_full[r], A_BYTES);
+        __syncwarp();
+        if (lane < 4) {
+            int row0 = 0;                         // query box `lane` of the tile
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int s = q / QPS;
-            const int row0 = it.chunk[s] >= 0 ? it.qs[s] + (q % QPS) * 32 : 0;
-            sm100::tma_load_2d(&tmQ, &sh.a_full[r], sA + q * (A_BYTES / 4), 0, row0);
+            for (int s = 0; s < NS; ++s)
+                if (lane / QPS == s && it.chunk[s] >= 0) row0 = it.qs[s] + (lane % QPS) * 32;
+            sm100::tma_load_2d(&tmQ, &sh.a_full[r], sA + lane * (A_BYTES / 4), 0, row0);
         }
         ++n_a;
         for (int k = 0; ok; ++k) {
@@ -729,17 +819,24 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
             for (int s = 0; s < NS; ++s) {
                 if (ok && k < 2 * U[s]) {
                     any = true;
-                    const int u = k % U[s];
-                    const int st = i % T::STAGES;
-                    if ((ok = pipe_wait(&sh.empty[st], ((i / T::STAGES) & 1) ^ 1, sh.abort_flag))) {
-                        uint8_t *dst = sh.sB + (size_t)st * T::STAGE_BYTES;
-                        const int nh = BN == 256 && 2 * u + 1 < nt[s] ? 2 : 1;   // 128-tiles of the unit
-                        sm100::mbar_arrive_expect_tx(&sh.full[st], nh * HALF_BYTES);
-                        for (int h = 0; h < nh; ++h) {
-                            const int row0 = __ldg(tl[s] + (BN == 256 ? 2 * u + h : u)).x;
-                            sm100::tma_load_2d(&tmC, &sh.full[st], dst + h * HALF_BYTES, 0, row0);
+                    const int u = k < U[s] ? k : k - U[s];
+                    const int w = issuer_of<NS>(k, s);
+                    if ((ok = warp_wait(&sh.empty[st], ph, sh.abort_flag))) {
+                        const int nh = BN == 256 && 2 * u + 1 >= nt[s] ? 1 : NH;
+                        uint64_t *full = sh.full + w * T::STAGES + (w == 0 ? n_w[0] : n_w[1]) % T::STAGES;
+                        if (lane == 0) sm100::mbar_arrive_expect_tx(full, nh * HALF_BYTES);
+                        __syncwarp();
+                        if (lane < nh)
+                            sm100::tma_load_2d(&tmC, full,
+                                               sh.sB + (size_t)st * T::STAGE_BYTES + lane * HALF_BYTES, 0, row[s]);
+                        const int un = u + 1 < U[s] ? u + 1 : 0, t = un * NH + lane;
+                        if (lane < NH && t < nt[s]) row[s] = __ldg(tl[s] + t).x;
+#pragma unroll
+                        for (int v = 0; v < MMA_WARPS; ++v) n_w[v] += v == w;
+                        if (++st == T::STAGES) {
+                            st = 0;
+                            ph ^= 1u;
                         }
-                        ++i;
                     }
                 }
             }
@@ -747,23 +844,32 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
         }
     }
     // every issued load has landed before the CTA exits
-    for (int j = (i > T::STAGES ? i - T::STAGES : 0); j < i; ++j)
-        sm100::mbar_drain(&sh.full[j % T::STAGES], (j / T::STAGES) & 1);
+#pragma unroll
+    for (int w = 0; w < MMA_WARPS; ++w)
+        for (int j = (n_w[w] > T::STAGES ? n_w[w] - T::STAGES : 0); j < n_w[w]; ++j)
+            sm100::mbar_drain(&sh.full[w * T::STAGES + j % T::STAGES], (j / T::STAGES) & 1);
     for (int j = (n_a > 2 ? n_a - 2 : 0); j < n_a; ++j) sm100::mbar_drain(&sh.a_full[j & 1], (j >> 1) & 1);
 }
 
-// MMA issuer (one thread), in the producer's order; unit g of slot s (counted
-// over the CTA's items) goes to accumulator s*BPS + g % BPS and is issued once
-// every epilogue warp of the slot released unit g - BPS of that buffer.  With
-// TAU the slot's first pass-2 unit of an item also waits until its epilogue
-// wrote the thresholds into the query tile (tau_ready[s], one phase per item
-// in which the slot has units).  After an item's last MMA a commit frees its
-// query tile.
-template <int BN, int NS, Fmt FMT, bool TAU>
+// MMA issuers (one thread of each of MMA_WARPS warps), in the producer's order,
+// each its own units (issuer_of).  One thread alone was the pipeline's
+// bound: its waits, the issue of the MMAs (which blocks for about as long as
+// they run) and the commits took ~1,450 cycles a unit in series, against ~300
+// of MMA time; two threads overlap one's waits with the other's MMAs.  Unit g
+// of slot s (counted over the CTA's items) goes to accumulator s*BPS + g % BPS
+// and is issued once every epilogue warp of the slot released unit g - BPS of
+// that buffer; a buffer, and with it every phase of its barriers, belongs to
+// one issuer, and so do the load barriers (a waiter that did not see every
+// phase could take an old phase's parity for the one it waits for).  With TAU
+// an issuer's first pass-2 unit of a slot in an item also waits until the
+// slot's epilogue wrote the thresholds into the query tile (tau_ready[s], one
+// phase per item in which the slot has units).  After an item's last unit each
+// issuer's commit lets its MMAs free the query tile.
+template <int BN, int NS, Fmt FMT, bool TAU, bool BIG>
 __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcItem *__restrict__ items, int nk,
-                                      uint32_t tmem, const Shared &sh)
+                                      uint32_t tmem, const Shared &sh, int w)
 {
-    using T = Tile<BN>;
+    using T = Tile<BN, BIG>;
     constexpr int BPS = T::NBUF / NS;
     // bf16 x bf16 or f16 x f16 (kind::f16, K = 16) or e4m3 x e4m3 (kind::f8f6f4, K = 32)
     // -> f32; either way one MMA consumes 32 bytes of every 128-byte operand row
@@ -771,7 +877,9 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
     unsigned g0[NS], taus[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) g0[s] = taus[s] = 0;
-    int i = 0;
+    int st = 0;                                   // stage of the next unit
+    int fw = 0;                                   // this issuer's next load barrier, and its parity
+    uint32_t ph = 0;
     bool ok = true;
     for (int seq = 0; ok; ++seq) {
         const int r = seq & 1;
@@ -781,8 +889,12 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
         if (idx < 0) break;
         const irc_tc::TcItem it = items[idx];
         int U[NS];
+        bool tau_wait[NS];
 #pragma unroll
-        for (int s = 0; s < NS; ++s) U[s] = units_per_pass<BN>(chunk_tiles(p, it.chunk[s]));
+        for (int s = 0; s < NS; ++s) {
+            U[s] = units_per_pass<BN>(chunk_tiles(p, it.chunk[s]));
+            tau_wait[s] = TAU;
+        }
         if (!(ok = pipe_wait(&sh.a_full[r], (seq >> 1) & 1, sh.abort_flag))) break;
         sm100::tc_fence_after();
         const uint64_t adesc = sm100::sdesc_sw128(sm100::smem_u32(sh.sA + (size_t)r * A_BYTES));
@@ -792,28 +904,40 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
             for (int s = 0; s < NS; ++s) {
                 if (ok && k < 2 * U[s]) {
                     any = true;
-                    const unsigned g = g0[s] + (unsigned)k, use = g / BPS;
-                    const int b = s * BPS + (int)(g % BPS), st = i % T::STAGES;
-                    ok = (use == 0 || pipe_wait(&sh.acc_empty[b], (use - 1) & 1, sh.abort_flag)) &&
-                         pipe_wait(&sh.full[st], (i / T::STAGES) & 1, sh.abort_flag) &&
-                         // the slot's thresholds are in the query tile before its pass 2
-                         (!TAU || k != U[s] || pipe_wait(&sh.tau_ready[s], taus[s] & 1, sh.abort_flag));
-                    if (ok) {
-                        sm100::tc_fence_after();
-                        const uint64_t bdesc =
-                            sm100::sdesc_sw128(sm100::smem_u32(sh.sB + (size_t)st * T::STAGE_BYTES));
+                    if (issuer_of<NS>(k, s) == w) {
+                        const unsigned g = g0[s] + (unsigned)k, use = g / BPS;
+                        const int b = s * BPS + (int)(g % BPS);
+                        // (the load is usually there long before the accumulator is free)
+                        ok = pipe_wait(&sh.full[w * T::STAGES + fw], ph, sh.abort_flag) &&
+                             (use == 0 || pipe_wait(&sh.acc_empty[b], (use - 1) & 1, sh.abort_flag));
+                        if (++fw == T::STAGES) {
+                            fw = 0;
+                            ph ^= 1u;
+                        }
+                        // the slot's thresholds are in the query tile before its pass 2 (after the
+                        // accumulator's wait: the slot's epilogue is then in this item, so no
+                        // earlier phase of tau_ready is open)
+                        if (TAU && ok && k >= U[s] && tau_wait[s]) {
+                            tau_wait[s] = false;
+                            ok = pipe_wait(&sh.tau_ready[s], taus[s] & 1, sh.abort_flag);
+                        }
+                        if (ok) {
+                            sm100::tc_fence_after();
+                            const uint64_t bdesc =
+                                sm100::sdesc_sw128(sm100::smem_u32(sh.sB + (size_t)st * T::STAGE_BYTES));
 #pragma unroll
-                        for (int kk = 0; kk < KP / 16; ++kk)
-                            if (kk >= nk)
-                                break;                    // the rest of every operand row is zero
-                            else if (FMT == Fmt::fp8)
-                                sm100::mma_f8(tmem + b * BN, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk > 0 ? 1u : 0u);
-                            else
-                                sm100::mma_f16(tmem + b * BN, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk > 0 ? 1u : 0u);
-                        sm100::mma_commit(&sh.empty[st]);
-                        sm100::mma_commit(&sh.acc_full[b]);
-                        ++i;
+                            for (int kk = 0; kk < KP / 16; ++kk)
+                                if (kk >= nk)
+                                    break;                // the rest of every operand row is zero
+                                else if (FMT == Fmt::fp8)
+                                    sm100::mma_f8(tmem + b * BN, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk > 0 ? 1u : 0u);
+                                else
+                                    sm100::mma_f16(tmem + b * BN, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk > 0 ? 1u : 0u);
+                            sm100::mma_commit(&sh.acc_full[b]);
+                            sm100::mma_commit(&sh.empty[st]);
+                        }
                     }
+                    if (++st == T::STAGES) st = 0;
                 }
             }
             if (!any) break;
@@ -826,9 +950,9 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
         }
         sm100::mma_commit(&sh.a_empty[r]);        // this item's MMAs done: its query tile may be replaced
     }
-    // every MMA has completed before TMEM is released
-    sm100::mma_commit(sh.mma_done);
-    sm100::mbar_drain(sh.mma_done, 0);
+    // every MMA of this thread has completed before TMEM is released
+    sm100::mma_commit(sh.mma_done + w);
+    sm100::mbar_drain(sh.mma_done + w, 0);
 }
 
 // The filter over the work items of one packing class (NS slots per item:
@@ -837,25 +961,25 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
 // is empty.  TAU: pass 2 reads the signs of d2 - tau (the thresholds written
 // into the query tile at K position tau_k), else it compares d2 with tau in
 // the epilogue.
-template <Fmt FMT, int BN, bool TAU, int NS>
+template <Fmt FMT, int BN, bool TAU, int NS, bool BIG>
 __global__ void __launch_bounds__(THREADS, 1)
 k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmC, irc::PlanDev p,
          const irc_tc::TcItem *__restrict__ items, int n_items, unsigned *queue, int nk, int tau_k, irc_tc::ListOut lo,
          int *__restrict__ scratch)
 {
-    using T = Tile<BN>;
+    using T = Tile<BN, BIG>;
     constexpr int QPS = 4 / NS;
     extern __shared__ unsigned char smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     Shared sh;
     sh.sA = base;
     sh.sB = base + 2 * A_BYTES;
-    sh.lists = reinterpret_cast<uint32_t *>(sh.sB + T::STAGES * T::STAGE_BYTES);   // [BM][LROW]
-    sh.sTau = reinterpret_cast<float *>(sh.lists + (size_t)LROW * BM);
+    sh.lists = sh.sB + T::STAGES * T::STAGE_BYTES;
+    sh.sTau = reinterpret_cast<float *>(sh.lists + 4 * T::QUARTER_BYTES);
     sh.sCnt = reinterpret_cast<int *>(sh.sTau + BM);
     uint64_t *bars = reinterpret_cast<uint64_t *>(sh.sCnt + BM);
     sh.full = bars;
-    sh.empty = sh.full + T::STAGES;
+    sh.empty = sh.full + MMA_WARPS * T::STAGES;
     sh.a_full = sh.empty + T::STAGES;
     sh.a_empty = sh.a_full + 2;
     sh.acc_full = sh.a_empty + 2;
@@ -864,24 +988,25 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
     sh.item_full = sh.tau_ready + 4;
     sh.item_empty = sh.item_full + 2;
     sh.mma_done = sh.item_empty + 2;
-    sh.item_idx = reinterpret_cast<int *>(sh.mma_done + 1);
+    sh.item_idx = reinterpret_cast<int *>(sh.mma_done + MMA_WARPS);
     sh.tmem_slot = reinterpret_cast<uint32_t *>(sh.item_idx + 2);
     sh.abort_flag = reinterpret_cast<volatile int *>(sh.tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < T::STAGES; ++s) { sm100::mbar_init(&sh.full[s], 1); sm100::mbar_init(&sh.empty[s], 1); }
+        for (int s = 0; s < MMA_WARPS * T::STAGES; ++s) sm100::mbar_init(&sh.full[s], 1);
+        for (int s = 0; s < T::STAGES; ++s) sm100::mbar_init(&sh.empty[s], 1);
         for (int r = 0; r < 2; ++r) {
             sm100::mbar_init(&sh.a_full[r], 1);
-            sm100::mbar_init(&sh.a_empty[r], 1);
+            sm100::mbar_init(&sh.a_empty[r], MMA_WARPS);
             sm100::mbar_init(&sh.item_full[r], 1);
-            sm100::mbar_init(&sh.item_empty[r], 1 + EPI_WARPS);   // the MMA thread and every epilogue warp
+            sm100::mbar_init(&sh.item_empty[r], MMA_WARPS + EPI_WARPS);   // the MMA threads and every epilogue warp
         }
         for (int b = 0; b < T::NBUF; ++b) {
             sm100::mbar_init(&sh.acc_full[b], 1);
             sm100::mbar_init(&sh.acc_empty[b], PARTS * QPS);       // the slot's epilogue warps
         }
-        sm100::mbar_init(sh.mma_done, 1);
+        for (int w = 0; w < MMA_WARPS; ++w) sm100::mbar_init(sh.mma_done + w, 1);
         for (int s = 0; s < 4; ++s) sm100::mbar_init(&sh.tau_ready[s], QPS);   // the slot's quarters' writers
         *sh.abort_flag = 0;
         sm100::fence_mbar_init();
@@ -893,13 +1018,13 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
     const uint32_t tmem = *sh.tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) produce<BN, NS>(tmQ, tmC, p, items, n_items, queue, sh);
+        produce<BN, NS, BIG>(tmQ, tmC, p, items, n_items, queue, sh, lane);
         __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) issue<BN, NS, FMT, TAU>(p, items, nk, tmem, sh);
+    } else if (warp == 1 || warp == 2 + EPI_WARPS) {
+        if (lane == 0) issue<BN, NS, FMT, TAU, BIG>(p, items, nk, tmem, sh, warp == 1 ? 0 : 1);
         __syncwarp();
     } else {
-        epilogue<BN, NS, FMT, TAU>(p, items, tau_rank(FMT), tmem, tau_k, sh, lo, scratch, warp, lane);
+        epilogue<BN, NS, FMT, TAU, BIG>(p, items, tau_rank(FMT), tmem, tau_k, sh, lo, scratch, warp, lane);
     }
     sm100::tc_fence_before();
     __syncthreads();
@@ -970,8 +1095,9 @@ static int launch_filter(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan 
                          int n_items, unsigned *queue, int nk, int tau_k, const ListOut &lo, int *scratch, cudaStream_t s)
 {
     if (n_items <= 0) return IRC_OK;
-    auto kern = k_knn_tc<FMT, BN, TAU, NS>;
-    const int smem = (int)Tile<BN>::SMEM_BYTES;
+    const bool big = pl->tc_max_tiles > MAX_SHORT_TILES;
+    auto kern = big ? k_knn_tc<FMT, BN, TAU, NS, true> : k_knn_tc<FMT, BN, TAU, NS, false>;
+    const int smem = (int)(big ? Tile<BN, true>::SMEM_BYTES : Tile<BN, false>::SMEM_BYTES);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int sms = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
