@@ -53,12 +53,11 @@ using irc_tc::Fmt;
 
 constexpr int kWarps = 8;                 // queries per block of the list kernels
 constexpr int kTile = 16;                 // queries per tile of the plain kernels
-constexpr int kMore = 12;                 // REF: list entries selected beyond knn (shared bins take places)
+constexpr int kRefKeys = 60;              // REF: list entries selected (shared bins take places; ws holds 64)
 
 // Counter words of a call's working memory (zeroed before it).
 constexpr int W_AMAX = 1;                 // bits of max |F|
 constexpr int W_ERR = irc::kScratchErr;   // a wait of the filter gave up
-constexpr int W_ITEMS = irc::kScratchItems;
 constexpr int W_TILES = 4;                // tiles left to the plain kernel
 constexpr int W_OVF = 5;                  // its overflow queue
 constexpr size_t kHdrBytes = 256;
@@ -125,7 +124,7 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
     unsigned long long kv[PER];
     irc_rr::list_keys<PER>(list, cL, c.Fp, irc_tc::fp_row4(c.nC), q, qs, nd, lane, kv);
     unsigned tb;
-    const int n = irc_rr::select_keys<PER>(kv, REF ? knn + kMore : knn, ws, lane, tb);
+    const int n = irc_rr::select_keys<PER>(kv, REF ? kRefKeys : knn, ws, lane, tb);
     const float x = __ldg(c.qnorm + o), s = __ldg(c.scale);
     if (n < knn || n > WARP_KEYS || !(s > 0.0f)) return false;
     if (!REF) {
@@ -142,8 +141,7 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
     __syncwarp();
     unsigned long long k2[2] = {~0ull, ~0ull};
     int nk = 0;                                   // bins found
-    unsigned long long ex = ~0ull;                // a left-over bin's key (at most one per lane is kept)
-    bool more = false;
+    unsigned long long ex[2] = {~0ull, ~0ull};    // keys of the left-over bins
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
         if (b * 32 >= n) break;
@@ -171,18 +169,18 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
             __syncwarp();
             if (f2) {
                 atomicOr(bits + (t2 >> 5), 1u << (t2 & 31));
-                const unsigned long long kx = key | ((unsigned long long)t2 << 16);
-                more |= ex != ~0ull;              // two in one lane: rare, left to the plain kernel
-                ex = kx;
+                ex[b] = key | ((unsigned long long)t2 << 16);
             }
             nk += __popc(__ballot_sync(0xffffffffu, f2));
         }
         __syncwarp();
     }
-    if (nk < knn || __any_sync(0xffffffffu, more)) return false;
+    if (nk < knn) return false;
     // the left-over bins' keys take free places (at most 64 keys are sorted)
-    const unsigned mx = __ballot_sync(0xffffffffu, ex != ~0ull);
-    if (mx) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const unsigned mx = __ballot_sync(0xffffffffu, ex[b] != ~0ull);
+        if (!mx) continue;
         const unsigned f0 = __ballot_sync(0xffffffffu, k2[0] == ~0ull), f1 = __ballot_sync(0xffffffffu, k2[1] == ~0ull);
         if (__popc(mx) > __popc(f0) + __popc(f1)) return false;
         // free place number i: the i-th set bit of f0, then of f1
@@ -190,7 +188,7 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
         const int p0 = __popc(f0 & lt), p1 = __popc(f0) + __popc(f1 & lt);
         unsigned rest = mx;
         for (int i = 0; rest; ++i, rest &= rest - 1u) {
-            const unsigned long long kx = __shfl_sync(0xffffffffu, ex, __ffs(rest) - 1);
+            const unsigned long long kx = __shfl_sync(0xffffffffu, ex[b], __ffs(rest) - 1);
             if (((f0 >> lane) & 1u) && p0 == i) k2[0] = kx;
             if (((f1 >> lane) & 1u) && p1 == i) k2[1] = kx;
         }
@@ -245,10 +243,10 @@ k_cert_knn(Call c, int knn, int nT, float *__restrict__ vrKnn, float *__restrict
 // REF delta of one query per warp: among its listed candidates with a higher
 // rho (the reference's mask), the smallest sqrt(d2), then the lowest bin, then
 // in the bin the smallest (d2, row).  Queries whose list holds none, or not
-// provably the nearest, are flagged for the drift-window search.
+// provably the nearest, are listed for the drift-window search.
 __global__ void __launch_bounds__(32 * kWarps, 4)
 k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ delta, int *__restrict__ nneigh,
-             int *__restrict__ flag)
+             int *__restrict__ counts, int *__restrict__ list_out)
 {
     __shared__ float4 qrows[kWarps * QROW4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -295,7 +293,9 @@ k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ de
             }
         }
     }
-    if (lane == 0) flag[o] = ok ? 0 : 1;
+    // (without a record the query is in no chunk, or a wait gave up and every query is searched again)
+    if (lane == 0 && !ok && ce.y >= 0)
+        list_out[__ldg(c.p.q0 + ce.y) - c.p.q_base + atomicAdd(counts + ce.y, 1)] = q;
 }
 
 // Working memory of the proven searches: one pool per device, shared by the
@@ -446,20 +446,16 @@ int irc_cert_site_delta_ref(irc_plan *pl, const float *F, int nC, const float *R
     // (a bin's step number has 20 bits in the drift-window search's keys: a
     // run of at most 2^20 rows always fits)
     if (!serves(pl, nC, false) || pl->max_rn > (1 << 20)) return IRC_CERT_PASS;
-    const size_t n = (size_t)pl->dev.n_out, q4 = up(n * 4), it = up(delta_items(n, pl->dev.nChunks) * sizeof(int2));
-    const size_t more = 2 * q4 + it + up(n * 8);
+    const size_t more = delta_bytes(pl->dev.n_out, pl->dev.nChunks);
     Work w(pl, lists_bytes(pl, nC, more), s);
     if (!w.base) return IRC_CERT_PASS;
     Lists L;
-    int rc = make_lists(pl, F, nC, (char *)w.base, more, 0, &L, s);
+    // (the counters lie at the front of the scratch)
+    int rc = make_lists(pl, F, nC, (char *)w.base, more, 4 * (4 + (size_t)pl->dev.nChunks), &L, s);
     if (rc != IRC_OK) return rc;
-    irc_delta_scratch sc;
-    sc.n_items = L.c.words + W_ITEMS;
-    sc.flags = (int *)L.more;
-    sc.list = (int *)(L.more + q4);
-    sc.items = (int2 *)(L.more + 2 * q4);
-    sc.keys = (unsigned long long *)(L.more + 2 * q4 + it);
-    k_cert_delta<<<(pl->dev.n_out + kWarps - 1) / kWarps, 32 * kWarps, 0, s>>>(L.c, R, nThreads, delta, nneigh, sc.flags);
+    const irc_delta_scratch sc = irc_delta_carve(pl, L.more, L.c.words + W_ERR);
+    k_cert_delta<<<(pl->dev.n_out + kWarps - 1) / kWarps, 32 * kWarps, 0, s>>>(L.c, R, nThreads, delta, nneigh, sc.counts,
+                                                                             sc.list);
     IRC_CHECK_LAUNCH("irc_site_delta lists");
     return irc_delta_window(pl, F, nC, R, nThreads, sc, delta, nneigh, s);
 }

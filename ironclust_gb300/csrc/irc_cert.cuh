@@ -18,17 +18,23 @@ int irc_ref_tiles(irc_plan *pl, const float *F, int nC, int knn, int nThreads, f
 int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
                     float *d2Knn, const irc::TileQueue &tq, int *cnt, int *ovf_list, cudaStream_t s);
 
-// Device scratch of the drift-window delta search: the unit counter, one flag
-// and one key per query, the compacted queries [n_out] and their units, up to
-// 8 parts of every 16-query tile.
+// Device scratch of the drift-window delta search: unit and list counters,
+// per chunk the number of queries to search and (a segment of list) which, the
+// queries searched one by one, per-query keys and the units of 16-query tiles,
+// up to 8 parts each.
 struct irc_delta_scratch {
-    int *n_items, *flags, *list;
-    int2 *items;                 // [delta_items(...)]
-    unsigned long long *keys;    // [n_out]
+    int *words, *counts, *list;
+    int2 *sparse, *items;
+    unsigned long long *keys;
+    const int *all;              // if not null and set: search every query
 };
-inline size_t delta_items(long long n_out, long long nChunks)
+inline size_t delta_part(size_t n) { return (n + 255) & ~(size_t)255; }
+inline size_t delta_bytes(long long n_out, long long nChunks)
 {
-    return 8 * ((size_t)n_out / 16 + (size_t)nChunks + 1);
+    const size_t n = (size_t)n_out, c = (size_t)nChunks;
+    return delta_part(4 * (4 + c)) + delta_part(4 * n) + 2 * delta_part(8 * n) + delta_part(8 * 8 * (n / 16 + c + 1));
 }
+irc_delta_scratch irc_delta_carve(const irc_plan *pl, void *mem, const int *all);
+cudaError_t irc_delta_clear(const irc_plan *pl, const irc_delta_scratch &sc, cudaStream_t s);
 int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int nT, const irc_delta_scratch &sc,
                      float *delta, int32_t *nneigh, cudaStream_t s);

@@ -20,12 +20,14 @@
 // exceeds the query's, whenever the list holds one (any closer higher-rho
 // spike would rank earlier in the list).  Queries without one -- local
 // density peaks -- go to a drift-window scan over all linked candidates.
+#include <climits>
 #include <cstdio>
 #include <mutex>
 
 #include "irc_cert.cuh"
 #include "irc_common.cuh"
 #include "irc_plan.cuh"
+#include "irc_rows.cuh"
 #include "irc_scan.cuh"
 
 namespace {
@@ -276,73 +278,112 @@ k_exact_overflow(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
     }
 }
 
-// delta from the kNN list; queries without a higher-rho list entry are queued.
-__global__ void k_delta_list(irc::PlanDev p, const float *__restrict__ R, int knn,
-                             const int *__restrict__ miKnn, const float *__restrict__ d2Knn,
-                             float *__restrict__ delta, int *__restrict__ nneigh,
-                             int *__restrict__ fb_flag)
+// delta from the kNN list, a thread per query, a warp per 32-query tile of a
+// chunk; queries without a higher-rho list entry go to the chunk's segment of
+// fb_list, in any order.  Entries are read four at a time (their rho gathers in
+// flight together): the first or second decides for most queries, and one at a
+// time the two dependent loads of each made a 3,000-query site take 10 us.
+constexpr int kListTile = 32, kListWarps = 4;
+
+__global__ void __launch_bounds__(32 * kListWarps)
+k_delta_list(irc::PlanDev p, int ntiles, const float *__restrict__ R, int knn, const int *__restrict__ miKnn,
+             const float *__restrict__ d2Knn, float *__restrict__ delta, int *__restrict__ nneigh,
+             int *__restrict__ counts, int *__restrict__ fb_list)
 {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= p.n_out) return;
-    const int q = o + p.q_base;
-    const float rq = __ldg(R + q);
-    const int *mi = miKnn + (size_t)knn * o;
-    const float *dk = d2Knn + (size_t)knn * o;
-    int miss = 1;
-    for (int k = 0; k < knn; ++k) {
-        const float d2 = __ldg(dk + k);
-        if (!(d2 < kInfSentinel)) break;                 // list exhausted
-        const int j = __ldg(mi + k) - 1;
-        if (!(__ldg(R + j) <= rq)) {                     // reference mask: rb <= ra is excluded
-            delta[o] = __fmul_rn(irc::ref_sqrt_abs(d2), rq);
-            nneigh[o] = j + 1;
-            miss = 0;
-            break;
+    const int lane = threadIdx.x & 31, tile = blockIdx.x * kListWarps + (threadIdx.x >> 5);
+    if (tile >= ntiles) return;
+    int chunk, qs, n;
+    irc::tile_lookup<kListTile>(p, tile, chunk, qs, n);
+    int miss = 0;
+    if (lane < n) {
+        const int q = qs + lane, o = q - p.q_base;
+        const float rq = __ldg(R + q);
+        const int *mi = miKnn + (size_t)knn * o;
+        const float *dk = d2Knn + (size_t)knn * o;
+        miss = 1;
+        bool more = true;
+        for (int k = 0; k < knn && more; k += 4) {
+            int j[4];
+            float d2[4], rj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                j[u] = k + u < knn ? __ldg(mi + k + u) - 1 : q;
+                d2[u] = k + u < knn ? __ldg(dk + k + u) : kInfSentinel;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) rj[u] = __ldg(R + j[u]);     // (a row without a neighbour names the query)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (!more) continue;
+                if (!(d2[u] < kInfSentinel)) more = false;           // list exhausted
+                else if (!(rj[u] <= rq)) {                           // reference mask: rb <= ra is excluded
+                    delta[o] = __fmul_rn(irc::ref_sqrt_abs(d2[u]), rq);
+                    nneigh[o] = j[u] + 1;
+                    miss = 0;
+                    more = false;
+                }
+            }
         }
     }
-    fb_flag[o] = miss;
+    const unsigned bal = __ballot_sync(0xffffffffu, miss);
+    if (!bal) return;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(counts + chunk, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (miss) fb_list[__ldg(p.q0 + chunk) - p.q_base + base + __popc(bal & ((1u << lane) - 1u))] = qs + lane;
 }
 
-// One CTA per chunk: compact the chunk's flagged queries (in order) into the
-// chunk's own segment of fb_list, then claim the (16-query tile, part) units
-// of the fallback scan: unit = {chunk | part << 28, (first << 5) | count}.
 constexpr int kParts = 8;        // most parts of one candidate window (part < 2^3: 3 bits at bit 28)
 constexpr int kMinPart = 2048;   // fewest candidates of a part
+constexpr int kWide = 512;       // candidates of a window that whole blocks search, in parts
+constexpr int kWideParts = 16;   // most parts (of kMinPart candidates and more)
+constexpr int kDense = 64;       // fewest queries of a chunk that are searched 16 at a time
 
-__global__ void __launch_bounds__(kThreads)
-k_delta_compact(irc::PlanDev p, const int *__restrict__ fb_flag, int *__restrict__ fb_list,
-                int *__restrict__ n_items, int2 *__restrict__ items, unsigned long long *__restrict__ keys)
+// Distributes the queries without a listed neighbour, a warp per chunk.  There
+// are few of them (0.1% of a drift site's queries, 1% of a probe's: density
+// peaks), and few candidates have a higher rho than one of them (2%): they are
+// searched one by one -- wide windows by blocks, a part each (sparse[0 ..
+// words[1])), the others by a warp (words[2] of them, from sparse's end).  (A
+// part, because a spike alone among noise has a low rho: nearly every candidate
+// of its window exceeds it.)  A chunk with at least kDense of
+// them and one in eight (a rho of another kind, a search that proved little)
+// has its windows read once for 16 queries: (16-query tile, part) units,
+// {chunk | part << 28, (first << 5) | count}.  all (may be null): a word that,
+// if set, sends every query there.
+__global__ void k_delta_items(irc::PlanDev p, const int *__restrict__ all, const int *__restrict__ counts,
+                              int *__restrict__ fb_list, int *__restrict__ words, int2 *__restrict__ sparse,
+                              int2 *__restrict__ items, unsigned long long *__restrict__ keys)
 {
-    __shared__ int wsum[kThreads / 32];
-    __shared__ int running, base;
-    const int chunk = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int q0 = __ldg(p.q0 + chunk), nq = __ldg(p.nq + chunk), seg = q0 - p.q_base;
-    if (threadIdx.x == 0) running = 0;
-    __syncthreads();
-    for (int start = 0; start < nq; start += kThreads) {
-        const int i = start + threadIdx.x;
-        const int f = i < nq ? fb_flag[seg + i] : 0;
-        const unsigned bal = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wsum[warp] = __popc(bal);
-        __syncthreads();
-        int off = running;
-        for (int w = 0; w < warp; ++w) off += wsum[w];
-        if (f) {
-            fb_list[seg + off + __popc(bal & ((1u << lane) - 1u))] = q0 + i;
-            keys[seg + i] = ~0ull;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) for (int w = 0; w < kThreads / 32; ++w) running += wsum[w];
-        __syncthreads();
+    const int chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (chunk >= p.nChunks) return;
+    const int q0 = __ldg(p.q0 + chunk), nq = __ldg(p.nq + chunk);
+    int *list = fb_list + (q0 - p.q_base);
+    int m = __ldg(counts + chunk);
+    if (all && __ldg(all)) {
+        m = nq;
+        for (int i = lane; i < m; i += 32) list[i] = q0 + i;
+        __syncwarp();
     }
-    const int total = running, ntile = (total + kQB - 1) / kQB;
-    // a long candidate window is split into np parts of at least kMinPart
-    const int np = min(kParts, max(1, __ldg(p.ncand + chunk) / kMinPart)), nunit = ntile * np;
-    if (threadIdx.x == 0) base = nunit ? atomicAdd(n_items, nunit) : 0;
-    __syncthreads();
-    for (int j = threadIdx.x; j < nunit; j += kThreads) {
-        const int t = j / np, part = j - t * np;
-        items[base + j] = make_int2(chunk | (part << 28), ((t * kQB) << 5) | min(kQB, total - t * kQB));
+    if (m == 0) return;
+    const int ncand = __ldg(p.ncand + chunk);
+    int base = 0;
+    if (m >= kDense && m * 8 >= nq) {
+        const int ntile = (m + kQB - 1) / kQB, np = min(kParts, max(1, ncand / kMinPart)), nunit = ntile * np;
+        if (lane == 0) base = atomicAdd(words, nunit);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int j = lane; j < nunit; j += 32) {
+            const int t = j / np, part = j - t * np;
+            items[base + j] = make_int2(chunk | (part << 28), ((t * kQB) << 5) | min(kQB, m - t * kQB));
+        }
+        for (int i = lane; i < m; i += 32) keys[list[i] - p.q_base] = ~0ull;
+    } else {
+        const bool wide = ncand > kWide;
+        if (lane == 0) base = atomicAdd(words + (wide ? 1 : 2), m);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int i = lane; i < m; i += 32)
+            sparse[wide ? base + i : p.n_out - 1 - (base + i)] = make_int2(list[i], chunk);
+        if (wide)
+            for (int i = lane; i < m; i += 32) keys[list[i] - p.q_base] = ~0ull;
     }
 }
 
@@ -360,29 +401,152 @@ __device__ __forceinline__ unsigned long long ref_key(float d2, int bin, int ste
            ((unsigned long long)(dd & 7u) << 20) | (unsigned)step;
 }
 
-// Drift-window fallback for the queued queries, one unit per (16-query tile
-// of a chunk, part of its candidate window; long windows have up to kParts
-// parts of at least kMinPart candidates): a unit loads every candidate of its
-// part once for the 16 queries, keeps per
-// query the candidates whose rho exceeds the query's (the search_delta_drift
-// mask), ties by (d2, index), and folds its best key into the query's key
-// with a 64-bit atomicMin -- the minimum of the same keys in any order, so
-// the split changes no result while giving the SMs kParts times more units
-// (a probe holds ~1,000 fallback tiles per site, too few to fill 152 SMs
-// when each scans a whole ~30K-candidate window).
+// delta and nneigh of query qq of a chunk from the best key of its window (~0:
+// no candidate, i.e. sqrt(SINGLE_INF) .* rho and the query itself, as
+// search_delta_drift_).
+template <bool REF>
+__device__ __forceinline__ void put_delta(const irc::PlanDev &p, const float *__restrict__ R, int chunk, int qq,
+                                          unsigned long long b, int nT, float *__restrict__ delta, int *__restrict__ nneigh)
+{
+    const bool ok = b != ~0ull;
+    float v;
+    int row = qq;
+    if (REF) {
+        v = ok ? __uint_as_float((unsigned)(b >> 33)) : irc::ref_sqrt_abs(kInfSentinel);
+        if (ok) {
+            const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
+            const int bin = (int)(b >> 23) & 1023;
+            row = __ldg(p.rsr + r0 + bin % nBB) + bin / nBB + (int)(b & 0xfffffu) * (nT / nBB);
+        }
+    } else {
+        v = irc::ref_sqrt_abs(ok ? __uint_as_float((unsigned)(b >> 32)) : kInfSentinel);
+        if (ok) row = (int)(b & 0xffffffffu);
+    }
+    const size_t o = (size_t)(qq - p.q_base);
+    delta[o] = __fmul_rn(v, __ldg(R + qq));
+    nneigh[o] = row + 1;
+}
 
+// One query's best key over positions [lo, hi) of its chunk's window, by `nw`
+// warps of which this is the w-th: the warp reads rho of 256 candidates at a
+// time, queues the rows that exceed the query's, and evaluates 32 queued rows
+// at once, copied to shared memory (a lane reading its row from global memory
+// touches 32 cache lines a feature: 240 us for a window of 28,500 such rows).
+// qrow: the warp's copy of the query's features; queue: 288 words; buf: 32 rows.
+template <bool REF>
+__device__ __forceinline__ unsigned long long scan_query(const irc::PlanDev &p, const float *__restrict__ F,
+                                                         const float *__restrict__ R, int nC, int nd, int chunk, int q,
+                                                         int nT, int lo, int hi, int w, int nw, float *qrow, int *queue,
+                                                         float *buf, int lane)
+{
+    constexpr int NL = 8;                                    // rho loads in flight
+    const float rq = __ldg(R + q);
+    const int P = irc::row_pitch(nC);
+    __syncwarp();
+    for (int c = lane; c < nd; c += 32) qrow[c] = __ldg(F + (size_t)q * nC + c);
+    __syncwarp();
+    unsigned long long best = ~0ull;
+    const int rr0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - rr0, step = REF ? nT / nBB : 1;
+    const irc::RowCopy<2> rc(nC, lane, 0);                   // rows 0 .. 31
+    int cnt = 0;
+    auto round = [&](int first, int m) {
+        __syncwarp();
+        const int iB = lane < m ? queue[first + lane] : -1;
+        const int rows[2] = {iB, -1};
+        rc.issue(buf, P, F, nC, rows);
+        irc::copies_commit();
+        irc::copies_wait<0>();
+        __syncwarp();
+        if (lane < m) {
+            const float *fb = buf + lane * P;
+            float acc = 0.0f;
+#pragma unroll 4
+            for (int c = 0; c < nd; ++c) acc = irc::dterm(acc, fb[c], qrow[c]);
+            if (acc > 0.0f && acc < kInfSentinel) {
+                unsigned long long key = dkey(acc, iB);
+                if (REF) {
+                    int a = 0, b = nBB;                      // the row's run (their starts ascend)
+                    while (b - a > 1) {
+                        const int mid = (a + b) >> 1;
+                        if (__ldg(p.rsr + rr0 + mid) <= iB) a = mid; else b = mid;
+                    }
+                    const int j = iB - __ldg(p.rsr + rr0 + a);
+                    key = ref_key(acc, (j % step) * nBB + a, j / step);
+                }
+                best = key < best ? key : best;
+            }
+        }
+        __syncwarp();
+    };
+    int pos = 0;                                             // position of run r's first candidate
+    for (int r = __ldg(p.roff + chunk); r < __ldg(p.roff + chunk + 1) && pos < hi; ++r) {
+        const int rs = __ldg(p.rs + r), rn = __ldg(p.rn + r);
+        const int a = max(lo - pos, 0), b = min(hi - pos, rn);
+        for (int i0 = a + w * 32 * NL; i0 < b; i0 += nw * 32 * NL) {
+            float rb[NL];
+#pragma unroll
+            for (int u = 0; u < NL; ++u) {
+                const int i = i0 + 32 * u + lane;
+                rb[u] = i < b ? __ldg(R + rs + i) : rq;
+            }
+#pragma unroll
+            for (int u = 0; u < NL; ++u) {
+                const bool hit = !(rb[u] <= rq) && i0 + 32 * u + lane < b;        // the search_delta_drift mask
+                const unsigned bal = __ballot_sync(0xffffffffu, hit);
+                if (hit) queue[cnt + __popc(bal & ((1u << lane) - 1u))] = rs + i0 + 32 * u + lane;
+                cnt += __popc(bal);
+            }
+            while (cnt >= 32) round(cnt -= 32, 32);          // the last 32 queued
+        }
+        pos += rn;
+    }
+    if (cnt) round(0, cnt);
+    return irc::warp_min_u64(best);
+}
+
+// The drift-window search of the queries that k_delta_items distributed.  The
+// 16-query units: a unit loads every candidate of its part once for the 16
+// queries, keeps per query the candidates whose rho exceeds the query's, and
+// folds its best key into the query's key with a 64-bit atomicMin -- the
+// minimum of the same keys in any order, so the split changes no result.
+// Before the queries were searched one by one, 16 of a chunk (2.6 on average)
+// shared a pass over all its candidates: 390 us for the 491 queries of a
+// 400,000-spike site.
 template <bool REF>
 __global__ void __launch_bounds__(kThreads)
-k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restrict__ R, int nC,
-              const uint8_t *__restrict__ row_dims, const int *__restrict__ n_items, const int2 *__restrict__ items,
-              const int *__restrict__ fb_list, unsigned long long *__restrict__ keys, int nT)
+k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restrict__ R, int nC,
+               const uint8_t *__restrict__ row_dims, const int *__restrict__ words, const int2 *__restrict__ sparse,
+               const int2 *__restrict__ items, const int *__restrict__ fb_list, unsigned long long *__restrict__ keys,
+               int nT, float *__restrict__ delta, int *__restrict__ nneigh)
 {
     __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
     __shared__ float sRA[kQB];
     __shared__ int sQ[kQB];
-    __shared__ unsigned long long red[kQB][kThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int total = *n_items;
+    __shared__ unsigned long long redt[kQB][kThreads / 32];
+    __shared__ int queues[kThreads / 32][288];
+    extern __shared__ __align__(16) float rows_sm[];         // 32 rows per warp
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kThreads / 32;
+    const int total = words[0], n_wide = words[1], n_narrow = words[2];
+    float *qrow = sA + warp * IRC_NC_MAX;                    // (kQB >= the warps of a block)
+    float *buf = rows_sm + warp * 32 * irc::row_pitch(nC);
+    for (int u = blockIdx.x; u < n_wide * kWideParts; u += gridDim.x) {
+        const int part = u / n_wide;
+        const int2 e = sparse[u - part * n_wide];
+        const int ntot = __ldg(p.ncand + e.y), per = max(kMinPart, (ntot + kWideParts - 1) / kWideParts);
+        if (part * per >= ntot) continue;
+        const int nd = row_dims ? min(nC, (int)__ldg(row_dims + e.x)) : nC;
+        const unsigned long long b = scan_query<REF>(p, F, R, nC, nd, e.y, e.x, nT, part * per, min(ntot, part * per + per),
+                                                     warp, nw, qrow, queues[warp], buf, lane);
+        if (lane == 0 && b != ~0ull) atomicMin(keys + (e.x - p.q_base), b);
+    }
+    for (int w = blockIdx.x * nw + warp; w < n_narrow; w += gridDim.x * nw) {
+        const int2 e = sparse[p.n_out - 1 - w];
+        const int nd = row_dims ? min(nC, (int)__ldg(row_dims + e.x)) : nC;
+        const unsigned long long b = scan_query<REF>(p, F, R, nC, nd, e.y, e.x, nT, 0, INT_MAX, 0, 1, qrow, queues[warp],
+                                                     buf, lane);
+        if (lane == 0) put_delta<REF>(p, R, e.y, e.x, b, nT, delta, nneigh);
+    }
+    __syncthreads();
     for (int u = blockIdx.x; u < total; u += gridDim.x) {
         const int2 item = items[u];
         const int chunk = item.x & 0x0fffffff, part = item.x >> 28, first = item.y >> 5, n = item.y & 31;
@@ -448,51 +612,38 @@ k_delta_tiles(irc::PlanDev p, const float *__restrict__ F, const float *__restri
 #pragma unroll
         for (int q = 0; q < kQB; ++q) {
             const unsigned long long b = irc::warp_min_u64(best[q]);
-            if (lane == 0) red[q][warp] = b;
+            if (lane == 0) redt[q][warp] = b;
         }
         __syncthreads();
         if (threadIdx.x < n) {
-            unsigned long long b = red[threadIdx.x][0];
-            for (int w = 1; w < kThreads / 32; ++w) b = red[threadIdx.x][w] < b ? red[threadIdx.x][w] : b;
+            unsigned long long b = redt[threadIdx.x][0];
+            for (int w = 1; w < kThreads / 32; ++w) b = redt[threadIdx.x][w] < b ? redt[threadIdx.x][w] : b;
             if (b != ~0ull) atomicMin(keys + (sQ[threadIdx.x] - p.q_base), b);
         }
         __syncthreads();
     }
 }
 
-// delta and nneigh of the queued queries from their keys (no candidate:
-// sqrt(SINGLE_INF) .* rho and the query itself, as search_delta_drift_).
+// delta and nneigh of the queries with keys: the wide windows' and the
+// 16-query units'.
 template <bool REF>
-__global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, const int *__restrict__ n_items,
-                               const int2 *__restrict__ items, const int *__restrict__ fb_list,
+__global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, const int *__restrict__ words,
+                               const int2 *__restrict__ sparse, const int2 *__restrict__ items, const int *__restrict__ fb_list,
                                const unsigned long long *__restrict__ keys, float *__restrict__ delta,
                                int *__restrict__ nneigh, int nT)
 {
-    const int total = *n_items * kQB;
+    const int total = words[0] * kQB, n_wide = words[1];
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_wide; t += gridDim.x * blockDim.x) {
+        const int2 e = sparse[t];
+        put_delta<REF>(p, R, e.y, e.x, keys[e.x - p.q_base], nT, delta, nneigh);
+    }
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         const int2 item = items[t / kQB];
         const int j = t - (t / kQB) * kQB;
         const int chunk = item.x & 0x0fffffff, first = item.y >> 5, n = item.y & 31;
         if ((item.x >> 28) != 0 || j >= n) continue;        // each tile once (its part 0)
         const int qq = fb_list[__ldg(p.q0 + chunk) - p.q_base + first + j];
-        const size_t o = (size_t)(qq - p.q_base);
-        const unsigned long long b = keys[o];
-        const bool ok = b != ~0ull;
-        if (REF) {
-            int row = qq;
-            if (ok) {
-                const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
-                const int bin = (int)(b >> 23) & 1023;
-                row = __ldg(p.rsr + r0 + bin % nBB) + bin / nBB + (int)(b & 0xfffffu) * (nT / nBB);
-            }
-            const float v = ok ? __uint_as_float((unsigned)(b >> 33)) : irc::ref_sqrt_abs(kInfSentinel);
-            delta[o] = __fmul_rn(v, __ldg(R + qq));
-            nneigh[o] = row + 1;
-            continue;
-        }
-        const float d2 = ok ? __uint_as_float((unsigned)(b >> 32)) : kInfSentinel;
-        delta[o] = __fmul_rn(irc::ref_sqrt_abs(d2), __ldg(R + qq));
-        nneigh[o] = (ok ? (int)(b & 0xffffffffu) : qq) + 1;
+        put_delta<REF>(p, R, chunk, qq, keys[qq - p.q_base], nT, delta, nneigh);
     }
 }
 
@@ -542,36 +693,58 @@ int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, in
                         const int32_t *miKnn, const float *d2Knn, float *delta, int32_t *nneigh,
                         cudaStream_t s)
 {
-    int *cnt, *la, *lb;
-    int rc = irc_plan_scratch(pl, &cnt, &la, &lb);
-    if (rc != IRC_OK) return rc;
-    // flags in list a, compacted queries in list b, (chunk, tile) items and keys after them
-    irc_delta_scratch sc;
-    sc.n_items = cnt + irc::kScratchItems;
-    const int n = pl->dev.n_out;
-    sc.flags = la;
-    sc.list = lb;
-    sc.items = reinterpret_cast<int2 *>(lb + n);      // (8-byte aligned: the two lists hold 2 n words)
-    sc.keys = reinterpret_cast<unsigned long long *>(sc.items + delta_items(n, pl->dev.nChunks));
-    k_delta_list<<<(n + 255) / 256, 256, 0, s>>>(pl->dev, R, knn, miKnn, d2Knn, delta, nneigh, la);
+    const irc_delta_scratch sc = irc_delta_carve(pl, pl->delta_mem, nullptr);
+    cudaError_t e = irc_delta_clear(pl, sc, s);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: memset");
+    const int tiles = pl->ntiles[irc::tile_slot(kListTile)];
+    k_delta_list<<<(tiles + kListWarps - 1) / kListWarps, 32 * kListWarps, 0, s>>>(
+        pl->dev, tiles, R, knn, miKnn, d2Knn, delta, nneigh, sc.counts, sc.list);
     IRC_CHECK_LAUNCH("irc_site_delta list");
     return irc_delta_window(pl, F, nC, R, 0, sc, delta, nneigh, s);
 }
 
-// The drift-window search of the flagged queries: ties by (d2, row), or by the
-// reference's rule over nT bins (nT > 0).
+// Scratch of the drift-window search in mem (delta_bytes(...)).
+irc_delta_scratch irc_delta_carve(const irc_plan *pl, void *mem, const int *all)
+{
+    const size_t n = (size_t)pl->dev.n_out;
+    char *b = (char *)mem;
+    irc_delta_scratch sc;
+    sc.all = all;
+    sc.words = (int *)b;
+    sc.counts = sc.words + 4;
+    b += delta_part(4 * (4 + (size_t)pl->dev.nChunks));
+    sc.list = (int *)b;
+    b += delta_part(4 * n);
+    sc.sparse = (int2 *)b;
+    b += delta_part(8 * n);
+    sc.keys = (unsigned long long *)b;
+    b += delta_part(8 * n);
+    sc.items = (int2 *)b;
+    return sc;
+}
+
+cudaError_t irc_delta_clear(const irc_plan *pl, const irc_delta_scratch &sc, cudaStream_t s)
+{
+    return cudaMemsetAsync(sc.words, 0, 4 * (4 + (size_t)pl->dev.nChunks), s);
+}
+
+// The drift-window search of the queries in sc.list (sc.counts of every
+// chunk): ties by (d2, row), or by the reference's rule over nT bins (nT > 0).
 int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int nT, const irc_delta_scratch &sc,
                      float *delta, int32_t *nneigh, cudaStream_t s)
 {
-    cudaError_t e = cudaMemsetAsync(sc.n_items, 0, sizeof(int), s);
-    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: memset");
-    k_delta_compact<<<pl->dev.nChunks, kThreads, 0, s>>>(pl->dev, sc.flags, sc.list, sc.n_items, sc.items, sc.keys);
-    IRC_CHECK_LAUNCH("irc_site_delta compact");
-    auto tiles = nT > 0 ? k_delta_tiles<true> : k_delta_tiles<false>;
+    k_delta_items<<<(pl->dev.nChunks + 7) / 8, 256, 0, s>>>(pl->dev, sc.all, sc.counts, sc.list, sc.words, sc.sparse,
+                                                            sc.items, sc.keys);
+    IRC_CHECK_LAUNCH("irc_site_delta items");
+    auto window = nT > 0 ? k_delta_window<true> : k_delta_window<false>;
     auto finish = nT > 0 ? k_delta_finish<true> : k_delta_finish<false>;
-    tiles<<<kQueueBlocks, kThreads, 0, s>>>(pl->dev, F, R, nC, pl->row_dims, sc.n_items, sc.items, sc.list, sc.keys, nT);
-    IRC_CHECK_LAUNCH("irc_site_delta tiles");
-    finish<<<kQueueBlocks, kThreads, 0, s>>>(pl->dev, R, sc.n_items, sc.items, sc.list, sc.keys, delta, nneigh, nT);
+    const size_t smem = (size_t)(kThreads / 32) * 32 * irc::row_pitch(nC) * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(window, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: smem attribute");
+    window<<<kQueueBlocks, kThreads, smem, s>>>(pl->dev, F, R, nC, pl->row_dims, sc.words, sc.sparse, sc.items, sc.list,
+                                             sc.keys, nT, delta, nneigh);
+    IRC_CHECK_LAUNCH("irc_site_delta window");
+    finish<<<kQueueBlocks / 4, kThreads, 0, s>>>(pl->dev, R, sc.words, sc.sparse, sc.items, sc.list, sc.keys, delta, nneigh, nT);
     IRC_CHECK_LAUNCH("irc_site_delta finish");
     return IRC_OK;
 }

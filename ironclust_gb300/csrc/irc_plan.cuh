@@ -4,11 +4,10 @@
 
 namespace irc {
 
-// Plan scratch words: [0] overflow-queue count, [1] delta-fallback count,
-// [2] device error word (a bounded wait gave up), [3] unused; the two query
-// lists of n_out entries follow.
+// Plan scratch words: [0] overflow-queue count, [1] largest magnitude (FP8's
+// scale), [2] device error word (a bounded wait gave up), [3] unused; the two
+// query lists of n_out entries follow.
 constexpr int kScratchErr = 2;
-constexpr int kScratchItems = 3;      // count of delta-fallback (chunk, tile) items
 constexpr int kScratchLists = 4;
 
 // Query-tile sizes for which a plan precomputes its tile tables.
@@ -82,6 +81,7 @@ struct irc_plan {
     irc::PlanDev dev;
     void *dmem;                            // single device allocation behind dev
     int32_t *scratch;                      // inside dmem: 4 words + 2 x n_out query lists
+    void *delta_mem;                       // inside dmem: scratch of the delta search (irc_cert.cuh)
     const irc::TcItem *tc_items;           // tensor-core work items: inside dmem, or tc_items_buf
     int n_tc_items;
     int n_tc_one;                          // items [0, n_tc_one) have one slot, [n_tc_one, n_tc_wide) two

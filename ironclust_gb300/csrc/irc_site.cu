@@ -465,7 +465,14 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     // 1-32 row remainders packed two and four per item (similar tile counts
     // together), all ordered by cost, largest first
     int n_one = 0, n_wide = 0;
-    std::vector<irc::TcItem> items = build_tc_items(q0, nq, moff.data(), mn.data(), nChunks, 4, 0, &n_one, &n_wide);
+    // When all items, unpacked, are at most two a SM, packing saves no turn of
+    // the machine and its classes run one after another: the leftover 32
+    // queries of a 20,000-spike static site, alone in a four-slot launch, took
+    // 285 us after the other 156 items' 237 (together 240).
+    long long unpacked = 0;
+    for (int i = 0; i < nChunks; ++i) unpacked += (nq[i] + 127) / 128;
+    std::vector<irc::TcItem> items = build_tc_items(q0, nq, moff.data(), mn.data(), nChunks, unpacked <= 2 * 152 ? 1 : 4, 0,
+                                                    &n_one, &n_wide);
     while (img.size() % 16) img.push_back(0);
     const size_t off_items = img.size();
     for (const irc::TcItem &it : items) {
@@ -474,14 +481,10 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     }
     cudaGetDevice(&pl->device);
     if (img.size() & 1) img.push_back(0);          // scratch starts 8-byte aligned (int2 items)
-    // 4 words, two query lists of n_out, and the (chunk, tile) items of the
-    // delta fallback: at most n_out/16 + nChunks pairs
-    // counters, two query lists, the delta fallback's (tile, part) units (up to 8 parts per
-    // 16-query tile) and its per-query 64-bit best keys (8-byte aligned: every term before
-    // them is even)
-    const size_t scratch_ints = irc::kScratchLists + 2 * (size_t)n_out + 2 * delta_items(n_out, nChunks) +
-                                2 * (size_t)n_out;
-    cudaError_t e = cudaMalloc(&pl->dmem, (img.size() + scratch_ints) * sizeof(int32_t));
+    // scratch: 4 words and two query lists of n_out, then the delta search's
+    const size_t scratch_ints = irc::kScratchLists + 2 * (size_t)n_out + 64;
+    const size_t delta_at = (img.size() + scratch_ints) / 64 * 64;          // 256-byte aligned
+    cudaError_t e = cudaMalloc(&pl->dmem, delta_at * sizeof(int32_t) + delta_bytes(n_out, nChunks));
     if (e != cudaSuccess) {
         free(pl->h_q0); free(pl->h_nq); free(pl->h_roff); free(pl->h_rs); free(pl->h_rn); free(pl);
         irc_host::cuda_status(e, "irc_plan_create: cudaMalloc");
@@ -503,6 +506,7 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     pl->dev.tc_tiles = reinterpret_cast<const int2 *>(base + off_tiles);
     for (int k = 0; k < irc::kNumTileSizes; ++k) pl->dev.tile_off[k] = base + off_tile[k];
     pl->scratch = (int32_t *)pl->dmem + img.size();
+    pl->delta_mem = (int32_t *)pl->dmem + delta_at;
     pl->tc_items = reinterpret_cast<const irc::TcItem *>((const int32_t *)pl->dmem + off_items);
     pl->n_tc_items = (int)items.size();
     pl->n_tc_one = n_one;
