@@ -60,6 +60,7 @@ constexpr int W_AMAX = 1;                 // bits of max |F|
 constexpr int W_ERR = irc::kScratchErr;   // a wait of the filter gave up
 constexpr int W_TILES = 4;                // tiles left to the plain kernel
 constexpr int W_OVF = 5;                  // its overflow queue
+constexpr int W_TICKET = 6;               // block ticket of the centring
 constexpr size_t kHdrBytes = 256;
 
 // Could a candidate outside a list with threshold tau have an FP32 distance
@@ -395,7 +396,7 @@ int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, si
     cudaError_t e = cudaMemsetAsync(base, 0, kHdrBytes + zero, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(cert, 0xff, (size_t)pl->dev.n_out * sizeof(int2), s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: memset");
-    int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, (unsigned *)words + W_AMAX, &L->op, s);
+    int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, (unsigned *)words + W_AMAX, (unsigned *)words + W_TICKET, &L->op, s);
     if (rc != IRC_OK) return rc;
     irc_tc::ListOut lo = irc_tc::list_area(la, pl->dev.n_out);
     lo.cert = cert;

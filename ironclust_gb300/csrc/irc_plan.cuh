@@ -5,9 +5,11 @@
 namespace irc {
 
 // Plan scratch words: [0] overflow-queue count, [1] largest magnitude (FP8's
-// scale), [2] device error word (a bounded wait gave up), [3] unused; the two
-// query lists of n_out entries follow.
+// scale), [2] device error word (a bounded wait gave up), [3] block ticket of the
+// centring (zero between launches); the two query lists of n_out entries
+// follow.
 constexpr int kScratchErr = 2;
+constexpr int kScratchTicket = 3;
 constexpr int kScratchLists = 4;
 
 // Query-tile sizes for which a plan precomputes its tile tables.

@@ -84,7 +84,7 @@ struct Operands {
     const float *qnorm;          // f16: upper bound of every query's scaled norm, [n_out]
 };
 size_t ops_bytes(const irc_plan *pl, int nC, Fmt fmt);
-int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, Operands *out,
-                  cudaStream_t s);
+int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, unsigned *ticket,
+                  Operands *out, cudaStream_t s);
 
 }  // namespace irc_tc

@@ -23,7 +23,6 @@ namespace {
 
 using irc_tc::Fmt;
 
-// F (f32 [nF x nC]) -> query / candidate BF16 rows of 64.
 // Centring of the tensor-core operands.  Distances do not change when every
 // feature vector is shifted by the same reference point, but the rounding
 // error of the BF16 / FP8 contraction grows with the operands' magnitude, and
@@ -32,53 +31,77 @@ using irc_tc::Fmt;
 // 64K of the plan's query rows (fixed summation order, so the rows are the
 // same on every call); the exact re-rank keeps reading the unshifted
 // features.
-constexpr int kMeanBlocks = 256;
+//
+// One launch: every block sums its rows (a thread per (row, column), so that a
+// block reads whole consecutive rows), and the block that ends last adds the
+// partial sums -- with all of its threads: one thread per column adding 256
+// partials in a kernel of its own took 25 us of every call, the sums before it
+// 4 to 12.  Latency-bound: 9 us for 3,000 rows, 24 for 65,536 rows out of 400,000.
+constexpr int kMeanBlocks = 152, kMeanThreads = 512;
 
-// FINITE: values that are not finite are left out of the sums (f16 operands:
-// one such spike must not spoil the centre and with it every proof).
-template <bool FINITE>
-__global__ void k_colsum_part(const float *__restrict__ F, int nC, int stride, int nS, float *__restrict__ part)
+// F16: values that are not finite are left out of the sums (one such spike must
+// not spoil the centre and with it every proof), and *scale becomes the power
+// of two that brings every finite |F - ref| to at most 8, from the finite |F|
+// maximum and the largest |ref| (their sum bounds the differences; what the
+// bound loses, a factor of two at most, only costs half-precision subnormals).
+// 0 when features reach 2^62, whose squared distances leave FP32's range:
+// nothing is proven with it.  ticket: zero, and zero again at the end.
+template <bool F16>
+__global__ void __launch_bounds__(kMeanThreads)
+k_centre(const float *__restrict__ F, int nC, int stride, int nS, float *__restrict__ part, unsigned *__restrict__ ticket,
+         float *__restrict__ ref, const unsigned *__restrict__ amax, float *__restrict__ scale)
 {
-    __shared__ float red[4][64];
-    const int c = threadIdx.x & 63, lane_r = threadIdx.x >> 6;   // 64 columns x 4 row lanes
+    __shared__ double red[kMeanThreads];
+    __shared__ bool last;
+    const int t = threadIdx.x, lanes = kMeanThreads / nC, rl = t / nC, c = t - rl * nC;
     const int per = (nS + gridDim.x - 1) / gridDim.x;
     const int k0 = blockIdx.x * per, k1 = min(nS, k0 + per);
     float acc = 0.0f;
-    if (c < nC)
-        for (int k = k0 + lane_r; k < k1; k += 4) {
+    if (rl < lanes) {
+#pragma unroll 8
+        for (int k = k0 + rl; k < k1; k += lanes) {
             const float v = __ldg(F + (size_t)k * stride * nC + c);
-            if (!FINITE || isfinite(v)) acc += v;
+            if (!F16 || isfinite(v)) acc += v;
         }
-    red[lane_r][c] = acc;
+    }
+    float *redf = reinterpret_cast<float *>(red);
+    redf[t] = acc;
     __syncthreads();
-    if (threadIdx.x < 64)
-        part[(size_t)blockIdx.x * 64 + c] = ((red[0][c] + red[1][c]) + red[2][c]) + red[3][c];
-}
-
-__global__ void k_colsum_final(const float *__restrict__ part, int nb, int nC, int nS, float *__restrict__ ref)
-{
-    const int c = threadIdx.x;
-    if (c >= nC) return;
-    double acc = 0.0;
-    for (int b = 0; b < nb; ++b) acc += (double)part[(size_t)b * 64 + c];
-    ref[c] = nS > 0 ? (float)(acc / (double)nS) : 0.0f;
-}
-
-// The power of two that brings every finite |F - ref| to at most 8, from the
-// finite |F| maximum and the largest |ref| (their sum bounds the differences;
-// what the bound loses, a factor of two at most, only costs half-precision
-// subnormals).  0 when features reach 2^62, whose squared distances leave
-// FP32's range: nothing is proven with it.
-__global__ void k_scale(const unsigned *__restrict__ amax, const float *__restrict__ ref, int nC,
-                        float *__restrict__ scale)
-{
-    float m = 0.0f;
-    for (int c = threadIdx.x; c < nC; c += 32) m = fmaxf(m, fabsf(ref[c]));
+    if (t < nC) {
+        float sum = 0.0f;
+#pragma unroll 4
+        for (int r = 0; r < lanes; ++r) sum += redf[r * nC + t];
+        part[(size_t)blockIdx.x * 64 + t] = sum;
+        __threadfence();
+    }
+    __syncthreads();
+    if (t == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double sum = 0.0;
+    if (rl < lanes) {
+#pragma unroll 4
+        for (int b = rl; b < gridDim.x; b += lanes) sum += (double)__ldcg(part + (size_t)b * 64 + c);
+    }
+    red[t] = sum;
+    __syncthreads();
+    if (t < nC) {
+        for (int r = 1; r < lanes; ++r) sum += red[r * nC + t];
+        ref[t] = nS > 0 ? (float)(sum / (double)nS) : 0.0f;
+    }
+    if (F16) {
+        __syncthreads();
+        if (t < 32) {
+            float m = 0.0f;
+            for (int k = t; k < nC; k += 32) m = fmaxf(m, fabsf(ref[k]));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) {
-        const float b = __uint_as_float(*amax) + m;
-        *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if (t == 0) {
+                const float b = __uint_as_float(*amax) + m;
+                *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
+            }
+        }
     }
 }
 
@@ -136,7 +159,10 @@ __device__ __forceinline__ int piece_exp(int t) { return t < 5 ? 8 - 4 * t : -9;
 // (BF16: above the file; FP8: above) and stages them in shared memory in
 // 16-byte pieces XOR-swizzled by row; the warp then writes its 32 rows of
 // every output -- the re-rank's FP32 rows padded to Dp4 float4 too -- with
-// contiguous stores.
+// contiguous stores.  Bound by the memory it writes once the instructions are
+// few and a warp's rows are all in flight at once: 52 us for 400,000 rows of
+// 33 features (220 MB).  With element counters by division, four loads in flight
+// and every operand element through the general form it took 79.
 constexpr int kPrepWarps = 4;
 
 size_t prep_smem(int nC)
@@ -155,6 +181,18 @@ template <Fmt FMT>
 __device__ __forceinline__ float val16(unsigned short v)
 {
     return FMT == Fmt::f16 ? __half2float(__ushort_as_half(v)) : __bfloat162float(__ushort_as_bfloat16(v));
+}
+
+__device__ __forceinline__ void copy_word(float *shared, const float *global)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(shared)), "l"(global)
+                 : "memory");
+}
+
+// 16-bit element `at` of a row that is otherwise written in 16-byte pieces.
+__device__ __forceinline__ void st_shared_u16(uint4 *row, int at, unsigned short v)
+{
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(row) + 2u * at), "h"(v) : "memory");
 }
 
 // qnorm (f16): an upper bound of every query's scaled norm |s (a - ref)|: the
@@ -179,16 +217,18 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
     if (r0 >= (long long)lo + n) return;
     const int nr = (int)min(32LL, (long long)lo + n - r0);
     const float *src = F + (size_t)r0 * nC;
-    for (int t = lane; t < nr * nC; t += 32) {
-        const int r = t / nC;
-        w[r * nCs + (t - r * nC)] = __ldg(src + t);
+    // (4-byte copies: the rows start on any word; all of them in flight at once)
+    for (int c = lane; c < nC; c += 32) {
+#pragma unroll 8
+        for (int r = 0; r < nr; ++r) copy_word(w + r * nCs + c, src + r * nC + c);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     const int W = 4 * Dp4;
     float *dst = Fp + (size_t)r0 * W;
-    for (int t = lane; t < nr * W; t += 32) {
-        const int r = t / W, c = t - r * W;
-        dst[t] = c < nC ? w[r * nCs + c] : 0.0f;
+    for (int c = lane; c < W; c += 32) {
+#pragma unroll 8
+        for (int r = 0; r < nr; ++r) dst[r * W + c] = c < nC ? w[r * nCs + c] : 0.0f;
     }
     if (lane < nr) {
         const float *a = w + lane * nCs;
@@ -197,39 +237,38 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
         if (FMT != Fmt::fp8) {
             const float s16 = FMT == Fmt::f16 ? *scale : 1.0f;         // a power of two: exact
             float na = 0.0f;
-            for (int k = 0; k < nC; ++k) {
-                const float f = val16<FMT>(op16<FMT>((a[k] - sref[k]) * s16));
-                na = __fmaf_rn(f, f, na);
-            }
-            const unsigned short h = op16<FMT>(na);
-            const float rem1 = na - val16<FMT>(h);
-            const unsigned short m = op16<FMT>(rem1);
-            const unsigned short l = op16<FMT>(rem1 - val16<FMT>(m));
-            const unsigned short one = op16<FMT>(1.0f), zero = 0;
 #pragma unroll 1
             for (int j = 0; j < irc_tc::KP / 8; ++j) {
                 __align__(16) unsigned short wq[8], wc[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const int k = j * 8 + e;
-                    unsigned short vq = zero, vc = zero;
+                    wq[e] = wc[e] = 0;
                     if (k < nC) {
-                        vc = op16<FMT>((a[k] - sref[k]) * s16);
-                        vq = op16<FMT>(-2.0f * val16<FMT>(vc));
-                    } else if (k < nC + 3) {
-                        vq = (k == nC) ? h : (k == nC + 1) ? m : l;
-                        vc = one;
-                    } else if (k < nC + 6) {
-                        vq = one;
-                        vc = (k == nC + 3) ? h : (k == nC + 4) ? m : l;
-                    } else if (k < nC + 9) {
-                        vc = one;                  // against the query's pass-2 threshold terms
+                        wc[e] = op16<FMT>((a[k] - sref[k]) * s16);
+                        const float f = val16<FMT>(wc[e]);
+                        na = __fmaf_rn(f, f, na);
+                        wq[e] = op16<FMT>(-2.0f * f);
                     }
-                    wq[e] = vq;
-                    wc[e] = vc;
                 }
                 oq[j ^ sw] = *reinterpret_cast<uint4 *>(wq);
                 oc[j ^ sw] = *reinterpret_cast<uint4 *>(wc);
+            }
+            // the 9 elements behind the features (nC + 9 may pass the row's
+            // end, where only the zeros of the query row are missing)
+            const unsigned short h = op16<FMT>(na);
+            const float rem1 = na - val16<FMT>(h);
+            const unsigned short m = op16<FMT>(rem1);
+            const unsigned short l = op16<FMT>(rem1 - val16<FMT>(m));
+            const unsigned short one = op16<FMT>(1.0f);
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+                const int k = nC + i;
+                if (k >= irc_tc::KP) break;
+                const int at = ((k >> 3) ^ sw) * 8 + (k & 7);
+                const unsigned short n3 = i % 3 == 0 ? h : i % 3 == 1 ? m : l;
+                if (i < 6) st_shared_u16(oq, at, i < 3 ? n3 : one);
+                st_shared_u16(oc, at, i >= 3 && i < 6 ? n3 : one);
             }
             const long long row = r0 + lane;
             if (FMT == Fmt::f16 && row >= q_lo && row < q_hi)
@@ -351,8 +390,8 @@ size_t ops_bytes(const irc_plan *pl, int nC, Fmt fmt)
     return 2 * (size_t)pl->dev.nF * 128 + fp_bytes(pl, nC) + kPartBytes + 256 + q;
 }
 
-int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, Operands *out,
-                  cudaStream_t s)
+int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, unsigned *ticket,
+                  Operands *out, cudaStream_t s)
 {
     const bool fp8 = fmt == Fmt::fp8, f16 = fmt == Fmt::f16;
     const int nF = pl->dev.nF, Dp4 = fp_row4(nC);
@@ -365,22 +404,22 @@ int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsi
     const int nQ = pl->dev.n_out;                                     // the query rows q_base ..
     const int stride = nQ > 65536 ? (nQ + 65535) / 65536 : 1;
     const int nS = (nQ + stride - 1) / stride;                        // sampled: q_base + k * stride
-    (f16 ? k_colsum_part<true> : k_colsum_part<false>)<<<kMeanBlocks, 256, 0, s>>>(F + (size_t)pl->dev.q_base * nC, nC,
-                                                                                   stride, nS, part);
-    k_colsum_final<<<1, 64, 0, s>>>(part, kMeanBlocks, nC, nS, ref);
-    IRC_CHECK_LAUNCH("irc_site_knn(tensor core) centre");
-    // operand rows for the rows the plan reads (its row intervals)
-    if (fp8 || f16) {
-        cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned), s);
-        if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): memset");
+    const float *Fq0 = F + (size_t)pl->dev.q_base * nC;
+    if (f16) {                                                        // (its scale takes the maximum)
         for (int v = 0; v < pl->n_row_iv; ++v) {
             const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
-            if (fp8) k_absmax<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
-            else k_absmax_finite<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, amax);
+            k_absmax_finite<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, amax);
         }
-        if (f16) k_scale<<<1, 32, 0, s>>>(amax, ref, nC, scale);
-        IRC_CHECK_LAUNCH("irc_site_knn(tensor core) absmax");
+        k_centre<true><<<kMeanBlocks, kMeanThreads, 0, s>>>(Fq0, nC, stride, nS, part, ticket, ref, amax, scale);
+    } else {
+        k_centre<false><<<kMeanBlocks, kMeanThreads, 0, s>>>(Fq0, nC, stride, nS, part, ticket, ref, nullptr, nullptr);
+        for (int v = 0; fp8 && v < pl->n_row_iv; ++v) {
+            const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
+            k_absmax<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
+        }
     }
+    IRC_CHECK_LAUNCH("irc_site_knn(tensor core) centre");
+    // operand rows for the rows the plan reads (its row intervals)
     const size_t psm = prep_smem(nC);
     auto prep = fp8 ? k_prep<Fmt::fp8> : f16 ? k_prep<Fmt::f16> : k_prep<Fmt::bf16>;
     cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
@@ -419,11 +458,12 @@ int irc_site_knn_tc(irc_plan *pl, const float *F, int nC, int knn, int mode, flo
     int rc = irc_plan_tc_buffer(pl, ops + irc_tc::list_area_bytes(pl->dev.n_out), &buf);
     if (rc != IRC_OK) return rc;
     const irc_tc::ListOut lo = irc_tc::list_area((char *)buf + ops, pl->dev.n_out);
-    cudaError_t e = cudaMemsetAsync(pl->scratch, 0, sizeof(int), s);       // overflow-queue count
+    cudaError_t e = cudaMemsetAsync(pl->scratch, 0, 2 * sizeof(int), s);   // overflow-queue count, largest magnitude
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(BF16): memset");
     irc_tc::Operands op;
-    unsigned *amax = reinterpret_cast<unsigned *>(pl->scratch + 1);       // free word of the plan scratch
-    if ((rc = irc_tc::make_operands(fmt, pl, F, nC, buf, amax, &op, s)) != IRC_OK) return rc;
+    unsigned *words = reinterpret_cast<unsigned *>(pl->scratch);
+    rc = irc_tc::make_operands(fmt, pl, F, nC, buf, words + 1, words + irc::kScratchTicket, &op, s);
+    if (rc != IRC_OK) return rc;
     rc = irc_tc::launch_knn_tc(fmt, op.mq, op.mc, pl, F, op.fp, nC, knn, vrKnn, rho, miKnn, d2Knn, lo, s);
     if (rc != IRC_OK) return rc;
     return irc_exact_overflow_drain(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, s);
