@@ -53,7 +53,7 @@ using irc_tc::Fmt;
 
 constexpr int kWarps = 8;                 // queries per block of the list kernels
 constexpr int kTile = 16;                 // queries per tile of the plain kernels
-constexpr int kRefKeys = 60;              // REF: list entries selected (shared bins take places; ws holds 64)
+constexpr int kRefKeys = 52;              // REF: list entries used (of 64 places; left-over bins take the others)
 
 // Counter words of a call's working memory (zeroed before it).
 constexpr int W_AMAX = 1;                 // bits of max |F|
@@ -125,7 +125,7 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
     unsigned long long kv[PER];
     irc_rr::list_keys<PER>(list, cL, c.Fp, irc_tc::fp_row4(c.nC), q, qs, nd, lane, kv);
     unsigned tb;
-    const int n = irc_rr::select_keys<PER>(kv, REF ? kRefKeys : knn, ws, lane, tb);
+    int n = irc_rr::select_keys<PER>(kv, REF ? kRefKeys : knn, ws, lane, tb);
     const float x = __ldg(c.qnorm + o), s = __ldg(c.scale);
     if (n < knn || n > WARP_KEYS || !(s > 0.0f)) return false;
     if (!REF) {
@@ -133,6 +133,10 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
         if (!complete && may_miss(D, tau, s, x)) return false;
         if (lane < knn) irc_rr::emit(lane, ws[lane], q, knn, (size_t)o, miKnn, d2Knn, vrKnn, rho);
         return true;
+    }
+    if (n > kRefKeys) {
+        tb = (unsigned)(ws[kRefKeys] >> 32);
+        n = kRefKeys;
     }
     // REF: the first candidate of every bin in (d2, row) order is the bin's
     // minimum; the bins' values sqrt(d2) in (value, bin) order are MATLAB's
@@ -198,7 +202,7 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
     const unsigned long long kth = __shfl_sync(0xffffffffu, ((knn - 1) & 1) ? k2[1] : k2[0], (knn - 1) >> 1);
     const float v = __uint_as_float((unsigned)(kth >> 32));
     // every candidate left out must have a larger square root than the knn-th
-    // value: the listed ones beyond ws (d2 > tb) and the unlisted ones
+    // value: the listed ones not used (d2 >= tb) and the unlisted ones
     if (tb < 0x7f800000u && !(__fsqrt_rn(__uint_as_float(tb)) > v)) return false;
     if (!complete && may_miss(__fmul_rn(v, v) * (1.0f + 1e-6f), tau, s, x)) return false;
 #pragma unroll
@@ -214,11 +218,11 @@ __device__ __forceinline__ bool from_list(const Call &c, const uint32_t *list, i
 }
 
 template <bool REF>
-__global__ void __launch_bounds__(32 * kWarps, 4)
+__global__ void __launch_bounds__(32 * kWarps, 5)
 k_cert_knn(Call c, int knn, int nT, float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
            float *__restrict__ d2Knn)
 {
-    __shared__ unsigned long long wkeys[kWarps * WARP_KEYS];
+    __shared__ __align__(16) unsigned long long wkeys[kWarps * WARP_KEYS];
     __shared__ float4 qrows[kWarps * QROW4];
     __shared__ unsigned wbits[REF ? kWarps * 32 : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -271,7 +275,10 @@ k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ de
         for (int e = lane; e < cL; e += 32) {
             const int idx = (int)__ldg(list + e);
             if (__ldg(R + idx) <= rq) continue;
-            const float d2 = irc_rr::row_dist2(c.Fp, Dp4, idx, qs, nd);
+            const int row[1] = {idx};
+            float acc[1];
+            irc_rr::row_dists<1>(c.Fp, Dp4, row, qs, nd, acc);
+            const float d2 = acc[0];
             if (!(d2 > 0.0f) || !(d2 < IRC_SINGLE_INF_F)) continue;
             const unsigned v = __float_as_uint(irc::ref_sqrt_abs(d2));
             if (v > bv) continue;

@@ -74,32 +74,45 @@ __device__ __forceinline__ void emit(int e, unsigned long long key, int q, int k
     }
 }
 
-// FP32 squared distance of row idx to the staged query row, reference
-// arithmetic, the first nd features.
-__device__ __forceinline__ float row_dist2(const float4 *__restrict__ Fp, int Dp4, int idx, const float4 *qs, int nd)
+// FP32 squared distances of NR rows to the staged query row, reference
+// arithmetic, the first nd features.  (Two rows at a time share the query's
+// shared-memory reads and keep twice the gathers in flight.)
+template <int NR>
+__device__ __forceinline__ void row_dists(const float4 *__restrict__ Fp, int Dp4, const int (&idx)[NR], const float4 *qs,
+                                          int nd, float (&acc)[NR])
 {
-                const float *bs = reinterpret_cast<const float *>(Fp + (size_t)idx * Dp4);
-                float acc = 0.0f;
-                const int full = nd >> 3, tail = nd & 7;   // whole groups of 8 features, then the rest
+    const float *bs[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        bs[r] = reinterpret_cast<const float *>(Fp + (size_t)idx[r] * Dp4);
+        acc[r] = 0.0f;
+    }
+    const int full = nd >> 3, tail = nd & 7;       // whole groups of 8 features, then the rest
 #pragma unroll 2
-                for (int c8 = 0; c8 < full; ++c8) {
-                    float bv[8];
-                    ld_nc_v8(bs + 8 * c8, bv);
-                    const float4 a0 = qs[2 * c8], a1 = qs[2 * c8 + 1];
-                    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    for (int c8 = 0; c8 < full; ++c8) {
+        float bv[NR][8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) acc = irc::dterm(acc, bv[u], av[u]);
-                }
-                if (tail) {
-                    float bv[8];
-                    ld_nc_v8(bs + 8 * full, bv);
-                    const float4 a0 = qs[2 * full], a1 = qs[2 * full + 1];
-                    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        for (int r = 0; r < NR; ++r) ld_nc_v8(bs[r] + 8 * c8, bv[r]);
+        const float4 a0 = qs[2 * c8], a1 = qs[2 * c8 + 1];
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (u < tail) acc = irc::dterm(acc, bv[u], av[u]);
-                }
-    return acc;
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int r = 0; r < NR; ++r) acc[r] = irc::dterm(acc[r], bv[r][u], av[u]);
+    }
+    if (tail) {
+        float bv[NR][8];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) ld_nc_v8(bs[r] + 8 * full, bv[r]);
+        const float4 a0 = qs[2 * full], a1 = qs[2 * full + 1];
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (u < tail) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r) acc[r] = irc::dterm(acc[r], bv[r][u], av[u]);
+            }
+    }
 }
 
 // Exact FP32 squared distances of the cL listed candidates of query q
@@ -123,16 +136,76 @@ __device__ __forceinline__ void list_keys(const uint32_t *__restrict__ list, int
     for (int i = 0; i < PER; ++i) kv[i] = ~0ull;
     __syncwarp();
 #pragma unroll
-    for (int bi = 0; bi < PER; ++bi) {
+    for (int bi = 0; bi < PER; bi += 2) {
         if (bi >= nbatch) break;
-        const int e = bi * 32 + lane;
-        if (e < cL) {
-            const int idx = (int)__ldg(list + e);
-            const float acc = row_dist2(Fp, Dp4, idx, qs, nd);
-            if (acc > 0.0f && acc < IRC_SINGLE_INF_F)
-                kv[bi] = ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned)idx;
+        int idx[2];                                   // (past the end: the query itself, at distance 0)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int e = (bi + r) * 32 + lane;
+            idx[r] = e < cL ? (int)__ldg(list + e) : q;
         }
+        float acc[2];
+        row_dists<2>(Fp, Dp4, idx, qs, nd, acc);
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            if (acc[r] > 0.0f && acc[r] < IRC_SINGLE_INF_F)
+                kv[bi + r] = ((unsigned long long)__float_as_uint(acc[r]) << 32) | (unsigned)idx[r];
     }
+}
+
+// Ascending bitonic sort of 64 32-bit keys, element 2 lane + i in v[i]; a
+// comparison is one shuffle and one minimum or maximum.
+__device__ __forceinline__ void warp_bitonic64(unsigned (&v)[2], int lane)
+{
+#pragma unroll
+    for (int size = 2; size <= 64; size <<= 1) {
+        const bool up = (2 * lane & size) == 0;
+#pragma unroll
+        for (int stride = size >> 1; stride > 1; stride >>= 1) {
+            const bool keep_min = ((2 * lane & stride) == 0) == up;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const unsigned o = __shfl_xor_sync(0xffffffffu, v[i], stride >> 1);
+                v[i] = keep_min ? min(v[i], o) : max(v[i], o);
+            }
+        }
+        const unsigned a = min(v[0], v[1]), b = max(v[0], v[1]);
+        v[0] = up ? a : b;
+        v[1] = up ? b : a;
+    }
+}
+
+// ws[0 .. 64) <- the keys of lists of at most 64 entries, all of them, ascending
+// and ~0 behind them; false (ws untouched) if the short keys cannot order
+// them.  A short key is the distance bits above the smallest one's (26 bits: d2
+// within a factor of 256, whatever the scale) and the entry (6 bits), so equal
+// distances are not ordered by it.  Sorting 64 short keys costs less than
+// finding the knn-th distance, compacting and sorting half as many 64-bit keys
+// (re-rank of 3,600 chunks' 625,000 queries 884 us so, 1,060 instructions a
+// query).
+__device__ __forceinline__ bool sort_short(const unsigned long long (&kv)[2], unsigned lo, unsigned hi,
+                                           unsigned long long *ws, int lane)
+{
+    if (lo > hi || hi - lo >= (1u << 26) - 1u) return false;       // (uniform)
+    unsigned v[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        v[i] = kv[i] == ~0ull ? ~0u : ((unsigned)(kv[i] >> 32) - lo) << 6 | (unsigned)(i * 32 + lane);
+    warp_bitonic64(v, lane);
+    const unsigned next = __shfl_down_sync(0xffffffffu, v[0], 1);
+    const bool tie = (v[0] >> 6 == v[1] >> 6 && v[1] != ~0u) || (lane < 31 && v[1] >> 6 == next >> 6 && next != ~0u);
+    if (__any_sync(0xffffffffu, tie)) return false;
+    unsigned long long out[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const unsigned i0 = __shfl_sync(0xffffffffu, (unsigned)kv[0], v[i] & 31u);
+        const unsigned i1 = __shfl_sync(0xffffffffu, (unsigned)kv[1], v[i] & 31u);
+        out[i] = v[i] == ~0u ? ~0ull : (unsigned long long)(lo + (v[i] >> 6)) << 32 | ((v[i] & 32u) ? i1 : i0);
+    }
+    __syncwarp();
+    *reinterpret_cast<ulonglong2 *>(ws + 2 * lane) = make_ulonglong2(out[0], out[1]);
+    __syncwarp();
+    return true;
 }
 
 // ws[0 .. n) <- the keys with distance bits <= tb, ascending, the rest of ws
@@ -140,7 +213,8 @@ __device__ __forceinline__ void list_keys(const uint32_t *__restrict__ list, int
 // search (stopped at TAU_LOW_BIT, rounded up), plus 2^-16 relative, so that
 // the FP64 band of the tensor-core forms lies inside it; +inf when there are
 // fewer than k keys.  The keys are a prefix of the full sort.  When more than
-// WARP_KEYS pass, ws is not usable.
+// WARP_KEYS pass, ws is not usable.  Lists of at most 64 entries are sorted
+// whole where sort_short can.
 template <int PER>
 __device__ __forceinline__ int select_keys(const unsigned long long (&kv)[PER], int k, unsigned long long *ws, int lane,
                                            unsigned &tb)
@@ -157,6 +231,12 @@ __device__ __forceinline__ int select_keys(const unsigned long long (&kv)[PER], 
         }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
+    if constexpr (PER == 2) {
+        if (sort_short(kv, lo, hi, ws, lane)) {
+            tb = 0x7f800000u;
+            return __popc(__ballot_sync(0xffffffffu, kv[0] != ~0ull)) + __popc(__ballot_sync(0xffffffffu, kv[1] != ~0ull));
+        }
+    }
     unsigned ans = 0;
     int top = 30;
     if (lo <= hi) {                               // some key: distances are below 2^31 as bit patterns
@@ -185,7 +265,7 @@ __device__ __forceinline__ int select_keys(const unsigned long long (&kv)[PER], 
         n += __popc(bal);
     }
     __syncwarp();
-    if (n <= 32) {                                // the common case: ~k keys, one per lane
+    if (n <= 32) {                                // ~k keys, one per lane
         unsigned long long v1[1] = {lane < n ? ws[lane] : ~0ull};
         __syncwarp();
         warp_bitonic<unsigned long long, 1>(v1, lane);

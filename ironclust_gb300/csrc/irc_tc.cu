@@ -1040,14 +1040,18 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
 // block's warps); queries without a list (qinfo.x < 0) belong to the exact
 // fallback or to no chunk.
 constexpr int RR_WARPS = 8;
+// Bound by L1's data pipe (a gathered 32-byte sector is about a pass through
+// it) and the latency of the gathers: 5 blocks a SM with a spilled register
+// measure 633 us for 400,000 queries of 61 entries of 33 features and 797 for
+// 3,600 chunks' 625,000, 4 without 665 and 844.
 
-__global__ void __launch_bounds__(32 * RR_WARPS, 4)
+__global__ void __launch_bounds__(32 * RR_WARPS, 5)
 k_rerank(const int2 *__restrict__ qinfo, const uint32_t *__restrict__ lists, int n_out, int q_base,
          const float *__restrict__ F, const float4 *__restrict__ Fp, int nC, const uint8_t *__restrict__ row_dims,
          int knn, float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
          float *__restrict__ d2Knn, int margin, int *__restrict__ scratch)
 {
-    __shared__ unsigned long long wkeys[RR_WARPS * WARP_KEYS];
+    __shared__ __align__(16) unsigned long long wkeys[RR_WARPS * WARP_KEYS];
     __shared__ float4 qrows[RR_WARPS * QROW4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int o = blockIdx.x * RR_WARPS + warp;
