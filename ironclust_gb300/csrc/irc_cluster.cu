@@ -486,7 +486,7 @@ struct Scratch {
     T *get(size_t n)
     {
         void *q = nullptr;
-        if (err == cudaSuccess) err = cudaMallocAsync(&q, sizeof(T) * (n ? n : 1), s);
+        if (err == cudaSuccess) err = irc_scratch_alloc(&q, sizeof(T) * (n ? n : 1), s);
         if (err != cudaSuccess) return nullptr;
         ptrs.push_back(q);
         return (T *)q;
@@ -585,17 +585,16 @@ extern "C" int irc_assign_cluster_knn(int32_t *viClu, int64_t *icl, int32_t *vnS
     // hdr: [0] error bits, [1] stop test of a cell2map_ repeat, [2] unassigned count, [3] state buffer
     int *hdr = sc.get<int>(4);
     const int nb = (int)((n + CTILE - 1) / CTILE);
-    int *bcount = sc.get<int>(nb), *boff = sc.get<int>(nb);
+    int *bcount = sc.get<int>(nb + 1), *boff = sc.get<int>(nb + 1);
     IRC_TRY(sc.err, "irc_assign_cluster_knn: scratch");
     IRC_TRY(cudaMemsetAsync(hdr, 0, 4 * sizeof(int), s), "irc_assign_cluster_knn");
 
     // viSpk_peak = find(vrDelta_spk(:) >= delta_cut)
     k_peak_count<<<nb, TPB, 0, s>>>(delta, n, delta_cut, bcount);
-    IRC_TRY(exclusive_sum(sc, bcount, boff, nb), "irc_assign_cluster_knn: scan");
-    int tail[2] = {0, 0};
-    IRC_TRY(read_back(&tail[0], boff + nb - 1, 1, s), "irc_assign_cluster_knn: peak count");
-    IRC_TRY(read_back(&tail[1], bcount + nb - 1, 1, s), "irc_assign_cluster_knn: peak count");
-    const int P = tail[0] + tail[1];
+    IRC_TRY(cudaMemsetAsync(bcount + nb, 0, sizeof(int), s), "irc_assign_cluster_knn");
+    IRC_TRY(exclusive_sum(sc, bcount, boff, nb + 1), "irc_assign_cluster_knn: scan");
+    int P = 0;
+    IRC_TRY(read_back(&P, boff + nb, 1, s), "irc_assign_cluster_knn: peak count");
     counts[0] = 0;
     counts[1] = P;
     counts[2] = 0;

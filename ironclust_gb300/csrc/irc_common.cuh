@@ -71,3 +71,8 @@ int check_plan(const char *who, const int32_t *q0, const int32_t *nq, const int3
         cudaError_t _e = cudaGetLastError();                                        \
         if (_e != cudaSuccess) return irc_host::cuda_status(_e, where);             \
     } while (0)
+
+// Stream-ordered scratch (irc_pool.cu), freed with cudaFreeAsync; a plan
+// created (+1) or destroyed (-1) on a device.
+cudaError_t irc_scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+void irc_scratch_plan(int dev, int change);

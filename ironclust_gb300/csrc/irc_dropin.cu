@@ -879,7 +879,7 @@ int launch_knn_bins(const char *name, float *K, int32_t *I, const float *B, cons
     if (e != cudaSuccess) return irc_host::cuda_status(e, name);
     int *bad = nullptr;
     if (IND) {
-        e = cudaMallocAsync(&bad, sizeof(int), s);
+        e = irc_scratch_alloc((void **)&bad, sizeof(int), s);
         if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), s);
         if (e != cudaSuccess) return irc_host::cuda_status(e, name);
     }

@@ -194,8 +194,8 @@ extern "C" int irc_fet_load_site(float *F, int *nC_out, const char *const *files
     if (nOut == 0 || nC == 0) return IRC_OK;
     char *rec = nullptr;
     int *dev = nullptr;                                // [0] bad flag, [1..] pcIdx
-    cudaError_t e = cudaMallocAsync((void **)&rec, (size_t)(nRec > 0 ? nRec : 1) * recBytes, s);
-    if (e == cudaSuccess) e = cudaMallocAsync((void **)&dev, sizeof(int) * (size_t)(nC + 1), s);
+    cudaError_t e = irc_scratch_alloc((void **)&rec, (size_t)(nRec > 0 ? nRec : 1) * recBytes, s);
+    if (e == cudaSuccess) e = irc_scratch_alloc((void **)&dev, sizeof(int) * (size_t)(nC + 1), s);
     if (e != cudaSuccess) {
         if (rec) cudaFreeAsync(rec, s);
         return irc_host::cuda_status(e, name);
@@ -263,8 +263,8 @@ extern "C" int irc_knn_save_site(const char *path, int append, const int32_t *mi
     if (n == 0) return IRC_OK;
     int64_t *out = nullptr;
     int *bad = nullptr;
-    cudaError_t e = cudaMallocAsync((void **)&out, sizeof(int64_t) * (size_t)(n * knnOut), s);
-    if (e == cudaSuccess) e = cudaMallocAsync((void **)&bad, sizeof(int), s);
+    cudaError_t e = irc_scratch_alloc((void **)&out, sizeof(int64_t) * (size_t)(n * knnOut), s);
+    if (e == cudaSuccess) e = irc_scratch_alloc((void **)&bad, sizeof(int), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), s);
     if (e != cudaSuccess) {
         if (out) cudaFreeAsync(out, s);
@@ -309,7 +309,7 @@ extern "C" int irc_sort_save(const char *path, const float *rho, const float *de
     }
     if (nSpk == 0) return IRC_OK;
     double *ord = nullptr;
-    cudaError_t e = cudaMallocAsync((void **)&ord, sizeof(double) * (size_t)nSpk, s);
+    cudaError_t e = irc_scratch_alloc((void **)&ord, sizeof(double) * (size_t)nSpk, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, name);
     k_i64_to_f64<<<grid_for(nSpk, 256), 256, 0, s>>>(ord, ordrho, nSpk);
     int rc = IRC_OK;
@@ -344,7 +344,7 @@ extern "C" int irc_sort_load(const char *path, float *rho, float *delta, int64_t
     }
     if (nSpk == 0) return IRC_OK;
     double *ord = nullptr;
-    cudaError_t e = cudaMallocAsync((void **)&ord, sizeof(double) * (size_t)nSpk, s);
+    cudaError_t e = irc_scratch_alloc((void **)&ord, sizeof(double) * (size_t)nSpk, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, name);
     int rc = IRC_OK;
     {

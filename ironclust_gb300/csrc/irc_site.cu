@@ -315,9 +315,9 @@ int irc_exact_chunk_fill(float *D, int32_t *I, const float *F, const int32_t *IB
     if (rc != IRC_OK) return rc;
     float *vr = nullptr, *d2 = nullptr;
     int32_t *mi = nullptr;
-    e = cudaMallocAsync(&vr, sizeof(float) * (size_t)nA, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d2, sizeof(float) * (size_t)nA * knn, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(&mi, sizeof(int32_t) * (size_t)nA * knn, s);
+    e = irc_scratch_alloc((void **)&vr, sizeof(float) * (size_t)nA, s);
+    if (e == cudaSuccess) e = irc_scratch_alloc((void **)&d2, sizeof(float) * (size_t)nA * knn, s);
+    if (e == cudaSuccess) e = irc_scratch_alloc((void **)&mi, sizeof(int32_t) * (size_t)nA * knn, s);
     if (e == cudaSuccess) {
         rc = irc_site_knn(pl, F, nC, knn, nT, IRC_MODE_EXACT, vr, nullptr, mi, d2, s);
         if (rc == IRC_OK) {
@@ -527,6 +527,7 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
             pl->max_rn = std::max(pl->max_rn, rn[r]);
             if (r > roff[i] && rs[r] < rs[r - 1] + rn[r - 1]) pl->runs_ascend = 0;
         }
+    irc_scratch_plan(pl->device, 1);
     *out = pl;
     return IRC_OK;
 }
@@ -536,6 +537,7 @@ int irc_plan_destroy(irc_plan *pl)
     if (!pl) return IRC_OK;
     cudaError_t e = cudaFree(pl->dmem);
     irc_cert_release(pl);
+    irc_scratch_plan(pl->device, -1);
     if (pl->tc_buf && !pl->tc_external) cudaFree(pl->tc_buf);
     if (pl->tc_items_buf) cudaFree(pl->tc_items_buf);
     if (pl->row_dims) cudaFree(pl->row_dims);

@@ -37,9 +37,9 @@ def matlab_round(x):
 def mi2ml_drift(mi_member):
     """mi2ml_drift_: column j of the result marks the chunks listed in column j."""
     mi_member = np.asarray(mi_member)
-    n_members, n_drift = mi_member.shape
+    n_drift = mi_member.shape[1]
     ml = np.zeros((n_drift, n_drift), bool)
-    ml[mi_member.ravel(order="F"), np.repeat(np.arange(n_drift), n_members)] = True
+    ml[mi_member, np.arange(n_drift)] = True
     return ml
 
 

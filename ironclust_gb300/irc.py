@@ -668,18 +668,19 @@ def calc_drift(vrAmp_spk, vrPos_spk, n_sites, nTime_drift, nTime_batch, nTime_ma
     n_spk = amp.numel()
     n_cap = max(int(nTime_drift), 1)
     nb = max(int(nTime_batch), 1)
-    mi = torch.empty((n_cap, nb), dtype=torch.int32, device=amp.device)
-    lim = torch.empty(n_cap + 1, dtype=torch.int64, device=amp.device)
+    both = torch.empty(n_cap + 1 + (n_cap * nb + 1) // 2, dtype=torch.int64, device=amp.device)
+    lim, mi = both[: n_cap + 1], both[n_cap + 1:].view(torch.int32)          # read back in one copy
     n_out = C.c_int(0)
     check(lib().irc_calc_drift(_p(mi), _p(lim), C.byref(n_out), _p(amp), _p(pos), C.c_int64(n_spk), int(n_sites),
                                int(nTime_drift), int(nTime_batch), int(nTime_max_drift), int(nQuantile_drift),
                                _stream()), "irc_calc_drift")
     n = n_out.value
-    lim_h = lim[: n + 1].cpu().numpy()
+    host = both.cpu().numpy()
+    lim_h = host[: n + 1].copy()
     if n == 1:
         ml = np.ones((1, 1), bool)
         mem = np.zeros((1, 1), np.int64)
     else:
-        mem = mi[:n].cpu().numpy().astype(np.int64).T          # [nTime_batch, n]
+        mem = host[n_cap + 1:].view(np.int32)[: n * nb].reshape(n, nb).T.astype(np.int64)    # [nTime_batch, n]
         ml = mi2ml_drift(mem)
     return (lim_h, ml, mem) if members else (lim_h, ml)

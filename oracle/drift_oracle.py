@@ -49,7 +49,7 @@ def subsample_vr(vi, n_max):
             vi = vi[::n_skip]
         if vi.size > n_max:
             n_remove = vi.size - n_max
-            rm = matlab_round(np.linspace(1, vi.size, n_remove)).astype(np.int64)
+            rm = matlab_round(np.linspace(1 if n_remove > 1 else vi.size, vi.size, n_remove)).astype(np.int64)  # (MATLAB's linspace(a, b, 1) is b)
             rm = np.clip(rm, 1, vi.size) - 1
             keep = np.ones(vi.size, bool)
             keep[rm] = False
