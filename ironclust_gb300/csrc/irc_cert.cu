@@ -390,7 +390,7 @@ struct Lists {
 size_t lists_bytes(irc_plan *pl, int nC, size_t more)
 {
     return kHdrBytes + up(more) + up((size_t)pl->dev.n_out * sizeof(int2)) + up(irc_tc::list_area_bytes(pl->dev.n_out)) +
-           irc_tc::ops_bytes(pl, nC, Fmt::f16);
+           irc_tc::ops_bytes(pl, nC, Fmt::f16) + irc_tc::split_bytes(pl, nC, Fmt::f16);
 }
 
 int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, size_t zero, Lists *L, cudaStream_t s)
@@ -406,6 +406,7 @@ int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, si
     int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, (unsigned *)words + W_AMAX, (unsigned *)words + W_TICKET, &L->op, s);
     if (rc != IRC_OK) return rc;
     irc_tc::ListOut lo = irc_tc::list_area(la, pl->dev.n_out);
+    irc_tc::split_area(pl, nC, Fmt::f16, ops + irc_tc::ops_bytes(pl, nC, Fmt::f16), &lo);
     lo.cert = cert;
     rc = irc_tc::launch_filters(Fmt::f16, L->op.mq, L->op.mc, pl, nC, lo, words, s);
     L->c = Call{pl->dev, lo.qinfo, cert, lo.lists, L->op.fp, nC, pl->row_dims, L->op.scale, L->op.qnorm, words, nullptr, nullptr};

@@ -61,6 +61,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <cfloat>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -93,7 +95,8 @@ constexpr int THREADS = 32 * (1 + MMA_WARPS + EPI_WARPS);
 constexpr uint32_t A_BYTES = BM * KP * 2;         // the query tile: 128 rows x 128 bytes
 constexpr uint32_t HALF_BYTES = 128 * KP * 2;     // one 128-candidate tile
 constexpr uint32_t TMEM_COLS = 512;               // all TMEM columns (one CTA per SM)
-constexpr int LISTCAP = 192;                      // candidate-list capacity per query (the four warps' hits pooled)
+constexpr int kSMs = 152;
+constexpr int LISTCAP = irc_tc::LIST_ROW;                      // candidate-list capacity per query (the four warps' hits pooled)
 constexpr int MAX_SHORT_TILES = 512;              // tiles per chunk that a 16-bit list entry can name
 // The threshold is the tau_rank-th smallest per-column minimum: tau_rank
 // distinct candidates lie at or below it, a margin over knn (<= 32) for the
@@ -157,6 +160,24 @@ template <int BN>
 __device__ __forceinline__ int units_per_pass(int nts)
 {
     return BN == 256 ? (nts + 1) >> 1 : nts;
+}
+
+// A CTA's units of an item of U units a pass: PASS 0 all of them twice (unit k
+// is unit k or k - U of the pass), else its part's, from u0.
+template <int PASS>
+__device__ __forceinline__ int span_of(int U, int idx, const irc_tc::SplitOut &sp, int &u0)
+{
+    u0 = 0;
+    if (PASS == 0) return 2 * U;
+    const int part = idx % sp.parts;
+    u0 = U * part / sp.parts;
+    return U * (part + 1) / sp.parts - u0;
+}
+
+template <int PASS>
+__device__ __forceinline__ const irc_tc::TcItem &item_of(const irc_tc::TcItem *items, int idx, const irc_tc::SplitOut &sp)
+{
+    return items[PASS == 0 ? idx : idx / sp.parts];
 }
 
 // The MMA issuer of unit k (both passes counted) of slot s: alternate units of
@@ -548,6 +569,35 @@ __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::Tc
     }
 }
 
+// The same for a part of a split item: its entries go behind the other parts'
+// in the query's list row; k_publish records the lists.
+template <class T>
+__device__ __forceinline__ void hand_off_part(const irc::PlanDev &p, const irc_tc::TcItem &it, int item, int piece, int quarter,
+                                              int part, int qrow, int nq_s, const int2 *__restrict__ tl,
+                                              const unsigned char *lists, const int *sCnt, const float *sTau,
+                                              const irc_tc::ListOut &lo, int lane)
+{
+    constexpr int RL = 32 / PARTS;
+    const int row = quarter * 32 + part * RL + lane;              // (lanes < RL: the warp's queries)
+    int n = 0, base = 0;
+    if (lane < RL && qrow + part * RL + lane < nq_s) {
+        n = sCnt[row];
+        if (n) base = atomicAdd(lo.split.cnt + item * BM + row, n);
+        if (lo.cert && piece == 0) lo.cert[it.qs[0] + row - p.q_base] = make_int2(__float_as_int(sTau[row]), it.chunk[0]);
+        if (n > LISTCAP || base + n > LISTCAP) n = 0;             // (the count, past LISTCAP, tells)
+    }
+#pragma unroll 1
+    for (int L = 0; L < RL; ++L) {
+        const int m = __shfl_sync(0xffffffffu, n, L), b = __shfl_sync(0xffffffffu, base, L);
+        const typename T::Entry *lr = T::row(lists, quarter, part * RL + L);
+        uint32_t *out = lo.lists + lo.split.area + (size_t)(item * BM + quarter * 32 + part * RL + L) * LISTCAP + b;
+        for (int e = lane; e < m; e += 32) {
+            const uint32_t v = lr[e];
+            out[e] = sizeof(typename T::Entry) == 4 ? v : (uint32_t)__ldg(tl + (v >> 7)).x + (v & 127u);
+        }
+    }
+}
+
 // Shared state of a persistent filter CTA: the item ring (the producer claims
 // items from the launch's work queue and publishes their indices), the
 // double-buffered query tile and the mbarriers of every stage.
@@ -574,7 +624,7 @@ struct Shared {
 // synchronise only among themselves (named barrier 1 + slot).  Unit g of a
 // slot (counted over all its items, both passes) goes to accumulator
 // s * BPS + g % BPS, whose barriers are in phase g / BPS.
-template <int BN, int NS, Fmt FMT, bool TAU, bool BIG>
+template <int BN, int NS, Fmt FMT, bool TAU, bool BIG, int PASS>
 __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::TcItem *__restrict__ items, int rank,
                                          uint32_t tmem, int tau_k, const Shared &sh, const irc_tc::ListOut &lo,
                                          int *scratch, int warp, int lane)
@@ -602,11 +652,14 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
         __syncwarp();
         if (lane == 0) sm100::mbar_arrive(&sh.item_empty[r]);
         if (idx < 0) break;                       // the queue is empty
-        const irc_tc::TcItem it = items[idx];
+        const irc_tc::TcItem it = item_of<PASS>(items, idx, lo.split);
         const int nq_s = it.chunk[s] >= 0 ? it.nq[s] : 0;
         const int nts = chunk_tiles(p, it.chunk[s]);
         const bool active = qrow < nq_s;          // warp-uniform: any valid query in this quarter
         const int U = units_per_pass<BN>(nts);
+        int u0;
+        const int K = span_of<PASS>(U, idx, lo.split, u0);
+        const int K1 = PASS == 0 ? U : PASS == 1 ? K : 0;      // units of pass 1
         // the slot's tile list: unit u is tile u (BN = 128) or tiles 2u, 2u + 1
         // (BN = 256; the second is (0, 0) past the end of an odd count)
         const int2 *tl = nts ? p.tc_tiles + __ldg(p.tc_toff + it.chunk[s]) : p.tc_tiles;
@@ -614,7 +667,7 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
         // Unit k of the two passes: (first row, columns) of its tile(s), loaded
         // one unit ahead of its use.
         auto load_unit = [&](int k) -> int4 {
-            const int u = k < U ? k : k - U;
+            const int u = PASS ? u0 + k : k < U ? k : k - U;
             if constexpr (BN == 256) {
                 return __ldg(reinterpret_cast<const int4 *>(tl) + u);
             } else {
@@ -622,11 +675,11 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
                 return make_int4(v.x, v.y, 0, 0);
             }
         };
-        int4 cu = U ? load_unit(0) : make_int4(0, 0, 0, 0);
+        int4 cu = K ? load_unit(0) : make_int4(0, 0, 0, 0);
         // this warp's columns of the unit: first rows ra, rb and valid counts
         // na, nb of its 32 columns in each tile (none: <= 0)
         auto unit = [&](int k, int &ra, int &na, int &rb, int &nb) {
-            const int4 nx = load_unit(k + 1 < 2 * U ? k + 1 : k);
+            const int4 nx = load_unit(k + 1 < K ? k + 1 : k);
             ra = cu.x;
             na = cu.y - part * PART;
             rb = cu.z;
@@ -638,7 +691,7 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
         float bm[PART];
 #pragma unroll
         for (int c = 0; c < PART; ++c) bm[c] = __int_as_float(0x7f800000);
-        for (int k = 0; k < U && ok; ++k) {
+        for (int k = 0; k < K1 && ok; ++k) {
             int ra, na, rb, nb;
             unit(k, ra, na, rb, nb);
             const unsigned g = g0 + (unsigned)k;
@@ -654,8 +707,21 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
                 release_acc(empty, lane);
             }
         }
+        // a part's minima meet the other parts' in global memory
+        if constexpr (PASS != 0) {
+            int *cm = lo.split.colmin + ((size_t)(idx / lo.split.parts) * 128 + part * PART) * BM + row;
+#pragma unroll
+            for (int c = 0; c < PART; ++c) {
+                if (PASS == 1) {
+                    if (active && bm[c] < FLT_MAX) atomicMin(cm + c * BM, __float_as_int(fmaxf(bm[c], 0.0f)));
+                } else {
+                    const int v = __ldg(cm + c * BM);
+                    bm[c] = __int_as_float(v < 0x7f7f7f7f ? v : 0x7f800000);
+                }
+            }
+        }
         // threshold: rank-th smallest of the 128 column minima of every query
-        {
+        if constexpr (PASS != 1) {
             float *brow = qarea + lane * BROW + part * PART;
 #pragma unroll
             for (int c = 0; c < PART; ++c) brow[c] = fmaxf(bm[c], 0.0f);
@@ -715,8 +781,8 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             }
             slot_barrier(s, slot_threads);        // minima rows are read; the list rows may be written
         }
-        const float tau = sh.sTau[row];
-        if (TAU && part == 0 && U > 0) {
+        const float tau = PASS == 1 ? 0.0f : sh.sTau[row];
+        if (TAU && PASS != 1 && part == 0 && K > 0) {
             // the thresholds into the item's query tile; visible to the tensor
             // core (async proxy) before the MMA thread, released by tau_ready,
             // issues the slot's pass-2 MMAs (one phase per item with units)
@@ -726,7 +792,7 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             if (lane == 0) sm100::mbar_arrive(&sh.tau_ready[s]);
         }
         // pass 2: collect the candidates at or below tau
-        for (int k = U; k < 2 * U && ok; ++k) {
+        for (int k = K1; k < K && ok; ++k) {
             int ra, na, rb, nb;
             unit(k, ra, na, rb, nb);
             const unsigned g = g0 + (unsigned)k;
@@ -738,7 +804,7 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
                 unsigned ma = 0u, mb = 0u;
                 mark<BN, BN == 256 && TAU>(tbase + b * BN, na, tbase + b * BN + 128, nb, tau, empty, lane, ma, mb);
                 // entries: rows, or (place of the tile in the list, column)
-                const uint32_t ea = BIG ? (uint32_t)ra : (uint32_t)((k - U) * (BN / 128)) << 7;
+                const uint32_t ea = BIG ? (uint32_t)ra : (uint32_t)((PASS ? u0 + k : k - U) * (BN / 128)) << 7;
                 const uint32_t eb = BIG ? (uint32_t)rb : ea + 128u;
                 append_hits(lrow, sh.sCnt + row, ma, ea + part * PART, mb, eb + part * PART);
             } else {
@@ -746,8 +812,11 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
             }
         }
         slot_barrier(s, slot_threads);
-        if (__all_sync(0xffffffffu, ok)) hand_off<T>(p, it, s, quarter, part, qrow, nq_s, tl, sh.lists, sh.sCnt, sh.sTau, lo, scratch, lane);
-        g0 += 2u * (unsigned)U;
+        if (PASS == 2 && __all_sync(0xffffffffu, ok))
+            hand_off_part<T>(p, it, idx / lo.split.parts, idx % lo.split.parts, quarter, part, qrow, nq_s, tl, sh.lists, sh.sCnt,
+                             sh.sTau, lo, lane);
+        if (PASS == 0 && __all_sync(0xffffffffu, ok)) hand_off<T>(p, it, s, quarter, part, qrow, nq_s, tl, sh.lists, sh.sCnt, sh.sTau, lo, scratch, lane);
+        g0 += (unsigned)K;
         // every warp of the slot is done with this item's lists before the
         // next item's minima overwrite them; after a timed-out wait all stop
         if (!slot_barrier_and(s, slot_threads, ok && !*sh.abort_flag)) break;
@@ -762,10 +831,10 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
 // tile's first row, which it fetched a unit ahead (the table lookup is off the
 // path between a free stage and its loads).  Stage and tile counters run on
 // across items, so the ring never drains between them.
-template <int BN, int NS, bool BIG>
+template <int BN, int NS, bool BIG, int PASS>
 __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMap &tmC, const irc::PlanDev &p,
                                         const irc_tc::TcItem *__restrict__ items, int n_items, unsigned *queue,
-                                        const Shared &sh, int lane)
+                                        const Shared &sh, const irc_tc::SplitOut &sp, int lane)
 {
     using T = Tile<BN, BIG>;
     constexpr int QPS = 4 / NS;
@@ -781,8 +850,12 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
     for (int seq = 0; ok; ++seq) {
         const int r = seq & 1;
         unsigned claim = 0;
-        if (lane == 0) claim = atomicAdd(queue, 1u);
-        claim = __shfl_sync(0xffffffffu, claim, 0);
+        if (PASS) {                               // (one: its unit count may be odd, which would move the next item's
+            claim = seq == 0 ? blockIdx.x : (unsigned)n_items;             // accumulators to the other issuer)
+        } else {
+            if (lane == 0) claim = atomicAdd(queue, 1u);
+            claim = __shfl_sync(0xffffffffu, claim, 0);
+        }
         const int idx = claim < (unsigned)n_items ? (int)claim : -1;
         if (!(ok = warp_wait(&sh.item_empty[r], ((seq >> 1) & 1) ^ 1, sh.abort_flag))) break;
         if (lane == 0) {
@@ -790,15 +863,18 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
             sm100::mbar_arrive(&sh.item_full[r]); // release: the index is visible to the waiters
         }
         if (idx < 0) break;
-        const irc_tc::TcItem it = items[idx];
+        const irc_tc::TcItem it = item_of<PASS>(items, idx, sp);
         const int2 *tl[NS];
         int U[NS], nt[NS], row[NS];               // row: this lane's tile of the slot's next unit
+        int K[NS], u0[NS];
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             nt[s] = chunk_tiles(p, it.chunk[s]);
             U[s] = units_per_pass<BN>(nt[s]);
             tl[s] = nt[s] ? p.tc_tiles + __ldg(p.tc_toff + it.chunk[s]) : p.tc_tiles;
-            row[s] = lane < NH && lane < nt[s] ? __ldg(tl[s] + lane).x : 0;
+            K[s] = span_of<PASS>(U[s], idx, sp, u0[s]);
+            const int t = u0[s] * NH + lane;
+            row[s] = lane < NH && t < nt[s] ? __ldg(tl[s] + t).x : 0;
         }
         // the query tile of item seq - 2 is free once that item's MMAs are done
         if (!(ok = warp_wait(&sh.a_empty[r], ((seq >> 1) & 1) ^ 1, sh.abort_flag))) break;
@@ -817,9 +893,9 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
             bool any = false;
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                if (ok && k < 2 * U[s]) {
+                if (ok && k < K[s]) {
                     any = true;
-                    const int u = k < U[s] ? k : k - U[s];
+                    const int u = PASS ? u0[s] + k : k < U[s] ? k : k - U[s];
                     const int w = issuer_of<NS>(k, s);
                     if ((ok = warp_wait(&sh.empty[st], ph, sh.abort_flag))) {
                         const int nh = BN == 256 && 2 * u + 1 >= nt[s] ? 1 : NH;
@@ -865,9 +941,9 @@ __device__ __forceinline__ void produce(const CUtensorMap &tmQ, const CUtensorMa
 // slot's epilogue wrote the thresholds into the query tile (tau_ready[s], one
 // phase per item in which the slot has units).  After an item's last unit each
 // issuer's commit lets its MMAs free the query tile.
-template <int BN, int NS, Fmt FMT, bool TAU, bool BIG>
+template <int BN, int NS, Fmt FMT, bool TAU, bool BIG, int PASS>
 __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcItem *__restrict__ items, int nk,
-                                      uint32_t tmem, const Shared &sh, int w)
+                                      uint32_t tmem, const Shared &sh, const irc_tc::SplitOut &sp, int w)
 {
     using T = Tile<BN, BIG>;
     constexpr int BPS = T::NBUF / NS;
@@ -887,13 +963,15 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
         const int idx = sh.item_idx[r];
         sm100::mbar_arrive(&sh.item_empty[r]);
         if (idx < 0) break;
-        const irc_tc::TcItem it = items[idx];
-        int U[NS];
+        const irc_tc::TcItem it = item_of<PASS>(items, idx, sp);
+        int U[NS], K[NS];
         bool tau_wait[NS];
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             U[s] = units_per_pass<BN>(chunk_tiles(p, it.chunk[s]));
-            tau_wait[s] = TAU;
+            int u0;
+            K[s] = span_of<PASS>(U[s], idx, sp, u0);
+            tau_wait[s] = TAU && PASS != 1;
         }
         if (!(ok = pipe_wait(&sh.a_full[r], (seq >> 1) & 1, sh.abort_flag))) break;
         sm100::tc_fence_after();
@@ -902,7 +980,7 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
             bool any = false;
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                if (ok && k < 2 * U[s]) {
+                if (ok && k < K[s]) {
                     any = true;
                     if (issuer_of<NS>(k, s) == w) {
                         const unsigned g = g0[s] + (unsigned)k, use = g / BPS;
@@ -917,7 +995,7 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
                         // the slot's thresholds are in the query tile before its pass 2 (after the
                         // accumulator's wait: the slot's epilogue is then in this item, so no
                         // earlier phase of tau_ready is open)
-                        if (TAU && ok && k >= U[s] && tau_wait[s]) {
+                        if (TAU && ok && (PASS == 2 || k >= U[s]) && tau_wait[s]) {
                             tau_wait[s] = false;
                             ok = pipe_wait(&sh.tau_ready[s], taus[s] & 1, sh.abort_flag);
                         }
@@ -945,8 +1023,8 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
         if (!ok) break;
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            g0[s] += 2u * (unsigned)U[s];
-            taus[s] += U[s] > 0 ? 1u : 0u;
+            g0[s] += (unsigned)K[s];
+            taus[s] += K[s] > 0 ? 1u : 0u;
         }
         sm100::mma_commit(&sh.a_empty[r]);        // this item's MMAs done: its query tile may be replaced
     }
@@ -960,8 +1038,9 @@ __device__ __forceinline__ void issue(const irc::PlanDev &p, const irc_tc::TcIte
 // from the class's work queue (queue: its head, items cost-ordered) until it
 // is empty.  TAU: pass 2 reads the signs of d2 - tau (the thresholds written
 // into the query tile at K position tau_k), else it compares d2 with tau in
-// the epilogue.
-template <Fmt FMT, int BN, bool TAU, int NS, bool BIG>
+// the epilogue.  PASS: 0 both passes; 1 or 2 one pass of a part of an item's
+// units (irc_tc::SplitOut), one (item, part) per CTA.
+template <Fmt FMT, int BN, bool TAU, int NS, bool BIG, int PASS = 0>
 __global__ void __launch_bounds__(THREADS, 1)
 k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmC, irc::PlanDev p,
          const irc_tc::TcItem *__restrict__ items, int n_items, unsigned *queue, int nk, int tau_k, irc_tc::ListOut lo,
@@ -1018,13 +1097,13 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
     const uint32_t tmem = *sh.tmem_slot;
 
     if (warp == 0) {
-        produce<BN, NS, BIG>(tmQ, tmC, p, items, n_items, queue, sh, lane);
+        produce<BN, NS, BIG, PASS>(tmQ, tmC, p, items, n_items, queue, sh, lo.split, lane);
         __syncwarp();
     } else if (warp == 1 || warp == 2 + EPI_WARPS) {
-        if (lane == 0) issue<BN, NS, FMT, TAU, BIG>(p, items, nk, tmem, sh, warp == 1 ? 0 : 1);
+        if (lane == 0) issue<BN, NS, FMT, TAU, BIG, PASS>(p, items, nk, tmem, sh, lo.split, warp == 1 ? 0 : 1);
         __syncwarp();
     } else {
-        epilogue<BN, NS, FMT, TAU, BIG>(p, items, tau_rank(FMT), tmem, tau_k, sh, lo, scratch, warp, lane);
+        epilogue<BN, NS, FMT, TAU, BIG, PASS>(p, items, tau_rank(FMT), tmem, tau_k, sh, lo, scratch, warp, lane);
     }
     sm100::tc_fence_before();
     __syncthreads();
@@ -1033,6 +1112,22 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
         sm100::tmem_dealloc(tmem, TMEM_COLS);
     }
     if (threadIdx.x == 0 && *sh.abort_flag) atomicExch(scratch + irc::kScratchErr, 1);
+}
+
+// The split items' lists: (offset, length) of every query, as hand_off.
+__global__ void __launch_bounds__(BM) k_publish(irc::PlanDev p, const irc_tc::TcItem *__restrict__ items,
+                                                irc_tc::ListOut lo, int *__restrict__ scratch)
+{
+    const irc_tc::TcItem &it = items[blockIdx.x];
+    const int row = threadIdx.x, slot = blockIdx.x * BM + row;
+    if (row >= it.nq[0]) return;
+    const int q = it.qs[0] + row, n = lo.split.cnt[slot];
+    if (n > LISTCAP) {
+        if (!lo.cert) scratch[irc::kScratchLists + atomicAdd(scratch + 0, 1)] = q;
+        return;
+    }
+    const int complete = n == __ldg(p.ncand + it.chunk[0]) ? (1 << 30) : 0;
+    lo.qinfo[q - p.q_base] = make_int2((int)(lo.split.area + (unsigned)slot * LISTCAP), n | complete);
 }
 
 // Exact re-rank kernel: one warp per query of the plan, in query order (the
@@ -1114,6 +1209,68 @@ static int launch_filter(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan 
     return IRC_OK;
 }
 
+// The items of lo.split: pass 1, pass 2, their lists published.
+template <Fmt FMT>
+static int launch_split(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, const irc_tc::TcItem *items, int nk,
+                        int tau_k, const ListOut &lo, int *scratch, cudaStream_t s)
+{
+    const bool big = pl->tc_max_tiles > MAX_SHORT_TILES;
+    auto pass1 = big ? k_knn_tc<FMT, 256, true, 1, true, 1> : k_knn_tc<FMT, 256, true, 1, false, 1>;
+    auto pass2 = big ? k_knn_tc<FMT, 256, true, 1, true, 2> : k_knn_tc<FMT, 256, true, 1, false, 2>;
+    const int smem = (int)(big ? Tile<256, true>::SMEM_BYTES : Tile<256, false>::SMEM_BYTES);
+    const SplitOut &sp = lo.split;
+    cudaError_t e = cudaFuncSetAttribute(pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pass2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(sp.colmin, 0x7f, (size_t)sp.items * BM * 128 * 4, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(sp.cnt, 0, (size_t)sp.items * BM * 4, s);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): split items");
+    const int n = sp.items * sp.parts;
+    pass1<<<n, THREADS, smem, s>>>(mq, mc, pl->dev, items, n, nullptr, nk, tau_k, lo, scratch);
+    pass2<<<n, THREADS, smem, s>>>(mq, mc, pl->dev, items, n, nullptr, nk, tau_k, lo, scratch);
+    k_publish<<<sp.items, BM, 0, s>>>(pl->dev, items, lo, scratch);
+    IRC_CHECK_LAUNCH("irc_site_knn(tensor core) split items");
+    return IRC_OK;
+}
+
+// The last one-slot items that leave SMs idle: n mod 152 of them take one more
+// turn, as long as a full one (1.42 us a unit, D = 24).  Cut into parts that
+// fill the machine they take two launches of a part's units and 57 us of their
+// own (memory cleared, prologues, the threshold search after pass 1, lists
+// published); 22 more than the launch they replace where they are all there
+// is.  us a call, whole -> split: 20,000 spikes in one chunk (157 items of 79
+// units) 302 -> 248, 21,000 273 -> 219, 60,001 in 30 chunks 675 -> 602,
+// 100,003 in 50 1,007 -> 959; not kept where it loses: 3,000 (24 of 12 units)
+// 71 -> 79, 8,000 (63 of 32, two parts) 100.5 -> 101.5.
+static SplitOut split_of(const irc_plan *pl, int nC, Fmt fmt)
+{
+    SplitOut sp{};
+    const int rest = pl->n_tc_one % kSMs, units = (pl->tc_max_tiles + 1) / 2;
+    if (fmt == Fmt::fp8 || nC + 9 > KP || pl->tc_wide_bn == 128 || rest == 0) return sp;
+    const int parts = std::min(kSMs / rest, units / 4), saved = units - units / std::max(parts, 1);
+    if (parts < 2 || saved < (pl->n_tc_one > kSMs ? 34 : 20)) return sp;
+    sp.items = rest;
+    sp.parts = parts;
+    return sp;
+}
+
+size_t split_bytes(const irc_plan *pl, int nC, Fmt fmt)
+{
+    return (size_t)split_of(pl, nC, fmt).items * BM * (128 + 1 + LIST_ROW) * 4;
+}
+
+void split_area(const irc_plan *pl, int nC, Fmt fmt, void *mem, ListOut *lo)
+{
+    SplitOut sp = split_of(pl, nC, fmt);
+    if (!sp.items) return;
+    sp.colmin = (int *)mem;
+    sp.cnt = sp.colmin + (size_t)sp.items * BM * 128;
+    uint32_t *rows = (uint32_t *)(sp.cnt + (size_t)sp.items * BM);
+    const size_t at = (size_t)(rows - lo->lists);
+    if (at + (size_t)sp.items * BM * LIST_ROW > (size_t)0x7fffff00) return;       // (offsets are int32)
+    sp.area = (unsigned)at;
+    lo->split = sp;
+}
+
 // The filter of every packing class of the plan on stream s.
 int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, int nC, const ListOut &lo,
                    int *scratch, cudaStream_t s)
@@ -1143,8 +1300,12 @@ int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_pl
     auto run = [&](auto fmt_c, auto tau_c) {
         constexpr Fmt F = decltype(fmt_c)::value;
         constexpr bool T = decltype(tau_c)::value;
+        const int rest = T && !narrow ? lo.split.items : 0;
         int r = narrow ? launch_filter<F, 128, false, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, scratch, s)
-                       : launch_filter<F, 256, T, 1>(mq, mc, pl, it1, n1, lo.count + 1, nk, tau_k, lo, scratch, s);
+                       : launch_filter<F, 256, T, 1>(mq, mc, pl, it1, n1 - rest, lo.count + 1, nk, tau_k, lo, scratch, s);
+        if constexpr (T)
+            if (r == IRC_OK && rest)
+                r = launch_split<F>(mq, mc, pl, it1 + n1 - rest, nk, tau_k, lo, scratch, s);
         if (r != IRC_OK) return r;
         r = narrow ? launch_filter<F, 128, false, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, scratch, s)
                    : launch_filter<F, 256, T, 2>(mq, mc, pl, it2, n2, lo.count + 2, nk, tau_k, lo, scratch, s);

@@ -24,6 +24,18 @@ enum class Fmt : int { bf16 = 0, fp8 = 1, f16 = 2 };
 // width in float4.
 inline __host__ __device__ int fp_row4(int nC) { return 2 * ((nC + 7) / 8); }
 
+// Items that do not fill a turn of the machine, split over their candidates:
+// `items` of them (the last one-slot ones) in `parts` pieces each, one piece per
+// CTA, one launch per pass.  colmin: the per-column minima of every item,
+// [items][128 columns][128 queries] (bits); cnt: list lengths, [items][128];
+// area: where the items' list rows (LIST_ROW entries a query) begin in lists.
+constexpr int LIST_ROW = 192;
+struct SplitOut {
+    int items, parts;
+    int *colmin, *cnt;
+    unsigned area;
+};
+
 // Candidate lists handed from the filter kernel to the re-rank kernel:
 // qinfo[o] = (offset into lists, length) of query q_base + o, or (-1, -1);
 // lists packed by a bump allocator (count) of cap entries.
@@ -33,6 +45,7 @@ struct ListOut {
     unsigned *count;             // count[0]: list entries used; count[1..3]: work-queue heads of the
     unsigned cap;                // filter's one-, two- and four-slot launches
     int2 *cert;                  // per query (threshold bits, chunk), or null when nobody asks
+    SplitOut split;
 };
 
 // Entries of the list area of a plan with n_out queries (offsets are int32).
@@ -59,8 +72,14 @@ inline ListOut list_area(void *base, long long n_out)
     lo.lists = (uint32_t *)(b + 256);
     lo.cap = (unsigned)list_cap(n_out);
     lo.cert = nullptr;
+    lo.split = SplitOut{};
     return lo;
 }
+
+// Memory of the split items (0: none), and its place in lo: behind lo.lists, in
+// the same allocation.
+size_t split_bytes(const irc_plan *pl, int nC, Fmt fmt);
+void split_area(const irc_plan *pl, int nC, Fmt fmt, void *mem, ListOut *lo);
 
 // The filter (one persistent launch per packing class: items of one or two
 // slots on 256-candidate units, four-slot items on 128-candidate units; mc is

@@ -455,9 +455,13 @@ int irc_site_knn_tc(irc_plan *pl, const float *F, int nC, int knn, int mode, flo
     if (knn > irc_tc::KNN_MAX) { irc_host::set_error("irc_site_knn(BF16): knn %d > %d", knn, irc_tc::KNN_MAX); return IRC_E_INVAL; }
     void *buf;
     const size_t ops = irc_tc::ops_bytes(pl, nC, fmt);
-    int rc = irc_plan_tc_buffer(pl, ops + irc_tc::list_area_bytes(pl->dev.n_out), &buf);
+    const size_t need = ops + irc_tc::list_area_bytes(pl->dev.n_out);
+    size_t split = irc_tc::split_bytes(pl, nC, fmt);
+    if (split && pl->tc_external && pl->tc_bytes < need + split) split = 0;      // the caller's memory is enough without
+    int rc = irc_plan_tc_buffer(pl, need + split, &buf);
     if (rc != IRC_OK) return rc;
-    const irc_tc::ListOut lo = irc_tc::list_area((char *)buf + ops, pl->dev.n_out);
+    irc_tc::ListOut lo = irc_tc::list_area((char *)buf + ops, pl->dev.n_out);
+    if (split) irc_tc::split_area(pl, nC, fmt, (char *)buf + need, &lo);
     cudaError_t e = cudaMemsetAsync(pl->scratch, 0, 2 * sizeof(int), s);   // overflow-queue count, largest magnitude
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(BF16): memset");
     irc_tc::Operands op;
