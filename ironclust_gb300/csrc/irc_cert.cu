@@ -362,22 +362,28 @@ struct Work {
 
 size_t up(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// Where the filter pays.  The plain kernels' time grows with the pairs of
-// their 16-query tiles and with the tiles; the search has a dozen launches to
-// make first.  Microseconds, plain -> proven (EXACT | REF | REF delta), D = 24:
-//     3,000 spikes, one chunk (9.0e6 pairs)      134 -> 159 | 177 -> 159 | 64 -> 214
-//     4,000, 8 chunks (1.6e7)                    163 -> 120 | 197 -> 124 | 86 -> 179
-//     20,000, 1,200 chunks (5.0e6, 2,400 tiles)  265 -> 147 | 714 -> 169 | 108 -> 199
-//     60,000, 1,200 chunks (4.5e7, 4,800 tiles)  845 -> 240 | 1,956 -> 324 | 381 -> 344
-//     8,000, 8 chunks, D = 33 (6.4e7)            639 -> 153 | 606 -> 161 | 384 -> 213
-constexpr long long kMinPairs = 12000000, kMinPairsDelta = 45000000;
-constexpr int kMinTiles = 1000;
+// Where the filter pays.  The plain kernels' time grows with the pairs times
+// the features and with the 16-query tiles; the search has a dozen launches to
+// make first.  Microseconds, plain -> proven (EXACT | REF | REF delta):
+//     1,000 spikes, one chunk, D = 24 (1.0e6 pairs)    55 -> 74  |  75 -> 73  |  17 -> 86
+//     2,048, D = 9 (4.2e6)                             54 -> 76  |  74 -> 77  |  17 -> 87
+//     2,048, D = 24                                    78 -> 79  |  82 -> 79  |  25 -> 99
+//     2,048, D = 45                                   118 -> 88  |  98 -> 85  |  40 -> 108
+//     4,000, D = 9 (1.6e7)                             94 -> 89  | 156 -> 92  |  41 -> 97
+//     5,000, D = 24 (2.5e7)                           264 -> 99  | 309 -> 104 | 143 -> 118
+//     4,000, 200 chunks (1.2e6, 400 tiles)             86 -> 89  | 172 -> 89  |  31 -> 101
+//     10,000, 400 chunks (3.8e6, 800 tiles)           144 -> 90  | 383 -> 98  |  55 -> 105
+//     20,000, 1,200 chunks (5.0e6, 2,400 tiles)       266 -> 109 | 725 -> 123 | 107 -> 125
+// Tiles alone count only where a window is likely to hold knn candidates.
+enum class Form { exact, ref, ref_delta };
 
-bool serves(const irc_plan *pl, int nC, bool knn)
+bool serves(const irc_plan *pl, int nC, Form f)
 {
-    return pl->runs_ascend && nC + 6 <= irc_tc::KP &&
-           (knn ? pl->pairs >= kMinPairs || pl->ntiles[irc::tile_slot(kTile)] >= kMinTiles
-                : pl->pairs >= kMinPairsDelta);
+    if (!pl->runs_ascend || nC + 6 > irc_tc::KP) return false;
+    const long long work = f == Form::exact ? 100000000 : f == Form::ref ? 20000000 : 500000000;
+    const int tiles = f == Form::exact ? 500 : f == Form::ref ? 150 : 4000;
+    return pl->pairs * nC >= work ||
+           (pl->ntiles[irc::tile_slot(kTile)] >= tiles && pl->pairs >= 64LL * pl->dev.n_out);
 }
 
 // Lists of every query on stream s: words | more (zeroed) ... | cert | lists | operands.
@@ -425,7 +431,7 @@ void irc_cert_release(irc_plan *pl)
 int irc_cert_site_knn(irc_plan *pl, const float *F, int nC, int knn, int nThreads, int mode, float *vrKnn, float *rho,
                       int32_t *miKnn, float *d2Knn, cudaStream_t s)
 {
-    if (!serves(pl, nC, true) || knn > irc_tc::KNN_MAX) return IRC_CERT_PASS;
+    if (!serves(pl, nC, mode == IRC_MODE_EXACT ? Form::exact : Form::ref) || knn > irc_tc::KNN_MAX) return IRC_CERT_PASS;
     const int tiles = pl->ntiles[irc::tile_slot(kTile)];
     const size_t flags = up((size_t)tiles * 4), queue = up((size_t)tiles * 4);
     const size_t ovf = mode == IRC_MODE_EXACT ? up((size_t)pl->dev.n_out * 4) : 0, more = flags + queue + ovf;
@@ -454,7 +460,7 @@ int irc_cert_site_delta_ref(irc_plan *pl, const float *F, int nC, const float *R
 {
     // (a bin's step number has 20 bits in the drift-window search's keys: a
     // run of at most 2^20 rows always fits)
-    if (!serves(pl, nC, false) || pl->max_rn > (1 << 20)) return IRC_CERT_PASS;
+    if (!serves(pl, nC, Form::ref_delta) || pl->max_rn > (1 << 20)) return IRC_CERT_PASS;
     const size_t more = delta_bytes(pl->dev.n_out, pl->dev.nChunks);
     Work w(pl, lists_bytes(pl, nC, more), s);
     if (!w.base) return IRC_CERT_PASS;

@@ -79,6 +79,9 @@ SHAPES = [
     ("plain", 7200, 58, 1, False, 30, 1024),
     ("plain", 7200, 59, 1, False, 30, 1024),
     ("plain", 20011, 24, 600, False, 30, 1024),
+    # the smallest sites of the search: fewer queries than a tile's columns, windows of a few hundred rows
+    ("plain", 905, 25, 1, False, 30, 1024), ("dup", 1100, 45, 2, True, 32, 1000), ("shift", 2101, 24, 3, False, 30, 512),
+    ("outlier", 2405, 9, 1, False, 30, 1024), ("coarse", 3001, 12, 40, False, 5, 1024), ("plain", 4003, 6, 200, False, 30, 1024),
 ]
 
 
