@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(32 * kWarps, 5)
 k_cert_knn(Call c, int knn, int nT, float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
            float *__restrict__ d2Knn)
 {
+    after_previous(c.qinfo, c.cert, c.lists, c.Fp, c.scale, c.qnorm);
     __shared__ __align__(16) unsigned long long wkeys[kWarps * WARP_KEYS];
     __shared__ float4 qrows[kWarps * QROW4];
     __shared__ unsigned wbits[REF ? kWarps * 32 : 1];
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4)
 k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ delta, int *__restrict__ nneigh,
              int *__restrict__ counts, int *__restrict__ list_out)
 {
+    after_previous(c.qinfo, c.cert, c.lists, c.Fp, c.scale, c.qnorm);
     __shared__ float4 qrows[kWarps * QROW4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int o = blockIdx.x * kWarps + warp;
@@ -406,14 +408,15 @@ int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, si
     int2 *cert = (int2 *)(L->more + up(more));
     char *la = (char *)cert + up((size_t)pl->dev.n_out * sizeof(int2));
     char *ops = la + up(irc_tc::list_area_bytes(pl->dev.n_out));
-    cudaError_t e = cudaMemsetAsync(base, 0, kHdrBytes + zero, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cert, 0xff, (size_t)pl->dev.n_out * sizeof(int2), s);
-    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: memset");
-    int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, (unsigned *)words + W_AMAX, (unsigned *)words + W_TICKET, &L->op, s);
-    if (rc != IRC_OK) return rc;
     irc_tc::ListOut lo = irc_tc::list_area(la, pl->dev.n_out);
     irc_tc::split_area(pl, nC, Fmt::f16, ops + irc_tc::ops_bytes(pl, nC, Fmt::f16), &lo);
     lo.cert = cert;
+    cudaError_t e = cudaMemsetAsync(base, 0, kHdrBytes + zero, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cert, 0xff, (size_t)pl->dev.n_out * sizeof(int2), s);
+    if (e == cudaSuccess) e = irc_tc::clear_lists(lo, pl->dev.n_out, s);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: memset");
+    int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, (unsigned *)words + W_AMAX, (unsigned *)words + W_TICKET, &L->op, s);
+    if (rc != IRC_OK) return rc;
     rc = irc_tc::launch_filters(Fmt::f16, L->op.mq, L->op.mc, pl, nC, lo, words, s);
     L->c = Call{pl->dev, lo.qinfo, cert, lo.lists, L->op.fp, nC, pl->row_dims, L->op.scale, L->op.qnorm, words, nullptr, nullptr};
     return rc;
@@ -444,9 +447,9 @@ int irc_cert_site_knn(irc_plan *pl, const float *F, int nC, int knn, int nThread
     L.c.tile_queue = (int *)(L.more + flags);
     const unsigned grid = (unsigned)((pl->dev.n_out + kWarps - 1) / kWarps);
     if (mode == IRC_MODE_EXACT)
-        k_cert_knn<false><<<grid, 32 * kWarps, 0, s>>>(L.c, knn, 1, vrKnn, rho, miKnn, d2Knn);
+        launch_next(k_cert_knn<false>, grid, 32 * kWarps, 0, s, L.c, knn, 1, vrKnn, rho, miKnn, d2Knn);
     else
-        k_cert_knn<true><<<grid, 32 * kWarps, 0, s>>>(L.c, knn, nThreads, vrKnn, rho, miKnn, nullptr);
+        launch_next(k_cert_knn<true>, grid, 32 * kWarps, 0, s, L.c, knn, nThreads, vrKnn, rho, miKnn, nullptr);
     IRC_CHECK_LAUNCH("irc_site_knn lists");
     const irc::TileQueue tq{L.c.tile_queue, L.c.words + W_TILES, L.c.words + W_ERR, tiles};
     if (mode == IRC_MODE_EXACT)
@@ -469,7 +472,7 @@ int irc_cert_site_delta_ref(irc_plan *pl, const float *F, int nC, const float *R
     int rc = make_lists(pl, F, nC, (char *)w.base, more, 4 * (4 + (size_t)pl->dev.nChunks), &L, s);
     if (rc != IRC_OK) return rc;
     const irc_delta_scratch sc = irc_delta_carve(pl, L.more, L.c.words + W_ERR);
-    k_cert_delta<<<(pl->dev.n_out + kWarps - 1) / kWarps, 32 * kWarps, 0, s>>>(L.c, R, nThreads, delta, nneigh, sc.counts,
+    launch_next(k_cert_delta, (pl->dev.n_out + kWarps - 1) / kWarps, 32 * kWarps, 0, s, L.c, R, nThreads, delta, nneigh, sc.counts,
                                                                              sc.list);
     IRC_CHECK_LAUNCH("irc_site_delta lists");
     return irc_delta_window(pl, F, nC, R, nThreads, sc, delta, nneigh, s);

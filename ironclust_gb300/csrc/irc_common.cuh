@@ -76,3 +76,45 @@ int check_plan(const char *who, const int32_t *q0, const int32_t *nq, const int3
 // created (+1) or destroyed (-1) on a device.
 cudaError_t irc_scratch_alloc(void **p, size_t bytes, cudaStream_t s);
 void irc_scratch_plan(int dev, int change);
+
+// Kernels of one call that follow each other without a copy or a memset in
+// between are launched so that the next one's blocks may start (and set up)
+// while the last blocks of the one before still run.  Every thread of such a
+// kernel calls after_previous() before it touches global memory, which waits
+// until the kernel before is complete and its writes are visible -- also the
+// threads with nothing to do: a kernel is then never complete before the one in
+// front of it.  Read-only loads (__ldg, const __restrict__) may be moved over
+// the wait by the compiler, so the pointers to what an earlier kernel of the
+// call wrote are passed in and come out of an asm behind it.
+// A call of ten kernels on 3,000 spikes takes 98 us instead of 111.  Kernels
+// of many blocks are launched the plain way: the wait is a cost of every block
+// (re-rank of 625,000 queries, 78,000 blocks, about 300 us in all).
+template <class T>
+__device__ __forceinline__ void behind_wait(T &p)
+{
+    static_assert(sizeof(T) == 8, "a pointer");
+    asm volatile("" : "+l"(p)::"memory");
+}
+
+template <class... T>
+__device__ __forceinline__ void after_previous(T &...p)
+{
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+    (behind_wait(p), ...);
+}
+
+template <class... P, class... A>
+cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = grid.x <= 152u * 8u ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}

@@ -127,6 +127,7 @@ k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
                  float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
                  float *__restrict__ d2Knn, int *__restrict__ ovf_count, int *__restrict__ ovf_list, irc::TileQueue tq)
 {
+    after_previous(tq.list, tq.count, tq.all);
     __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
     __shared__ float sTau[kQB];
     __shared__ int sCnt[kQB];
@@ -230,6 +231,7 @@ k_exact_overflow(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
                  float *__restrict__ vrKnn, float *__restrict__ rho,
                  int *__restrict__ miKnn, float *__restrict__ d2Knn)
 {
+    after_previous(ovf_count, ovf_list);
     __shared__ unsigned long long red[kThreads / 32];
     __shared__ unsigned long long sBest;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -290,6 +292,7 @@ k_delta_list(irc::PlanDev p, int ntiles, const float *__restrict__ R, int knn, c
              const float *__restrict__ d2Knn, float *__restrict__ delta, int *__restrict__ nneigh,
              int *__restrict__ counts, int *__restrict__ fb_list)
 {
+    after_previous();
     const int lane = threadIdx.x & 31, tile = blockIdx.x * kListWarps + (threadIdx.x >> 5);
     if (tile >= ntiles) return;
     int chunk, qs, n;
@@ -354,6 +357,7 @@ __global__ void k_delta_items(irc::PlanDev p, const int *__restrict__ all, const
                               int *__restrict__ fb_list, int *__restrict__ words, int2 *__restrict__ sparse,
                               int2 *__restrict__ items, unsigned long long *__restrict__ keys)
 {
+    after_previous(all, counts);
     const int chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (chunk >= p.nChunks) return;
     const int q0 = __ldg(p.q0 + chunk), nq = __ldg(p.nq + chunk);
@@ -519,6 +523,7 @@ k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restr
                const int2 *__restrict__ items, const int *__restrict__ fb_list, unsigned long long *__restrict__ keys,
                int nT, float *__restrict__ delta, int *__restrict__ nneigh)
 {
+    after_previous(words, sparse, items, fb_list);
     __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
     __shared__ float sRA[kQB];
     __shared__ int sQ[kQB];
@@ -632,6 +637,7 @@ __global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, cons
                                const unsigned long long *__restrict__ keys, float *__restrict__ delta,
                                int *__restrict__ nneigh, int nT)
 {
+    after_previous(words, sparse, items, fb_list, keys);
     const int total = words[0] * kQB, n_wide = words[1];
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_wide; t += gridDim.x * blockDim.x) {
         const int2 e = sparse[t];
@@ -668,10 +674,10 @@ int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn,
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): smem attribute");
     const int tiles = pl->ntiles[irc::tile_slot(kQB)];
     const int grid = tq.list && tiles > kQueueBlocks ? kQueueBlocks : tiles;
-    k_site_knn_exact<<<grid, kThreads, smem, s>>>(pl->dev, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, ovf_list, tq);
+    launch_next(k_site_knn_exact, grid, kThreads, smem, s, pl->dev, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, ovf_list, tq);
     IRC_CHECK_LAUNCH("irc_site_knn(EXACT)");
     // the overflow list is usually empty; size the grid for the worst case
-    k_exact_overflow<<<kQueueBlocks, 256, 0, s>>>(
+    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, 
         pl->dev, F, nC, knn, cnt, ovf_list, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn(EXACT) overflow");
     return IRC_OK;
@@ -697,7 +703,7 @@ int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, in
     cudaError_t e = irc_delta_clear(pl, sc, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: memset");
     const int tiles = pl->ntiles[irc::tile_slot(kListTile)];
-    k_delta_list<<<(tiles + kListWarps - 1) / kListWarps, 32 * kListWarps, 0, s>>>(
+    launch_next(k_delta_list, (tiles + kListWarps - 1) / kListWarps, 32 * kListWarps, 0, s, 
         pl->dev, tiles, R, knn, miKnn, d2Knn, delta, nneigh, sc.counts, sc.list);
     IRC_CHECK_LAUNCH("irc_site_delta list");
     return irc_delta_window(pl, F, nC, R, 0, sc, delta, nneigh, s);
@@ -733,7 +739,7 @@ cudaError_t irc_delta_clear(const irc_plan *pl, const irc_delta_scratch &sc, cud
 int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int nT, const irc_delta_scratch &sc,
                      float *delta, int32_t *nneigh, cudaStream_t s)
 {
-    k_delta_items<<<(pl->dev.nChunks + 7) / 8, 256, 0, s>>>(pl->dev, sc.all, sc.counts, sc.list, sc.words, sc.sparse,
+    launch_next(k_delta_items, (pl->dev.nChunks + 7) / 8, 256, 0, s, pl->dev, sc.all, sc.counts, sc.list, sc.words, sc.sparse,
                                                             sc.items, sc.keys);
     IRC_CHECK_LAUNCH("irc_site_delta items");
     auto window = nT > 0 ? k_delta_window<true> : k_delta_window<false>;
@@ -741,10 +747,10 @@ int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int n
     const size_t smem = (size_t)(kThreads / 32) * 32 * irc::row_pitch(nC) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(window, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_delta: smem attribute");
-    window<<<kQueueBlocks, kThreads, smem, s>>>(pl->dev, F, R, nC, pl->row_dims, sc.words, sc.sparse, sc.items, sc.list,
+    launch_next(window, kQueueBlocks, kThreads, smem, s, pl->dev, F, R, nC, pl->row_dims, sc.words, sc.sparse, sc.items, sc.list,
                                              sc.keys, nT, delta, nneigh);
     IRC_CHECK_LAUNCH("irc_site_delta window");
-    finish<<<kQueueBlocks / 4, kThreads, 0, s>>>(pl->dev, R, sc.words, sc.sparse, sc.items, sc.list, sc.keys, delta, nneigh, nT);
+    launch_next(finish, kQueueBlocks / 4, kThreads, 0, s, pl->dev, R, sc.words, sc.sparse, sc.items, sc.list, sc.keys, delta, nneigh, nT);
     IRC_CHECK_LAUNCH("irc_site_delta finish");
     return IRC_OK;
 }
@@ -756,7 +762,7 @@ int irc_exact_overflow_drain(irc_plan *pl, const float *F, int nC, int knn, floa
 {
     int *cnt, *la, *lb;
     irc_plan_scratch(pl, &cnt, &la, &lb);
-    k_exact_overflow<<<kQueueBlocks, 256, 0, s>>>(pl->dev, F, nC, knn, cnt, la, vrKnn, rho, miKnn, d2Knn);
+    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, pl->dev, F, nC, knn, cnt, la, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn overflow drain");
     return IRC_OK;
 }
@@ -902,9 +908,9 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn_exact_noalloc: smem attribute");
     int32_t *cnt = base, *queue = base + irc::kScratchLists;
-    k_site_knn_exact<<<(unsigned)tiles, kThreads, smem, s>>>(p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, irc::TileQueue{});
+    launch_next(k_site_knn_exact, (unsigned)tiles, kThreads, smem, s, p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, irc::TileQueue{});
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc");
-    k_exact_overflow<<<kQueueBlocks, 256, 0, s>>>(p, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
+    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, p, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc overflow");
     return IRC_OK;
 }

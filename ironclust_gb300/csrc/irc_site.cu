@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(kThreads)
 k_site_knn_ref(irc::PlanDev p, const float *__restrict__ F, int nC, int nT, int knn,
                float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn, irc::TileQueue tq)
 {
+    after_previous(tq.list, tq.count, tq.all);
     constexpr int QB = kKnnQB;
     __shared__ __align__(16) float sA[IRC_NC_MAX * QB];
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -345,7 +346,7 @@ int irc_ref_tiles(irc_plan *pl, const float *F, int nC, int knn, int nThreads, f
     cudaError_t e = cudaFuncSetAttribute(k_site_knn_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: smem attribute");
     const int tiles = tiles_for(pl, kKnnQB), grid = tq.list ? std::min(tiles, 152) : tiles;
-    k_site_knn_ref<<<grid, kThreads, smem, s>>>(pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
+    launch_next(k_site_knn_ref, grid, kThreads, smem, s, pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
     IRC_CHECK_LAUNCH("irc_site_knn(REF)");
     return IRC_OK;
 }

@@ -1095,6 +1095,7 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
     __syncthreads();
     sm100::tc_fence_after();
     const uint32_t tmem = *sh.tmem_slot;
+    after_previous();
 
     if (warp == 0) {
         produce<BN, NS, BIG, PASS>(tmQ, tmC, p, items, n_items, queue, sh, lo.split, lane);
@@ -1118,6 +1119,7 @@ k_knn_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
 __global__ void __launch_bounds__(BM) k_publish(irc::PlanDev p, const irc_tc::TcItem *__restrict__ items,
                                                 irc_tc::ListOut lo, int *__restrict__ scratch)
 {
+    after_previous(lo.split.cnt);
     const irc_tc::TcItem &it = items[blockIdx.x];
     const int row = threadIdx.x, slot = blockIdx.x * BM + row;
     if (row >= it.nq[0]) return;
@@ -1146,6 +1148,7 @@ k_rerank(const int2 *__restrict__ qinfo, const uint32_t *__restrict__ lists, int
          int knn, float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
          float *__restrict__ d2Knn, int margin, int *__restrict__ scratch)
 {
+    after_previous(qinfo, lists, Fp);
     __shared__ __align__(16) unsigned long long wkeys[RR_WARPS * WARP_KEYS];
     __shared__ float4 qrows[RR_WARPS * QROW4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1204,7 +1207,7 @@ static int launch_filter(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan 
     // persistent: one CTA per SM (shared memory and TMEM allow one), each
     // taking items from the queue until it is empty
     const int grid = n_items < sms ? n_items : sms;
-    kern<<<grid, THREADS, smem, s>>>(mq, mc, pl->dev, items, n_items, queue, nk, tau_k, lo, scratch);
+    launch_next(kern, grid, THREADS, smem, s, mq, mc, pl->dev, items, n_items, queue, nk, tau_k, lo, scratch);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core)");
     return IRC_OK;
 }
@@ -1221,13 +1224,11 @@ static int launch_split(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *
     const SplitOut &sp = lo.split;
     cudaError_t e = cudaFuncSetAttribute(pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(pass2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaMemsetAsync(sp.colmin, 0x7f, (size_t)sp.items * BM * 128 * 4, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(sp.cnt, 0, (size_t)sp.items * BM * 4, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): split items");
     const int n = sp.items * sp.parts;
-    pass1<<<n, THREADS, smem, s>>>(mq, mc, pl->dev, items, n, nullptr, nk, tau_k, lo, scratch);
-    pass2<<<n, THREADS, smem, s>>>(mq, mc, pl->dev, items, n, nullptr, nk, tau_k, lo, scratch);
-    k_publish<<<sp.items, BM, 0, s>>>(pl->dev, items, lo, scratch);
+    launch_next(pass1, n, THREADS, smem, s, mq, mc, pl->dev, items, n, nullptr, nk, tau_k, lo, scratch);
+    launch_next(pass2, n, THREADS, smem, s, mq, mc, pl->dev, items, n, nullptr, nk, tau_k, lo, scratch);
+    launch_next(k_publish, sp.items, BM, 0, s, pl->dev, items, lo, scratch);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core) split items");
     return IRC_OK;
 }
@@ -1271,14 +1272,20 @@ void split_area(const irc_plan *pl, int nC, Fmt fmt, void *mem, ListOut *lo)
     lo->split = sp;
 }
 
+cudaError_t clear_lists(const ListOut &lo, int n_out, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(lo.qinfo, 0xff, (size_t)n_out * sizeof(int2), s);   // (-1, -1): no list
+    if (e == cudaSuccess) e = cudaMemsetAsync(lo.count, 0, 4 * sizeof(unsigned), s);     // count, queue heads
+    const SplitOut &sp = lo.split;
+    if (e == cudaSuccess && sp.items) e = cudaMemsetAsync(sp.colmin, 0x7f, (size_t)sp.items * BM * 128 * 4, s);
+    if (e == cudaSuccess && sp.items) e = cudaMemsetAsync(sp.cnt, 0, (size_t)sp.items * BM * 4, s);
+    return e;
+}
+
 // The filter of every packing class of the plan on stream s.
 int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, int nC, const ListOut &lo,
                    int *scratch, cudaStream_t s)
 {
-    const int n_out = pl->dev.n_out;
-    cudaError_t e = cudaMemsetAsync(lo.qinfo, 0xff, (size_t)n_out * sizeof(int2), s);   // (-1, -1): no list
-    if (e == cudaSuccess) e = cudaMemsetAsync(lo.count, 0, 4 * sizeof(unsigned), s);     // count, queue heads
-    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): memset");
     // BF16, F16: the pass-2 thresholds go into K positions nC + 6 .. nC + 8 of
     // the query rows when they fit (else, and for FP8, pass 2 compares in the
     // epilogue).  MMAs per unit: only the 32-byte K slices that hold data
@@ -1332,7 +1339,7 @@ int launch_knn_tc(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_pla
     const int rc = launch_filters(fmt, mq, mc, pl, nC, lo, pl->scratch, s);
     if (rc != IRC_OK) return rc;
     if (ev) cudaEventRecord(ev[1], s);
-    k_rerank<<<(n_out + RR_WARPS - 1) / RR_WARPS, 32 * RR_WARPS, 0, s>>>(
+    launch_next(k_rerank, (n_out + RR_WARPS - 1) / RR_WARPS, 32 * RR_WARPS, 0, s, 
         lo.qinfo, lo.lists, n_out, pl->dev.q_base, F, Fp, nC, pl->row_dims, knn, vrKnn, rho, miKnn, d2Knn,
         crowd_margin(fmt), pl->scratch);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core) re-rank");

@@ -88,6 +88,10 @@ int launch_knn_tc(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_pla
                   const float4 *Fp, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn, float *d2Knn,
                   const ListOut &lo, cudaStream_t s);
 
+// What the filter expects cleared (before the operands are made: nothing then
+// stands between the kernels).
+cudaError_t clear_lists(const ListOut &lo, int n_out, cudaStream_t s);
+
 // The filter alone; scratch: the counter words of its overflow queue and error
 // word (irc_plan.cuh), the queue after them (unused when lo.cert is set).
 int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *pl, int nC, const ListOut &lo,

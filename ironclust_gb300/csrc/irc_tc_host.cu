@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(kMeanThreads)
 k_centre(const float *__restrict__ F, int nC, int stride, int nS, float *__restrict__ part, unsigned *__restrict__ ticket,
          float *__restrict__ ref, const unsigned *__restrict__ amax, float *__restrict__ scale)
 {
+    after_previous(amax);
     __shared__ double red[kMeanThreads];
     __shared__ bool last;
     const int t = threadIdx.x, lanes = kMeanThreads / nC, rl = t / nC, c = t - rl * nC;
@@ -109,6 +110,7 @@ k_centre(const float *__restrict__ F, int nC, int stride, int nS, float *__restr
 // integer max == float max).
 __global__ void k_absmax_finite(const float *__restrict__ F, size_t n, unsigned *__restrict__ out)
 {
+    after_previous();
     unsigned m = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const unsigned b = __float_as_uint(fabsf(__ldg(F + i)));
@@ -122,6 +124,7 @@ __global__ void k_absmax_finite(const float *__restrict__ F, size_t n, unsigned 
 __global__ void k_absmax(const float *__restrict__ F, size_t n, int nC, const float *__restrict__ ref,
                          unsigned *__restrict__ out)
 {
+    after_previous(ref);
     unsigned m = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         m = max(m, __float_as_uint(fabsf(__ldg(F + i) - __ldg(ref + i % nC))));
@@ -204,6 +207,7 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
        const unsigned *__restrict__ amax, uint4 *__restrict__ Fq, uint4 *__restrict__ Fc, float *__restrict__ Fp,
        int Dp4, int q_lo, int q_hi, const float *__restrict__ scale, float *__restrict__ qnorm)
 {
+    after_previous(ref, amax, scale);
     extern __shared__ __align__(16) unsigned char prep_sm[];
     const int nCs = nC | 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -408,14 +412,14 @@ int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsi
     if (f16) {                                                        // (its scale takes the maximum)
         for (int v = 0; v < pl->n_row_iv; ++v) {
             const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
-            k_absmax_finite<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, amax);
+            launch_next(k_absmax_finite, 152 * 4, 256, 0, s, F + (size_t)lo * nC, (size_t)n * nC, amax);
         }
-        k_centre<true><<<kMeanBlocks, kMeanThreads, 0, s>>>(Fq0, nC, stride, nS, part, ticket, ref, amax, scale);
+        launch_next(k_centre<true>, kMeanBlocks, kMeanThreads, 0, s, Fq0, nC, stride, nS, part, ticket, ref, amax, scale);
     } else {
-        k_centre<false><<<kMeanBlocks, kMeanThreads, 0, s>>>(Fq0, nC, stride, nS, part, ticket, ref, nullptr, nullptr);
+        launch_next(k_centre<false>, kMeanBlocks, kMeanThreads, 0, s, Fq0, nC, stride, nS, part, ticket, ref, nullptr, nullptr);
         for (int v = 0; fp8 && v < pl->n_row_iv; ++v) {
             const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
-            k_absmax<<<152 * 4, 256, 0, s>>>(F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
+            launch_next(k_absmax, 152 * 4, 256, 0, s, F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
         }
     }
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core) centre");
@@ -427,7 +431,7 @@ int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsi
     for (int v = 0; v < pl->n_row_iv; ++v) {
         const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
         const int rows_per_block = 32 * kPrepWarps;
-        prep<<<(n + rows_per_block - 1) / rows_per_block, 32 * kPrepWarps, psm, s>>>(
+        launch_next(prep, (n + rows_per_block - 1) / rows_per_block, 32 * kPrepWarps, psm, s, 
             F, lo, n, nC, ref, amax, (uint4 *)fq, (uint4 *)fc, (float *)fp, Dp4, pl->dev.q_base,
             pl->dev.q_base + pl->dev.n_out, scale, qnorm);
     }
@@ -463,6 +467,7 @@ int irc_site_knn_tc(irc_plan *pl, const float *F, int nC, int knn, int mode, flo
     irc_tc::ListOut lo = irc_tc::list_area((char *)buf + ops, pl->dev.n_out);
     if (split) irc_tc::split_area(pl, nC, fmt, (char *)buf + need, &lo);
     cudaError_t e = cudaMemsetAsync(pl->scratch, 0, 2 * sizeof(int), s);   // overflow-queue count, largest magnitude
+    if (e == cudaSuccess) e = irc_tc::clear_lists(lo, pl->dev.n_out, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(BF16): memset");
     irc_tc::Operands op;
     unsigned *words = reinterpret_cast<unsigned *>(pl->scratch);
