@@ -214,13 +214,15 @@ int irc_plan_tc_units(irc_plan *plan, int width);
  * row_base[k] .. row_base[k+1]-1 of F belong to site k, whose features past
  * dims[k] are zero in every row (as irc_batch_stack writes them); row_base
  * spans the plan's nF rows, and every chunk's queries and candidates must lie
- * in one site (checked).  The tensor-core re-rank and the delta fallback
+ * in one site (checked).  The tensor-core re-rank and the delta window
  * scan then skip each query's zero features: same results, less work.
  * nSites = 0 clears it.  No reference counterpart. */
 int irc_plan_set_site_dims(irc_plan *plan, int nSites, const int64_t *row_base, const int32_t *dims);
 
 /* Working memory of the tensor-core modes: bytes a plan needs for nC
- * features (operand rows of all nF columns + their padded FP32 copy).  By
+ * features (operand rows of all nF columns + their padded FP32 copy, candidate
+ * lists; with less than this, down to what the plan cannot do without, calls
+ * run without splitting work items).  By
  * default a plan allocates it on its first tensor-core call and keeps it;
  * irc_plan_set_tc_buffer hands it caller-owned device memory of `bytes`
  * instead, which several plans can share when their calls are serialised on
@@ -253,7 +255,11 @@ int irc_profile_end(float *filter_ms, float *rerank_ms, int *calls);
  * vrKnn [n_out]: distance of the knn-th neighbour; rho [n_out] (optional) =
  * 1 ./ vrKnn; miKnn [knn x n_out]: 1-based indices into F; d2Knn
  * [knn x n_out] (optional, not in REF mode): squared distances.
- * REF mode = search_min_drift with nThreads bins + MATLAB sort, bit-exact. */
+ * REF mode = search_min_drift with nThreads bins + MATLAB sort, bit-exact.
+ * Large enough REF and EXACT calls search with the tensor cores and prove
+ * every query's result (else its tile is searched in plain FP32): same bits.
+ * They take stream-ordered working memory from a pool of the library's, or do
+ * without it when there is none. */
 int irc_site_knn(irc_plan *plan, const float *F, int nC, int knn, int nThreads, int mode,
                  float *vrKnn, float *rho, int32_t *miKnn, float *d2Knn, void *stream);
 

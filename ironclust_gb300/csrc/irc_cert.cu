@@ -32,8 +32,9 @@
 // because the candidate's norm is bounded through the triangle inequality.
 //
 // Measured: EXACT kNN + delta of 100,003 spikes (D = 33, 50 chunks, 3.0e9
-// pairs) 22.2 -> 1.42 ms; REF kNN + delta of 60,001 spikes and 12,001 copies
-// (D = 24, 30 chunks, 2.2e9 pairs) 29.4 -> 2.74 ms.  The contraction's error,
+// pairs) 22.2 -> 1.09 ms; REF kNN + delta of 60,001 spikes and 12,001 copies
+// (D = 24, 30 chunks, 2.2e9 pairs) 29.2 -> 1.46 ms (a site with one
+// query without a proof: 0.2 to 0.3 more, a 16-query tile on one SM).  The contraction's error,
 // on rows of this layout against FP64, is at most 2^-20.7 of the sum that c
 // multiplies.
 #include <algorithm>

@@ -46,10 +46,11 @@
 //           against 1s in the candidate rows, so the accumulators are
 //           d2 - tau and a hit is a sign bit (one funnel shift per pair);
 //           elsewhere every pair is compared with tau in the epilogue.
-// The minima partition is the same at both widths, so results never depend
-// on the width or the work layout.  Measured on 400,000 spikes, D = 33 (1.2e10
+// The minima partition, and with it tau, is the same at both widths and in every
+// layout (the lists of folded thresholds also hold what lies within 2^-10 above
+// tau).  Measured on 400,000 spikes, D = 33 (1.2e10
 // pairs, one launch): 3.65 ms with one MMA issuer, three stages and late
-// releases, 3.10 ms as above; without any epilogue work the pipeline takes
+// releases, 3.02 ms as above; without any epilogue work the pipeline takes
 // 1.81, and folding, marking and appending add 0.35, 0.48 and 0.46.
 // Every listed candidate is then re-ranked
 // with the reference FP32 arithmetic (exact), zero distances dropped, sorted
@@ -154,8 +155,8 @@ struct Tile {
 // stage (the second absent when the count is odd).  Either way epilogue warp
 // w of a lane quarter reads columns 32w .. 32w + 31 of every 128-tile, and
 // per-column minimum i of that warp covers column 32w + i of every tile, so
-// the minima, the threshold and the candidate lists do not depend on the
-// width, nor on the work layout.
+// the minima and the threshold do not depend on the width, nor on the work
+// layout.
 template <int BN>
 __device__ __forceinline__ int units_per_pass(int nts)
 {
