@@ -35,9 +35,10 @@
 //  * Cluster sizes.  A shared-memory histogram (or warp-aggregated global
 //    atomics for many clusters), a scan of the keep flags, one remap pass.
 //
-// Host round trips: the peak count, each cell2map_ repeat's stop test, the
-// cluster count, each pass's unassigned count and convergence checks of the
-// jumping rounds, the final counts.  The call synchronises its stream.
+// Host round trips (about 12 us each): the peak count, every second cell2map_
+// repeat's stop test, the cluster count, after every eight jumping rounds of a
+// pass what is unresolved and unassigned, the final counts.  The call
+// synchronises its stream.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -213,8 +214,9 @@ __global__ void k_row_count(const uint32_t *__restrict__ S, int P, int W, int *_
 // member; owner[m] = the largest such i whose union holds m (cvi_clu1(viClu1)
 // = {viClu1} visits iClu ascending, so the last writer is the largest).
 __global__ void k_union(const uint32_t *__restrict__ S, const int *__restrict__ cnt, int P, int W,
-                        uint32_t *__restrict__ U, int *__restrict__ ucnt, int *__restrict__ owner)
+                        uint32_t *__restrict__ U, int *__restrict__ ucnt, int *__restrict__ owner, const int *before)
 {
+    if (before && !*before) return;               // (uniform) the repeat before changed nothing: the loop has ended
     extern __shared__ uint32_t sm[];
     uint32_t *row = sm, *acc = sm + W;
     const int i = blockIdx.x;
@@ -253,8 +255,10 @@ __global__ void k_union(const uint32_t *__restrict__ S, const int *__restrict__ 
 
 // the new set sizes, and whether any differs from the old (the stop test)
 __global__ void k_new_count(const int *__restrict__ owner, const int *__restrict__ ucnt,
-                            const int *__restrict__ cnt, int P, int *__restrict__ ncnt, int *__restrict__ changed)
+                            const int *__restrict__ cnt, int P, int *__restrict__ ncnt, int *__restrict__ changed,
+                            const int *before)
 {
+    if (before && !*before) return;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= P) return;
     const int o = owner[m];
@@ -265,8 +269,9 @@ __global__ void k_new_count(const int *__restrict__ owner, const int *__restrict
 
 // cvi_clu = cvi_clu1: row m becomes its owner's union (empty without owner)
 __global__ void k_gather(const int *__restrict__ owner, const uint32_t *__restrict__ U, int W,
-                         uint32_t *__restrict__ S, int *__restrict__ cnt, const int *__restrict__ ncnt)
+                         uint32_t *__restrict__ S, int *__restrict__ cnt, const int *__restrict__ ncnt, const int *changed)
 {
+    if (!*changed) return;
     const int m = blockIdx.x, o = owner[m];
     uint32_t *Sm = S + (size_t)m * W;
     if (o >= 0) {
@@ -400,8 +405,9 @@ __global__ void k_jump(const unsigned long long *__restrict__ src, unsigned long
 
 __global__ void k_pass_finish(const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
                               const int *__restrict__ lastbuf, const int64_t *__restrict__ ordrho, int64_t n,
-                              int32_t *__restrict__ viClu, int *__restrict__ zeros)
+                              int32_t *__restrict__ viClu, int *__restrict__ zeros, const int *left)
 {
+    if (left && *left) return;                    // more rounds follow
     const int64_t r0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t r = r0 < n ? r0 : n - 1;
     const unsigned long long w = (*lastbuf ? b : a)[r];
@@ -460,9 +466,10 @@ __global__ void k_remap(int32_t *__restrict__ viClu, int64_t n, int nIcl, const 
 
 __global__ void k_centres(const int64_t *__restrict__ icl_tmp, const int *__restrict__ cnt, int nIcl,
                           const int *__restrict__ keep, const int *__restrict__ newid, int64_t cap,
-                          int64_t *__restrict__ icl, int32_t *__restrict__ vn)
+                          int64_t *__restrict__ icl, int32_t *__restrict__ vn, int *__restrict__ n_keep)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    if (c == nIcl) *n_keep = newid[nIcl];
     if (c > nIcl || !keep[c]) return;
     const int64_t o = newid[c] - 1;
     if (o < cap) {
@@ -537,6 +544,7 @@ cudaError_t exclusive_sum(Scratch &sc, const int *in, int *out, int n)
 
 constexpr int JUMP_BATCH = 8;      // pointer-jumping rounds between convergence checks
 constexpr int JUMP_MAX = 32;       // 2^32 > any chain length
+constexpr int REPEATS = 10;        // cell2map_'s
 
 }  // namespace
 
@@ -582,12 +590,14 @@ extern "C" int irc_assign_cluster_knn(int32_t *viClu, int64_t *icl, int32_t *vnS
     }
     const int64_t n = nSpk;
     Scratch sc(s);
-    // hdr: [0] error bits, [1] stop test of a cell2map_ repeat, [2] unassigned count, [3] state buffer
-    int *hdr = sc.get<int>(4);
+    // hdr: [0] error bits, [1] clusters kept, [2] unassigned count, [3] state buffer, the unresolved
+    // counts of a pass's rounds, the stop tests of the cell2map_ repeats
+    constexpr int kHdr = 4 + (JUMP_MAX + 1) + REPEATS;
+    int *hdr = sc.get<int>(kHdr), *act = hdr + 4, *chg = act + JUMP_MAX + 1;
     const int nb = (int)((n + CTILE - 1) / CTILE);
     int *bcount = sc.get<int>(nb + 1), *boff = sc.get<int>(nb + 1);
     IRC_TRY(sc.err, "irc_assign_cluster_knn: scratch");
-    IRC_TRY(cudaMemsetAsync(hdr, 0, 4 * sizeof(int), s), "irc_assign_cluster_knn");
+    IRC_TRY(cudaMemsetAsync(hdr, 0, kHdr * sizeof(int), s), "irc_assign_cluster_knn");
 
     // viSpk_peak = find(vrDelta_spk(:) >= delta_cut)
     k_peak_count<<<nb, TPB, 0, s>>>(delta, n, delta_cut, bcount);
@@ -637,15 +647,19 @@ extern "C" int irc_assign_cluster_knn(int32_t *viClu, int64_t *icl, int32_t *vnS
         if (usmem > 48 * 1024)
             IRC_TRY(cudaFuncSetAttribute(k_union, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem),
                     "irc_assign_cluster_knn: union smem");
-        for (int rep = 0; rep < 10; ++rep) {
+        // (the kernels of a repeat find out on the device whether the loop has
+        // ended; the host asks after every second one)
+        for (int rep = 0; rep < REPEATS; ++rep) {
+            const int *before = rep ? chg + rep - 1 : nullptr;
             IRC_TRY(cudaMemsetAsync(owner, 0xff, sizeof(int) * (size_t)P, s), "irc_assign_cluster_knn");
-            IRC_TRY(cudaMemsetAsync(hdr + 1, 0, sizeof(int), s), "irc_assign_cluster_knn");
-            k_union<<<P, 128, usmem, s>>>(S, cnt, P, W, U, ucnt, owner);
-            k_new_count<<<blocks_for(P), TPB, 0, s>>>(owner, ucnt, cnt, P, ncnt, hdr + 1);
-            int changed = 0;
-            IRC_TRY(read_back(&changed, hdr + 1, 1, s), "irc_assign_cluster_knn: cell2map_");
-            if (!changed) break;
-            k_gather<<<P, 128, 0, s>>>(owner, U, W, S, cnt, ncnt);
+            k_union<<<P, 128, usmem, s>>>(S, cnt, P, W, U, ucnt, owner, before);
+            k_new_count<<<blocks_for(P), TPB, 0, s>>>(owner, ucnt, cnt, P, ncnt, chg + rep, before);
+            k_gather<<<P, 128, 0, s>>>(owner, U, W, S, cnt, ncnt, chg + rep);
+            if (rep % 2 == 1) {
+                int changed = 0;
+                IRC_TRY(read_back(&changed, chg + rep, 1, s), "irc_assign_cluster_knn: cell2map_");
+                if (!changed) break;
+            }
         }
         // viMapClu, viUniq_ and the compacted map
         IRC_TRY(cudaMemsetAsync(isrep, 0, sizeof(int) * (size_t)(P + 1), s), "irc_assign_cluster_knn");
@@ -665,28 +679,25 @@ extern "C" int irc_assign_cluster_knn(int32_t *viClu, int64_t *icl, int32_t *vnS
         // ranks (ordrho must be a permutation), then at most ten passes
         int32_t *rank = sc.get<int32_t>(n);
         unsigned long long *stA = sc.get<unsigned long long>(n), *stB = sc.get<unsigned long long>(n);
-        int *act = sc.get<int>(JUMP_MAX + 1);
         IRC_TRY(sc.err, "irc_assign_cluster_knn: propagation scratch");
         IRC_TRY(cudaMemsetAsync(rank, 0xff, sizeof(int32_t) * (size_t)n, s), "irc_assign_cluster_knn");
         k_rank<<<blocks_for(n), TPB, 0, s>>>(ordrho, n, rank, hdr);
         for (int pass = 0; pass < 10; ++pass) {
-            IRC_TRY(cudaMemsetAsync(act, 0, sizeof(int) * (JUMP_MAX + 1), s), "irc_assign_cluster_knn");
-            IRC_TRY(cudaMemsetAsync(hdr + 2, 0, sizeof(int), s), "irc_assign_cluster_knn");
+            IRC_TRY(cudaMemsetAsync(hdr + 2, 0, sizeof(int) * (2 + JUMP_MAX + 1), s), "irc_assign_cluster_knn");
             k_pass_state<<<blocks_for(n), TPB, 0, s>>>(ordrho, nneigh, rank, viClu, n, stA, act, hdr, hdr + 3);
+            int back[2 + JUMP_MAX + 1] = {};              // hdr[2 ..]: unassigned, state buffer, the rounds
             for (int round = 1; round <= JUMP_MAX; ++round) {
                 const bool odd = round & 1;
                 k_jump<<<blocks_for(n), TPB, 0, s>>>(odd ? stA : stB, odd ? stB : stA, n, act, round, hdr + 3,
                                                       odd ? 1 : 0);
                 if (round % JUMP_BATCH == 0) {
-                    int left = 0;
-                    IRC_TRY(read_back(&left, act + round, 1, s), "irc_assign_cluster_knn: propagation");
-                    if (left == 0) break;
+                    k_pass_finish<<<blocks_for(n), TPB, 0, s>>>(stA, stB, hdr + 3, ordrho, n, viClu, hdr + 2,
+                                                                round < JUMP_MAX ? act + round : nullptr);
+                    IRC_TRY(read_back(back, hdr + 2, 2 + round + 1, s), "irc_assign_cluster_knn: propagation");
+                    if (back[2 + round] == 0) break;
                 }
             }
-            k_pass_finish<<<blocks_for(n), TPB, 0, s>>>(stA, stB, hdr + 3, ordrho, n, viClu, hdr + 2);
-            int zeros = 0;
-            IRC_TRY(read_back(&zeros, hdr + 2, 1, s), "irc_assign_cluster_knn: propagation");
-            if (zeros == 0) break;
+            if (back[0] == 0) break;
         }
     }
     counts[2] = nIcl;
@@ -699,13 +710,12 @@ extern "C" int irc_assign_cluster_knn(int32_t *viClu, int64_t *icl, int32_t *vnS
     k_hist<<<gh, TPB, 0, s>>>(viClu, n, nIcl, ccnt);
     k_keep<<<blocks_for(nIcl + 1), TPB, 0, s>>>(ccnt, nIcl, min_count, keep);
     IRC_TRY(inclusive_sum(sc, keep, newid, nIcl + 1), "irc_assign_cluster_knn: keep scan");
-    int nKeep = 0;
-    IRC_TRY(read_back(&nKeep, newid + nIcl, 1, s), "irc_assign_cluster_knn: cluster count");
-    if (nKeep < nIcl) k_remap<<<blocks_for(n), TPB, 0, s>>>(viClu, n, nIcl, keep, newid);
-    k_centres<<<blocks_for(nIcl), TPB, 0, s>>>(icl_tmp, ccnt, nIcl, keep, newid, cap, icl, vnSpk_clu);
+    k_remap<<<blocks_for(n), TPB, 0, s>>>(viClu, n, nIcl, keep, newid);
+    k_centres<<<blocks_for(nIcl), TPB, 0, s>>>(icl_tmp, ccnt, nIcl, keep, newid, cap, icl, vnSpk_clu, hdr + 1);
+    int last[2] = {0, 0};
+    IRC_TRY(read_back(last, hdr, 2, s), "irc_assign_cluster_knn");
+    const int err = last[0], nKeep = last[1];
     counts[0] = nKeep;
-    int err = 0;
-    IRC_TRY(read_back(&err, hdr, 1, s), "irc_assign_cluster_knn");
     IRC_CHECK_LAUNCH("irc_assign_cluster_knn");
     if (err & ERR_ORDRHO_RANGE) {
         irc_host::set_error("irc_assign_cluster_knn: an ordrho entry is outside 1..nSpk");
