@@ -53,6 +53,9 @@ namespace {
 constexpr int TPB = 256;
 constexpr int CTILE = 2048;                         // compaction tile (8 items per thread)
 constexpr unsigned long long DONE = 1ull << 63;     // propagation state: resolved
+constexpr int JUMP_BATCH = 8;      // pointer-jumping rounds between convergence checks
+constexpr int JUMP_MAX = 32;       // 2^32 > any chain length
+constexpr int REPEATS = 10;        // cell2map_'s
 constexpr int ERR_ORDRHO_RANGE = 1, ERR_ORDRHO_PERM = 2, ERR_NNEIGH_RANGE = 4;
 
 unsigned blocks_for(int64_t n, int per = TPB)
@@ -353,37 +356,78 @@ __device__ __forceinline__ void count_warp(bool pred, int *ctr)
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(ctr, __popc(b));
 }
 
-// The state of one pass: resolved spikes carry DONE | label; an unassigned
-// spike whose nneigh is unassigned and ranked earlier points to that rank.
+// The state of rank r in one pass: resolved spikes carry DONE | label; an
+// unassigned spike whose nneigh is unassigned and ranked earlier points to
+// that rank.
+__device__ __forceinline__ unsigned long long pass_state(const int64_t *ordrho, const int64_t *nneigh, const int32_t *rank,
+                                                         const int32_t *viClu, int64_t n, int64_t r, int *err)
+{
+    const int64_t o = ordrho[r] - 1;
+    if (o < 0 || o >= n) return DONE;
+    const int32_t L = viClu[o];
+    if (L > 0) return DONE | (uint32_t)L;
+    const int64_t nn = nneigh[o];
+    if (nn < 1 || nn > n) {
+        atomicOr(err, ERR_NNEIGH_RANGE);
+        return DONE;
+    }
+    const int32_t Ln = viClu[nn - 1];
+    if (Ln > 0) return DONE | (uint32_t)Ln;
+    const int32_t t = rank[nn - 1];
+    return t >= 0 && t < r ? (unsigned long long)(uint32_t)t : DONE;   // else: nneigh is visited later (or itself): label 0
+}
+
 __global__ void k_pass_state(const int64_t *__restrict__ ordrho, const int64_t *__restrict__ nneigh,
                              const int32_t *__restrict__ rank, const int32_t *__restrict__ viClu, int64_t n,
                              unsigned long long *__restrict__ st, int *__restrict__ act, int *__restrict__ err,
                              int *__restrict__ lastbuf)
 {
-    const int64_t r0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r0 == 0) *lastbuf = 0;
-    const int64_t r = r0 < n ? r0 : n - 1;
-    unsigned long long w = DONE;
-    const int64_t o = ordrho[r] - 1;
-    if (o >= 0 && o < n) {
-        const int32_t L = viClu[o];
-        if (L > 0) {
-            w = DONE | (uint32_t)L;
-        } else {
-            const int64_t nn = nneigh[o];
-            if (nn < 1 || nn > n) {
-                if (r0 < n) atomicOr(err, ERR_NNEIGH_RANGE);
-            } else {
-                const int32_t Ln = viClu[nn - 1];
-                const int32_t t = rank[nn - 1];
-                if (Ln > 0) w = DONE | (uint32_t)Ln;
-                else if (t >= 0 && t < r) w = (unsigned long long)(uint32_t)t;
-                // else: nneigh is visited later (or is the spike itself): label 0
-            }
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r == 0) *lastbuf = 0;
+    const unsigned long long w = r < n ? pass_state(ordrho, nneigh, rank, viClu, n, r, err) : DONE;
+    if (r < n) st[r] = w;
+    count_warp(!(w & DONE), &act[0]);
+}
+
+// All passes of a small site in one block: nothing to ask the host, and one
+// launch where a pass takes ten.  From a few thousand spikes on the rounds of the whole
+// machine are faster than a block's.
+constexpr int SMALL_SITE = 4096;
+
+__global__ void __launch_bounds__(1024) k_passes(const int64_t *ordrho, const int64_t *nneigh, const int32_t *rank,
+                                                 int32_t *viClu, int n, unsigned long long *st0, unsigned long long *st1,
+                                                 int *err)
+{
+    for (int pass = 0; pass < 10; ++pass) {
+        unsigned long long *src = st0, *dst = st1;
+        int open = 0;
+        for (int r = threadIdx.x; r < n; r += 1024) {
+            const unsigned long long w = pass_state(ordrho, nneigh, rank, viClu, n, r, err);
+            src[r] = w;
+            open |= !(w & DONE);
         }
+        for (int round = 0; __syncthreads_or(open) && round < JUMP_MAX; ++round) {
+            open = 0;
+            for (int r = threadIdx.x; r < n; r += 1024) {
+                unsigned long long w = src[r];
+                if (!(w & DONE)) w = src[(uint32_t)w];
+                dst[r] = w;
+                open |= !(w & DONE);
+            }
+            unsigned long long *t = src;
+            src = dst;
+            dst = t;
+        }
+        int zeros = 0;
+        for (int r = threadIdx.x; r < n; r += 1024) {
+            const unsigned long long w = src[r];
+            const int32_t L = (w & DONE) ? (int32_t)(uint32_t)w : 0;
+            const int64_t o = ordrho[r] - 1;
+            if (o >= 0 && o < n) viClu[o] = L;
+            zeros |= L <= 0;
+        }
+        if (!__syncthreads_or(zeros)) break;
     }
-    if (r0 < n) st[r] = w;
-    count_warp(r0 < n && !(w & DONE), &act[0]);
 }
 
 // One pointer-jumping round, src -> dst; returns at once when the previous
@@ -542,9 +586,6 @@ cudaError_t exclusive_sum(Scratch &sc, const int *in, int *out, int n)
     return cub::DeviceScan::ExclusiveSum(tmp, tb, in, out, n, sc.s);
 }
 
-constexpr int JUMP_BATCH = 8;      // pointer-jumping rounds between convergence checks
-constexpr int JUMP_MAX = 32;       // 2^32 > any chain length
-constexpr int REPEATS = 10;        // cell2map_'s
 
 }  // namespace
 
@@ -682,7 +723,8 @@ extern "C" int irc_assign_cluster_knn(int32_t *viClu, int64_t *icl, int32_t *vnS
         IRC_TRY(sc.err, "irc_assign_cluster_knn: propagation scratch");
         IRC_TRY(cudaMemsetAsync(rank, 0xff, sizeof(int32_t) * (size_t)n, s), "irc_assign_cluster_knn");
         k_rank<<<blocks_for(n), TPB, 0, s>>>(ordrho, n, rank, hdr);
-        for (int pass = 0; pass < 10; ++pass) {
+        if (n <= SMALL_SITE) k_passes<<<1, 1024, 0, s>>>(ordrho, nneigh, rank, viClu, (int)n, stA, stB, hdr);
+        for (int pass = 0; n > SMALL_SITE && pass < 10; ++pass) {
             IRC_TRY(cudaMemsetAsync(hdr + 2, 0, sizeof(int) * (2 + JUMP_MAX + 1), s), "irc_assign_cluster_knn");
             k_pass_state<<<blocks_for(n), TPB, 0, s>>>(ordrho, nneigh, rank, viClu, n, stA, act, hdr, hdr + 3);
             int back[2 + JUMP_MAX + 1] = {};              // hdr[2 ..]: unassigned, state buffer, the rounds
