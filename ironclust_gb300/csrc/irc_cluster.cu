@@ -528,23 +528,39 @@ namespace {
 
 // Device scratch of one call: stream-ordered allocations, released in stream
 // order when the call returns.
+// Scratch of a call: pieces of a few blocks, given back with it.  (A block per
+// array was some fifty allocations and frees a call, 1 to 2 us each.)
 struct Scratch {
+    static constexpr size_t kBlock = 1 << 20;
     cudaStream_t s;
-    std::vector<void *> ptrs;
+    std::vector<void *> blocks;
+    char *at = nullptr;
+    size_t left = 0;
     cudaError_t err = cudaSuccess;
     explicit Scratch(cudaStream_t st) : s(st) {}
     template <class T>
     T *get(size_t n)
     {
-        void *q = nullptr;
-        if (err == cudaSuccess) err = irc_scratch_alloc(&q, sizeof(T) * (n ? n : 1), s);
+        const size_t bytes = (sizeof(T) * (n ? n : 1) + 255) & ~(size_t)255;
         if (err != cudaSuccess) return nullptr;
-        ptrs.push_back(q);
-        return (T *)q;
+        if (bytes > left) {
+            void *q = nullptr;
+            const size_t size = bytes > kBlock ? bytes : kBlock;
+            err = irc_scratch_alloc(&q, size, s);
+            if (err != cudaSuccess) return nullptr;
+            blocks.push_back(q);
+            if (size - bytes < left) return (T *)q;       // (the block before has more room left)
+            at = (char *)q;
+            left = size;
+        }
+        T *p = (T *)at;
+        at += bytes;
+        left -= bytes;
+        return p;
     }
     ~Scratch()
     {
-        for (void *q : ptrs) cudaFreeAsync(q, s);
+        for (void *q : blocks) cudaFreeAsync(q, s);
     }
 };
 
