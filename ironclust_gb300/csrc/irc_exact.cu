@@ -908,7 +908,7 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn_exact_noalloc: smem attribute");
     int32_t *cnt = base, *queue = base + irc::kScratchLists;
-    launch_next(k_site_knn_exact, (unsigned)tiles, kThreads, smem, s, p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, irc::TileQueue{});
+    k_site_knn_exact<<<(unsigned)tiles, kThreads, smem, s>>>(p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, irc::TileQueue{});
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc");
     launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, p, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc overflow");

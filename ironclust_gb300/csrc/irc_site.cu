@@ -346,7 +346,11 @@ int irc_ref_tiles(irc_plan *pl, const float *F, int nC, int knn, int nThreads, f
     cudaError_t e = cudaFuncSetAttribute(k_site_knn_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: smem attribute");
     const int tiles = tiles_for(pl, kKnnQB), grid = tq.list ? std::min(tiles, 152) : tiles;
-    launch_next(k_site_knn_ref, grid, kThreads, smem, s, pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
+    // (alone it follows what the caller launched, whose results it reads: the plain launch)
+    if (tq.list)
+        launch_next(k_site_knn_ref, grid, kThreads, smem, s, pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
+    else
+        k_site_knn_ref<<<grid, kThreads, smem, s>>>(pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
     IRC_CHECK_LAUNCH("irc_site_knn(REF)");
     return IRC_OK;
 }
