@@ -192,6 +192,15 @@ int irc_plan_destroy(irc_plan *plan);
  * flag.  No reference counterpart: the reference kernels have no waits. */
 int irc_plan_check(irc_plan *plan, void *stream);
 
+/* Where the plan's calls since the last one of this function went (host,
+ * counts[5]): {REF and EXACT kNN searches by proven lists, 16-query tiles
+ * they left to the plain kernels, queries that any kNN form finished by
+ * ordered scans (mass ties, lists that overflowed), REF delta searches by
+ * proven lists, queries they left to the window search}; clears them.
+ * Results never depend on it, only speed.  Synchronises `stream`.  No
+ * reference counterpart. */
+int irc_plan_search_counts(irc_plan *plan, int64_t *counts, void *stream);
+
 /* Layout of the plan's tensor-core work items (IRC_MODE_BF16 / FP8): chunks
  * with more than 64 queries run as 128-query CTAs; the remaining queries of
  * each chunk are packed up to max_slots chunks per CTA (1, 2 or 4; default

@@ -40,6 +40,7 @@ SIGNATURES = {
     "irc_plan_create": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I],
     "irc_plan_destroy": [_P],
     "irc_plan_check": [_P, _P],
+    "irc_plan_search_counts": [_P, _P, _P],
     "irc_plan_tc_layout": [_P, _I, _I],
     "irc_plan_tc_units": [_P, _I],
     "irc_plan_set_site_dims": [_P, _I, _P, _P],

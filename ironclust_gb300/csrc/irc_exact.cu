@@ -134,6 +134,10 @@ k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
     extern __shared__ __align__(16) unsigned char dyn[];
     unsigned long long *sList = reinterpret_cast<unsigned long long *>(dyn);   // [kQB][kCap]
     float *sMin = reinterpret_cast<float *>(sList + kQB * kCap);              // [kQB][kThreads]
+    if (tq.list && blockIdx.x == 0 && threadIdx.x == 0) {
+        irc::count_stat(p, irc::kStatSearches, 1);
+        irc::count_stat(p, irc::kStatTiles, tq.size());
+    }
     for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
         int chunk, qs, n;
         irc::tile_lookup<kQB>(p, tq.tile(w), chunk, qs, n);
@@ -236,6 +240,7 @@ k_exact_overflow(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
     __shared__ unsigned long long sBest;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = *ovf_count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) irc::count_stat(p, irc::kStatScans, n);
     for (int w = blockIdx.x; w < n; w += gridDim.x) {
         const int q = ovf_list[w];
         int lo = 0, hi = p.nChunks;
@@ -367,6 +372,10 @@ __global__ void k_delta_items(irc::PlanDev p, const int *__restrict__ all, const
         m = nq;
         for (int i = lane; i < m; i += 32) list[i] = q0 + i;
         __syncwarp();
+    }
+    if (all && lane == 0) {
+        irc::count_stat(p, irc::kStatDeltas, chunk == 0);
+        irc::count_stat(p, irc::kStatWindows, m);
     }
     if (m == 0) return;
     const int ncand = __ldg(p.ncand + chunk);
@@ -903,6 +912,7 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     p.ncand = nullptr;                                    // read only by the delta kernels
     p.tc_toff = nullptr;                                  // read only by the tensor-core filter
     p.tc_tiles = nullptr;
+    p.stat = nullptr;
     p.nChunks = nChunks; p.q_base = q_base; p.n_out = n_out; p.nF = nF; p.nRuns = nRuns;
     const size_t smem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
     e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -12,6 +12,12 @@ constexpr int kScratchErr = 2;
 constexpr int kScratchTicket = 3;
 constexpr int kScratchLists = 4;
 
+// Counters of irc_plan_search_counts (PlanDev::stat), summed by the kernels:
+// proven searches and the 16-query tiles they left to the plain kernel, queries
+// finished by ordered scans, proven delta searches and the queries they left
+// to the window search.
+enum { kStatSearches, kStatTiles, kStatScans, kStatDeltas, kStatWindows, kStatWords };
+
 // Query-tile sizes for which a plan precomputes its tile tables.
 constexpr int kTileSizes[] = {8, 16, 32, 64, 128};
 constexpr int kNumTileSizes = 5;
@@ -48,8 +54,14 @@ struct PlanDev {
     // so a 256-wide unit is one aligned int4.  Null in plans without it.
     const int32_t *tc_toff;                   // [nChunks+1]
     const int2 *tc_tiles;
+    unsigned long long *stat;                 // [kStatWords], or null: not counted
     int nChunks, q_base, n_out, nF, nRuns;
 };
+
+__device__ __forceinline__ void count_stat(const PlanDev &p, int which, int n)
+{
+    if (p.stat && n) atomicAdd(p.stat + which, (unsigned long long)n);
+}
 
 // The 16-query tiles a plain-form kernel works on: every tile of the plan, one
 // per block (list null), or the tiles a proven search left open (irc_cert.cu):

@@ -38,6 +38,10 @@ k_site_knn_ref(irc::PlanDev p, const float *__restrict__ F, int nC, int nT, int 
     extern __shared__ __align__(16) unsigned char dyn[];
     float *sV = reinterpret_cast<float *>(dyn);            // [QB][nT]  sqrt(|bin min|)
     int *sI = reinterpret_cast<int *>(sV + QB * nT);       // [QB][nT]  1-based index
+    if (tq.list && blockIdx.x == 0 && threadIdx.x == 0) {
+        irc::count_stat(p, irc::kStatSearches, 1);
+        irc::count_stat(p, irc::kStatTiles, tq.size());
+    }
     for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
         int chunk, qs, n;
         irc::tile_lookup<QB>(p, tq.tile(w), chunk, qs, n);
@@ -489,7 +493,8 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     // scratch: 4 words and two query lists of n_out, then the delta search's
     const size_t scratch_ints = irc::kScratchLists + 2 * (size_t)n_out + 64;
     const size_t delta_at = (img.size() + scratch_ints) / 64 * 64;          // 256-byte aligned
-    cudaError_t e = cudaMalloc(&pl->dmem, delta_at * sizeof(int32_t) + delta_bytes(n_out, nChunks));
+    const size_t stat_at = delta_at * sizeof(int32_t) + delta_bytes(n_out, nChunks);
+    cudaError_t e = cudaMalloc(&pl->dmem, stat_at + irc::kStatWords * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         free(pl->h_q0); free(pl->h_nq); free(pl->h_roff); free(pl->h_rs); free(pl->h_rn); free(pl);
         irc_host::cuda_status(e, "irc_plan_create: cudaMalloc");
@@ -512,11 +517,13 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     for (int k = 0; k < irc::kNumTileSizes; ++k) pl->dev.tile_off[k] = base + off_tile[k];
     pl->scratch = (int32_t *)pl->dmem + img.size();
     pl->delta_mem = (int32_t *)pl->dmem + delta_at;
+    pl->dev.stat = reinterpret_cast<unsigned long long *>((char *)pl->dmem + stat_at);
     pl->tc_items = reinterpret_cast<const irc::TcItem *>((const int32_t *)pl->dmem + off_items);
     pl->n_tc_items = (int)items.size();
     pl->n_tc_one = n_one;
     pl->n_tc_wide = n_wide;
     e = cudaMemset(pl->scratch, 0, irc::kScratchLists * sizeof(int32_t));      // counters and error word
+    if (e == cudaSuccess) e = cudaMemset(pl->dev.stat, 0, irc::kStatWords * sizeof(unsigned long long));
     if (e != cudaSuccess) { cudaFree(pl->dmem); free(pl); return irc_host::cuda_status(e, "irc_plan_create: clear"); }
     pl->dev.nChunks = nChunks;
     pl->dev.q_base = q_base;
@@ -670,6 +677,17 @@ int irc_plan_check(irc_plan *pl, void *stream)
         return IRC_E_TIMEOUT;
     }
     return IRC_OK;
+}
+
+int irc_plan_search_counts(irc_plan *pl, int64_t *counts, void *stream)
+{
+    if (!pl || !counts) { irc_host::set_error("irc_plan_search_counts: null pointer"); return IRC_E_INVAL; }
+    cudaStream_t s = (cudaStream_t)stream;
+    const size_t bytes = irc::kStatWords * sizeof(unsigned long long);
+    cudaError_t e = cudaMemcpyAsync(counts, pl->dev.stat, bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(pl->dev.stat, 0, bytes, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    return e == cudaSuccess ? IRC_OK : irc_host::cuda_status(e, "irc_plan_search_counts");
 }
 
 int irc_site_knn(irc_plan *pl, const float *F, int nC, int knn, int nThreads, int mode,

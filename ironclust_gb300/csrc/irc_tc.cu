@@ -786,7 +786,11 @@ __device__ __forceinline__ void epilogue(const irc::PlanDev &p, const irc_tc::Tc
         if (TAU && PASS != 1 && part == 0 && K > 0) {
             // the thresholds into the item's query tile; visible to the tensor
             // core (async proxy) before the MMA thread, released by tau_ready,
-            // issues the slot's pass-2 MMAs (one phase per item with units)
+            // issues the slot's pass-2 MMAs (one phase per item with units).
+            // Accumulators of pass 1 show that the tile has landed; where pass 1
+            // was another launch, its load is waited for here: landing later, it
+            // would put the rows' zeros over the thresholds.
+            if (PASS == 2) ok = warp_wait(&sh.a_full[r], (seq >> 1) & 1, sh.abort_flag) && ok;
             put_tau<FMT>(sh.sA + (size_t)r * A_BYTES, row, tau_k, tau);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();

@@ -306,6 +306,12 @@ class Plan:
                                            dd.ctypes.data_as(C.c_void_p)), "irc_plan_set_site_dims")
         return self
 
+    def search_counts(self):
+        """irc_plan_search_counts: where the calls since the last one went (waits for the stream)."""
+        c = (C.c_int64 * 5)()
+        check(lib().irc_plan_search_counts(self.h, c, _stream()), "irc_plan_search_counts")
+        return dict(zip(("searches", "tiles", "scans", "deltas", "windows"), c))
+
     def close(self):
         if self.h:
             lib().irc_plan_destroy(self.h)
