@@ -311,19 +311,23 @@ k_delta_list(irc::PlanDev p, int ntiles, const float *__restrict__ R, int knn, c
         miss = 1;
         bool more = true;
         for (int k = 0; k < knn && more; k += 4) {
-            int j[4];
+            int j[4];                                        // -1: no entry
             float d2[4], rj[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                j[u] = k + u < knn ? __ldg(mi + k + u) - 1 : q;
+                j[u] = k + u < knn ? __ldg(mi + k + u) - 1 : -1;
                 d2[u] = k + u < knn ? __ldg(dk + k + u) : kInfSentinel;
             }
+            // (a list may be padded with any index, and rows of a search that gave up were never written)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) rj[u] = __ldg(R + j[u]);     // (a row without a neighbour names the query)
+            for (int u = 0; u < 4; ++u) {
+                if (!(d2[u] < kInfSentinel) || (unsigned)j[u] >= (unsigned)p.nF) j[u] = -1;
+                rj[u] = j[u] >= 0 ? __ldg(R + j[u]) : 0.0f;
+            }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 if (!more) continue;
-                if (!(d2[u] < kInfSentinel)) more = false;           // list exhausted
+                if (j[u] < 0) more = false;                          // list exhausted
                 else if (!(rj[u] <= rq)) {                           // reference mask: rb <= ra is excluded
                     delta[o] = __fmul_rn(irc::ref_sqrt_abs(d2[u]), rq);
                     nneigh[o] = j[u] + 1;
