@@ -306,7 +306,7 @@ k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ de
     }
     // (without a record the query is in no chunk, or a wait gave up and every query is searched again)
     if (lane == 0 && !ok && ce.y >= 0)
-        list_out[__ldg(c.p.q0 + ce.y) - c.p.q_base + atomicAdd(counts + ce.y, 1)] = q;
+        list_out[__ldg(c.p.qseg + ce.y) + atomicAdd(counts + ce.y, 1)] = q;
 }
 
 // Working memory of the proven searches: one pool per device, shared by the
@@ -382,7 +382,7 @@ enum class Form { exact, ref, ref_delta };
 
 bool serves(const irc_plan *pl, int nC, Form f)
 {
-    if (!pl->runs_ascend || nC + 6 > irc_tc::KP) return false;
+    if (!pl->runs_ascend || !pl->disjoint || nC + 6 > irc_tc::KP) return false;
     const long long work = f == Form::exact ? 100000000 : f == Form::ref ? 20000000 : 500000000;
     const int tiles = f == Form::exact ? 500 : f == Form::ref ? 150 : 4000;
     return pl->pairs * nC >= work ||
@@ -465,7 +465,7 @@ int irc_cert_site_delta_ref(irc_plan *pl, const float *F, int nC, const float *R
     // (a bin's step number has 20 bits in the drift-window search's keys: a
     // run of at most 2^20 rows always fits)
     if (!serves(pl, nC, Form::ref_delta) || pl->max_rn > (1 << 20)) return IRC_CERT_PASS;
-    const size_t more = delta_bytes(pl->dev.n_out, pl->dev.nChunks);
+    const size_t more = delta_bytes(pl->dev.n_out, pl->dev.n_qry, pl->dev.nChunks);
     Work w(pl, lists_bytes(pl, nC, more), s);
     if (!w.base) return IRC_CERT_PASS;
     Lists L;

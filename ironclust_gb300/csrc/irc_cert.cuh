@@ -23,16 +23,17 @@ int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn,
 // queries searched one by one, per-query keys and the units of 16-query tiles,
 // up to 8 parts each.
 struct irc_delta_scratch {
-    int *words, *counts, *list;
+    int *words, *counts, *list;  // (a chunk's segment of list: from PlanDev::qseg)
     int2 *sparse, *items;
     unsigned long long *keys;
     const int *all;              // if not null and set: search every query
 };
 inline size_t delta_part(size_t n) { return (n + 255) & ~(size_t)255; }
-inline size_t delta_bytes(long long n_out, long long nChunks)
+inline size_t delta_bytes(long long n_out, long long n_qry, long long nChunks)
 {
-    const size_t n = (size_t)n_out, c = (size_t)nChunks;
-    return delta_part(4 * (4 + c)) + delta_part(4 * n) + 2 * delta_part(8 * n) + delta_part(8 * 8 * (n / 16 + c + 1));
+    const size_t n = (size_t)n_qry, c = (size_t)nChunks;
+    return delta_part(4 * (4 + c)) + delta_part(4 * n) + delta_part(8 * n) + delta_part(8 * (size_t)n_out) +
+           delta_part(8 * 8 * (n / 16 + c + 1));
 }
 irc_delta_scratch irc_delta_carve(const irc_plan *pl, void *mem, const int *all);
 cudaError_t irc_delta_clear(const irc_plan *pl, const irc_delta_scratch &sc, cudaStream_t s);

@@ -342,7 +342,7 @@ k_delta_list(irc::PlanDev p, int ntiles, const float *__restrict__ R, int knn, c
     int base = 0;
     if (lane == 0) base = atomicAdd(counts + chunk, __popc(bal));
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (miss) fb_list[__ldg(p.q0 + chunk) - p.q_base + base + __popc(bal & ((1u << lane) - 1u))] = qs + lane;
+    if (miss) fb_list[__ldg(p.qseg + chunk) + base + __popc(bal & ((1u << lane) - 1u))] = qs + lane;
 }
 
 constexpr int kParts = 8;        // most parts of one candidate window (part < 2^3: 3 bits at bit 28)
@@ -370,7 +370,7 @@ __global__ void k_delta_items(irc::PlanDev p, const int *__restrict__ all, const
     const int chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (chunk >= p.nChunks) return;
     const int q0 = __ldg(p.q0 + chunk), nq = __ldg(p.nq + chunk);
-    int *list = fb_list + (q0 - p.q_base);
+    int *list = fb_list + __ldg(p.qseg + chunk);
     int m = __ldg(counts + chunk);
     if (all && __ldg(all)) {
         m = nq;
@@ -398,7 +398,7 @@ __global__ void k_delta_items(irc::PlanDev p, const int *__restrict__ all, const
         if (lane == 0) base = atomicAdd(words + (wide ? 1 : 2), m);
         base = __shfl_sync(0xffffffffu, base, 0);
         for (int i = lane; i < m; i += 32)
-            sparse[wide ? base + i : p.n_out - 1 - (base + i)] = make_int2(list[i], chunk);
+            sparse[wide ? base + i : p.n_qry - 1 - (base + i)] = make_int2(list[i], chunk);
         if (wide)
             for (int i = lane; i < m; i += 32) keys[list[i] - p.q_base] = ~0ull;
     }
@@ -558,7 +558,7 @@ k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restr
         if (lane == 0 && b != ~0ull) atomicMin(keys + (e.x - p.q_base), b);
     }
     for (int w = blockIdx.x * nw + warp; w < n_narrow; w += gridDim.x * nw) {
-        const int2 e = sparse[p.n_out - 1 - w];
+        const int2 e = sparse[p.n_qry - 1 - w];
         const int nd = row_dims ? min(nC, (int)__ldg(row_dims + e.x)) : nC;
         const unsigned long long b = scan_query<REF>(p, F, R, nC, nd, e.y, e.x, nT, 0, INT_MAX, 0, 1, qrow, queues[warp],
                                                      buf, lane);
@@ -574,7 +574,7 @@ k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restr
         const int32_t *prs = REF ? p.rsr : p.rs, *prn = REF ? p.rnr : p.rn;
         const int r0 = __ldg((REF ? p.roffr : p.roff) + chunk), r1 = __ldg((REF ? p.roffr : p.roff) + chunk + 1);
         const int nBB = r1 - r0, nT0 = REF ? nT / nBB : 1;
-        const int seg = __ldg(p.q0 + chunk) - p.q_base;
+        const int seg = __ldg(p.qseg + chunk);
         // features that can be non-zero for this chunk's queries and candidates
         // (their site's width, irc_plan_set_site_dims): the rest add exactly 0
         const int nd = row_dims ? min(nC, (int)__ldg(row_dims + __ldg(p.q0 + chunk))) : nC;
@@ -661,24 +661,15 @@ __global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, cons
         const int j = t - (t / kQB) * kQB;
         const int chunk = item.x & 0x0fffffff, first = item.y >> 5, n = item.y & 31;
         if ((item.x >> 28) != 0 || j >= n) continue;        // each tile once (its part 0)
-        const int qq = fb_list[__ldg(p.q0 + chunk) - p.q_base + first + j];
+        const int qq = fb_list[__ldg(p.qseg + chunk) + first + j];
         put_delta<REF>(p, R, chunk, qq, keys[qq - p.q_base], nT, delta, nneigh);
     }
 }
 
 }  // namespace
 
-// Plan-owned scratch: two counters and two query lists of n_out entries.
-static int irc_plan_scratch(irc_plan *pl, int **counters, int **list_a, int **list_b)
-{
-    *counters = pl->scratch;
-    *list_a = pl->scratch + irc::kScratchLists;
-    *list_b = pl->scratch + irc::kScratchLists + pl->dev.n_out;
-    return IRC_OK;
-}
-
 // The EXACT kernel over the tiles of tq (all of the plan's by default) and its
-// overflow queue (*cnt, zeroed; up to n_out entries).
+// overflow queue (*cnt, zeroed; up to n_qry entries).
 int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
                     float *d2Knn, const irc::TileQueue &tq, int *cnt, int *ovf_list, cudaStream_t s)
 {
@@ -700,12 +691,10 @@ int irc_site_knn_exact(irc_plan *pl, const float *F, int nC, int knn, float *vrK
                        int32_t *miKnn, float *d2Knn, cudaStream_t s)
 {
     if (knn > kCap / 2) { irc_host::set_error("irc_site_knn(EXACT): knn %d > %d", knn, kCap / 2); return IRC_E_INVAL; }
-    int *cnt, *la, *lb;
-    int rc = irc_plan_scratch(pl, &cnt, &la, &lb);
-    if (rc != IRC_OK) return rc;
+    int *cnt = pl->scratch, *queue = pl->scratch + irc::kScratchLists;
     cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * sizeof(int), s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): memset");
-    return irc_exact_tiles(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, irc::TileQueue{}, cnt, la, s);
+    return irc_exact_tiles(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, irc::TileQueue{}, cnt, queue, s);
 }
 
 int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, int knn,
@@ -725,7 +714,7 @@ int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, in
 // Scratch of the drift-window search in mem (delta_bytes(...)).
 irc_delta_scratch irc_delta_carve(const irc_plan *pl, void *mem, const int *all)
 {
-    const size_t n = (size_t)pl->dev.n_out;
+    const size_t n = (size_t)pl->dev.n_qry;
     char *b = (char *)mem;
     irc_delta_scratch sc;
     sc.all = all;
@@ -737,7 +726,7 @@ irc_delta_scratch irc_delta_carve(const irc_plan *pl, void *mem, const int *all)
     sc.sparse = (int2 *)b;
     b += delta_part(8 * n);
     sc.keys = (unsigned long long *)b;
-    b += delta_part(8 * n);
+    b += delta_part(8 * (size_t)pl->dev.n_out);
     sc.items = (int2 *)b;
     return sc;
 }
@@ -769,13 +758,12 @@ int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int n
 }
 
 // Finish the queries the tensor-core kernel queued (list overflow) with the
-// exact ordered-scan kernel; the queue is the plan's first scratch list.
+// exact ordered-scan kernel; the queue lies in the plan's scratch.
 int irc_exact_overflow_drain(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho,
                              int32_t *miKnn, float *d2Knn, cudaStream_t s)
 {
-    int *cnt, *la, *lb;
-    irc_plan_scratch(pl, &cnt, &la, &lb);
-    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, pl->dev, F, nC, knn, cnt, la, vrKnn, rho, miKnn, d2Knn);
+    int *cnt = pl->scratch, *queue = pl->scratch + irc::kScratchLists;
+    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, pl->dev, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn overflow drain");
     return IRC_OK;
 }
@@ -825,7 +813,8 @@ int noalloc_scratch(int32_t **out)
 }
 
 // Word offsets of everything the entry point keeps in the fixed array, in
-// order: the plan scratch words (queue counters), two query queues of n_out,
+// order: the plan scratch words (queue counters), the overflow queue (2 n_out,
+// or all chunks' queries where a query is in several),
 // q0 [nChunks], nq [nChunks], roff [nChunks+1], rs [nRuns], rn [nRuns] and
 // the 16-query tile table [nChunks+1].  The size check and the pointers both
 // come from here, so they cannot disagree.
@@ -833,10 +822,10 @@ struct NoAllocLayout {
     size_t q0, nq, roff, rs, rn, tile, total;
 };
 
-NoAllocLayout noalloc_layout(long long n_out, long long nChunks, long long nRuns)
+NoAllocLayout noalloc_layout(long long n_out, long long n_qry, long long nChunks, long long nRuns)
 {
     NoAllocLayout L;
-    L.q0 = (size_t)irc::kScratchLists + 2 * (size_t)n_out;
+    L.q0 = (size_t)irc::kScratchLists + (size_t)(n_qry > 2 * n_out ? n_qry : 2 * n_out);
     L.nq = L.q0 + (size_t)nChunks;
     L.roff = L.nq + (size_t)nChunks;
     L.rs = L.roff + (size_t)nChunks + 1;
@@ -886,7 +875,9 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     int rc = irc_host::check_plan(me, q0, nq, roff, rs, rn, nChunks, q_base, n_out, nF, nullptr, nullptr);
     if (rc != IRC_OK) return rc;
     const int nRuns = roff[nChunks];
-    const NoAllocLayout L = noalloc_layout(n_out, nChunks, nRuns);
+    long long n_qry = 0;
+    for (int i = 0; i < nChunks; ++i) n_qry += nq[i];
+    const NoAllocLayout L = noalloc_layout(n_out, n_qry, nChunks, nRuns);
     if (L.total > kNoAllocWords) {
         irc_host::set_error("%s: plan needs %zu scratch words (4 + 2*n_out + 4*chunks + 2 + 2*runs), "
                             "the fixed array holds %zu", me, L.total, kNoAllocWords);
@@ -913,10 +904,11 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     p.q0 = d_q0; p.nq = d_nq; p.roff = d_roff; p.rs = d_rs; p.rn = d_rn;
     p.roffr = d_roff; p.rsr = d_rs; p.rnr = d_rn;         // the EXACT kernels take any run split
     for (int k = 0; k < irc::kNumTileSizes; ++k) p.tile_off[k] = d_tile;     // only the 16-query table is read
-    p.ncand = nullptr;                                    // read only by the delta kernels
+    p.ncand = p.qseg = nullptr;                           // read only by the delta kernels
     p.tc_toff = nullptr;                                  // read only by the tensor-core filter
     p.tc_tiles = nullptr;
     p.stat = nullptr;
+    p.n_qry = (int)(n_qry < INT32_MAX ? n_qry : INT32_MAX);
     p.nChunks = nChunks; p.q_base = q_base; p.n_out = n_out; p.nF = nF; p.nRuns = nRuns;
     const size_t smem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
     e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -6,8 +6,7 @@ namespace irc {
 
 // Plan scratch words: [0] overflow-queue count, [1] largest magnitude (FP8's
 // scale), [2] device error word (a bounded wait gave up), [3] block ticket of the
-// centring (zero between launches); the two query lists of n_out entries
-// follow.
+// centring (zero between launches); the overflow queue follows.
 constexpr int kScratchErr = 2;
 constexpr int kScratchTicket = 3;
 constexpr int kScratchLists = 4;
@@ -48,6 +47,7 @@ struct PlanDev {
     const int32_t *roffr, *rsr, *rnr;
     const int32_t *tile_off[kNumTileSizes];   // [nChunks+1] prefix sums of ceil(nq/QB)
     const int32_t *ncand;                     // [nChunks] candidates of each chunk (sum of its runs)
+    const int32_t *qseg;                      // [nChunks] queries of the chunks before (a query may be in several chunks)
     // 128-candidate tiles of every chunk's intervals for the tensor-core
     // filter: tile j of chunk c is tc_tiles[tc_toff[c] + j] = (first row,
     // columns); each chunk's list is padded to an even length with (0, 0),
@@ -56,6 +56,7 @@ struct PlanDev {
     const int2 *tc_tiles;
     unsigned long long *stat;                 // [kStatWords], or null: not counted
     int nChunks, q_base, n_out, nF, nRuns;
+    int n_qry;                                // queries of all chunks
 };
 
 __device__ __forceinline__ void count_stat(const PlanDev &p, int which, int n)
@@ -94,7 +95,7 @@ __device__ __forceinline__ void tile_lookup(const PlanDev &p, int tile, int &chu
 struct irc_plan {
     irc::PlanDev dev;
     void *dmem;                            // single device allocation behind dev
-    int32_t *scratch;                      // inside dmem: 4 words + 2 x n_out query lists
+    int32_t *scratch;                      // inside dmem: 4 words + the overflow queue (n_qry + n_out queries)
     void *delta_mem;                       // inside dmem: scratch of the delta search (irc_cert.cuh)
     const irc::TcItem *tc_items;           // tensor-core work items: inside dmem, or tc_items_buf
     int n_tc_items;
@@ -114,6 +115,7 @@ struct irc_plan {
     int max_nq;                            // largest query chunk
     int max_rn;                            // longest candidate run
     int runs_ascend;                       // every chunk's runs ascend without overlap (a row is in at most one)
+    int disjoint;                          // no query is in two chunks
     int uses_pool;                         // the plan took working memory from the library's pool (irc_cert.cu)
     long long pairs;                       // (query, candidate) pairs of the plan
     int device;

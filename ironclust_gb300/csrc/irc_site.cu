@@ -409,6 +409,12 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
                                          &pairs, &max_nq);
     if (vrc != IRC_OK) return vrc;
     const int nRuns = roff[nChunks];
+    long long n_qry = 0;
+    for (int i = 0; i < nChunks; ++i) n_qry += nq[i];
+    if (n_qry > INT32_MAX) {
+        irc_host::set_error("irc_plan_create: %lld queries in all chunks (at most 2^31 - 1)", n_qry);
+        return IRC_E_INVAL;
+    }
     irc_plan *pl = (irc_plan *)calloc(1, sizeof(irc_plan));
     if (!pl) return IRC_E_NOMEM;
     // host copies
@@ -443,6 +449,8 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
         for (int r = roff[i]; r < roff[i + 1]; ++r) c += rn[r];
         img.push_back(c);
     }
+    const size_t off_qseg = img.size();
+    for (int i = 0, at = 0; i < nChunks; at += nq[i++]) img.push_back(at);
     // tensor-core tiles: every chunk's intervals cut into 128-row tiles,
     // each chunk's list padded to an even length
     const size_t off_toff = img.size();
@@ -490,10 +498,11 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     }
     cudaGetDevice(&pl->device);
     if (img.size() & 1) img.push_back(0);          // scratch starts 8-byte aligned (int2 items)
-    // scratch: 4 words and two query lists of n_out, then the delta search's
-    const size_t scratch_ints = irc::kScratchLists + 2 * (size_t)n_out + 64;
+    // scratch: 4 words and the overflow queue (every query of every chunk, then
+    // every row of the re-rank), then the delta search's
+    const size_t scratch_ints = irc::kScratchLists + (size_t)n_qry + (size_t)n_out + 64;
     const size_t delta_at = (img.size() + scratch_ints) / 64 * 64;          // 256-byte aligned
-    const size_t stat_at = delta_at * sizeof(int32_t) + delta_bytes(n_out, nChunks);
+    const size_t stat_at = delta_at * sizeof(int32_t) + delta_bytes(n_out, n_qry, nChunks);
     cudaError_t e = cudaMalloc(&pl->dmem, stat_at + irc::kStatWords * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         free(pl->h_q0); free(pl->h_nq); free(pl->h_roff); free(pl->h_rs); free(pl->h_rn); free(pl);
@@ -512,6 +521,8 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     pl->dev.rsr = base + off_rsr;
     pl->dev.rnr = base + off_rnr;
     pl->dev.ncand = base + off_ncand;
+    pl->dev.qseg = base + off_qseg;
+    pl->dev.n_qry = (int)n_qry;
     pl->dev.tc_toff = base + off_toff;
     pl->dev.tc_tiles = reinterpret_cast<const int2 *>(base + off_tiles);
     for (int k = 0; k < irc::kNumTileSizes; ++k) pl->dev.tile_off[k] = base + off_tile[k];
@@ -533,6 +544,12 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     pl->max_nq = max_nq;
     pl->pairs = pairs;
     row_intervals(q0, nq, rs, rn, nChunks, nRuns, pl);
+    std::vector<std::pair<int32_t, int32_t>> qs;
+    for (int i = 0; i < nChunks; ++i) qs.emplace_back(q0[i], nq[i]);
+    std::sort(qs.begin(), qs.end());
+    pl->disjoint = 1;
+    for (int i = 1; i < nChunks; ++i)
+        if (qs[i].first < qs[i - 1].first + qs[i - 1].second) pl->disjoint = 0;
     pl->runs_ascend = 1;
     for (int i = 0; i < nChunks; ++i)
         for (int r = roff[i]; r < roff[i + 1]; ++r) {
