@@ -14,8 +14,8 @@ constexpr int kScratchLists = 4;
 // Counters of irc_plan_search_counts (PlanDev::stat), summed by the kernels:
 // proven searches and the 16-query tiles they left to the plain kernel, queries
 // finished by ordered scans, proven delta searches and the queries they left
-// to the window search.
-enum { kStatSearches, kStatTiles, kStatScans, kStatDeltas, kStatWindows, kStatWords };
+// to the window search, work items split over their candidates.
+enum { kStatSearches, kStatTiles, kStatScans, kStatDeltas, kStatWindows, kStatSplits, kStatWords };
 
 // Query-tile sizes for which a plan precomputes its tile tables.
 constexpr int kTileSizes[] = {8, 16, 32, 64, 128};
@@ -102,6 +102,7 @@ struct irc_plan {
     int n_tc_one;                          // items [0, n_tc_one) have one slot, [n_tc_one, n_tc_wide) two
     int n_tc_wide;                         // (both on 256-candidate units), the rest four (128-candidate units)
     int tc_max_tiles;                      // most 128-row candidate tiles of a chunk
+    int tc_rest_tiles;                     // the same of the one-slot items behind the last full turn of the machine
     int tc_wide_bn;                        // unit width of the one- and two-slot items: 256 (0 = default) or 128
     uint8_t *row_dims;                     // [nF] features of each row's site (irc_plan_set_site_dims) or null
     void *tc_items_buf;                    // items of irc_plan_tc_layout, when called
@@ -118,7 +119,7 @@ struct irc_plan {
     int disjoint;                          // no query is in two chunks
     int uses_pool;                         // the plan took working memory from the library's pool (irc_cert.cu)
     long long pairs;                       // (query, candidate) pairs of the plan
-    int device;
+    int device, sms;
     // host copies (for the per-chunk drop-in emulation and validation)
     int32_t *h_q0, *h_nq, *h_roff, *h_rs, *h_rn;
 };

@@ -173,7 +173,7 @@ struct Slot {
 // them in L2); order 1: chunk order.
 std::vector<irc::TcItem> build_tc_items(const int32_t *q0, const int32_t *nq, const int32_t *roff,
                                         const int32_t *rn, int nChunks, int max_slots, int order_mode,
-                                        int *n_one, int *n_wide)
+                                        int sms, int *n_one, int *n_wide, int *rest_tiles)
 {
     std::vector<irc::TcItem> items;
     std::vector<int> cost;
@@ -236,6 +236,8 @@ std::vector<irc::TcItem> build_tc_items(const int32_t *q0, const int32_t *nq, co
     }
     *n_one = n1;
     *n_wide = nw;
+    *rest_tiles = 0;
+    for (int k = n1 - n1 % sms; k < n1; ++k) *rest_tiles = std::max(*rest_tiles, cost[order[k]]);
     return out;
 }
 
@@ -481,29 +483,34 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     // tensor-core work items: 128-row tiles of large chunks, then the 33-64 and
     // 1-32 row remainders packed two and four per item (similar tile counts
     // together), all ordered by cost, largest first
-    int n_one = 0, n_wide = 0;
+    int n_one = 0, n_wide = 0, rest = 0;
+    cudaError_t e = cudaGetDevice(&pl->device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&pl->sms, cudaDevAttrMultiProcessorCount, pl->device);
+    if (e != cudaSuccess) {
+        free(pl->h_q0); free(pl->h_nq); free(pl->h_roff); free(pl->h_rs); free(pl->h_rn); free(pl);
+        return irc_host::cuda_status(e, "irc_plan_create: device");
+    }
     // When all items, unpacked, are at most two a SM, packing saves no turn of
     // the machine and its classes run one after another: the leftover 32
     // queries of a 20,000-spike static site, alone in a four-slot launch, took
     // 285 us after the other 156 items' 237 (together 240).
     long long unpacked = 0;
     for (int i = 0; i < nChunks; ++i) unpacked += (nq[i] + 127) / 128;
-    std::vector<irc::TcItem> items = build_tc_items(q0, nq, moff.data(), mn.data(), nChunks, unpacked <= 2 * 152 ? 1 : 4, 0,
-                                                    &n_one, &n_wide);
+    std::vector<irc::TcItem> items = build_tc_items(q0, nq, moff.data(), mn.data(), nChunks, unpacked <= 2 * pl->sms ? 1 : 4, 0,
+                                                    pl->sms, &n_one, &n_wide, &rest);
     while (img.size() % 16) img.push_back(0);
     const size_t off_items = img.size();
     for (const irc::TcItem &it : items) {
         const int32_t *w = reinterpret_cast<const int32_t *>(&it);
         img.insert(img.end(), w, w + 16);
     }
-    cudaGetDevice(&pl->device);
     if (img.size() & 1) img.push_back(0);          // scratch starts 8-byte aligned (int2 items)
     // scratch: 4 words and the overflow queue (every query of every chunk, then
     // every row of the re-rank), then the delta search's
     const size_t scratch_ints = irc::kScratchLists + (size_t)n_qry + (size_t)n_out + 64;
     const size_t delta_at = (img.size() + scratch_ints) / 64 * 64;          // 256-byte aligned
     const size_t stat_at = delta_at * sizeof(int32_t) + delta_bytes(n_out, n_qry, nChunks);
-    cudaError_t e = cudaMalloc(&pl->dmem, stat_at + irc::kStatWords * sizeof(unsigned long long));
+    e = cudaMalloc(&pl->dmem, stat_at + irc::kStatWords * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         free(pl->h_q0); free(pl->h_nq); free(pl->h_roff); free(pl->h_rs); free(pl->h_rn); free(pl);
         irc_host::cuda_status(e, "irc_plan_create: cudaMalloc");
@@ -533,6 +540,7 @@ int irc_plan_create(irc_plan **out, const int32_t *q0, const int32_t *nq, const 
     pl->n_tc_items = (int)items.size();
     pl->n_tc_one = n_one;
     pl->n_tc_wide = n_wide;
+    pl->tc_rest_tiles = rest;
     e = cudaMemset(pl->scratch, 0, irc::kScratchLists * sizeof(int32_t));      // counters and error word
     if (e == cudaSuccess) e = cudaMemset(pl->dev.stat, 0, irc::kStatWords * sizeof(unsigned long long));
     if (e != cudaSuccess) { cudaFree(pl->dmem); free(pl); return irc_host::cuda_status(e, "irc_plan_create: clear"); }
@@ -604,9 +612,9 @@ int irc_plan_tc_layout(irc_plan *pl, int max_slots, int order)
     const int nChunks = pl->dev.nChunks;
     std::vector<int32_t> moff, ms, mn;
     merge_runs(pl->h_roff, pl->h_rs, pl->h_rn, nChunks, moff, ms, mn);
-    int n_one = 0, n_wide = 0;
+    int n_one = 0, n_wide = 0, rest = 0;
     std::vector<irc::TcItem> items = build_tc_items(pl->h_q0, pl->h_nq, moff.data(), mn.data(), nChunks, max_slots,
-                                                    order, &n_one, &n_wide);
+                                                    order, pl->sms, &n_one, &n_wide, &rest);
     void *buf = nullptr;
     cudaError_t e = cudaMalloc(&buf, sizeof(irc::TcItem) * (items.size() ? items.size() : 1));
     if (e == cudaSuccess)
@@ -621,6 +629,7 @@ int irc_plan_tc_layout(irc_plan *pl, int max_slots, int order)
     pl->n_tc_items = (int)items.size();
     pl->n_tc_one = n_one;
     pl->n_tc_wide = n_wide;
+    pl->tc_rest_tiles = rest;
     return IRC_OK;
 }
 

@@ -96,7 +96,6 @@ constexpr int THREADS = 32 * (1 + MMA_WARPS + EPI_WARPS);
 constexpr uint32_t A_BYTES = BM * KP * 2;         // the query tile: 128 rows x 128 bytes
 constexpr uint32_t HALF_BYTES = 128 * KP * 2;     // one 128-candidate tile
 constexpr uint32_t TMEM_COLS = 512;               // all TMEM columns (one CTA per SM)
-constexpr int kSMs = 152;
 constexpr int LISTCAP = irc_tc::LIST_ROW;                      // candidate-list capacity per query (the four warps' hits pooled)
 constexpr int MAX_SHORT_TILES = 512;              // tiles per chunk that a 16-bit list entry can name
 // The threshold is the tau_rank-th smallest per-column minimum: tau_rank
@@ -1125,6 +1124,7 @@ __global__ void __launch_bounds__(BM) k_publish(irc::PlanDev p, const irc_tc::Tc
                                                 irc_tc::ListOut lo, int *__restrict__ scratch)
 {
     after_previous(lo.split.cnt);
+    if (blockIdx.x == 0 && threadIdx.x == 0) irc::count_stat(p, irc::kStatSplits, gridDim.x);
     const irc_tc::TcItem &it = items[blockIdx.x];
     const int row = threadIdx.x, slot = blockIdx.x * BM + row;
     if (row >= it.nq[0]) return;
@@ -1206,12 +1206,10 @@ static int launch_filter(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan 
     auto kern = big ? k_knn_tc<FMT, BN, TAU, NS, true> : k_knn_tc<FMT, BN, TAU, NS, false>;
     const int smem = (int)(big ? Tile<BN, true>::SMEM_BYTES : Tile<BN, false>::SMEM_BYTES);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int sms = 0;
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(tensor core): launch attributes");
     // persistent: one CTA per SM (shared memory and TMEM allow one), each
     // taking items from the queue until it is empty
-    const int grid = n_items < sms ? n_items : sms;
+    const int grid = n_items < pl->sms ? n_items : pl->sms;
     launch_next(kern, grid, THREADS, smem, s, mq, mc, pl->dev, items, n_items, queue, nk, tau_k, lo, scratch);
     IRC_CHECK_LAUNCH("irc_site_knn(tensor core)");
     return IRC_OK;
@@ -1239,7 +1237,7 @@ static int launch_split(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *
 }
 
 // The last one-slot items that leave SMs idle: n mod 152 of them take one more
-// turn, as long as a full one (1.42 us a unit, D = 24).  Cut into parts that
+// turn, as long as the longest of them (1.42 us a unit, D = 24).  Cut into parts that
 // fill the machine they take two launches of a part's units and 57 us of their
 // own (memory cleared, prologues, the threshold search after pass 1, lists
 // published); 22 more than the launch they replace where they are all there
@@ -1250,10 +1248,10 @@ static int launch_split(const CUtensorMap &mq, const CUtensorMap &mc, irc_plan *
 static SplitOut split_of(const irc_plan *pl, int nC, Fmt fmt)
 {
     SplitOut sp{};
-    const int rest = pl->n_tc_one % kSMs, units = (pl->tc_max_tiles + 1) / 2;
+    const int rest = pl->n_tc_one % pl->sms, units = (pl->tc_rest_tiles + 1) / 2;
     if (fmt == Fmt::fp8 || nC + 9 > KP || pl->tc_wide_bn == 128 || rest == 0) return sp;
-    const int parts = std::min(kSMs / rest, units / 4), saved = units - units / std::max(parts, 1);
-    if (parts < 2 || saved < (pl->n_tc_one > kSMs ? 34 : 20)) return sp;
+    const int parts = std::min(pl->sms / rest, units / 4), saved = units - units / std::max(parts, 1);
+    if (parts < 2 || saved < (pl->n_tc_one > pl->sms ? 34 : 20)) return sp;
     sp.items = rest;
     sp.parts = parts;
     return sp;
