@@ -587,7 +587,7 @@ size_t irc_plan_tc_bytes(const irc_plan *pl, int nC)
 {
     if (!pl || nC < 1) return 0;
     return irc_tc::ops_bytes(pl, nC, irc_tc::Fmt::bf16) + irc_tc::list_area_bytes(pl->dev.n_out) +
-           irc_tc::split_bytes(pl, nC, irc_tc::Fmt::bf16);
+           irc_tc::split_reserve(pl);
 }
 
 int irc_plan_set_tc_buffer(irc_plan *pl, void *buf, size_t bytes)

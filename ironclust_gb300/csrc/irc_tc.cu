@@ -1257,9 +1257,14 @@ static SplitOut split_of(const irc_plan *pl, int nC, Fmt fmt)
     return sp;
 }
 
-size_t split_bytes(const irc_plan *pl, int nC, Fmt fmt)
+static size_t item_bytes(int items) { return (size_t)items * BM * (128 + 1 + LIST_ROW) * 4; }
+
+size_t split_bytes(const irc_plan *pl, int nC, Fmt fmt) { return item_bytes(split_of(pl, nC, fmt).items); }
+
+// (parts >= 2: at most half as many items as SMs; below 24 units nothing is saved)
+size_t split_reserve(const irc_plan *pl)
 {
-    return (size_t)split_of(pl, nC, fmt).items * BM * (128 + 1 + LIST_ROW) * 4;
+    return (pl->tc_max_tiles + 1) / 2 < 24 ? 0 : item_bytes(pl->sms / 2);
 }
 
 void split_area(const irc_plan *pl, int nC, Fmt fmt, void *mem, ListOut *lo)

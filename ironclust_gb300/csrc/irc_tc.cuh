@@ -76,9 +76,12 @@ inline ListOut list_area(void *base, long long n_out)
     return lo;
 }
 
-// Memory of the split items (0: none), and its place in lo: behind lo.lists, in
-// the same allocation.
+// Memory of the split items (0: none), the most that any layout, width or form
+// of the plan takes (a buffer that the plan keeps has room for it: it is not
+// allocated again, and captured graphs that use it stay valid), and its place
+// in lo: behind lo.lists, in the same allocation.
 size_t split_bytes(const irc_plan *pl, int nC, Fmt fmt);
+size_t split_reserve(const irc_plan *pl);
 void split_area(const irc_plan *pl, int nC, Fmt fmt, void *mem, ListOut *lo);
 
 // The filter (one persistent launch per packing class: items of one or two

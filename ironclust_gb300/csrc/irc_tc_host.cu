@@ -460,12 +460,12 @@ int irc_site_knn_tc(irc_plan *pl, const float *F, int nC, int knn, int mode, flo
     void *buf;
     const size_t ops = irc_tc::ops_bytes(pl, nC, fmt);
     const size_t need = ops + irc_tc::list_area_bytes(pl->dev.n_out);
-    size_t split = irc_tc::split_bytes(pl, nC, fmt);
-    if (split && pl->tc_external && pl->tc_bytes < need + split) split = 0;      // the caller's memory is enough without
-    int rc = irc_plan_tc_buffer(pl, need + split, &buf);
+    size_t reserve = irc_tc::split_reserve(pl);
+    if (pl->tc_external && pl->tc_bytes < need + reserve) reserve = 0;      // the caller's memory is enough without
+    int rc = irc_plan_tc_buffer(pl, need + reserve, &buf);
     if (rc != IRC_OK) return rc;
     irc_tc::ListOut lo = irc_tc::list_area((char *)buf + ops, pl->dev.n_out);
-    if (split) irc_tc::split_area(pl, nC, fmt, (char *)buf + need, &lo);
+    if (reserve) irc_tc::split_area(pl, nC, fmt, (char *)buf + need, &lo);
     cudaError_t e = cudaMemsetAsync(pl->scratch, 0, 2 * sizeof(int), s);   // overflow-queue count, largest magnitude
     if (e == cudaSuccess) e = irc_tc::clear_lists(lo, pl->dev.n_out, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(BF16): memset");
