@@ -122,105 +122,125 @@ __device__ __forceinline__ void warp_sort_keys(unsigned long long *keys, int lan
     for (int i = 0; i < PER; ++i) keys[lane * PER + i] = v[i];
 }
 
-__global__ void __launch_bounds__(kThreads)
-k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
-                 float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
-                 float *__restrict__ d2Knn, int *__restrict__ ovf_count, int *__restrict__ ovf_list, irc::TileQueue tq)
+// One 16-query tile.
+__device__ __forceinline__ void
+exact_tile(const irc::PlanDev &p, int tile, const float *__restrict__ F, int nC, int knn, float *__restrict__ vrKnn,
+           float *__restrict__ rho, int *__restrict__ miKnn, float *__restrict__ d2Knn, int *__restrict__ ovf_count,
+           int *__restrict__ ovf_list)
 {
-    after_previous(tq.list, tq.count, tq.all);
     __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
     __shared__ float sTau[kQB];
     __shared__ int sCnt[kQB];
     extern __shared__ __align__(16) unsigned char dyn[];
     unsigned long long *sList = reinterpret_cast<unsigned long long *>(dyn);   // [kQB][kCap]
     float *sMin = reinterpret_cast<float *>(sList + kQB * kCap);              // [kQB][kThreads]
-    if (tq.list && blockIdx.x == 0 && threadIdx.x == 0) {
+    int chunk, qs, n;
+    irc::tile_lookup<kQB>(p, tile, chunk, qs, n);
+    const int r0 = __ldg(p.roff + chunk), r1 = __ldg(p.roff + chunk + 1);
+    irc::stage_queries<kQB>(F, nC, qs, n, sA);
+    if (threadIdx.x < kQB) sCnt[threadIdx.x] = 0;
+    __syncthreads();
+    const int t = threadIdx.x;
+    // pass 1: stripe minima
+    float mn[kQB];
+#pragma unroll
+    for (int q = 0; q < kQB; ++q) mn[q] = __int_as_float(0x7f800000);
+    walk_stripe(p, r0, r1, t, [&](int iB) {
+        float acc[kQB];
+        dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
+#pragma unroll
+        for (int q = 0; q < kQB; ++q)
+            if (acc[q] > 0.0f && acc[q] < mn[q]) mn[q] = acc[q];
+    });
+#pragma unroll
+    for (int q = 0; q < kQB; ++q) sMin[q * kThreads + t] = mn[q];
+    __syncthreads();
+    // tau = k-th smallest stripe minimum (by value); +inf if fewer than k finite
+    const int lane = t & 31, warp = t >> 5, nw = kThreads / 32;
+    for (int q = warp; q < kQB; q += nw) {
+        float *m = sMin + q * kThreads;
+        float kth = __int_as_float(0x7f800000);
+        for (int k = 0; k < knn; ++k) {
+            unsigned long long best = ~0ull;
+            for (int s = lane; s < kThreads; s += 32) {
+                const unsigned long long key = dkey(m[s], s);
+                best = key < best ? key : best;
+            }
+            best = irc::warp_min_u64(best);
+            const int s = (int)(best & 0xffffffffu);
+            kth = __uint_as_float((unsigned)(best >> 32));
+            __syncwarp();
+            if (lane == 0) m[s] = __int_as_float(0x7fffffff);      // NaN bits: sorts last
+            __syncwarp();
+            if (!(kth < __int_as_float(0x7f800000))) break;
+        }
+        if (lane == 0) sTau[q] = kth;
+    }
+    __syncthreads();
+    // pass 2: collect d2 <= tau
+    walk_stripe(p, r0, r1, t, [&](int iB) {
+        float acc[kQB];
+        dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
+#pragma unroll
+        for (int q = 0; q < kQB; ++q)
+            if (acc[q] > 0.0f && acc[q] <= sTau[q]) {
+                const int slot = atomicAdd(&sCnt[q], 1);
+                if (slot < kCap) sList[q * kCap + slot] = dkey(acc[q], iB);
+            }
+    });
+    __syncthreads();
+    for (int q = warp; q < n; q += nw) {
+        const int cnt = sCnt[q];
+        const size_t o = (size_t)(qs + q - p.q_base);
+        if (cnt > kCap) {                          // overflow: finished by the fallback kernel
+            if (lane == 0) { int i = atomicAdd(ovf_count, 1); ovf_list[i] = qs + q; }
+            continue;
+        }
+        unsigned long long *L = sList + q * kCap;
+        for (int i = cnt + lane; i < kCap; i += 32) L[i] = ~0ull;
+        __syncwarp();
+        warp_sort_keys(L, lane);
+        __syncwarp();
+        for (int k = lane; k < knn; k += 32) {
+            const unsigned long long key = L[k];
+            const bool ok = k < cnt;
+            const float d2 = ok ? __uint_as_float((unsigned)(key >> 32)) : kInfSentinel;
+            const int idx = ok ? (int)(key & 0xffffffffu) : qs + q;
+            miKnn[(size_t)k + (size_t)knn * o] = idx + 1;
+            if (d2Knn) d2Knn[(size_t)k + (size_t)knn * o] = d2;
+            if (k == knn - 1) {
+                const float v = irc::ref_sqrt_abs(d2);
+                vrKnn[o] = v;
+                if (rho) rho[o] = __fdiv_rn(1.0f, v);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// A tile per block.
+__global__ void __launch_bounds__(kThreads)
+k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn, float *__restrict__ vrKnn,
+                 float *__restrict__ rho, int *__restrict__ miKnn, float *__restrict__ d2Knn, int *__restrict__ ovf_count,
+                 int *__restrict__ ovf_list)
+{
+    exact_tile(p, blockIdx.x, F, nC, knn, vrKnn, rho, miKnn, d2Knn, ovf_count, ovf_list);
+}
+
+// The tiles of a queue.  (A kernel of its own: with the loop around it the tile
+// spills, 4% on a site of 1,500 spikes.)
+__global__ void __launch_bounds__(kThreads)
+k_site_knn_exact_queue(irc::PlanDev p, const float *__restrict__ F, int nC, int knn, float *__restrict__ vrKnn,
+                       float *__restrict__ rho, int *__restrict__ miKnn, float *__restrict__ d2Knn,
+                       int *__restrict__ ovf_count, int *__restrict__ ovf_list, irc::TileQueue tq)
+{
+    after_previous(tq.list, tq.count, tq.all);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         irc::count_stat(p, irc::kStatSearches, 1);
         irc::count_stat(p, irc::kStatTiles, tq.size());
     }
     for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
-        int chunk, qs, n;
-        irc::tile_lookup<kQB>(p, tq.tile(w), chunk, qs, n);
-        const int r0 = __ldg(p.roff + chunk), r1 = __ldg(p.roff + chunk + 1);
-        irc::stage_queries<kQB>(F, nC, qs, n, sA);
-        if (threadIdx.x < kQB) sCnt[threadIdx.x] = 0;
-        __syncthreads();
-        const int t = threadIdx.x;
-        // pass 1: stripe minima
-        float mn[kQB];
-#pragma unroll
-        for (int q = 0; q < kQB; ++q) mn[q] = __int_as_float(0x7f800000);
-        walk_stripe(p, r0, r1, t, [&](int iB) {
-            float acc[kQB];
-            dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
-#pragma unroll
-            for (int q = 0; q < kQB; ++q)
-                if (acc[q] > 0.0f && acc[q] < mn[q]) mn[q] = acc[q];
-        });
-#pragma unroll
-        for (int q = 0; q < kQB; ++q) sMin[q * kThreads + t] = mn[q];
-        __syncthreads();
-        // tau = k-th smallest stripe minimum (by value); +inf if fewer than k finite
-        const int lane = t & 31, warp = t >> 5, nw = kThreads / 32;
-        for (int q = warp; q < kQB; q += nw) {
-            float *m = sMin + q * kThreads;
-            float kth = __int_as_float(0x7f800000);
-            for (int k = 0; k < knn; ++k) {
-                unsigned long long best = ~0ull;
-                for (int s = lane; s < kThreads; s += 32) {
-                    const unsigned long long key = dkey(m[s], s);
-                    best = key < best ? key : best;
-                }
-                best = irc::warp_min_u64(best);
-                const int s = (int)(best & 0xffffffffu);
-                kth = __uint_as_float((unsigned)(best >> 32));
-                __syncwarp();
-                if (lane == 0) m[s] = __int_as_float(0x7fffffff);      // NaN bits: sorts last
-                __syncwarp();
-                if (!(kth < __int_as_float(0x7f800000))) break;
-            }
-            if (lane == 0) sTau[q] = kth;
-        }
-        __syncthreads();
-        // pass 2: collect d2 <= tau
-        walk_stripe(p, r0, r1, t, [&](int iB) {
-            float acc[kQB];
-            dist_qb<kQB>(F + (size_t)iB * nC, nC, sA, acc);
-#pragma unroll
-            for (int q = 0; q < kQB; ++q)
-                if (acc[q] > 0.0f && acc[q] <= sTau[q]) {
-                    const int slot = atomicAdd(&sCnt[q], 1);
-                    if (slot < kCap) sList[q * kCap + slot] = dkey(acc[q], iB);
-                }
-        });
-        __syncthreads();
-        for (int q = warp; q < n; q += nw) {
-            const int cnt = sCnt[q];
-            const size_t o = (size_t)(qs + q - p.q_base);
-            if (cnt > kCap) {                          // overflow: finished by the fallback kernel
-                if (lane == 0) { int i = atomicAdd(ovf_count, 1); ovf_list[i] = qs + q; }
-                continue;
-            }
-            unsigned long long *L = sList + q * kCap;
-            for (int i = cnt + lane; i < kCap; i += 32) L[i] = ~0ull;
-            __syncwarp();
-            warp_sort_keys(L, lane);
-            __syncwarp();
-            for (int k = lane; k < knn; k += 32) {
-                const unsigned long long key = L[k];
-                const bool ok = k < cnt;
-                const float d2 = ok ? __uint_as_float((unsigned)(key >> 32)) : kInfSentinel;
-                const int idx = ok ? (int)(key & 0xffffffffu) : qs + q;
-                miKnn[(size_t)k + (size_t)knn * o] = idx + 1;
-                if (d2Knn) d2Knn[(size_t)k + (size_t)knn * o] = d2;
-                if (k == knn - 1) {
-                    const float v = irc::ref_sqrt_abs(d2);
-                    vrKnn[o] = v;
-                    if (rho) rho[o] = __fdiv_rn(1.0f, v);
-                }
-            }
-            __syncwarp();
-        }
+        exact_tile(p, tq.tile(w), F, nC, knn, vrKnn, rho, miKnn, d2Knn, ovf_count, ovf_list);
         __syncthreads();
     }
 }
@@ -668,23 +688,32 @@ __global__ void k_delta_finish(irc::PlanDev p, const float *__restrict__ R, cons
 
 }  // namespace
 
-// The EXACT kernel over the tiles of tq (all of the plan's by default) and its
-// overflow queue (*cnt, zeroed; up to n_qry entries).
+constexpr size_t kExactSmem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
+constexpr int kExactBlocks = 3;          // resident on an SM (registers)
+
+static int exact_overflow(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
+                          float *d2Knn, int *cnt, int *ovf_list, cudaStream_t s)
+{
+    // the overflow list is usually empty; size the grid for the worst case
+    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, pl->dev, F, nC, knn, cnt, ovf_list, vrKnn, rho, miKnn, d2Knn);
+    IRC_CHECK_LAUNCH("irc_site_knn(EXACT) overflow");
+    return IRC_OK;
+}
+
+// The EXACT kernel over the tiles of tq and its overflow queue (*cnt, zeroed;
+// up to n_qry entries).  As many blocks as run at once: a second wave would
+// find its share of the tiles still waiting (100,003 spikes, every tile: 26.0
+// ms with four blocks an SM asked for, 22.3 a tile per block).
 int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
                     float *d2Knn, const irc::TileQueue &tq, int *cnt, int *ovf_list, cudaStream_t s)
 {
-    const size_t smem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
-    cudaError_t e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_site_knn_exact_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExactSmem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): smem attribute");
-    const int tiles = pl->ntiles[irc::tile_slot(kQB)];
-    const int grid = tq.list && tiles > kQueueBlocks ? kQueueBlocks : tiles;
-    launch_next(k_site_knn_exact, grid, kThreads, smem, s, pl->dev, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, ovf_list, tq);
+    const int tiles = pl->ntiles[irc::tile_slot(kQB)], most = pl->sms * kExactBlocks;
+    launch_next(k_site_knn_exact_queue, tiles < most ? tiles : most, kThreads, kExactSmem, s, pl->dev, F, nC, knn, vrKnn, rho,
+                miKnn, d2Knn, cnt, ovf_list, tq);
     IRC_CHECK_LAUNCH("irc_site_knn(EXACT)");
-    // the overflow list is usually empty; size the grid for the worst case
-    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, 
-        pl->dev, F, nC, knn, cnt, ovf_list, vrKnn, rho, miKnn, d2Knn);
-    IRC_CHECK_LAUNCH("irc_site_knn(EXACT) overflow");
-    return IRC_OK;
+    return exact_overflow(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, ovf_list, s);
 }
 
 int irc_site_knn_exact(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho,
@@ -694,7 +723,12 @@ int irc_site_knn_exact(irc_plan *pl, const float *F, int nC, int knn, float *vrK
     int *cnt = pl->scratch, *queue = pl->scratch + irc::kScratchLists;
     cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * sizeof(int), s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): memset");
-    return irc_exact_tiles(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, irc::TileQueue{}, cnt, queue, s);
+    e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExactSmem);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): smem attribute");
+    k_site_knn_exact<<<pl->ntiles[irc::tile_slot(kQB)], kThreads, kExactSmem, s>>>(pl->dev, F, nC, knn, vrKnn, rho, miKnn, d2Knn,
+                                                                                   cnt, queue);
+    IRC_CHECK_LAUNCH("irc_site_knn(EXACT)");
+    return exact_overflow(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, s);
 }
 
 int irc_site_delta_list(irc_plan *pl, const float *F, int nC, const float *R, int knn,
@@ -762,10 +796,7 @@ int irc_delta_window(irc_plan *pl, const float *F, int nC, const float *R, int n
 int irc_exact_overflow_drain(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho,
                              int32_t *miKnn, float *d2Knn, cudaStream_t s)
 {
-    int *cnt = pl->scratch, *queue = pl->scratch + irc::kScratchLists;
-    launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, pl->dev, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
-    IRC_CHECK_LAUNCH("irc_site_knn overflow drain");
-    return IRC_OK;
+    return exact_overflow(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, pl->scratch, pl->scratch + irc::kScratchLists, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -910,11 +941,10 @@ extern "C" int irc_site_knn_exact_noalloc(const float *F, int nC, const int32_t 
     p.stat = nullptr;
     p.n_qry = (int)(n_qry < INT32_MAX ? n_qry : INT32_MAX);
     p.nChunks = nChunks; p.q_base = q_base; p.n_out = n_out; p.nF = nF; p.nRuns = nRuns;
-    const size_t smem = (size_t)kQB * kCap * 8 + (size_t)kQB * kThreads * 4;
-    e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(k_site_knn_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExactSmem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn_exact_noalloc: smem attribute");
     int32_t *cnt = base, *queue = base + irc::kScratchLists;
-    k_site_knn_exact<<<(unsigned)tiles, kThreads, smem, s>>>(p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue, irc::TileQueue{});
+    k_site_knn_exact<<<(unsigned)tiles, kThreads, kExactSmem, s>>>(p, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, queue);
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc");
     launch_next(k_exact_overflow, kQueueBlocks, 256, 0, s, p, F, nC, knn, cnt, queue, vrKnn, rho, miKnn, d2Knn);
     IRC_CHECK_LAUNCH("irc_site_knn_exact_noalloc overflow");

@@ -64,14 +64,13 @@ __device__ __forceinline__ void count_stat(const PlanDev &p, int which, int n)
     if (p.stat && n) atomicAdd(p.stat + which, (unsigned long long)n);
 }
 
-// The 16-query tiles a plain-form kernel works on: every tile of the plan, one
-// per block (list null), or the tiles a proven search left open (irc_cert.cu):
-// list[0 .. *count), or all ntiles of them when *all is set.
+// The 16-query tiles a proven search left open (irc_cert.cu): list[0 .. *count),
+// or all ntiles of the plan's when *all is set.
 struct TileQueue {
     const int *list, *count, *all;
     int ntiles;
-    __device__ __forceinline__ int size() const { return !list ? (int)gridDim.x : *all ? ntiles : *count; }
-    __device__ __forceinline__ int tile(int w) const { return !list || *all ? w : list[w]; }
+    __device__ __forceinline__ int size() const { return *all ? ntiles : *count; }
+    __device__ __forceinline__ int tile(int w) const { return *all ? w : list[w]; }
 };
 
 // Map a flat tile id to (chunk, first query, query count) for tile size QB.

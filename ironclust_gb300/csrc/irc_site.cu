@@ -27,69 +27,84 @@ constexpr int kThreads = 256;
 constexpr int kKnnQB = 16;     // queries per CTA, kNN kernel (bin table 16 x nT in smem)
 constexpr int kDeltaQB = 16;   // queries per CTA, delta kernel
 
-// kNN (search_min_drift + sort): bin table sV/sI [QB][nT] in dynamic smem.
-__global__ void __launch_bounds__(kThreads)
-k_site_knn_ref(irc::PlanDev p, const float *__restrict__ F, int nC, int nT, int knn,
-               float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn, irc::TileQueue tq)
+// kNN (search_min_drift + sort) of one tile: bin table sV/sI [QB][nT] in dynamic smem.
+__device__ __forceinline__ void
+ref_tile(const irc::PlanDev &p, int tile, const float *__restrict__ F, int nC, int nT, int knn, float *__restrict__ vrKnn,
+         float *__restrict__ rho, int *__restrict__ miKnn)
 {
-    after_previous(tq.list, tq.count, tq.all);
     constexpr int QB = kKnnQB;
     __shared__ __align__(16) float sA[IRC_NC_MAX * QB];
     extern __shared__ __align__(16) unsigned char dyn[];
     float *sV = reinterpret_cast<float *>(dyn);            // [QB][nT]  sqrt(|bin min|)
     int *sI = reinterpret_cast<int *>(sV + QB * nT);       // [QB][nT]  1-based index
-    if (tq.list && blockIdx.x == 0 && threadIdx.x == 0) {
+    int chunk, qs, n;
+    irc::tile_lookup<QB>(p, tile, chunk, qs, n);
+    const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
+    irc::stage_queries<QB>(F, nC, qs, n, sA);
+    __syncthreads();
+    const int nT0 = nT / nBB;
+    for (int t = threadIdx.x; t < nT; t += blockDim.x) {
+        const int b = t % nBB;
+        const int ib0 = __ldg(p.rsr + r0 + b), nb0 = __ldg(p.rnr + r0 + b);
+        float mn[QB];
+        int mi[QB];
+#pragma unroll
+        for (int q = 0; q < QB; ++q) { mn[q] = IRC_SINGLE_INF_F; mi[q] = qs + min(q, n - 1); }
+        irc::scan_bin<QB, false>(F, nullptr, nC, ib0 + t / nBB, ib0 + nb0, nT0, sA, nullptr, mn, mi);
+#pragma unroll
+        for (int q = 0; q < QB; ++q) { sV[q * nT + t] = irc::ref_sqrt_abs(mn[q]); sI[q * nT + t] = mi[q] + 1; }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const float kTaken = -1.0f;
+    for (int q = warp; q < n; q += nw) {
+        float *v = sV + q * nT;
+        const int *ix = sI + q * nT;
+        const size_t o = (size_t)(qs + q - p.q_base);
+        float last = 0.0f;
+        for (int k = 0; k < knn; ++k) {
+            unsigned long long best = ~0ull;
+            for (int t = lane; t < nT; t += 32) {
+                const float x = v[t];
+                const unsigned long long key = (x == kTaken) ? ~0ull : irc::sort_key(x, t);
+                best = key < best ? key : best;
+            }
+            best = irc::warp_min_u64(best);
+            const int t = (int)(best & 0xffffffffu);
+            last = v[t];
+            __syncwarp();
+            if (lane == 0) {
+                miKnn[(size_t)k + (size_t)knn * o] = ix[t];
+                v[t] = kTaken;
+            }
+            __syncwarp();
+        }
+        if (lane == 0) {
+            vrKnn[o] = last;
+            if (rho) rho[o] = __fdiv_rn(1.0f, last);
+        }
+    }
+}
+
+// A tile per block, and the tiles of a queue.
+__global__ void __launch_bounds__(kThreads)
+k_site_knn_ref(irc::PlanDev p, const float *__restrict__ F, int nC, int nT, int knn, float *__restrict__ vrKnn,
+               float *__restrict__ rho, int *__restrict__ miKnn)
+{
+    ref_tile(p, blockIdx.x, F, nC, nT, knn, vrKnn, rho, miKnn);
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_site_knn_ref_queue(irc::PlanDev p, const float *__restrict__ F, int nC, int nT, int knn, float *__restrict__ vrKnn,
+                     float *__restrict__ rho, int *__restrict__ miKnn, irc::TileQueue tq)
+{
+    after_previous(tq.list, tq.count, tq.all);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         irc::count_stat(p, irc::kStatSearches, 1);
         irc::count_stat(p, irc::kStatTiles, tq.size());
     }
     for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
-        int chunk, qs, n;
-        irc::tile_lookup<QB>(p, tq.tile(w), chunk, qs, n);
-        const int r0 = __ldg(p.roffr + chunk), nBB = __ldg(p.roffr + chunk + 1) - r0;
-        irc::stage_queries<QB>(F, nC, qs, n, sA);
-        __syncthreads();
-        const int nT0 = nT / nBB;
-        for (int t = threadIdx.x; t < nT; t += blockDim.x) {
-            const int b = t % nBB;
-            const int ib0 = __ldg(p.rsr + r0 + b), nb0 = __ldg(p.rnr + r0 + b);
-            float mn[QB];
-            int mi[QB];
-#pragma unroll
-            for (int q = 0; q < QB; ++q) { mn[q] = IRC_SINGLE_INF_F; mi[q] = qs + min(q, n - 1); }
-            irc::scan_bin<QB, false>(F, nullptr, nC, ib0 + t / nBB, ib0 + nb0, nT0, sA, nullptr, mn, mi);
-#pragma unroll
-            for (int q = 0; q < QB; ++q) { sV[q * nT + t] = irc::ref_sqrt_abs(mn[q]); sI[q * nT + t] = mi[q] + 1; }
-        }
-        __syncthreads();
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        const float kTaken = -1.0f;
-        for (int q = warp; q < n; q += nw) {
-            float *v = sV + q * nT;
-            const int *ix = sI + q * nT;
-            const size_t o = (size_t)(qs + q - p.q_base);
-            float last = 0.0f;
-            for (int k = 0; k < knn; ++k) {
-                unsigned long long best = ~0ull;
-                for (int t = lane; t < nT; t += 32) {
-                    const float x = v[t];
-                    const unsigned long long key = (x == kTaken) ? ~0ull : irc::sort_key(x, t);
-                    best = key < best ? key : best;
-                }
-                best = irc::warp_min_u64(best);
-                const int t = (int)(best & 0xffffffffu);
-                last = v[t];
-                __syncwarp();
-                if (lane == 0) {
-                    miKnn[(size_t)k + (size_t)knn * o] = ix[t];
-                    v[t] = kTaken;
-                }
-                __syncwarp();
-            }
-            if (lane == 0) {
-                vrKnn[o] = last;
-                if (rho) rho[o] = __fdiv_rn(1.0f, last);
-            }
-        }
+        ref_tile(p, tq.tile(w), F, nC, nT, knn, vrKnn, rho, miKnn);
         __syncthreads();
     }
 }
@@ -344,19 +359,30 @@ int irc_exact_chunk_fill(float *D, int32_t *I, const float *F, const int32_t *IB
     return rc;
 }
 
-// search_min_drift + sort over the tiles of tq (all of the plan's by default).
+// search_min_drift + sort over the tiles of tq, by as many blocks as run at
+// once (bin tables, registers): 152 whatever nThreads left two thirds of the
+// machine idle at 256 bins (every tile of 10,000 spikes: 1,277 us, 425 a tile
+// per block).
 int irc_ref_tiles(irc_plan *pl, const float *F, int nC, int knn, int nThreads, float *vrKnn, float *rho,
                   int32_t *miKnn, const irc::TileQueue &tq, cudaStream_t s)
+{
+    const size_t smem = (size_t)kKnnQB * nThreads * 8, own = smem + sizeof(float) * IRC_NC_MAX * kKnnQB + 1024;
+    cudaError_t e = cudaFuncSetAttribute(k_site_knn_ref_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: smem attribute");
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(3, (size_t)233472 / own));
+    launch_next(k_site_knn_ref_queue, std::min(tiles_for(pl, kKnnQB), per_sm * pl->sms), kThreads, smem, s, pl->dev, F, nC,
+                nThreads, knn, vrKnn, rho, miKnn, tq);
+    IRC_CHECK_LAUNCH("irc_site_knn(REF)");
+    return IRC_OK;
+}
+
+static int irc_site_knn_ref(irc_plan *pl, const float *F, int nC, int knn, int nThreads, float *vrKnn, float *rho,
+                            int32_t *miKnn, cudaStream_t s)
 {
     const size_t smem = (size_t)kKnnQB * nThreads * 8;
     cudaError_t e = cudaFuncSetAttribute(k_site_knn_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: smem attribute");
-    const int tiles = tiles_for(pl, kKnnQB), grid = tq.list ? std::min(tiles, 152) : tiles;
-    // (alone it follows what the caller launched, whose results it reads: the plain launch)
-    if (tq.list)
-        launch_next(k_site_knn_ref, grid, kThreads, smem, s, pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
-    else
-        k_site_knn_ref<<<grid, kThreads, smem, s>>>(pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn, tq);
+    k_site_knn_ref<<<tiles_for(pl, kKnnQB), kThreads, smem, s>>>(pl->dev, F, nC, nThreads, knn, vrKnn, rho, miKnn);
     IRC_CHECK_LAUNCH("irc_site_knn(REF)");
     return IRC_OK;
 }
@@ -735,7 +761,7 @@ int irc_site_knn(irc_plan *pl, const float *F, int nC, int knn, int nThreads, in
             }
         const int rc = irc_cert_site_knn(pl, F, nC, knn, nThreads, mode, vrKnn, rho, miKnn, nullptr, s);
         if (rc != IRC_CERT_PASS) return rc;
-        return irc_ref_tiles(pl, F, nC, knn, nThreads, vrKnn, rho, miKnn, irc::TileQueue{}, s);
+        return irc_site_knn_ref(pl, F, nC, knn, nThreads, vrKnn, rho, miKnn, s);
     }
     if (mode == IRC_MODE_EXACT) {
         const int rc = irc_cert_site_knn(pl, F, nC, knn, 0, mode, vrKnn, rho, miKnn, d2Knn, s);
