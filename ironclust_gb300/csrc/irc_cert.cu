@@ -314,8 +314,14 @@ k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ de
 // thread gets other memory, so concurrent calls on one plan stay independent,
 // as the plain kernels' are).  It keeps at most 1/32 of the device's memory
 // between calls and gives everything back when the last plan that used it is
-// destroyed.  Under stream capture the allocation becomes a node of the graph.
+// destroyed.
+//
+// A captured call takes a block of its own, which the plan keeps (a graph is
+// of no use without its plan), so that the graph holds no allocations: one
+// that does can be instantiated only once at a time and be no child graph.
+// Beyond kMaxCaptured captured calls of a plan, the plain kernels are captured.
 constexpr int kMaxDevices = 64;
+constexpr int kMaxCaptured = sizeof(irc_plan::captured) / sizeof(void *);
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices];
 int g_pool_plans[kMaxDevices];
@@ -331,6 +337,7 @@ cudaMemPool_t pool_of(irc_plan *pl)
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         cudaMemPool_t pool = nullptr;
+        irc_host::Uncaptured mode;
         if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         size_t fr = 0, total = 0;
         cudaMemGetInfo(&fr, &total);
@@ -345,12 +352,30 @@ cudaMemPool_t pool_of(irc_plan *pl)
     return g_pool[dev];
 }
 
+void *captured_block(irc_plan *pl, size_t bytes)
+{
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (pl->n_captured == kMaxCaptured) return nullptr;
+    irc_host::Uncaptured mode;
+    void *p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return pl->captured[pl->n_captured++] = p;
+}
+
 // Stream-ordered working memory of one call, returned in stream order.
 struct Work {
     cudaStream_t s;
     void *base = nullptr;
+    bool kept = false;
     Work(irc_plan *pl, size_t bytes, cudaStream_t st) : s(st)
     {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cudaGetLastError();
+        if (cs != cudaStreamCaptureStatusNone) {
+            kept = true;
+            base = captured_block(pl, bytes);
+            return;
+        }
         cudaMemPool_t pool = pool_of(pl);
         if (!pool || cudaMallocFromPoolAsync(&base, bytes, pool, s) != cudaSuccess) {
             cudaGetLastError();                   // not served: the plain kernels need no memory
@@ -359,7 +384,7 @@ struct Work {
     }
     ~Work()
     {
-        if (base) cudaFreeAsync(base, s);
+        if (base && !kept) cudaFreeAsync(base, s);
     }
 };
 
@@ -427,6 +452,7 @@ int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, si
 
 void irc_cert_release(irc_plan *pl)
 {
+    for (int i = 0; i < pl->n_captured; ++i) cudaFree(pl->captured[i]);
     if (!pl->uses_pool) return;
     std::lock_guard<std::mutex> lk(g_pool_mu);
     if (--g_pool_plans[pl->device] == 0 && g_pool[pl->device]) cudaMemPoolTrimTo(g_pool[pl->device], 0);

@@ -64,6 +64,14 @@ int cuda_status(cudaError_t e, const char *where);
 // its largest query chunk.
 int check_plan(const char *who, const int32_t *q0, const int32_t *nq, const int32_t *roff, const int32_t *rs,
                const int32_t *rn, int nChunks, int q_base, int n_out, int nF, long long *pairs, int *max_nq);
+
+// While it lives, calls of this thread that no graph records (allocations) are
+// allowed although a stream, this thread's or another's, is being captured.
+struct Uncaptured {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 }  // namespace irc_host
 
 #define IRC_CHECK_LAUNCH(where)                                                    \

@@ -34,6 +34,7 @@ cudaError_t irc_scratch_alloc(void **p, size_t bytes, cudaStream_t s)
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
+            irc_host::Uncaptured mode;
             if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
                 unsigned long long keep = kKeep;
                 cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
