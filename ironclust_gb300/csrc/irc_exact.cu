@@ -369,13 +369,20 @@ constexpr int kParts = 8;        // most parts of one candidate window (part < 2
 constexpr int kMinPart = 2048;   // fewest candidates of a part
 constexpr int kWide = 512;       // candidates of a window that whole blocks search, in parts
 constexpr int kWideParts = 16;   // most parts (of kMinPart candidates and more)
+// A part costs a block some 5 us before its first round, so many queries are
+// searched in few parts: as many as make four units a block, taken from a
+// counter (their work differs by the rows of higher rho).  us, window search and
+// the rest of delta, 16 parts each -> so: 3,200 queries of a random rho among 100,000
+// spikes 705 -> 293; 491 of a 400,000-spike site 228 -> 206 (two units 247, eight 226).
+constexpr int kWideTurns = 4;
 constexpr int kDense = 64;       // fewest queries of a chunk that are searched 16 at a time
 
 // Distributes the queries without a listed neighbour, a warp per chunk.  There
 // are few of them (0.1% of a drift site's queries, 1% of a probe's: density
 // peaks), and few candidates have a higher rho than one of them (2%): they are
 // searched one by one -- wide windows by blocks, a part each (sparse[0 ..
-// words[1])), the others by a warp (words[2] of them, from sparse's end).  (A
+// words[1]); words[3] counts the units taken), the others by a warp (words[2] of
+// them, from sparse's end).  (A
 // part, because a spike alone among noise has a low rho: nearly every candidate
 // of its window exceeds it.)  A chunk with at least kDense of
 // them and one in eight (a rho of another kind, a search that proved little)
@@ -552,7 +559,7 @@ __device__ __forceinline__ unsigned long long scan_query(const irc::PlanDev &p, 
 template <bool REF>
 __global__ void __launch_bounds__(kThreads)
 k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restrict__ R, int nC,
-               const uint8_t *__restrict__ row_dims, const int *__restrict__ words, const int2 *__restrict__ sparse,
+               const uint8_t *__restrict__ row_dims, int *words, const int2 *__restrict__ sparse,
                const int2 *__restrict__ items, const int *__restrict__ fb_list, unsigned long long *__restrict__ keys,
                int nT, float *__restrict__ delta, int *__restrict__ nneigh)
 {
@@ -567,15 +574,20 @@ k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restr
     const int total = words[0], n_wide = words[1], n_narrow = words[2];
     float *qrow = sA + warp * IRC_NC_MAX;                    // (kQB >= the warps of a block)
     float *buf = rows_sm + warp * 32 * irc::row_pitch(nC);
-    for (int u = blockIdx.x; u < n_wide * kWideParts; u += gridDim.x) {
+    const int parts = n_wide ? min(kWideParts, (kWideTurns * (int)gridDim.x - 1) / n_wide + 1) : 0;
+    __shared__ int sNext[2];                                 // (in turns: read after the barrier, written before the next)
+    for (int u = blockIdx.x, turn = 0; u < n_wide * parts; u = sNext[turn & 1], ++turn) {
+        if (threadIdx.x == 0) sNext[turn & 1] = (int)gridDim.x + atomicAdd(words + 3, 1);
         const int part = u / n_wide;
         const int2 e = sparse[u - part * n_wide];
-        const int ntot = __ldg(p.ncand + e.y), per = max(kMinPart, (ntot + kWideParts - 1) / kWideParts);
-        if (part * per >= ntot) continue;
-        const int nd = row_dims ? min(nC, (int)__ldg(row_dims + e.x)) : nC;
-        const unsigned long long b = scan_query<REF>(p, F, R, nC, nd, e.y, e.x, nT, part * per, min(ntot, part * per + per),
-                                                     warp, nw, qrow, queues[warp], buf, lane);
-        if (lane == 0 && b != ~0ull) atomicMin(keys + (e.x - p.q_base), b);
+        const int ntot = __ldg(p.ncand + e.y), per = max(kMinPart, (ntot + parts - 1) / parts);
+        if (part * per < ntot) {
+            const int nd = row_dims ? min(nC, (int)__ldg(row_dims + e.x)) : nC;
+            const unsigned long long b = scan_query<REF>(p, F, R, nC, nd, e.y, e.x, nT, part * per, min(ntot, part * per + per),
+                                                         warp, nw, qrow, queues[warp], buf, lane);
+            if (lane == 0 && b != ~0ull) atomicMin(keys + (e.x - p.q_base), b);
+        }
+        __syncthreads();
     }
     for (int w = blockIdx.x * nw + warp; w < n_narrow; w += gridDim.x * nw) {
         const int2 e = sparse[p.n_qry - 1 - w];
