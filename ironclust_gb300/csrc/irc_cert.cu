@@ -16,8 +16,9 @@
 // The proof.  Scaled by the power of two s, a row is x = s (a - ref) and its
 // operand x^ = half(x): |x^ - x| <= u |x| + e0 (u = 2^-11 for the rounding,
 // enlarged to cover the FP32 subtraction; e0 the subnormals of 64 features).
-// A candidate outside the list has a computed value v > tau (or NaN: a row
-// that is not finite is never a result of these forms), where
+// A candidate outside the list has a computed value v > tau, or no operand: a
+// row that is not finite is never a result of these forms, one longer than
+// kNorm is met below.  With an operand,
 //     |v - |x^ - y^|^2| <= c (|x|^2 + |y|^2 + tau) + e1
 // (FP32 norms of <= 64 terms, their three half-precision pieces, and <= 64
 // products accumulated in FP32 by at most five MMAs: 2^-16 covers them with
@@ -27,9 +28,13 @@
 // most |x| + s delta, so its operands' distance is at most
 //     h = s delta + u (2 |x| + s delta) + 2 e0
 // and v <= h^2 + c (|x|^2 + (|x| + s delta)^2 + tau) + e1.  If the right-hand
-// side is below tau, no such candidate exists.  |x| comes from the operand
-// preparation (an upper bound); far-away outliers do not weaken the proof,
-// because the candidate's norm is bounded through the triangle inequality.
+// side is below tau and |x| + s delta at most kNorm (the candidate then has an
+// operand), no such candidate exists.  |x| comes from the operand preparation
+// (an upper bound).  What weakens the proof: queries far from the centre
+// (rounding grows with |x|: units 30 times their noise apart leave a few
+// percent of the queries open, 60 times most) and a scale that many far rows
+// have pulled down.  A few far rows change neither (k_centre_robust), because a
+// candidate's norm is bounded through the triangle inequality.
 //
 // Measured: EXACT kNN + delta of 100,003 spikes (D = 33, 50 chunks, 3.0e9
 // pairs) 22.2 -> 1.09 ms; REF kNN + delta of 60,001 spikes and 12,001 copies
@@ -57,12 +62,14 @@ constexpr int kTile = 16;                 // queries per tile of the plain kerne
 constexpr int kRefKeys = 52;              // REF: list entries used (of 64 places; left-over bins take the others)
 
 // Counter words of a call's working memory (zeroed before it).
-constexpr int W_AMAX = 1;                 // bits of max |F|
 constexpr int W_ERR = irc::kScratchErr;   // a wait of the filter gave up
 constexpr int W_TILES = 4;                // tiles left to the plain kernel
 constexpr int W_OVF = 5;                  // its overflow queue
 constexpr int W_TICKET = 6;               // block ticket of the centring
 constexpr size_t kHdrBytes = 256;
+
+constexpr float kNorm = 240.0f;           // rows up to here have operands: kNorm^2 < F16_NORM2, with the rounding's room
+static_assert(kNorm * kNorm * 1.002f < irc_tc::F16_NORM2, "rows within kNorm have operands");
 
 // Could a candidate outside a list with threshold tau have an FP32 distance
 // <= D?  False only if it cannot (the proof above).
@@ -73,7 +80,7 @@ __device__ __forceinline__ bool may_miss(float D, float tau, float s, float x)
     const float h = sd + u * (2.0f * x + sd) + 2.0f * e0;
     const float y = x + sd;
     const float rhs = (h * h + c * (x * x + y * y + tau) + e1) * (1.0f + 1e-5f);
-    return !(rhs < tau) && !(tau == __int_as_float(0x7f800000));     // tau = inf: nothing was cut
+    return !(rhs < tau) || !(y <= kNorm);
 }
 
 // The reference's bin of row idx for the queries of a chunk: bin t scans run
@@ -441,7 +448,7 @@ int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, si
     if (e == cudaSuccess) e = cudaMemsetAsync(cert, 0xff, (size_t)pl->dev.n_out * sizeof(int2), s);
     if (e == cudaSuccess) e = irc_tc::clear_lists(lo, pl->dev.n_out, s);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn: memset");
-    int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, (unsigned *)words + W_AMAX, (unsigned *)words + W_TICKET, &L->op, s);
+    int rc = irc_tc::make_operands(Fmt::f16, pl, F, nC, ops, nullptr, (unsigned *)words + W_TICKET, &L->op, s);
     if (rc != IRC_OK) return rc;
     rc = irc_tc::launch_filters(Fmt::f16, L->op.mq, L->op.mc, pl, nC, lo, words, s);
     L->c = Call{pl->dev, lo.qinfo, cert, lo.lists, L->op.fp, nC, pl->row_dims, L->op.scale, L->op.qnorm, words, nullptr, nullptr};

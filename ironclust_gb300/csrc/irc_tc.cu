@@ -445,7 +445,7 @@ __device__ __forceinline__ void mark(uint32_t ta, int la, uint32_t tb, int lb, f
 // absolute) at K positions tau_k ..
 // tau_k + 2, against 1, 1, 1 in every candidate row, so the pass-2
 // accumulators are d2 - tau'.  tau' = tau (1 + 2^-10), capped at 1e30 (F16:
-// 60000, above every distance its scaled operands can form): the
+// 60000; a cap that cuts is in the record of the proof, F16_TAU_MAX): the
 // small margin keeps every candidate at or below tau negative whatever the
 // rounding of the extra terms.  The tile is 128-byte swizzled: the 16-byte
 // piece c of row r sits at piece c ^ (r % 8).
@@ -543,7 +543,7 @@ __device__ __forceinline__ void hand_off(const irc::PlanDev &p, const irc_tc::Tc
     if (lane < RL && cL != -1) {
         const int q = it.qs[s] + qrow + part * RL + lane;
         if (lo.cert)                              // the list's bound and its chunk, for the proof of completeness
-            lo.cert[q - p.q_base] = make_int2(__float_as_int(sTau[quarter * 32 + part * RL + lane]), it.chunk[s]);
+            lo.cert[q - p.q_base] = make_int2(__float_as_int(fminf(sTau[quarter * 32 + part * RL + lane], irc_tc::F16_TAU_MAX)), it.chunk[s]);
         if (cL == -2 || !fits) {
             if (!lo.cert) {                       // (with the record above, its tile is searched again)
                 const int k = atomicAdd(scratch + 0, 1);
@@ -583,7 +583,7 @@ __device__ __forceinline__ void hand_off_part(const irc::PlanDev &p, const irc_t
     if (lane < RL && qrow + part * RL + lane < nq_s) {
         n = sCnt[row];
         if (n) base = atomicAdd(lo.split.cnt + item * BM + row, n);
-        if (lo.cert && piece == 0) lo.cert[it.qs[0] + row - p.q_base] = make_int2(__float_as_int(sTau[row]), it.chunk[0]);
+        if (lo.cert && piece == 0) lo.cert[it.qs[0] + row - p.q_base] = make_int2(__float_as_int(fminf(sTau[row], irc_tc::F16_TAU_MAX)), it.chunk[0]);
         if (n > LISTCAP || base + n > LISTCAP) n = 0;             // (the count, past LISTCAP, tells)
     }
 #pragma unroll 1

@@ -15,9 +15,16 @@ using TcItem = irc::TcItem;
 
 // Operand formats of the filter (128-byte rows in all of them).  f16: the
 // BF16 row layout in half precision, the features scaled by a power of two to
-// at most 8 in magnitude; 8 times BF16's resolution at the same MMA cost, so
+// about 8 in magnitude at most; 8 times BF16's resolution at the same MMA cost, so
 // that a query's candidate list can be proven complete (irc_cert.cu).
 enum class Fmt : int { bf16 = 0, fp8 = 1, f16 = 2 };
+
+// f16: the longest scaled row (squared) whose norm the operand rows can hold
+// (half precision ends at 65,504).
+constexpr float F16_NORM2 = 60000.0f;
+// f16: distances up to here are listed whenever the threshold says so (the
+// threshold in the operand rows ends at 60,000).
+constexpr float F16_TAU_MAX = 59900.0f;
 
 // The re-rank's FP32 copy of a feature row, zero-padded to a multiple of 8
 // floats (32 bytes) so that it is read with whole-sector 256-bit loads:
@@ -105,11 +112,11 @@ int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_pl
 struct Operands {
     CUtensorMap mq, mc;
     const float4 *fp;            // padded FP32 rows of the re-rank
-    const float *ref;            // the centre, [nC]
     const float *scale;          // f16: the power of two the features were scaled by
     const float *qnorm;          // f16: upper bound of every query's scaled norm, [n_out]
 };
 size_t ops_bytes(const irc_plan *pl, int nC, Fmt fmt);
+// amax (fp8): the largest magnitude, zero before; ticket: zero.
 int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsigned *amax, unsigned *ticket,
                   Operands *out, cudaStream_t s);
 

@@ -39,19 +39,11 @@ using irc_tc::Fmt;
 // 4 to 12.  Latency-bound: 9 us for 3,000 rows, 24 for 65,536 rows out of 400,000.
 constexpr int kMeanBlocks = 152, kMeanThreads = 512;
 
-// F16: values that are not finite are left out of the sums (one such spike must
-// not spoil the centre and with it every proof), and *scale becomes the power
-// of two that brings every finite |F - ref| to at most 8, from the finite |F|
-// maximum and the largest |ref| (their sum bounds the differences; what the
-// bound loses, a factor of two at most, only costs half-precision subnormals).
-// 0 when features reach 2^62, whose squared distances leave FP32's range:
-// nothing is proven with it.  ticket: zero, and zero again at the end.
-template <bool F16>
 __global__ void __launch_bounds__(kMeanThreads)
 k_centre(const float *__restrict__ F, int nC, int stride, int nS, float *__restrict__ part, unsigned *__restrict__ ticket,
-         float *__restrict__ ref, const unsigned *__restrict__ amax, float *__restrict__ scale)
+         float *__restrict__ ref)
 {
-    after_previous(amax);
+    after_previous();
     __shared__ double red[kMeanThreads];
     __shared__ bool last;
     const int t = threadIdx.x, lanes = kMeanThreads / nC, rl = t / nC, c = t - rl * nC;
@@ -60,10 +52,7 @@ k_centre(const float *__restrict__ F, int nC, int stride, int nS, float *__restr
     float acc = 0.0f;
     if (rl < lanes) {
 #pragma unroll 8
-        for (int k = k0 + rl; k < k1; k += lanes) {
-            const float v = __ldg(F + (size_t)k * stride * nC + c);
-            if (!F16 || isfinite(v)) acc += v;
-        }
+        for (int k = k0 + rl; k < k1; k += lanes) acc += __ldg(F + (size_t)k * stride * nC + c);
     }
     float *redf = reinterpret_cast<float *>(red);
     redf[t] = acc;
@@ -91,33 +80,133 @@ k_centre(const float *__restrict__ F, int nC, int stride, int nS, float *__restr
         for (int r = 1; r < lanes; ++r) sum += red[r * nC + t];
         ref[t] = nS > 0 ? (float)(sum / (double)nS) : 0.0f;
     }
-    if (F16) {
-        __syncthreads();
-        if (t < 32) {
-            float m = 0.0f;
-            for (int k = t; k < nC; k += 32) m = fmaxf(m, fabsf(ref[k]));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (t == 0) {
-                const float b = __uint_as_float(*amax) + m;
-                *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
-            }
-        }
-    }
 }
 
-// |F| maximum over the finite values (bits of a non-negative float, so
-// integer max == float max).
-__global__ void k_absmax_finite(const float *__restrict__ F, size_t n, unsigned *__restrict__ out)
+// Bits of x in ascending order of x.
+__device__ __forceinline__ unsigned ordered(float x)
+{
+    const unsigned u = __float_as_uint(x);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// The warp's key of rank k (0-based) among the N a lane holds (~0: none); where
+// `rough`, any value with 40 to 60 percent of the m keys below it will do.
+template <int N>
+__device__ __forceinline__ unsigned key_of_rank(const unsigned (&key)[N], unsigned k, unsigned m, bool rough)
+{
+    unsigned ans = 0;
+    for (int b = 31; b >= 0; --b) {
+        const unsigned t = ans | (1u << b);
+        unsigned c = 0;
+#pragma unroll
+        for (int i = 0; i < N; ++i) c += key[i] < t;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c <= k) ans = t;
+        if (rough && 5 * c >= 2 * m && 5 * c <= 3 * m) return t;
+    }
+    return ans;
+}
+
+// Centre and scale of the F16 operands, of which each query's proof needs that
+// most rows are well inside the half-precision range.  A few spikes far out
+// (artefacts), or not finite, must not move either: with the mean and the
+// largest magnitude, five rows of 10,000 at 1,000 times the others left every
+// query without a proof.  Every block takes the column means of its rows and
+// their largest distance from its first row; ref is the median of the means per
+// column, and *scale the power of two that brings the upper quartile over the
+// blocks of (that distance + the mean's distance from ref) to at most 8.  Rows
+// that are then too long for F16 get no operand (k_prep), which the proof takes
+// into account.  Values that are not finite are left out.  *scale 0 (nothing is
+// proven): the squared distances leave FP32's range.  part, the magnitudes in
+// column 63 (nC <= 58); ticket: zero, and zero again at the end.
+__global__ void __launch_bounds__(kMeanThreads)
+k_centre_robust(const float *__restrict__ F, int nC, int stride, int nS, float *__restrict__ part,
+                unsigned *__restrict__ ticket, float *__restrict__ ref, float *__restrict__ scale)
 {
     after_previous();
-    unsigned m = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const unsigned b = __float_as_uint(fabsf(__ldg(F + i)));
-        if (b < 0x7f800000u) m = max(m, b);
+    __shared__ float means[kMeanBlocks][64];
+    __shared__ float red[kMeanThreads], mags[kMeanThreads / 32], sref[64];
+    __shared__ int cnt[kMeanThreads];
+    __shared__ bool last;
+    const float none = __int_as_float(0x7fc00000);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int lanes = kMeanThreads / nC, rl = t / nC, c = t - rl * nC;
+    const int per = (nS + gridDim.x - 1) / gridDim.x;
+    const int k0 = blockIdx.x * per, k1 = min(nS, k0 + per);
+    float acc = 0.0f, mx = 0.0f, first = 0.0f;               // sums from the first row: no offset to lose digits to
+    int n = 0;
+    if (rl < lanes && k0 < k1) {
+        first = __ldg(F + (size_t)k0 * stride * nC + c);
+        if (!isfinite(first)) first = 0.0f;
+#pragma unroll 8
+        for (int k = k0 + rl; k < k1; k += lanes) {
+            const float v = __ldg(F + (size_t)k * stride * nC + c);
+            if (!isfinite(v)) continue;
+            acc += v - first;
+            mx = fmaxf(mx, fabsf(v - first));
+            ++n;
+        }
     }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+    red[t] = acc;
+    cnt[t] = n;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) mags[warp] = mx;
+    __syncthreads();
+    if (t < nC) {
+        for (int r = 1; r < lanes; ++r) {
+            acc += red[r * nC + t];
+            n += cnt[r * nC + t];
+        }
+        part[(size_t)blockIdx.x * 64 + t] = n ? first + acc / (float)n : none;
+    } else if (t == 63) {
+        for (int w = 0; w < kMeanThreads / 32; ++w) mx = fmaxf(mx, mags[w]);
+        part[(size_t)blockIdx.x * 64 + 63] = k0 < k1 ? mx : none;
+    }
+    if (t < 64) __threadfence();
+    __syncthreads();
+    if (t == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = t; i < kMeanBlocks * 64; i += kMeanThreads) means[i >> 6][i & 63] = __ldcg(part + i);
+    __syncthreads();
+    constexpr int N = (kMeanBlocks + 31) / 32;
+    for (int k = warp; k < nC; k += kMeanThreads / 32) {
+        unsigned key[N], m = 0;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float v = i * 32 + lane < kMeanBlocks ? means[i * 32 + lane][k] : none;
+            key[i] = isfinite(v) ? ordered(v) : ~0u;
+            m += isfinite(v);
+        }
+        m = __reduce_add_sync(0xffffffffu, m);
+        const unsigned u = key_of_rank(key, m / 2, m, true);
+        if (lane == 0) sref[k] = m ? __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u) : 0.0f;
+    }
+    __syncthreads();
+    if (t < nC) ref[t] = sref[t];
+    float size = none;
+    if (t < kMeanBlocks) {
+        size = means[t][63];
+        float d = 0.0f;
+        for (int k = 0; k < nC; ++k) d = fmaxf(d, fabsf(means[t][k] - sref[k]));
+        size += d;
+    }
+    red[t] = size;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned key[N], m = 0;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float v = red[i * 32 + lane];
+            key[i] = v != v ? ~0u : __float_as_uint(v);
+            m += v == v;
+        }
+        m = __reduce_add_sync(0xffffffffu, m);
+        const float b = m ? __uint_as_float(key_of_rank(key, (3 * m + 3) / 4 - 1, m, false)) : 0.0f;
+        if (lane == 0) *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
+    }
 }
 
 // |F| maximum (bits of a non-negative float, so integer max == float max).
@@ -200,7 +289,8 @@ __device__ __forceinline__ void st_shared_u16(uint4 *row, int at, unsigned short
 
 // qnorm (f16): an upper bound of every query's scaled norm |s (a - ref)|: the
 // rounded row's norm, plus the rounding (2^-11 relative, 2^-25 absolute per
-// feature), with room.
+// feature), with room.  A row longer than irc_tc::F16_NORM2 allows, or not
+// finite, gets an operand without features: as a candidate at distance inf.
 template <Fmt FMT>
 __global__ void __launch_bounds__(32 * kPrepWarps)
 k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restrict__ ref,
@@ -258,6 +348,10 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
                 oq[j ^ sw] = *reinterpret_cast<uint4 *>(wq);
                 oc[j ^ sw] = *reinterpret_cast<uint4 *>(wc);
             }
+            const bool out = FMT == Fmt::f16 && !(na <= irc_tc::F16_NORM2);
+            if (out) {
+                for (int j = 0; j < irc_tc::KP / 8; ++j) oq[j] = oc[j] = make_uint4(0u, 0u, 0u, 0u);
+            }
             // the 9 elements behind the features (nC + 9 may pass the row's
             // end, where only the zeros of the query row are missing)
             const unsigned short h = op16<FMT>(na);
@@ -271,8 +365,8 @@ k_prep(const float *__restrict__ F, int lo, int n, int nC, const float *__restri
                 if (k >= irc_tc::KP) break;
                 const int at = ((k >> 3) ^ sw) * 8 + (k & 7);
                 const unsigned short n3 = i % 3 == 0 ? h : i % 3 == 1 ? m : l;
-                if (i < 6) st_shared_u16(oq, at, i < 3 ? n3 : one);
-                st_shared_u16(oc, at, i >= 3 && i < 6 ? n3 : one);
+                if (i < 6) st_shared_u16(oq, at, i >= 3 ? one : out ? 0 : n3);
+                st_shared_u16(oc, at, i < 3 || i >= 6 ? one : !out ? n3 : i == 3 ? op16<FMT>(__int_as_float(0x7f800000)) : 0);
             }
             const long long row = r0 + lane;
             if (FMT == Fmt::f16 && row >= q_lo && row < q_hi)
@@ -409,14 +503,10 @@ int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsi
     const int stride = nQ > 65536 ? (nQ + 65535) / 65536 : 1;
     const int nS = (nQ + stride - 1) / stride;                        // sampled: q_base + k * stride
     const float *Fq0 = F + (size_t)pl->dev.q_base * nC;
-    if (f16) {                                                        // (its scale takes the maximum)
-        for (int v = 0; v < pl->n_row_iv; ++v) {
-            const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
-            launch_next(k_absmax_finite, 152 * 4, 256, 0, s, F + (size_t)lo * nC, (size_t)n * nC, amax);
-        }
-        launch_next(k_centre<true>, kMeanBlocks, kMeanThreads, 0, s, Fq0, nC, stride, nS, part, ticket, ref, amax, scale);
+    if (f16) {
+        launch_next(k_centre_robust, kMeanBlocks, kMeanThreads, 0, s, Fq0, nC, stride, nS, part, ticket, ref, scale);
     } else {
-        launch_next(k_centre<false>, kMeanBlocks, kMeanThreads, 0, s, Fq0, nC, stride, nS, part, ticket, ref, nullptr, nullptr);
+        launch_next(k_centre, kMeanBlocks, kMeanThreads, 0, s, Fq0, nC, stride, nS, part, ticket, ref);
         for (int v = 0; fp8 && v < pl->n_row_iv; ++v) {
             const int lo = pl->row_iv[2 * v], n = pl->row_iv[2 * v + 1] - lo;
             launch_next(k_absmax, 152 * 4, 256, 0, s, F + (size_t)lo * nC, (size_t)n * nC, nC, ref, amax);
@@ -439,7 +529,6 @@ int make_operands(Fmt fmt, irc_plan *pl, const float *F, int nC, void *buf, unsi
     int rc = make_map(&out->mq, fq, nF, 32, fmt);                     // 32 query rows per lane quarter
     if (rc == IRC_OK) rc = make_map(&out->mc, fc, nF, 128, fmt);      // 128-row candidate tiles
     out->fp = (const float4 *)fp;
-    out->ref = ref;
     out->scale = scale;
     out->qnorm = qnorm;
     return rc;
