@@ -193,11 +193,12 @@ int irc_plan_destroy(irc_plan *plan);
 int irc_plan_check(irc_plan *plan, void *stream);
 
 /* Where the plan's calls since the last one of this function went (host,
- * counts[6]): {REF and EXACT kNN searches by proven lists, 16-query tiles
+ * counts[7]): {REF and EXACT kNN searches by proven lists, 16-query tiles
  * they left to the plain kernels, queries that any kNN form finished by
  * ordered scans (mass ties, lists that overflowed), REF delta searches by
  * proven lists, queries they left to the window search, tensor-core work
- * items split over their candidates}; clears them.
+ * items split over their candidates, queries of proven kNN searches whose
+ * windows were read again}; clears them.
  * Results never depend on it, only speed.  Synchronises `stream`.  No
  * reference counterpart. */
 int irc_plan_search_counts(irc_plan *plan, int64_t *counts, void *stream);

@@ -16,7 +16,7 @@ void irc_cert_release(irc_plan *pl);
 int irc_ref_tiles(irc_plan *pl, const float *F, int nC, int knn, int nThreads, float *vrKnn, float *rho,
                   int32_t *miKnn, const irc::TileQueue &tq, cudaStream_t s);
 int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
-                    float *d2Knn, const irc::TileQueue &tq, int *cnt, int *ovf_list, cudaStream_t s);
+                    float *d2Knn, const irc::TileQueue &tq, cudaStream_t s);
 
 // Device scratch of the drift-window delta search: unit and list counters,
 // per chunk the number of queries to search and (a segment of list) which, the

@@ -227,28 +227,82 @@ k_site_knn_exact(irc::PlanDev p, const float *__restrict__ F, int nC, int knn, f
     exact_tile(p, blockIdx.x, F, nC, knn, vrKnn, rho, miKnn, d2Knn, ovf_count, ovf_list);
 }
 
+// One query by k ordered scans of all linked candidates, each a block-wide
+// minimum of the keys above the previous one.  Serves the rare queries whose
+// candidate list overflowed (mass ties, or an unlucky spread of the tensor-core
+// filter's list parts).
+__device__ __forceinline__ void ordered_scans(const irc::PlanDev &p, const float *__restrict__ F, int nC, int knn, int q,
+                                              float *__restrict__ vrKnn, float *__restrict__ rho, int *__restrict__ miKnn,
+                                              float *__restrict__ d2Knn)
+{
+    __shared__ unsigned long long red[kThreads / 32];
+    __shared__ unsigned long long sBest;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int lo = 0, hi = p.nChunks;
+    while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (__ldg(p.q0 + mid) <= q) lo = mid; else hi = mid; }
+    const int r0 = __ldg(p.roff + lo), r1 = __ldg(p.roff + lo + 1);
+    const float *a = F + (size_t)q * nC;
+    const size_t o = (size_t)(q - p.q_base);
+    unsigned long long prev = 0;
+    bool have_prev = false;
+    for (int k = 0; k < knn; ++k) {
+        unsigned long long best = ~0ull;
+        walk_stripe(p, r0, r1, threadIdx.x, [&](int iB) {
+            const float *b = F + (size_t)iB * nC;
+            float acc = 0.0f;
+            for (int c = 0; c < nC; ++c) acc = irc::dterm(acc, __ldg(b + c), __ldg(a + c));
+            if (!(acc > 0.0f) || !(acc < kInfSentinel)) return;
+            const unsigned long long key = dkey(acc, iB);
+            if ((!have_prev || key > prev) && key < best) best = key;
+        });
+        best = irc::warp_min_u64(best);
+        if (lane == 0) red[warp] = best;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long b = red[0];
+            for (int i = 1; i < kThreads / 32; ++i) b = red[i] < b ? red[i] : b;
+            sBest = b;
+            const bool ok = b != ~0ull;
+            const float d2 = ok ? __uint_as_float((unsigned)(b >> 32)) : kInfSentinel;
+            const int idx = ok ? (int)(b & 0xffffffffu) : q;
+            miKnn[(size_t)k + (size_t)knn * o] = idx + 1;
+            if (d2Knn) d2Knn[(size_t)k + (size_t)knn * o] = d2;
+            if (k == knn - 1) {
+                const float v = irc::ref_sqrt_abs(d2);
+                vrKnn[o] = v;
+                if (rho) rho[o] = __fdiv_rn(1.0f, v);
+            }
+        }
+        __syncthreads();
+        best = sBest;
+        if (best != ~0ull) { prev = best; have_prev = true; }
+    }
+}
+
 // The tiles of a queue.  (A kernel of its own: with the loop around it the tile
-// spills, 4% on a site of 1,500 spikes.)
+// spills, 4% on a site of 1,500 spikes.)  A tile's overflowed queries follow it.
 __global__ void __launch_bounds__(kThreads)
 k_site_knn_exact_queue(irc::PlanDev p, const float *__restrict__ F, int nC, int knn, float *__restrict__ vrKnn,
-                       float *__restrict__ rho, int *__restrict__ miKnn, float *__restrict__ d2Knn,
-                       int *__restrict__ ovf_count, int *__restrict__ ovf_list, irc::TileQueue tq)
+                       float *__restrict__ rho, int *__restrict__ miKnn, float *__restrict__ d2Knn, irc::TileQueue tq)
 {
     after_previous(tq.list, tq.count, tq.all);
+    __shared__ int sOvf[kQB], sOvfN;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         irc::count_stat(p, irc::kStatSearches, 1);
         irc::count_stat(p, irc::kStatTiles, tq.size());
     }
     for (int w = blockIdx.x, n_tiles = tq.size(); w < n_tiles; w += gridDim.x) {
-        exact_tile(p, tq.tile(w), F, nC, knn, vrKnn, rho, miKnn, d2Knn, ovf_count, ovf_list);
+        if (threadIdx.x == 0) sOvfN = 0;                     // (the tile has barriers before it counts)
+        exact_tile(p, tq.tile(w), F, nC, knn, vrKnn, rho, miKnn, d2Knn, &sOvfN, sOvf);
+        __syncthreads();
+        const int n = sOvfN;
+        for (int i = 0; i < n; ++i) ordered_scans(p, F, nC, knn, sOvf[i], vrKnn, rho, miKnn, d2Knn);
+        if (threadIdx.x == 0) irc::count_stat(p, irc::kStatScans, n);
         __syncthreads();
     }
 }
 
-// One CTA per queued query: k ordered scans of all linked candidates, each a
-// block-wide minimum of the keys above the previous one.  Serves the rare
-// queries whose candidate list overflowed (mass ties, or an unlucky spread of
-// the tensor-core filter's list parts).
+// The queued queries, one per block.
 __global__ void __launch_bounds__(kThreads)
 k_exact_overflow(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
                  const int *__restrict__ ovf_count, const int *__restrict__ ovf_list,
@@ -256,53 +310,9 @@ k_exact_overflow(irc::PlanDev p, const float *__restrict__ F, int nC, int knn,
                  int *__restrict__ miKnn, float *__restrict__ d2Knn)
 {
     after_previous(ovf_count, ovf_list);
-    __shared__ unsigned long long red[kThreads / 32];
-    __shared__ unsigned long long sBest;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = *ovf_count;
     if (blockIdx.x == 0 && threadIdx.x == 0) irc::count_stat(p, irc::kStatScans, n);
-    for (int w = blockIdx.x; w < n; w += gridDim.x) {
-        const int q = ovf_list[w];
-        int lo = 0, hi = p.nChunks;
-        while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (__ldg(p.q0 + mid) <= q) lo = mid; else hi = mid; }
-        const int r0 = __ldg(p.roff + lo), r1 = __ldg(p.roff + lo + 1);
-        const float *a = F + (size_t)q * nC;
-        const size_t o = (size_t)(q - p.q_base);
-        unsigned long long prev = 0;
-        bool have_prev = false;
-        for (int k = 0; k < knn; ++k) {
-            unsigned long long best = ~0ull;
-            walk_stripe(p, r0, r1, threadIdx.x, [&](int iB) {
-                const float *b = F + (size_t)iB * nC;
-                float acc = 0.0f;
-                for (int c = 0; c < nC; ++c) acc = irc::dterm(acc, __ldg(b + c), __ldg(a + c));
-                if (!(acc > 0.0f) || !(acc < kInfSentinel)) return;
-                const unsigned long long key = dkey(acc, iB);
-                if ((!have_prev || key > prev) && key < best) best = key;
-            });
-            best = irc::warp_min_u64(best);
-            if (lane == 0) red[warp] = best;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                unsigned long long b = red[0];
-                for (int i = 1; i < kThreads / 32; ++i) b = red[i] < b ? red[i] : b;
-                sBest = b;
-                const bool ok = b != ~0ull;
-                const float d2 = ok ? __uint_as_float((unsigned)(b >> 32)) : kInfSentinel;
-                const int idx = ok ? (int)(b & 0xffffffffu) : q;
-                miKnn[(size_t)k + (size_t)knn * o] = idx + 1;
-                if (d2Knn) d2Knn[(size_t)k + (size_t)knn * o] = d2;
-                if (k == knn - 1) {
-                    const float v = irc::ref_sqrt_abs(d2);
-                    vrKnn[o] = v;
-                    if (rho) rho[o] = __fdiv_rn(1.0f, v);
-                }
-            }
-            __syncthreads();
-            best = sBest;
-            if (best != ~0ull) { prev = best; have_prev = true; }
-        }
-    }
+    for (int w = blockIdx.x; w < n; w += gridDim.x) ordered_scans(p, F, nC, knn, ovf_list[w], vrKnn, rho, miKnn, d2Knn);
 }
 
 // delta from the kNN list, a thread per query, a warp per 32-query tile of a
@@ -712,20 +722,19 @@ static int exact_overflow(irc_plan *pl, const float *F, int nC, int knn, float *
     return IRC_OK;
 }
 
-// The EXACT kernel over the tiles of tq and its overflow queue (*cnt, zeroed;
-// up to n_qry entries).  As many blocks as run at once: a second wave would
-// find its share of the tiles still waiting (100,003 spikes, every tile: 26.0
-// ms with four blocks an SM asked for, 22.3 a tile per block).
+// The EXACT kernel over the tiles of tq.  As many blocks as run at once: a second
+// wave would find its share of the tiles still waiting (100,003 spikes, every
+// tile: 26.0 ms with four blocks an SM asked for, 22.3 a tile per block).
 int irc_exact_tiles(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho, int32_t *miKnn,
-                    float *d2Knn, const irc::TileQueue &tq, int *cnt, int *ovf_list, cudaStream_t s)
+                    float *d2Knn, const irc::TileQueue &tq, cudaStream_t s)
 {
     cudaError_t e = cudaFuncSetAttribute(k_site_knn_exact_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExactSmem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_site_knn(EXACT): smem attribute");
     const int tiles = pl->ntiles[irc::tile_slot(kQB)], most = pl->sms * kExactBlocks;
     launch_next(k_site_knn_exact_queue, tiles < most ? tiles : most, kThreads, kExactSmem, s, pl->dev, F, nC, knn, vrKnn, rho,
-                miKnn, d2Knn, cnt, ovf_list, tq);
+                miKnn, d2Knn, tq);
     IRC_CHECK_LAUNCH("irc_site_knn(EXACT)");
-    return exact_overflow(pl, F, nC, knn, vrKnn, rho, miKnn, d2Knn, cnt, ovf_list, s);
+    return IRC_OK;
 }
 
 int irc_site_knn_exact(irc_plan *pl, const float *F, int nC, int knn, float *vrKnn, float *rho,

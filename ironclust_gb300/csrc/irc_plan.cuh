@@ -14,8 +14,9 @@ constexpr int kScratchLists = 4;
 // Counters of irc_plan_search_counts (PlanDev::stat), summed by the kernels:
 // proven searches and the 16-query tiles they left to the plain kernel, queries
 // finished by ordered scans, proven delta searches and the queries they left
-// to the window search, work items split over their candidates.
-enum { kStatSearches, kStatTiles, kStatScans, kStatDeltas, kStatWindows, kStatSplits, kStatWords };
+// to the window search, work items split over their candidates, queries of
+// proven searches whose windows were read again.
+enum { kStatSearches, kStatTiles, kStatScans, kStatDeltas, kStatWindows, kStatSplits, kStatSecond, kStatWords };
 
 // Query-tile sizes for which a plan precomputes its tile tables.
 constexpr int kTileSizes[] = {8, 16, 32, 64, 128};

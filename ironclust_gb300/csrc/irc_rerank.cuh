@@ -123,8 +123,9 @@ __device__ __forceinline__ void row_dists(const float4 *__restrict__ Fp, int Dp4
 // rows padded to Dp4 float4 (whole 32-byte sectors); nd: the features that can
 // be non-zero for this query and its candidates (the width of their site): the
 // rest are zero in both rows and add exactly 0 to every distance, so they are
-// skipped.  qs: the warp's staging row.
-template <int PER>
+// skipped.  qs: the warp's staging row.  FRESH: other blocks of this kernel wrote
+// the list.
+template <int PER, bool FRESH = false>
 __device__ __forceinline__ void list_keys(const uint32_t *__restrict__ list, int cL, const float4 *__restrict__ Fp,
                                           int Dp4, int q, float4 *__restrict__ qs, int nd, int lane,
                                           unsigned long long (&kv)[PER])
@@ -142,7 +143,7 @@ __device__ __forceinline__ void list_keys(const uint32_t *__restrict__ list, int
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const int e = (bi + r) * 32 + lane;
-            idx[r] = e < cL ? (int)__ldg(list + e) : q;
+            idx[r] = e >= cL ? q : FRESH ? (int)__ldcg(list + e) : (int)__ldg(list + e);
         }
         float acc[2];
         row_dists<2>(Fp, Dp4, idx, qs, nd, acc);

@@ -89,31 +89,13 @@ __device__ __forceinline__ unsigned ordered(float x)
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// The warp's key of rank k (0-based) among the N a lane holds (~0: none); where
-// `rough`, any value with 40 to 60 percent of the m keys below it will do.
-template <int N>
-__device__ __forceinline__ unsigned key_of_rank(const unsigned (&key)[N], unsigned k, unsigned m, bool rough)
-{
-    unsigned ans = 0;
-    for (int b = 31; b >= 0; --b) {
-        const unsigned t = ans | (1u << b);
-        unsigned c = 0;
-#pragma unroll
-        for (int i = 0; i < N; ++i) c += key[i] < t;
-        c = __reduce_add_sync(0xffffffffu, c);
-        if (c <= k) ans = t;
-        if (rough && 5 * c >= 2 * m && 5 * c <= 3 * m) return t;
-    }
-    return ans;
-}
-
 // Centre and scale of the F16 operands, of which each query's proof needs that
 // most rows are well inside the half-precision range.  A few spikes far out
 // (artefacts), or not finite, must not move either: with the mean and the
 // largest magnitude, five rows of 10,000 at 1,000 times the others left every
 // query without a proof.  Every block takes the column means of its rows and
-// their largest distance from its first row; ref is the median of the means per
-// column, and *scale the power of two that brings the upper quartile over the
+// their largest distance from its first row; ref is the median of 32 blocks' means
+// per column, and *scale the power of two that brings the upper quartile over the
 // blocks of (that distance + the mean's distance from ref) to at most 8.  Rows
 // that are then too long for F16 get no operand (k_prep), which the proof takes
 // into account.  Values that are not finite are left out.  *scale 0 (nothing is
@@ -124,7 +106,7 @@ k_centre_robust(const float *__restrict__ F, int nC, int stride, int nS, float *
                 unsigned *__restrict__ ticket, float *__restrict__ ref, float *__restrict__ scale)
 {
     after_previous();
-    __shared__ float means[kMeanBlocks][64];
+    __shared__ float means[kMeanBlocks][65];                 // (a warp reads a column)
     __shared__ float red[kMeanThreads], mags[kMeanThreads / 32], sref[64];
     __shared__ int cnt[kMeanThreads];
     __shared__ bool last;
@@ -141,10 +123,11 @@ k_centre_robust(const float *__restrict__ F, int nC, int stride, int nS, float *
 #pragma unroll 8
         for (int k = k0 + rl; k < k1; k += lanes) {
             const float v = __ldg(F + (size_t)k * stride * nC + c);
-            if (!isfinite(v)) continue;
-            acc += v - first;
-            mx = fmaxf(mx, fabsf(v - first));
-            ++n;
+            const bool in = isfinite(v);
+            const float d = in ? v - first : 0.0f;
+            acc += d;
+            mx = fmaxf(mx, fabsf(d));
+            n += in;
         }
     }
     red[t] = acc;
@@ -169,20 +152,27 @@ k_centre_robust(const float *__restrict__ F, int nC, int stride, int nS, float *
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int i = t; i < kMeanBlocks * 64; i += kMeanThreads) means[i >> 6][i & 63] = __ldcg(part + i);
-    __syncthreads();
-    constexpr int N = (kMeanBlocks + 31) / 32;
-    for (int k = warp; k < nC; k += kMeanThreads / 32) {
-        unsigned key[N], m = 0;
+    static_assert(kMeanBlocks * 64 % kMeanThreads == 0, "whole turns");
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float v = i * 32 + lane < kMeanBlocks ? means[i * 32 + lane][k] : none;
-            key[i] = isfinite(v) ? ordered(v) : ~0u;
-            m += isfinite(v);
+    for (int k = 0; k < kMeanBlocks * 64 / kMeanThreads; ++k) {
+        const int i = k * kMeanThreads + t;
+        means[i >> 6][i & 63] = __ldcg(part + i);
+    }
+    __syncthreads();
+    // median of 32 blocks' means per column, a warp per column, by rank
+#pragma unroll 1
+    for (int k = warp; k < nC; k += kMeanThreads / 32) {
+        const float v = means[lane * kMeanBlocks / 32][k];
+        const unsigned key = isfinite(v) ? ordered(v) : ~0u;
+        unsigned rank = 0;
+#pragma unroll
+        for (int o = 0; o < 32; ++o) {
+            const unsigned other = __shfl_sync(0xffffffffu, key, o);
+            rank += other < key || (other == key && o < lane);
         }
-        m = __reduce_add_sync(0xffffffffu, m);
-        const unsigned u = key_of_rank(key, m / 2, m, true);
-        if (lane == 0) sref[k] = m ? __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u) : 0.0f;
+        const unsigned m = __popc(__ballot_sync(0xffffffffu, key != ~0u));
+        if (key != ~0u && rank == m / 2) sref[k] = v;
+        if (m == 0 && lane == 0) sref[k] = 0.0f;
     }
     __syncthreads();
     if (t < nC) ref[t] = sref[t];
@@ -194,18 +184,22 @@ k_centre_robust(const float *__restrict__ F, int nC, int stride, int nS, float *
         size += d;
     }
     red[t] = size;
+    if (t == 0) mags[0] = 0.0f;
     __syncthreads();
-    if (warp == 0) {
-        unsigned key[N], m = 0;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float v = red[i * 32 + lane];
-            key[i] = v != v ? ~0u : __float_as_uint(v);
-            m += v == v;
+    if (t < kMeanBlocks) {
+        int rank = 0, m = 0;
+#pragma unroll 8
+        for (int b = 0; b < kMeanBlocks; ++b) {
+            const float o = red[b];
+            m += o == o;
+            rank += o < size || (o == size && b < t);
         }
-        m = __reduce_add_sync(0xffffffffu, m);
-        const float b = m ? __uint_as_float(key_of_rank(key, (3 * m + 3) / 4 - 1, m, false)) : 0.0f;
-        if (lane == 0) *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
+        if (size == size && rank == (3 * m + 3) / 4 - 1) mags[0] = size;
+    }
+    __syncthreads();
+    if (t == 0) {
+        const float b = mags[0];
+        *scale = !(b > 0.0f) ? 1.0f : !(b < 0x1p62f) ? 0.0f : ldexpf(1.0f, min(30, 2 - ilogbf(b)));
     }
 }
 

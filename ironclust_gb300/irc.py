@@ -308,9 +308,9 @@ class Plan:
 
     def search_counts(self):
         """irc_plan_search_counts: where the calls since the last one went (waits for the stream)."""
-        c = (C.c_int64 * 6)()
+        c = (C.c_int64 * 7)()
         check(lib().irc_plan_search_counts(self.h, c, _stream()), "irc_plan_search_counts")
-        return dict(zip(("searches", "tiles", "scans", "deltas", "windows", "splits"), c))
+        return dict(zip(("searches", "tiles", "scans", "deltas", "windows", "splits", "second"), c))
 
     def close(self):
         if self.h:
