@@ -377,6 +377,7 @@ k_delta_list(irc::PlanDev p, int ntiles, const float *__restrict__ R, int knn, c
 
 constexpr int kParts = 8;        // most parts of one candidate window (part < 2^3: 3 bits at bit 28)
 constexpr int kMinPart = 2048;   // fewest candidates of a part
+constexpr int kMinDense = 512;   // the same where 16 queries share it (968 queries of 6,000 spikes: 203 -> 171 us)
 constexpr int kWide = 512;       // candidates of a window that whole blocks search, in parts
 constexpr int kWideParts = 16;   // most parts (of kMinPart candidates and more)
 // A part costs a block some 5 us before its first round, so many queries are
@@ -422,7 +423,7 @@ __global__ void k_delta_items(irc::PlanDev p, const int *__restrict__ all, const
     const int ncand = __ldg(p.ncand + chunk);
     int base = 0;
     if (m >= kDense && m * 8 >= nq) {
-        const int ntile = (m + kQB - 1) / kQB, np = min(kParts, max(1, ncand / kMinPart)), nunit = ntile * np;
+        const int ntile = (m + kQB - 1) / kQB, np = min(kParts, max(1, ncand / kMinDense)), nunit = ntile * np;
         if (lane == 0) base = atomicAdd(words, nunit);
         base = __shfl_sync(0xffffffffu, base, 0);
         for (int j = lane; j < nunit; j += 32) {
@@ -611,7 +612,7 @@ k_delta_window(irc::PlanDev p, const float *__restrict__ F, const float *__restr
         const int2 item = items[u];
         const int chunk = item.x & 0x0fffffff, part = item.x >> 28, first = item.y >> 5, n = item.y & 31;
         const int ntot = __ldg(p.ncand + chunk);
-        const int np = min(kParts, max(1, ntot / kMinPart));
+        const int np = min(kParts, max(1, ntot / kMinDense));
         // REF: the runs as the reference passes them (its bins depend on them)
         const int32_t *prs = REF ? p.rsr : p.rs, *prn = REF ? p.rnr : p.rn;
         const int r0 = __ldg((REF ? p.roffr : p.roff) + chunk), r1 = __ldg((REF ? p.roffr : p.roff) + chunk + 1);
