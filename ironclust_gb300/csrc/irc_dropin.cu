@@ -152,10 +152,68 @@ k_search_drift(float *__restrict__ D, int *__restrict__ I, const float *__restri
         }
 }
 
+// The same for short scans: 16 queries a CTA, a bin a thread, rows read where
+// they are.  A bin of a few rows is over before the kernel above has staged
+// them.
+constexpr int kDirectThreads = 256;
+
 template <bool DELTA>
-int launch_search(float *D, int32_t *I, const float *F, const float *R, const int32_t *IBB, const int32_t *NBB, int nC,
-                  int nBB, int iA0, int nA, int nT, cudaStream_t s, const char *who)
+__global__ void __launch_bounds__(kDirectThreads)
+k_search_direct(float *__restrict__ D, int *__restrict__ I, const float *__restrict__ F,
+                const float *__restrict__ R, const int *__restrict__ IBB,
+                const int *__restrict__ NBB, int nC, int nBB, int iA0, int nA, int nT)
 {
+    __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
+    __shared__ float sRA[kQB];
+    const int a0 = blockIdx.x * kQB;                 // first query of this CTA (chunk-relative)
+    const int n = min(kQB, nA - a0);
+    irc::stage_queries<kQB>(F, nC, iA0 + a0, n, sA);
+    if (DELTA && threadIdx.x < kQB) sRA[threadIdx.x] = __ldg(R + iA0 + a0 + min((int)threadIdx.x, n - 1));
+    __syncthreads();
+    const int nT0 = nT / nBB;
+    for (int t = threadIdx.x; t < nT; t += blockDim.x) {
+        const int b = t % nBB;
+        const int ib0 = __ldg(IBB + b), nb0 = __ldg(NBB + b);
+        float mn[kQB];
+        int mi[kQB];
+#pragma unroll
+        for (int q = 0; q < kQB; ++q) { mn[q] = IRC_SINGLE_INF_F; mi[q] = iA0 + a0 + min(q, n - 1); }
+        irc::scan_bin<kQB, DELTA>(F, R, nC, ib0 + t / nBB, ib0 + nb0, nT0, sA, sRA, mn, mi);
+#pragma unroll
+        for (int q = 0; q < kQB; ++q)
+            if (q < n) {
+                const size_t o = (size_t)t + (size_t)nT * (a0 + q);
+                D[o] = irc::ref_sqrt_abs(mn[q]);
+                I[o] = mi[q] + 1;
+            }
+    }
+}
+
+// Which of the two: by the row features that a thread of k_search_direct reads
+// (bins a thread x rows a bin, if the window is all of F, x nC), among windows of
+// some thousand rows at most, or queries for two turns of the chip.  Several runs
+// cost the kernel above more (its blocks of 64 bins straddle them).  us, direct |
+// staged, D = 12 (kNN with 1,024 bins, delta with 512): 300 x 300 one run 8.6 | 9.1,
+// 7.3 | 9.0; 1,000 x 1,000 in 15 runs 11.1 | 15.9, 10.5 | 13.8, one run 10.7 | 10.1,
+// 10.6 | 12.4; 50 x 1,000 11.0 | 8.7, 10.4 | 11.9; 5,000 x 5,000 in 15 runs 55 | 59, 77 | 62.
+template <bool DELTA>
+inline bool direct_search(int nF, int nC, int nBB, int nA, int nT)
+{
+    if (nF <= 0) return false;
+    const long long w = (long long)((nT + kDirectThreads - 1) / kDirectThreads) * ((nF - 1) / nT + 1) * nC;
+    if (nBB > 1 && nA >= 2 * 152 * kQB && w <= (DELTA ? 120 : 240)) return true;
+    return DELTA ? nF <= 2048 && w <= (nBB > 1 ? 100 : 72) : nF <= 1024 && nA > 64 && w <= (nBB > 1 ? 180 : 48);
+}
+
+template <bool DELTA>
+int launch_search(float *D, int32_t *I, const float *F, const float *R, const int32_t *IBB, const int32_t *NBB, int nF,
+                  int nC, int nBB, int iA0, int nA, int nT, cudaStream_t s, const char *who)
+{
+    if (direct_search<DELTA>(nF, nC, nBB, nA, nT)) {
+        k_search_direct<DELTA><<<(nA + kQB - 1) / kQB, kDirectThreads, 0, s>>>(D, I, F, R, IBB, NBB, nC, nBB, iA0, nA, nT);
+        IRC_CHECK_LAUNCH(who);
+        return IRC_OK;
+    }
     // 64 queries share the staged rows when there are so many; 8 warps a CTA when 4 would leave the
     // SMs fewer than three CTAs (kNN, 1,024 bins: 512 CTAs of 4; delta, 512 bins: 256 of 8)
     const int cols = (nT + 63) / 64, ng = nA > 32 ? 4 : nA > 16 ? 2 : 1;
@@ -478,6 +536,69 @@ k_delta_knn(float *__restrict__ D, unsigned *__restrict__ N, const float *__rest
         N[qa] = (found ? ((lo & 0x1ffffffu) << 7 | lo >> 25) : (unsigned)qa) + 1u;
     }
     cluster.sync();                                          // the other CTAs' keys are read
+}
+
+// The same without staging: 16 queries a CTA of the reference's 128 threads, rows
+// read where they are.
+__global__ void __launch_bounds__(128)
+k_delta_direct(float *__restrict__ D, unsigned *__restrict__ N, const float *__restrict__ B,
+               const float *__restrict__ A, const float *__restrict__ RB, const float *__restrict__ RA,
+               int nB, int nA, int nC)
+{
+    __shared__ __align__(16) float sA[IRC_NC_MAX * kQB];
+    __shared__ __align__(16) float sRA[kQB];
+    __shared__ unsigned long long sKey[kQB][4];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int a0 = blockIdx.x * kQB;
+    const int n = min(kQB, nA - a0);
+    irc::stage_queries<kQB>(A, nC, a0, n, sA);
+    if (t < kQB) sRA[t] = __ldg(RA + a0 + min(t, n - 1));
+    __syncthreads();
+    float mn[kQB];
+    int mi[kQB];
+#pragma unroll
+    for (int q = 0; q < kQB; ++q) { mn[q] = IRC_SINGLE_INF_F; mi[q] = 0; }
+    for (int iB = t; iB < nB; iB += 128) {
+        const unsigned live = irc::strictly_higher_rho<kQB>(__ldg(RB + iB), sRA);
+        if (!live) continue;
+        const float *fb = B + (size_t)iB * nC;
+        float acc[kQB];
+#pragma unroll
+        for (int q = 0; q < kQB; ++q) acc[q] = 0.0f;
+        for (int c = 0; c < nC; ++c) {
+            const float bv = __ldg(fb + c);
+            const float4 *a4 = reinterpret_cast<const float4 *>(sA + c * kQB);
+#pragma unroll
+            for (int j = 0; j < kQB / 4; ++j) {
+                const float4 a = a4[j];
+                acc[4 * j + 0] = irc::dterm(acc[4 * j + 0], bv, a.x);
+                acc[4 * j + 1] = irc::dterm(acc[4 * j + 1], bv, a.y);
+                acc[4 * j + 2] = irc::dterm(acc[4 * j + 2], bv, a.z);
+                acc[4 * j + 3] = irc::dterm(acc[4 * j + 3], bv, a.w);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kQB; ++q)
+            if (((live >> q) & 1u) && acc[q] < mn[q]) { mn[q] = acc[q]; mi[q] = iB; }
+    }
+#pragma unroll
+    for (int q = 0; q < kQB; ++q) {
+        // (a thread's rows share iB % 128, its first strict minimum is the first)
+        unsigned long long k = ~0ull;
+        if (mn[q] < IRC_SINGLE_INF_F)
+            k = ((unsigned long long)__float_as_uint(mn[q]) << 32) | ((unsigned)t << 25) | (unsigned)(mi[q] >> 7);
+        k = irc::warp_min_u64(k);
+        if (lane == 0) sKey[q][warp] = k;
+    }
+    __syncthreads();
+    if (t < n) {
+        unsigned long long k = sKey[t][0];
+        for (int w = 1; w < 4; ++w) k = sKey[t][w] < k ? sKey[t][w] : k;
+        const bool found = k != ~0ull;
+        const unsigned lo = (unsigned)k;
+        D[a0 + t] = irc::ref_sqrt_abs(found ? __uint_as_float((unsigned)(k >> 32)) : IRC_SINGLE_INF_F);
+        N[a0 + t] = (found ? ((lo & 0x1ffffffu) << 7 | lo >> 25) : (unsigned)(a0 + t)) + 1u;
+    }
 }
 
 // jrc3_cuda_rho_drift (DELTA false): the fraction of site-matched candidates
@@ -829,7 +950,7 @@ int irc_search_min_drift(float *D, int32_t *I, const float *F, const int32_t *IB
         return irc_exact_chunk_fill(D, I, F, IBB, NBB, nC, nBB, iA0, nA, nThreads, knn, vnConst[1], s);
     }
     if (mode != IRC_MODE_REF) { irc_host::set_error("irc_search_min_drift: unsupported mode %d", mode); return IRC_E_UNSUPPORTED; }
-    return launch_search<false>(D, I, F, nullptr, IBB, NBB, nC, nBB, iA0, nA, nThreads, s, "irc_search_min_drift");
+    return launch_search<false>(D, I, F, nullptr, IBB, NBB, vnConst[1], nC, nBB, iA0, nA, nThreads, s, "irc_search_min_drift");
 }
 
 int irc_search_delta_drift(float *D, int32_t *I, const float *F, const float *R,
@@ -847,7 +968,7 @@ int irc_search_delta_drift(float *D, int32_t *I, const float *F, const float *R,
         return IRC_E_INVAL;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    return launch_search<true>(D, I, F, R, IBB, NBB, nC, nBB, iA0, nA, nThreads, s, "irc_search_delta_drift");
+    return launch_search<true>(D, I, F, R, IBB, NBB, vnConst[1], nC, nBB, iA0, nA, nThreads, s, "irc_search_delta_drift");
 }
 
 }  // extern "C"
@@ -980,6 +1101,14 @@ int irc_cuda_delta_knn(float *D, uint32_t *N, const float *B, const float *A, co
     if (nC <= 0 || nA <= 0 || nB < 0 || nThreads != 128) {
         irc_host::set_error("irc_cuda_delta_knn: bad sizes (nThreads must be 128, the reference block size)");
         return IRC_E_INVAL;
+    }
+    // short scans are over before the kernel below has staged them; with few features and queries for
+    // two turns of the chip its minima cost more than the distances (us, direct | staged: 300 x 300 of
+    // 24 features 8.8 | 15.9, 1,000 x 1,000 17.2 | 20.6, 300 x 2,000 of 9 19 | 15; 5,000 x 5,000 of 6 41 | 52)
+    if (nB <= 1024 || (nC <= 9 && nA >= 2 * 152 * kQB)) {
+        k_delta_direct<<<cdiv(nA, kQB), 128, 0, (cudaStream_t)stream>>>(D, N, B, A, R_B, R_A, nB, nA, nC);
+        IRC_CHECK_LAUNCH("irc_cuda_delta_knn");
+        return IRC_OK;
     }
     const int ng = nA > 32 ? 4 : nA > 16 ? 2 : 1;
     auto bytes = [&](int nw) { return scan_smem(nC, ng, nw) + (size_t)kQB * 64 * nw * sizeof(int); };
