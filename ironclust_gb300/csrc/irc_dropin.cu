@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <climits>
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "irc_common.cuh"
 #include "irc_rerank.cuh"
@@ -354,7 +355,6 @@ k_knn_bins(float *__restrict__ K, int *__restrict__ I, const float *__restrict__
     cluster.sync();
     // 1-based B column of a list position (1 for a bin without candidates)
     auto column = [&](int at) { return at < 0 ? 1 : IND ? __ldg(IB + at) : at + 1; };
-    constexpr int PER = 16;
     for (int q = rank * kBinWarps + warp; q < n; q += nr * kBinWarps) {
         float *d = rowd;
         int *ix = reinterpret_cast<int *>(rowd + nT);
@@ -369,29 +369,29 @@ k_knn_bins(float *__restrict__ K, int *__restrict__ I, const float *__restrict__
         }
         __syncwarp();
         const int qa = a0 + q;
-        if (nT <= 32 * PER) {
+        // the knn smallest by selection; false where ties want the reference's steps
+        auto select = [&](auto per) {
+            constexpr int PER = decltype(per)::value;
             unsigned long long kv[PER], *ws = wkeys[warp];
 #pragma unroll
             for (int i = 0; i < PER; ++i) kv[i] = i * 32 + lane < nT ? irc::sort_key(d[i * 32 + lane], i * 32 + lane) : ~0ull;
             unsigned tbits;
             const int m = irc_rr::select_keys<PER>(kv, knn, ws, lane, tbits);
-            bool plain = m >= knn && m <= irc_rr::WARP_KEYS;
-            if (plain) {
-                bool tie = false;
-                for (int e = lane; e < knn; e += 32) tie |= e + 1 < m && (ws[e] >> 32) == (ws[e + 1] >> 32);
-                plain = !__any_sync(0xffffffffu, tie);
+            if (m < knn || m > irc_rr::WARP_KEYS) return false;
+            bool tie = false;
+            for (int e = lane; e < knn; e += 32) tie |= e + 1 < m && (ws[e] >> 32) == (ws[e + 1] >> 32);
+            if (__any_sync(0xffffffffu, tie)) return false;
+            for (int e = lane; e < knn; e += 32) {
+                const float v = irc::ref_sqrt_abs(__uint_as_float((unsigned)(ws[e] >> 32)));
+                if (KALL) K[e + (size_t)knn * qa] = v;
+                else if (e == knn - 1) K[qa] = v;
+                if (I) I[e + (size_t)knn * qa] = column(ix[(int)(ws[e] & 0xffffffffu)]);
             }
-            if (plain) {
-                for (int e = lane; e < knn; e += 32) {
-                    const float v = irc::ref_sqrt_abs(__uint_as_float((unsigned)(ws[e] >> 32)));
-                    if (KALL) K[e + (size_t)knn * qa] = v;
-                    else if (e == knn - 1) K[qa] = v;
-                    if (I) I[e + (size_t)knn * qa] = column(ix[(int)(ws[e] & 0xffffffffu)]);
-                }
-                __syncwarp();
-                continue;
-            }
-        }
+            __syncwarp();
+            return true;
+        };
+        // (above 512 bins the steps took 58 of 103 us for 2,000 queries x 2,000 candidates)
+        if (nT <= 512 ? select(std::integral_constant<int, 16>{}) : select(std::integral_constant<int, 32>{})) continue;
         for (int iK = 0; iK < knn; ++iK) {
             unsigned long long best = ~0ull;
             for (int p = iK + lane; p < nT; p += 32) {
