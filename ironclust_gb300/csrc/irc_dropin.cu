@@ -1118,14 +1118,15 @@ int irc_cuda_delta_knn(float *D, uint32_t *N, const float *B, const float *A, co
                         : (ng == 4 ? k_delta_knn<4, 4> : ng == 2 ? k_delta_knn<2, 4> : k_delta_knn<1, 4>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return irc_host::cuda_status(e, "irc_cuda_delta_knn");
-    // up to 8 CTAs share a query tile's candidates, as many as give the shortest turns of the chip (a
-    // CTA costs some two steps besides its own): 154 tiles on 152 SMs are two turns, 8 x 154 eighths of
-    // a tile nine eighths (9,800 queries of 20,000 candidates: 1,006 us whole, 690 so)
+    // up to 8 CTAs share a query tile's candidates, as many as keep the fullest SM busy for the shortest
+    // time: two CTAs run together, one alone takes two thirds of their time, each costs some two steps
+    // besides its own.  154 tiles put two whole tiles on some SMs, or nine eighths (9,800 queries of
+    // 20,000 candidates: 1,006 us whole, 597 so; 1,507 of 15,000, 24 tiles: 8 CTAs 10 us faster than 4)
     const int tiles = cdiv(nA, kQB * ng);
     int split = 1;
     long long best = LLONG_MAX;
     for (int k = 1; k <= 8 && (k == 1 || nB >= k * 2 * block); k *= 2) {
-        const long long t = (long long)cdiv((long long)tiles * k, 152) * (cdiv(nB, (long long)k * block) + 2);
+        const long long c = cdiv((long long)tiles * k, 152), t = (c / 2 * 3 + c % 2 * 2) * (cdiv(nB, (long long)k * block) + 2);
         if (t < best) { best = t; split = k; }
     }
     e = launch_cluster(kern, dim3(tiles, split), split, 32 * nw, smem, (cudaStream_t)stream, D, N, B, A, R_B, R_A, nB, nA, nC);
