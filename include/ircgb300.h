@@ -271,8 +271,8 @@ int irc_profile_end(float *filter_ms, float *rerank_ms, int *calls);
  * every query's result (else its tile is searched in plain FP32): same bits.
  * They take stream-ordered working memory from a pool of the library's, or do
  * without it when there is none.  A captured call takes memory that the plan
- * keeps until irc_plan_destroy, for eight captured calls of a plan; later ones
- * capture the plain kernels.  The graphs hold no allocations. */
+ * keeps until irc_plan_destroy, for eight captured searches of a plan (REF's
+ * delta is one of its own); later ones capture the plain kernels.  The graphs hold no allocations. */
 int irc_site_knn(irc_plan *plan, const float *F, int nC, int knn, int nThreads, int mode,
                  float *vrKnn, float *rho, int32_t *miKnn, float *d2Knn, void *stream);
 

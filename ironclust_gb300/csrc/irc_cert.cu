@@ -651,52 +651,20 @@ k_cert_delta(Call c, const float *__restrict__ R, int nT, float *__restrict__ de
         list_out[__ldg(c.p.qseg + ce.y) + atomicAdd(counts + ce.y, 1)] = q;
 }
 
-// Working memory of the proven searches: one pool per device, shared by the
-// plans, its blocks handed out in stream order (a call of another stream or
-// thread gets other memory, so concurrent calls on one plan stay independent,
-// as the plain kernels' are).  It keeps at most 1/32 of the device's memory
-// between calls and gives everything back when the last plan that used it is
-// destroyed.
+// Working memory of the proven searches: a block of the library's pool per call
+// (a call of another stream or thread gets other memory, so concurrent calls on
+// one plan stay independent, as the plain kernels' are).
 //
 // A captured call takes a block of its own, which the plan keeps (a graph is
 // of no use without its plan), so that the graph holds no allocations: one
 // that does can be instantiated only once at a time and be no child graph.
 // Beyond kMaxCaptured captured calls of a plan, the plain kernels are captured.
-constexpr int kMaxDevices = 64;
 constexpr int kMaxCaptured = sizeof(irc_plan::captured) / sizeof(void *);
-std::mutex g_pool_mu;
-cudaMemPool_t g_pool[kMaxDevices];
-int g_pool_plans[kMaxDevices];
-
-cudaMemPool_t pool_of(irc_plan *pl)
-{
-    const int dev = pl->device;
-    if (dev < 0 || dev >= kMaxDevices) return nullptr;
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (!g_pool[dev]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        irc_host::Uncaptured mode;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        size_t fr = 0, total = 0;
-        cudaMemGetInfo(&fr, &total);
-        unsigned long long keep = total / 32;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        g_pool[dev] = pool;
-    }
-    if (!pl->uses_pool) {
-        pl->uses_pool = 1;
-        ++g_pool_plans[dev];
-    }
-    return g_pool[dev];
-}
+std::mutex g_captured_mu;
 
 void *captured_block(irc_plan *pl, size_t bytes)
 {
-    std::lock_guard<std::mutex> lk(g_pool_mu);
+    std::lock_guard<std::mutex> lk(g_captured_mu);
     if (pl->n_captured == kMaxCaptured) return nullptr;
     irc_host::Uncaptured mode;
     void *p = nullptr;
@@ -718,8 +686,7 @@ struct Work {
             base = captured_block(pl, bytes);
             return;
         }
-        cudaMemPool_t pool = pool_of(pl);
-        if (!pool || cudaMallocFromPoolAsync(&base, bytes, pool, s) != cudaSuccess) {
+        if (irc_search_alloc(&base, bytes, pl->device, s) != cudaSuccess) {
             cudaGetLastError();                   // not served: the plain kernels need no memory
             base = nullptr;
         }
@@ -800,9 +767,6 @@ int make_lists(irc_plan *pl, const float *F, int nC, char *base, size_t more, si
 void irc_cert_release(irc_plan *pl)
 {
     for (int i = 0; i < pl->n_captured; ++i) cudaFree(pl->captured[i]);
-    if (!pl->uses_pool) return;
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (--g_pool_plans[pl->device] == 0 && g_pool[pl->device]) cudaMemPoolTrimTo(g_pool[pl->device], 0);
 }
 
 int irc_cert_site_knn(irc_plan *pl, const float *F, int nC, int knn, int nThreads, int mode, float *vrKnn, float *rho,

@@ -80,9 +80,11 @@ struct Uncaptured {
         if (_e != cudaSuccess) return irc_host::cuda_status(_e, where);             \
     } while (0)
 
-// Stream-ordered scratch (irc_pool.cu), freed with cudaFreeAsync; a plan
-// created (+1) or destroyed (-1) on a device.
+// Stream-ordered scratch, and working memory of a proven search
+// (irc_pool.cu), freed with cudaFreeAsync; a plan created (+1) or destroyed
+// (-1) on a device.
 cudaError_t irc_scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+cudaError_t irc_search_alloc(void **p, size_t bytes, int dev, cudaStream_t s);
 void irc_scratch_plan(int dev, int change);
 
 // Kernels of one call that follow each other without a copy or a memset in

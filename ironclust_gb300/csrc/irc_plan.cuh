@@ -117,7 +117,6 @@ struct irc_plan {
     int max_rn;                            // longest candidate run
     int runs_ascend;                       // every chunk's runs ascend without overlap (a row is in at most one)
     int disjoint;                          // no query is in two chunks
-    int uses_pool;                         // the plan took working memory from the library's pool (irc_cert.cu)
     void *captured[8];                     // working memory of the plan's captured calls, n_captured blocks
     int n_captured;
     long long pairs;                       // (query, candidate) pairs of the plan
