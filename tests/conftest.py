@@ -34,4 +34,7 @@ def gpu():
 def refk(gpu):
     """The reference's own kernels (PTX compiled from its sources)."""
     from oracle.oracle import RefKernels
-    return RefKernels()
+    try:
+        return RefKernels()
+    except FileNotFoundError as e:                             # the PTX is made where the reference's sources are
+        pytest.skip(str(e))
