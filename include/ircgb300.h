@@ -206,19 +206,22 @@ int irc_plan_search_counts(irc_plan *plan, int64_t *counts, void *stream);
 /* Layout of the plan's tensor-core work items (IRC_MODE_BF16 / FP8): chunks
  * with more than 64 queries run as 128-query CTAs; the remaining queries of
  * each chunk are packed up to max_slots chunks per CTA (1, 2 or 4; default
- * 4); order 0 = costliest first with a chunk's CTAs adjacent (default),
- * 1 = chunk order.  Results do not depend on the layout, only speed does
- * (ironclust_gb300.autotune picks it by timing).  Synchronises the device;
- * call it outside stream capture.  No reference counterpart. */
+ * 4, or 1 where that makes at most two CTAs an SM); order 0 = costliest first
+ * with a chunk's CTAs adjacent (default), 1 = chunk order.  The layout is for
+ * speed (ironclust_gb300.autotune picks it by timing).  A BF16 list may hold
+ * some candidates more in one layout than in another, which changes a result
+ * only where so many exact copies of a spike crowd its list that the exact
+ * search takes it over in one of them.  Synchronises the device; call it
+ * outside stream capture.  No reference counterpart. */
 int irc_plan_tc_layout(irc_plan *plan, int max_slots, int order);
 
 /* Candidate-unit width of the plan's one- and two-slot tensor-core work items
  * (IRC_MODE_BF16 / FP8): 256 (default: one N = 256 MMA per K slice, two
  * 256-column accumulators, the threshold folded into the MMA for BF16) or 128
  * (N = 128, four 128-column accumulators, the threshold compared in the
- * epilogue).  Four-slot items always use 128.  Results do not depend on it,
- * only speed does (ironclust_gb300.autotune picks it with the layout).  No
- * reference counterpart. */
+ * epilogue).  Four-slot items always use 128.  For speed, as the layout
+ * (ironclust_gb300.autotune picks it with the layout).  No reference
+ * counterpart. */
 int irc_plan_tc_units(irc_plan *plan, int width);
 
 /* Site widths of a plan over stacked sites (host arrays): rows
@@ -330,7 +333,8 @@ int irc_batch_stack(float *F, int nCmax, const float *const *F_sites, const int3
  * plan, its tile table and the overflow queue live in one fixed 8 MiB array
  * inside the library, held by every GPU that loads it until the process
  * exits.  The plan must fit that array: 4 + 2*n_out + 4*nChunks + 2 +
- * 2*nRuns int32 words <= 2^21 (about a million queries); larger plans are
+ * 2*nRuns int32 words <= 2^21 (about a million queries; where queries are in
+ * more than two chunks, all chunks' queries in place of 2*n_out); larger plans are
  * rejected with IRC_E_INVAL and a message, as are plans irc_plan_create
  * rejects.  The first call on a device looks up the array's device address
  * (cudaGetSymbolAddress) with that device current and keeps it; make that

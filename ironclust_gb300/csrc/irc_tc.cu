@@ -1143,9 +1143,10 @@ __global__ void __launch_bounds__(BM) k_publish(irc::PlanDev p, const irc_tc::Tc
 // fallback or to no chunk.
 constexpr int RR_WARPS = 8;
 // Bound by L1's data pipe (a gathered 32-byte sector is about a pass through
-// it) and the latency of the gathers: 5 blocks a SM with a spilled register
-// measure 633 us for 400,000 queries of 61 entries of 33 features and 797 for
-// 3,600 chunks' 625,000, 4 without 665 and 844.
+// it) and the latency of the gathers: 5 blocks a SM with some registers spilled
+// (56 bytes of stores, 220 of loads a thread) measure 633 us for 400,000 queries
+// of 61 entries of 33 features and 797 for 3,600 chunks' 625,000, 4 without 665
+// and 844.
 
 __global__ void __launch_bounds__(32 * RR_WARPS, 5)
 k_rerank(const int2 *__restrict__ qinfo, const uint32_t *__restrict__ lists, int n_out, int q_base,
@@ -1308,7 +1309,8 @@ int launch_filters(Fmt fmt, const CUtensorMap &mq, const CUtensorMap &mc, irc_pl
     // narrower ones compare in the epilogue.  Four-slot items (small chunks)
     // keep the compare: their CTAs are short, and waiting for the thresholds
     // before the pass-2 MMAs would put the threshold step on their critical
-    // path.  Neither the width nor the packing changes the results.
+    // path.  Every form lists all candidates at or below tau; with folded
+    // thresholds a list also holds what lies within 2^-10 above it.
     const int n1 = pl->n_tc_one, n2 = pl->n_tc_wide - pl->n_tc_one, n4 = pl->n_tc_items - pl->n_tc_wide;
     const irc_tc::TcItem *it1 = pl->tc_items, *it2 = it1 + n1, *it4 = it2 + n2;
     const bool narrow = pl->tc_wide_bn == 128;
