@@ -238,8 +238,18 @@ __device__ __forceinline__ void ordered_scans(const irc::PlanDev &p, const float
     __shared__ unsigned long long red[kThreads / 32];
     __shared__ unsigned long long sBest;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int lo = 0, hi = p.nChunks;
+    int lo = 0, hi = p.nChunks;                // the query's chunk, where the chunks ascend
     while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (__ldg(p.q0 + mid) <= q) lo = mid; else hi = mid; }
+    if (q < __ldg(p.q0 + lo) || q >= __ldg(p.q0 + lo) + __ldg(p.nq + lo)) {      // else the first that holds it
+        __shared__ int sChunk;
+        if (threadIdx.x == 0) sChunk = INT_MAX;
+        __syncthreads();
+        for (int c = threadIdx.x; c < p.nChunks; c += kThreads)
+            if (q >= __ldg(p.q0 + c) && q < __ldg(p.q0 + c) + __ldg(p.nq + c)) atomicMin(&sChunk, c);
+        __syncthreads();
+        lo = min(sChunk, p.nChunks - 1);
+        __syncthreads();
+    }
     const int r0 = __ldg(p.roff + lo), r1 = __ldg(p.roff + lo + 1);
     const float *a = F + (size_t)q * nC;
     const size_t o = (size_t)(q - p.q_base);
