@@ -350,7 +350,8 @@ k_cert_knn(Call c, Second z, int knn, int nT, float *__restrict__ vrKnn, float *
 // Before it, an open query sent its 16-query tile there, two passes over the
 // window on one SM: a single one cost 3,000 spikes as much as all of them in the
 // plain kernel, and every query of a site with far apart units 20% more than no
-// search at all.
+// search at all.  With all of 100,000 spikes open (3.0e9 pairs of 33 features) it
+// takes some 8 ms: 12 of the FP32 pipe's 38 T terms a second, as k_search_drift.
 constexpr int kSecondWarps = 8;
 constexpr int kSecondBlocks = 8;              // blocks of 64 rows in shared memory, in use or on their way
 constexpr int kSecondPart = 256;              // fewest rows of a part

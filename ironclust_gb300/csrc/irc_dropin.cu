@@ -390,7 +390,7 @@ k_knn_bins(float *__restrict__ K, int *__restrict__ I, const float *__restrict__
             __syncwarp();
             return true;
         };
-        // (above 512 bins the steps took 58 of 103 us for 2,000 queries x 2,000 candidates)
+        // (2,000 queries x 2,000 candidates, 1,024 bins: 103 us with the steps, 60 so)
         if (nT <= 512 ? select(std::integral_constant<int, 16>{}) : select(std::integral_constant<int, 32>{})) continue;
         for (int iK = 0; iK < knn; ++iK) {
             unsigned long long best = ~0ull;
